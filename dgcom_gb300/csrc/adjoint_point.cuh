@@ -442,14 +442,7 @@ DG_PT void tide_elevation_rev(const Condition& c, double t, double etab, double*
 // h^(-4/3) as manning_rate evaluates it (for its derivatives)
 DG_PT double manning_z4(double h) {
 #if DGSWE_FAST_PATH
-    const int64_t b = fp::bits(h);
-    double z = (b >= 0x3820000000000000ll && b < 0x47C0000000000000ll)
-                   ? f64_of(rcbrtf(f32_seed(h)))
-                   : 1.0 / cbrt(h);
-    const double e = fma(-h, z * z * z, 1.0);
-    z = fma(z * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), z);
-    const double z2 = z * z;
-    return z2 * z2;
+    return vpow_m43(h);
 #else
     return 1.0 / (ref_cbrt(h) * h);
 #endif

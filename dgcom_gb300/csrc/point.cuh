@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "device.hpp"
+#include "fixed64.hpp"
 #include "fp64_bits.hpp"
 
 #if defined(__CUDACC__)
@@ -43,36 +44,18 @@ constexpr int kIncomingWave = 1;
 using fp::lmax;
 using fp::lmin;
 
-// Square roots and reciprocals. DGSWE_FAST: faithful (within an ulp of the
-// correctly rounded value) from a single-precision seed refined in FP64,
-// ≈ 5 FP64-pipe operations against ≈ 8 for sqrt and ≈ 5 for 1/y measured
-// on GB300; the float views of the seed are built on the integer pipes,
-// since F2F conversions run on the FP64 pipe. Arguments outside the seed's
-// range (zero, subnormal, negative, huge, non-finite) take the IEEE
-// operation. Otherwise, and always without DGSWE_FAST, the IEEE operation.
-#if DGSWE_FAST_PATH
-// The float at or below a positive double in [2^-126, 2^128): the exponent
-// rebiased, the mantissa truncated
-__device__ __forceinline__ float f32_seed(double x) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    return __uint_as_float((unsigned int)(b >> 29) - (896u << 23));
-}
-// The double of a positive normal float
-__device__ __forceinline__ double f64_of(float f) {
-    return __longlong_as_double(
-        (long long)(((unsigned long long)__float_as_uint(f) << 29) + (896ull << 52)));
-}
-#endif
-
+// Square roots and reciprocals. DGSWE_FAST: in 64-bit fixed point on the
+// integer pipes (fixed64.hpp), within 0.75 ulp: ≈ 30 integer instructions,
+// 60–70 cycles of a sub-partition, against 5 and 4 FP64 operations of 64
+// cycles each for the refinement of a float seed in FP64 that they replace.
+// Arguments outside the range where the seed is a normal float (zero,
+// subnormal, negative, huge, non-finite) take the IEEE operation. Otherwise,
+// and always without DGSWE_FAST, the IEEE operation.
 DG_PT double vsqrt(double x) {
 #if DGSWE_FAST_PATH
     const int64_t b = fp::bits(x);
     if (b < 0x3810000000000000ll || b >= 0x47E0000000000000ll) return sqrt(x);  // 2^-126, 2^127
-    const float r0 = rsqrtf(f32_seed(x));
-    const double h0 = f64_of(0.5f * r0);  // 1/(2√x), single precision
-    double c = x * f64_of(r0);
-    c = fma(h0, fma(-c, c, x), c);     // relative error ≈ 2^-42
-    return fma(h0, fma(-c, c, x), c);  // ≈ 2^-63 before the last rounding
+    return fx::sqrt_pos(x);
 #else
     return sqrt(x);
 #endif
@@ -82,11 +65,7 @@ DG_PT double vrcp(double y) {
 #if DGSWE_FAST_PATH
     const int64_t b = fp::bits(y);
     if (b < 0x3820000000000000ll || b >= 0x47C0000000000000ll) return 1.0 / y;  // 2^-125, 2^125
-    double r = f64_of(__frcp_rn(f32_seed(y)));
-    double e = fma(-y, r, 1.0);
-    r = fma(r, e, r);  // Newton: relative error ≈ 2^-44
-    e = fma(-y, r, 1.0);
-    return fma(r, e, r);
+    return fx::rcp_pos(y);
 #else
     return 1.0 / y;
 #endif
@@ -116,7 +95,7 @@ DG_PT Sd side(const Q& q) { return {q.h, q.u, q.v, q.b}; }
 DG_PT void node_velocity(double h, double hu, double hv, double h_min,
                                               double& u, double& v) {
     const bool wet = fp::gt(h, h_min);
-    const double inv_h = vrcp(h);
+    const double inv_h = vrcp(wet ? h : 1.0);
     u = wet ? hu * inv_h : 0.0;
     v = wet ? hv * inv_h : 0.0;
 }
@@ -243,20 +222,20 @@ DG_PT double ref_cbrt(double x) {
     return y;
 }
 
+// h^(-4/3) of a floored depth h > 0 (DGSWE_FAST; fixed64.hpp)
+DG_PT double vpow_m43(double h) {
+#if DGSWE_FAST_PATH
+    const int64_t b = fp::bits(h);
+    if (b >= 0x3820000000000000ll && b < 0x47C0000000000000ll) return fx::pow_m43(h);  // 2^±125
+#endif
+    const double z = 1.0 / cbrt(h);
+    return (z * z) * (z * z);
+}
+
 // Manning's rate g n² |u| / h^{4/3} at a floored depth h
 DG_PT double manning_rate(double g_n2, double h, double speed) {
 #if DGSWE_FAST_PATH
-    // h^{-1/3} from a single-precision seed (relative error δ ≈ 2^-22) and
-    // one step of third order, z ← z(1 + e/3 + 2e²/9) with e = 1 − h z³
-    // (error ≈ 5δ³ ≈ 2^-61); then the rate is g n² |u| z⁴, no division
-    const int64_t b = fp::bits(h);
-    double z = (b >= 0x3820000000000000ll && b < 0x47C0000000000000ll)  // 2^-125, 2^125
-                   ? f64_of(rcbrtf(f32_seed(h)))
-                   : 1.0 / cbrt(h);
-    const double e = fma(-h, z * z * z, 1.0);
-    z = fma(z * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), z);
-    const double z2 = z * z;
-    return g_n2 * speed * (z2 * z2);
+    return g_n2 * speed * vpow_m43(h);
 #else
     return g_n2 * speed / (ref_cbrt(h) * h);
 #endif
