@@ -51,6 +51,17 @@ int upload_vec(dgswe_handle* h, const std::vector<T>& v, const T** out) {
     return DGSWE_OK;
 }
 
+template <class T>
+int device_array(dgswe_handle* h, size_t n, T** out) {
+    *out = nullptr;
+    if (n == 0) return DGSWE_OK;
+    void* p = nullptr;
+    CK(cudaMalloc(&p, n * sizeof(T)));
+    h->allocations.push_back(p);
+    *out = (T*)p;
+    return DGSWE_OK;
+}
+
 int ensure_buffer(dgswe_handle* h, int id) {
     DeviceBuffer& b = h->buf[id];
     if (b.base) return DGSWE_OK;
@@ -586,9 +597,33 @@ int create_impl(dgswe_handle* h, const dgswe_form* f, int device) {
     for (size_t q = 0; q < hcoef.size(); ++q) hcoef[q] = 0.5 * sched.accum_coef[q];
     UP(sched_hcoef, hcoef);
     UP(pair_coef, pair_coef_table(sched));
-#undef UP
 
     fill_physics(*f, ops, !t.fcor.empty(), h->P, h->X);
+    if (h->ks->has_fixed) {
+        std::vector<FxLimb> coef;
+        const bool usable = fixed_constants(sched, h->P, T, coef);
+        UP(fx_coef, coef);
+        const size_t nh = (size_t)h->n_values * (ops.n1 - 1), nl = (size_t)h->K * 4 * ops.n1;
+        FxPair *hm = nullptr, *gdb = nullptr;
+        FxLimb* lift = nullptr;
+        FxExp* exps = nullptr;
+        FxPair* normal = nullptr;
+        if ((s = device_array(h, nh, &hm)) || (s = device_array(h, (size_t)h->n_values, &gdb)) ||
+            (s = device_array(h, nl, &lift)) || (s = device_array(h, (size_t)h->K, &exps)) ||
+            (s = device_array(h, (size_t)T.n_edges, &normal)))
+            return bail(s);
+        // on the uploads' own stream, and done before any other stream reads them
+        h->ks->fixed_tables(h->n1, T, hm, gdb, lift, exps, normal, nullptr);
+        CK(cudaGetLastError());
+        if (!usable) CK(cudaMemsetAsync(exps, 0, (size_t)h->K * sizeof(FxExp), nullptr));
+        CK(cudaStreamSynchronize(nullptr));
+        T.fx_hm = hm;
+        T.fx_gdb = gdb;
+        T.fx_lift = lift;
+        T.fx_exp = exps;
+        if (usable) T.fx_normal = normal;  // null: every face in FP64
+    }
+#undef UP
     h->P.n_conditions = f->n_boundaries;
     for (int b = 0; b < f->n_boundaries; ++b) h->P.cond[b] = make_condition(f->boundaries[b]);
     if ((s = boundary_node_tables(h, *f, ops, topo, t))) return bail(s);

@@ -20,6 +20,24 @@ struct DevBuf {
     double *u, *v;        // node velocity (hu, hv)/h, 0 at h ≤ h_min
 };
 
+// Fixed-point table entries (fixed64.hpp), one load each: a number's two
+// limbs, a pair of numbers, an element's exponents
+struct alignas(8) FxLimb {
+    int32_t lo, hi;
+};
+struct alignas(16) FxPair {
+    FxLimb x, y;
+};
+struct alignas(16) FxExp {
+    int32_t et, eg, el, ok;
+};
+// √g and g/2 at 2^(62 − e), their exponents and g's and h_min's (the least e
+// with x < 2^e)
+struct FxFaceConstants {
+    FxLimb sqrt_g, half_g;
+    int e_sqrt_g, e_half_g, e_g, e_h_min;
+};
+
 struct DevTables {
     int64_t K = 0;
     int64_t n_edges = 0, n_bfaces = 0;
@@ -37,6 +55,19 @@ struct DevTables {
     const double* sched_coef;   // [nn][2(n1-1)]
     const double* sched_hcoef;  // [nn][2(n1-1)] sched_coef / 2
     const double* pair_coef;    // [nn·(n1-1)][4] per owned slot: both nodes' coefficients, halves
+    // the wet stage's tables in fixed point (fixed64.hpp), made on the device
+    // from the ones above: pair_hm, gdb and lift_scale as limbs with their
+    // element's exponents {et, eg, el, usable}, sched_coef as limbs at
+    // 2^(62 − fx_ec), 2g at 2^(62 − fx_e2g). Null without DGSWE_FAST.
+    const FxPair* fx_hm = nullptr;    // [K·nn·(n1−1)]
+    const FxPair* fx_gdb = nullptr;   // [K·nn]
+    const FxLimb* fx_lift = nullptr;  // [K·4·n1]
+    const FxExp* fx_exp = nullptr;    // [K]
+    const FxLimb* fx_coef = nullptr;  // [nn][2(n1−1)]
+    const FxPair* fx_normal = nullptr;  // [E] the edges' unit normals at 2^61
+    FxLimb fx_two_g{};
+    FxFaceConstants fx_face{};
+    int fx_ec = 0, fx_e2g = 0;
     // An ensemble's concatenated members: each element's member (its
     // StepCtl is ctl[member]) and the members' boundary conditions, which
     // bface_cond indexes. Both null for one mesh (ctl[0], Physics::cond).

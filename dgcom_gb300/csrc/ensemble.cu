@@ -204,8 +204,33 @@ int build_group(dgswe_ensemble* h, Group& G, std::vector<Tables>& tabs,
     for (size_t q = 0; q < hcoef.size(); ++q) hcoef[q] = 0.5 * sched.accum_coef[q];
     UP(sched_hcoef, hcoef);
     UP(pair_coef, pair_coef_table(sched));
-#undef UP
     fill_physics(h->form0, ops, fcor, G.P, G.X);
+    if (h->ks->has_fixed) {
+        std::vector<FxLimb> coef;
+        const bool usable = fixed_constants(sched, G.P, T, coef);
+        UP(fx_coef, coef);
+        FxPair *hm = nullptr, *gdb = nullptr;
+        FxLimb* lift = nullptr;
+        FxExp* exps = nullptr;
+        FxPair* normal = nullptr;
+        if ((s = device_array(h, (size_t)G.n_values * (n1 - 1), &hm)) ||
+            (s = device_array(h, (size_t)G.n_values, &gdb)) ||
+            (s = device_array(h, (size_t)G.K * 4 * n1, &lift)) ||
+            (s = device_array(h, (size_t)G.K, &exps)) ||
+            (s = device_array(h, (size_t)T.n_edges, &normal)))
+            return s;
+        // on the uploads' own stream, and done before any other stream reads them
+        h->ks->fixed_tables(n1, T, hm, gdb, lift, exps, normal, nullptr);
+        CK(cudaGetLastError());
+        if (!usable) CK(cudaMemsetAsync(exps, 0, (size_t)G.K * sizeof(FxExp), nullptr));
+        CK(cudaStreamSynchronize(nullptr));
+        T.fx_hm = hm;
+        T.fx_gdb = gdb;
+        T.fx_lift = lift;
+        T.fx_exp = exps;
+        if (usable) T.fx_normal = normal;  // null: every face in FP64
+    }
+#undef UP
     G.P.has_bed = h->form0.bathymetry ? 1 : 0;
     G.P.friction = friction ? DGSWE_FRICTION_MANNING_NODES : DGSWE_FRICTION_NONE;
     G.P.n_conditions = 0;  // the conditions are in T.cond

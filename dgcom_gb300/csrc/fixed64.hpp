@@ -1,9 +1,12 @@
-// Square roots, reciprocals and h^(-4/3) of doubles in 64-bit fixed point.
+// 64-bit fixed-point arithmetic on doubles: square roots, reciprocals and
+// h^(-4/3), and the sums and products of the flux-differencing volume term.
 //
 // GB300 takes one FP64 instruction of a warp in 64 cycles of an SM
 // sub-partition, one 32×32+64-bit integer multiply-add in 2 (measured: 67.6
-// and 2.3 cycles, in parallel on their two pipes), so a Newton step of
-// 64-bit integers costs a tenth of one in FP64. Each function takes a
+// and 2.3 cycles, in parallel on their two pipes), so a product of 62-bit
+// integers costs a tenth of an FP64 one and a sum a sixteenth.
+//
+// The roots: each function takes a
 // single-precision seed from the special-function unit, refines it on the
 // mantissa as an integer to a relative error below 2^-55 and rounds once to
 // the nearest double: at most 0.5 + 2^-2 ulp, where the FP64 sequences these
@@ -18,6 +21,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "device.hpp"
 #include "fp64_bits.hpp"
 
 #ifndef DGSWE_SEED_ERROR
@@ -93,26 +97,29 @@ DG_HD int64_t smulhi(int64_t a, int64_t b) {
 #endif
 }
 
+// Leading zeros; 64 for 0
+DG_HD int clz64(uint64_t x) {
+#if defined(__CUDA_ARCH__)
+    return __clzll((long long)x);
+#else
+    return x ? __builtin_clzll(x) : 64;
+#endif
+}
+
 constexpr uint64_t kMantissa = 0x000FFFFFFFFFFFFFull, kImplicit = 0x0010000000000000ull;
 
 // Biased exponent field and the mantissa with its implicit bit (2^52..2^53)
 DG_HD int expo(double x) { return (int)((uint64_t)fp::bits(x) >> 52) & 0x7FF; }
 DG_HD uint64_t mant(double x) { return ((uint64_t)fp::bits(x) & kMantissa) | kImplicit; }
-// The float in [1, 2) of a mantissa, truncated
-DG_HD float mant_f32(uint64_t m) { return as_float((uint32_t)(m >> 29) + 0x3F000000u); }
-
-// √x for x in [2^-126, 2^127) (the caller's guard). With X = x·4^-k in
-// [1, 4): s0 = X·rsqrt(X) to 2^-21 in 31 bits, one Newton step to 2^-42 in
-// 47, a second from the exact residual X − s1² (its high bits cancel, so
-// arithmetic modulo 2^64 holds it whole) to 2^-60.
-DG_HD double sqrt_pos(double x) {
-    const uint64_t m = mant(x);
-    const int e = expo(x);            // x = m·2^(e − 1075)
-    const int odd = (e & 1) ^ 1;      // 1023 is odd: an even field is an odd power of two
-    const uint64_t X = m << (8 + odd);                  // 2^60·X
-    const float xf = as_float((uint32_t)(m >> 29) + 0x3F000000u + ((uint32_t)odd << 23));
+// 2^62·√X from 2^60·X, X in [1, 4): s0 = X·rsqrt(X) to 2^-21 in 31 bits, one
+// Newton step to 2^-42 in 47, a second from the exact residual X − s1² (its
+// high bits cancel, so arithmetic modulo 2^64 holds it whole) to 2^-60
+DG_HD uint64_t root62(uint64_t X) {
+    // the float of X, truncated: 24 bits below the leading one
+    const uint32_t two = (uint32_t)(X >> 61);  // 1 where X ≥ 2
+    const float xf = as_float((uint32_t)((X >> two) >> 37) + 0x3F000000u + (two << 23));
     const uint32_t r = (uint32_t)(seed_rsqrt(xf) * 2147483648.0f);  // 2^31/√X, in [2^30, 2^31]
-    // X·2^60 / 2^32 (29–31 bits) times 2^31/√X → √X·2^59, to 2^30·√X < 2^31
+    // X·2^28 times 2^31/√X → √X·2^59, to 2^30·√X < 2^31
     uint32_t s0 = (uint32_t)(madu(hi32(X), r, 0) >> 29);
     s0 = s0 > 0x7FFFFFFFu ? 0x7FFFFFFFu : s0;
     const int64_t d0 = mads((int32_t)s0, -(int32_t)s0, (int64_t)X);  // 2^60·(X − s0²)
@@ -124,32 +131,43 @@ DG_HD double sqrt_pos(double x) {
     const int64_t d1 = (int64_t)((X << 32) - sq);  // 2^92·(X − s1²), below 2^54 in size
     const int64_t c2 = mads((int32_t)(d1 >> 25), (int32_t)(r >> 1), 0) >> 36;
     // d1·2^-25 (2^67) · r/2 (2^30) = 2^97; half of it at 2^62 is >> 36
-    const uint64_t s = (s1 << 16) + (uint64_t)c2;  // 2^62·√X in [2^62, 2^63)
-    const uint64_t q = (s + 512u) >> 10;           // rounded to 53 bits (2^52..2^53)
+    return (s1 << 16) + (uint64_t)c2;
+}
+
+// √x for x in [2^-126, 2^127) (the caller's guard)
+DG_HD double sqrt_pos(double x) {
+    const int e = expo(x);
+    const int odd = (e & 1) ^ 1;  // 1023 is odd: an even field is an odd power of two
+    const uint64_t s = root62(mant(x) << (8 + odd));
+    const uint64_t q = (s + 512u) >> 10;  // rounded to 53 bits (2^52..2^53)
     // exponent field of √x: 1023 + k, k = (e − 1023 − odd)/2
     return fp::from_bits((int64_t)(q + ((uint64_t)((e - 1023 - odd) / 2 + 1022) << 52)));
 }
 
-// 1/y for y in [2^-125, 2^125) (the caller's guard): r0 to 2^-22, then
+// 2^61/Y in (2^60, 2^61] from 2^63·Y, Y in [1, 2): r0 to 2^-22, then
 // r0·(1 + e + e²) with e = 1 − Y·r0 (relative error e³ = 2^-63)
-DG_HD double rcp_pos(double y) {
-    const uint64_t m = mant(y);
-    const int e = expo(y);
-    const uint64_t Y = m << 11;  // 2^63·Y, Y in [1, 2)
-    const uint32_t r = (uint32_t)(seed_rcp(mant_f32(m)) * 2147483648.0f);  // [2^30, 2^31]
+DG_HD uint64_t reciprocal61(uint64_t Y) {
+    const float yf = as_float((uint32_t)((Y >> 40) & 0x7FFFFFu) | 0x3F800000u);
+    const uint32_t r = (uint32_t)(seed_rcp(yf) * 2147483648.0f);  // [2^30, 2^31]
     // 2^62·Y·r0
     const uint64_t p = madu(hi32(Y), r, hi32(madu(lo32(Y), r, 0)));
     const int64_t e1 = (int64_t)((1ull << 62) - p);  // 2^62·e, |e| < 2^-20
     const int32_t es = (int32_t)(e1 >> 12);          // 2^50·e
-    const int64_t e2 = e1 + (mads(es, es, 0) >> 38);  // 2^62·(e + e²)
-    // r0·(e + e²): 2^62 · 2^31 / 2^32
-    const int64_t c = mads((int32_t)(e2 >> 32), (int32_t)(r >> 1), 0) * 2 +
-                      (int64_t)hi32(madu(lo32((uint64_t)e2), r, 0)) +
-                      ((r & 1) ? (e2 >> 32) : 0);
-    const uint64_t q = ((uint64_t)r << 30) + (uint64_t)c;  // 2^61/Y in (2^60, 2^61]
-    const uint64_t rounded = (q + 128u) >> 8;              // (2^52, 2^53]
+    const int64_t e2 = e1 + (mads(es, es, 0) >> 38);  // 2^62·(e + e²), below 2^42 in size
+    // r0·(e + e²): 2^62 · 2^31 / 2^32; the high word times r in a signed
+    // product of r's half, twice, and its odd bit
+    const int32_t eh = (int32_t)(e2 >> 32);
+    const int64_t c = mads(eh, (int32_t)(r >> 1), 0) * 2 + ((r & 1) ? eh : 0) +
+                      (int64_t)hi32(madu(lo32((uint64_t)e2), r, 0));
+    return ((uint64_t)r << 30) + (uint64_t)c;
+}
+
+// 1/y for y in [2^-125, 2^125) (the caller's guard)
+DG_HD double rcp_pos(double y) {
+    const uint64_t q = reciprocal61(mant(y) << 11);
+    const uint64_t rounded = (q + 128u) >> 8;  // (2^52, 2^53]
     // 1/y = (1/Y)·2^(1023 − e), 1/Y in (½, 1]
-    return fp::from_bits((int64_t)(rounded + ((uint64_t)(2044 - e) << 52)));
+    return fp::from_bits((int64_t)(rounded + ((uint64_t)(2044 - expo(y)) << 52)));
 }
 
 // h^(-4/3) for h in [2^-125, 2^125) (the caller's guard): with m = h·8^-k
@@ -179,17 +197,347 @@ DG_HD double pow_m43(double h) {
     const uint64_t w = z4 + (uint64_t)(smulhi((int64_t)z4, p << 22) >> 16);
     // z⁴ (2^62) · p·2^22 (2^80) / 2^64 = 2^78; >> 16 for 2^62
     // w in (2^58, 2^62]: normalise (0..4 bits) and round to 53
-#if defined(__CUDA_ARCH__)
-    const int c = __clz((int)hi32(w));
-#else
-    const int c = __builtin_clzll(w);
-#endif
+    const int c = clz64(w);
     const uint64_t n = w << c;  // top bit 63
     const uint64_t rounded = (n >> 11) + ((n >> 10) & 1);
     // n·2^-63 in [1, 2): w·2^-62 = n·2^(-62 − c), so the exponent of
     // m^(-4/3) is 1 − c, of the result 1 − c − 4k, k = k3 − 342
     const int field = 1023 + 1 - c - 4 * ((int)k3 - 342);
     return fp::from_bits((int64_t)(rounded + ((uint64_t)(field - 1) << 52)));
+}
+
+// ---- fixed-point numbers ----------------------------------------------------
+//
+// A number is an int64 whose scale (the power of two it is multiplied by) is
+// known from the quantities' largest exponents; a double is cut to it
+// exactly where its last bit fits, else towards zero. Products take the two
+// 32-bit limbs, the low one signed, so that three multiply-adds give the
+// high 64 of the 128 bits: the low × low part, at most a quarter of the last
+// place, is left out.
+
+using Lim = FxLimb;  // hi·2^32 + lo
+
+DG_HD Lim split(int64_t v) {
+    const int32_t lo = (int32_t)v;
+    return {lo, (int32_t)(v >> 32) - (lo >> 31)};
+}
+
+// A sum of products: r counts 2^64, t 2^32
+struct Acc {
+    int64_t t, r;
+};
+
+DG_HD void mac(Acc& s, const Lim& a, const Lim& b) {
+    s.t = mads(a.hi, b.lo, s.t);
+    s.t = mads(a.lo, b.hi, s.t);
+    s.r = mads(a.hi, b.hi, s.r);
+}
+
+// The sum divided by 2^(64 − K), rounded: an accumulator starts at
+// {half<K>(), 0}
+template <int K>
+DG_HD constexpr int64_t half() {
+    return 1ll << (31 - K);
+}
+template <int K>
+DG_HD int64_t fold(const Acc& s) {
+    return (int64_t)((uint64_t)s.r << K) + (s.t >> (32 - K));
+}
+
+// A node's sum over its pairs, whose terms lie well below the accumulator's
+// range: with the low × low parts, a quarter of each (l counts 4)
+struct PairSum {
+    Acc s;
+    int64_t l;
+};
+DG_HD PairSum pair_sum() { return {{half<4>(), 0}, 0}; }
+DG_HD void mac(PairSum& p, const Lim& coef, const Lim& f) {
+    mac(p.s, coef, f);
+    p.l = mads(coef.lo >> 2, f.lo, p.l);
+}
+DG_HD int64_t fold(const PairSum& p) {
+    return fold<4>(Acc{p.s.t + (p.l >> 30), p.s.r});
+}
+
+// x·2^(1085 − K), towards zero: |x| < 2^(K − 1023), so the result is below
+// 2^62. Subnormal x count as zero (K is far above their exponent).
+DG_HD int64_t to_fixed(double x, int K) {
+    const int64_t b = fp::bits(x);
+    const uint64_t m = mant(x) << 10;
+    const int r = K - expo(x);
+    const int64_t v = (int64_t)(m >> (r > 63 ? 63 : r));
+    const int64_t sign = b >> 63;
+    return (v ^ sign) - sign;
+}
+
+// v·2^-s rounded to the nearest double, for results in the normal range
+DG_HD double from_fixed(int64_t v, int s) {
+    const int64_t sign = v >> 63;
+    const uint64_t a = (uint64_t)((v ^ sign) - sign);
+    if (a == 0) return 0.0;
+    const int c = clz64(a);
+    const uint64_t m = a << c;
+    const uint64_t q = (m >> 11) + ((m >> 10) & 1);
+    const uint64_t bits = q + ((uint64_t)(1085 - c - s) << 52);
+    return fp::from_bits((int64_t)(bits | ((uint64_t)sign & 0x8000000000000000ull)));
+}
+
+// ---- the wet element's right-hand side --------------------------------------
+//
+// Volume pairs, bed slope, surface lift and 1/J of a wet element, the FP64
+// sums' terms in fixed point with one scale per element and quantity. Where
+// the exponents go (E of a quantity: |x| < 2^E over the element):
+//   h          2^(62 − eh)       exact: the element's depths lie within 2^9
+//   hu, hv     2^(60 − em)       (u, v at 2^(61 − ev)); exact down to 2^-8
+//   pair metric 2^(62 − et), bed slope 2^(62 − eg), lift 2^(61 − el)
+//   mass flux of a pair 2^(58 − em − et), its momentum flux 2^(58 − eP − et),
+//   eP covering 2g·h² and the advected momentum, whichever is larger
+// Every sum stays below 2^63 with its last place below 2^-57 of the largest
+// term, where FP64 rounds each operation at 2^-53 of its result.
+
+struct Exps {  // biased exponent fields over an element; 0: all zero
+    int h_max, h_min, m, v, fh, fm;  // depth, momentum, velocity, face fluxes
+};
+
+struct Scale {
+    bool ok;
+    int kh, km, ku;   // to_fixed's K of h, of hu and hv, of u and v
+    int g_shift;      // of 2g·h, and of the bed slope's products
+    int b_shift;
+    int kfh, kfm;     // K of the face fluxes
+    int sh, sm;       // the sums are values times 2^sh (mass), 2^sm (momentum)
+};
+
+// exponent fields within 2^±120 (beyond it the element takes FP64)
+constexpr int kExpLo = 1023 - 120, kExpHi = 1023 + 120;
+
+DG_HD Scale scales(const Exps& x, const FxExp& t, int ec, int e2g) {
+    Scale s;
+    s.ok = t.ok && x.h_max <= kExpHi && x.h_max >= kExpLo && x.h_min >= x.h_max - 9 &&
+           x.m <= kExpHi && (x.m == 0 || x.m >= kExpLo) && x.v <= kExpHi && x.fh <= kExpHi &&
+           x.fm <= kExpHi;
+    const int eh = x.h_max - 1022;
+    const int lift = t.el - t.et - ec - 1022;
+    int em = (x.m > kExpLo ? x.m : kExpLo) - 1022;
+    if (x.fh && em < x.fh + lift + 1) em = x.fh + lift + 1;
+    int eP = e2g + 2 * eh;
+    if (x.v && eP < em + x.v - 1022 + 3) eP = em + x.v - 1022 + 3;
+    if (x.fm && eP < x.fm + lift + 2) eP = x.fm + lift + 2;
+    const int steep = t.eg + eh + 1 - t.et - ec;
+    if (eP < steep) eP = steep;
+    s.kh = 1023 + eh;
+    s.km = 1025 + em;
+    s.ku = 1021 + eP - em;
+    s.g_shift = eP - e2g - 2 * eh;
+    s.b_shift = eP - steep;
+    s.sh = 60 - em - t.et - ec;
+    s.sm = 61 - eP - t.et - ec;
+    s.kfh = 1082 - s.sh - t.el;
+    s.kfm = 1082 - s.sm - t.el;
+    return s;
+}
+
+// 2g·h at 2^(62 − eP + eh) from h and 2g (two_g: at 2^(62 − e2g))
+DG_HD Lim two_g_h(const Lim& H, const Lim& two_g, const Scale& s) {
+    Acc a{half<2>(), 0};
+    mac(a, H, two_g);
+    const int64_t v = fold<2>(a);
+    return split(v >> (s.g_shift > 63 ? 63 : s.g_shift));
+}
+
+struct Flux {
+    Lim h, hu, hv;
+};
+
+// The two-point flux of a pair along its half metric (m0, m1), twice for the
+// momentum: mass = Σhu·m0 + Σhv·m1, mass·Σu + 2g·h_a·h_c·m0, …; the sums of
+// momentum and velocity over the two nodes
+DG_HD Flux pair_flux(const Lim& G, const Lim& H, int64_t M0, int64_t M1, int64_t U0, int64_t U1,
+                     const Lim& m0, const Lim& m1) {
+    Flux f;
+    Acc a{half<0>(), 0};
+    mac(a, split(M0), m0);
+    mac(a, split(M1), m1);
+    f.h = split(fold<0>(a));
+    Acc p{half<0>(), 0};
+    mac(p, G, H);
+    const Lim gp = split(fold<0>(p));
+    Acc b{half<0>(), 0};
+    mac(b, f.h, split(U0));
+    mac(b, gp, m0);
+    f.hu = split(fold<0>(b));
+    Acc c{half<0>(), 0};
+    mac(c, f.h, split(U1));
+    mac(c, gp, m1);
+    f.hv = split(fold<0>(c));
+    return f;
+}
+
+// h times the bed slope at the momentum sums' scale
+DG_HD int64_t bed_term(const Lim& H, const Lim& slope, const Scale& s) {
+    Acc a{half<0>(), 0};
+    mac(a, H, slope);
+    return fold<0>(a) >> (s.b_shift > 63 ? 63 : s.b_shift);
+}
+
+// V·2^-s/J as a double
+DG_HD double over_jacobian(int64_t V, int s, double jinv) {
+    Acc a{half<1>(), 0};
+    mac(a, split(V), split((int64_t)(mant(jinv) << 9)));
+    return from_fixed(fold<1>(a), s + 1021 - expo(jinv));
+}
+
+// ---- the interior face's flux ------------------------------------------------
+//
+// hydro_hll (point.cuh) between two wet sides in sub-critical flow, each
+// quantity at a scale of the face node's own exponents (E: |x| < 2^E):
+//   depths 2^(61 − eh), velocities 2^(60 − ev), speeds of waves 2^(60 − eS),
+//   mass flux 2^(60 − eM), momentum flux 2^(59 − eQ), weights 2^61.
+// With α = S_R/(S_R − S_L), β = 1 − α and w = −α·S_L the star flux is
+//   α·F_l + β·F_r − w·(q_r − q_l),
+// whose differences of depths are exact, so that a face at rest has no mass
+// flux; eM follows the depths' difference, not their size.
+
+using FaceConstants = FxFaceConstants;
+
+struct FaceFlux {
+    double h, hu_a, hv_a, hu_b, hv_b;  // seen along the normal from both sides
+};
+
+DG_HD int64_t min64(int64_t a, int64_t b) { return a < b ? a : b; }
+DG_HD int64_t max64(int64_t a, int64_t b) { return a > b ? a : b; }
+DG_HD int imax(int a, int b) { return a > b ? a : b; }
+DG_HD int64_t shr(int64_t v, int n) { return v >> (n > 63 ? 63 : n); }
+DG_HD int64_t abs64(int64_t v) { return v < 0 ? -v : v; }
+
+template <int K>
+DG_HD int64_t mul(const Lim& a, const Lim& b) {
+    Acc s{half<K>(), 0};
+    mac(s, a, b);
+    return fold<K>(s);
+}
+
+// √(g·x) at 2^(60 − eC) for x > 0 at 2^s (below 2^62), √(g·x) < 2^eC
+DG_HD int64_t celerity(int64_t x, int s, const FaceConstants& c, int eC) {
+    int up = clz64((uint64_t)x) - 2;     // x·2^up in [2^61, 2^62)
+    up -= (60 - up - s) & 1;             // one less where that makes the exponent even
+    const uint64_t X = up >= 0 ? (uint64_t)x << up : (uint64_t)x >> 1;
+    const int p = 60 - up - s;           // x's value is X·2^(p − 60)
+    const int64_t v = mul<2>(split((int64_t)(root62(X) >> 1)), c.sqrt_g);
+    return shr(v, 1 - c.e_sqrt_g - p / 2 + eC);
+}
+
+// a/(a + b) at 2^61 for 0 ≤ a, b < 2^61, not both 0
+DG_HD int64_t share(int64_t a, int64_t b) {
+    const uint64_t d = (uint64_t)(a + b);
+    const int up = clz64(d) - 2;  // (a + b)·2^up in [2^61, 2^62)
+    const uint64_t q = reciprocal61(d << (up + 2));
+    return mul<3>(split((int64_t)((uint64_t)a << up)), split((int64_t)q));
+}
+
+// False where the sides are not both wet, or the exponents spread too far:
+// nothing is written then
+template <class Side>
+DG_HD bool face_flux(const Side& qa, const Side& qb, const FxPair& n, const FaceConstants& c,
+                     FaceFlux& out) {
+    const int xa = (int)((uint64_t)fp::bits(qa.h) >> 52), xb = (int)((uint64_t)fp::bits(qb.h) >> 52);
+    const int xh = imax(xa, xb);
+    const int xl = imax(xh, imax(expo(qa.b), expo(qb.b)));
+    const int xv = imax(imax(expo(qa.u), expo(qa.v)), imax(expo(qb.u), expo(qb.v)));
+    // depths within 2^±120 (a negative one's sign field is above) and within
+    // 2^7 of the bed's elevation, so that the surface's sums hold them whole
+    if (xl > kExpHi || imax(xv, xh) > kExpHi || (xa < xb ? xa : xb) < imax(kExpLo, xl - 7))
+        return false;
+    const int eh = xh - 1022, up = xl - xh + 1;
+    // hydrostatic reconstruction: the surfaces over the higher bed, exact
+    const int64_t la = to_fixed(qa.h, xl + 3), lb = to_fixed(qb.h, xl + 3);  // 2^(60 − eL)
+    const int64_t ba = to_fixed(qa.b, xl + 3), bb = to_fixed(qb.b, xl + 3);
+    const int64_t top = max64(ba, bb);
+    const int64_t ha = (int64_t)((uint64_t)la << up), hb = (int64_t)((uint64_t)lb << up);
+    const int64_t sa = (int64_t)((uint64_t)(la + ba - top) << up);
+    const int64_t sb = (int64_t)((uint64_t)(lb + bb - top) << up);
+    // every depth above twice h_min (its side wet beyond rounding)
+    const int64_t least = min64(sa, sb);
+    if (least <= 0 || 63 - clz64((uint64_t)least) + eh - 61 <= c.e_h_min) return false;
+    const int eC = (eh + c.e_g + 1) >> 1;
+    const int ev = imax(xv - 1022, eC - 30);
+    const int kv = 1024 + ev;
+    auto rotate = [&](const Lim& u, const Lim& v, int64_t& normal, int64_t& along) {
+        Acc a{half<2>(), 0}, t{half<2>(), 0};
+        mac(a, u, n.x);
+        mac(a, v, n.y);
+        normal = fold<2>(a);
+        mac(t, v, n.x);
+        Acc o{0, 0};
+        mac(o, u, n.y);
+        t.t -= o.t;
+        t.r -= o.r;
+        along = fold<2>(t);
+    };
+    int64_t un_a, ut_a, un_b, ut_b;  // 2^(60 − ev)
+    rotate(split(to_fixed(qa.u, kv)), split(to_fixed(qa.v, kv)), un_a, ut_a);
+    rotate(split(to_fixed(qb.u, kv)), split(to_fixed(qb.v, kv)), un_b, ut_b);
+    // wave speeds (Einfeldt)
+    const int64_t c_a = celerity(sa, 61 - eh, c, eC), c_b = celerity(sb, 61 - eh, c, eC);
+    const int64_t c_m = celerity(sa + sb, 62 - eh, c, eC);
+    const Lim ul = split(un_a), ur = split(un_b);
+    const int64_t u_m = un_b + mul<3>(split(share(c_a, c_b)), split(un_a - un_b));
+    const int eS = imax(ev + 1, eC) + 1;
+    const int dv = eS - ev, dc = eS - eC;
+    const int64_t s_l = min64(shr(un_a, dv) - shr(c_a, dc), shr(u_m, dv) - shr(c_m, dc));
+    const int64_t s_r = max64(shr(un_b, dv) + shr(c_b, dc), shr(u_m, dv) + shr(c_m, dc));
+    if (s_l >= 0 || s_r <= 0) return false;
+    const int64_t alpha = share(s_r, -s_l);
+    const Lim al = split(alpha), be = split((1ll << 61) - alpha);
+    const Lim w = split(mul<3>(al, split(-s_l)));  // 2^(60 − eS)
+    // momenta hs·un, hs·ut at 2^(60 − eh − ev)
+    const Lim da = split(sa), db = split(sb);
+    const int64_t m_a = mul<3>(da, ul), m_b = mul<3>(db, ur);
+    const Lim tl = split(ut_a), tr = split(ut_b);
+    const int64_t t_a = mul<3>(da, tl), t_b = mul<3>(db, tr);
+    const Lim ml = split(m_a), mr = split(m_b);
+    // mass
+    const int64_t dh = sb - sa;
+    const int grow = clz64((uint64_t)abs64(dh)) - 3;  // dh·2^grow below 2^61
+    const int eD = eh - grow;
+    const int eM = imax(eh + ev + 1, eS + eD);
+    Acc f{half<3>(), 0};
+    mac(f, al, ml);
+    mac(f, be, mr);
+    const int64_t f_h = shr(fold<3>(f), eM - eh - ev) -
+                        shr(mul<3>(w, split((int64_t)((uint64_t)dh << grow))), eM - eS - eD);
+    out.h = from_fixed(f_h, 60 - eM);
+    // momentum
+    const int eP = 2 * eh + c.e_half_g;
+    const int eQ = imax(imax(eP, eh + 2 * ev + 1), eS + eh + ev - 1);
+    const int dp = 1 + eQ - eP, dm = 1 + eQ - eh - 2 * ev, dw = 1 + eQ - eS - eh - ev;
+    auto pressure = [&](int64_t x, int64_t y) {  // ½g·x·y of depths' scale, at 2^(59 − eQ)
+        return shr(mul<1>(split(mul<3>(split(x), split(y))), c.half_g), dp);
+    };
+    Acc g{half<3>(), 0};
+    mac(g, al, split(pressure(sa, sa) + shr(mul<4>(ml, ul), dm)));
+    mac(g, be, split(pressure(sb, sb) + shr(mul<4>(mr, ur), dm)));
+    const int64_t f_n = fold<3>(g) - shr(mul<4>(w, split(m_b - m_a)), dw);
+    Acc t{half<3>(), 0};
+    mac(t, al, split(shr(mul<4>(ml, tl), dm)));
+    mac(t, be, split(shr(mul<4>(mr, tr), dm)));
+    const Lim f_t = split(fold<3>(t) - shr(mul<4>(w, split(t_b - t_a)), dw));
+    // each side's own pressure over the reconstructed one, and back
+    auto back = [&](int64_t normal, double& x, double& y) {
+        const Lim fn = split(normal);
+        Acc a{half<2>(), 0}, o{0, 0}, b{half<2>(), 0};
+        mac(a, fn, n.x);
+        mac(o, f_t, n.y);
+        a.t -= o.t;
+        a.r -= o.r;
+        mac(b, fn, n.y);
+        mac(b, f_t, n.x);
+        x = from_fixed(fold<2>(a), 58 - eQ);
+        y = from_fixed(fold<2>(b), 58 - eQ);
+    };
+    back(f_n + pressure(ha - sa, ha + sa), out.hu_a, out.hv_a);
+    back(f_n + pressure(hb - sb, hb + sb), out.hu_b, out.hv_b);
+    return true;
 }
 
 }  // namespace fx

@@ -12,6 +12,7 @@
 
 #include "../../include/dgswe.h"
 #include "device.hpp"
+#include "fixed64.hpp"
 #include "setup.hpp"
 
 namespace dgswe {
@@ -262,6 +263,36 @@ inline std::vector<double> pair_coef_table(const PairSchedule& sched) {
             pc[(size_t)sl * 4 + 2 + side] = 0.5 * c;
         }
     return pc;
+}
+
+// The fixed-point constants of the wet stage and of the interior faces
+// (fixed64.hpp): the accumulation coefficients as limbs at 2^(62 − fx_ec),
+// each node's adding up to at most 2^fx_ec in size, 2g, √g, g/2 and the
+// exponents of g and h_min; false where g is outside their range
+inline bool fixed_constants(const PairSchedule& sched, const Physics& P, DevTables& T,
+                            std::vector<FxLimb>& coef) {
+    const size_t na = 2 * ((size_t)sched.n1 - 1);
+    double most = 0.0;
+    for (int i = 0; i < sched.nn; ++i) {
+        double sum = 0.0;
+        for (size_t q = 0; q < na; ++q) sum += std::fabs(sched.accum_coef[(size_t)i * na + q]);
+        most = std::fmax(most, sum);
+    }
+    std::frexp(most, &T.fx_ec);
+    coef.clear();
+    for (double c : sched.accum_coef) coef.push_back(fx::split(fx::to_fixed(c, 1023 + T.fx_ec)));
+    auto constant = [](double x, int& e) {
+        std::frexp(x, &e);
+        return fx::split(fx::to_fixed(x, 1023 + e));
+    };
+    T.fx_two_g = constant(P.two_g, T.fx_e2g);
+    FxFaceConstants& c = T.fx_face;
+    c.sqrt_g = constant(P.sqrt_g, c.e_sqrt_g);
+    c.half_g = constant(P.half_g, c.e_half_g);
+    std::frexp(P.g, &c.e_g);
+    std::frexp(P.h_min, &c.e_h_min);
+    if (P.h_min == 0.0) c.e_h_min = -1100;
+    return T.fx_e2g >= -60 && T.fx_e2g <= 60;
 }
 
 // The ready lists of a state uploaded in `chunks` element chunks of

@@ -83,6 +83,11 @@ struct KernelSet {
     void (*dt_listed)(int n1, const DevTables&, const Physics&, const DevBuf& q, const DtParams&,
                       double* dt_el, StepCtl* ctl, const int* active, const int32_t* list,
                       int64_t n, cudaStream_t);
+    // the fixed-point tables from pair_hm, gdb, lift_scale and edge_geo
+    // (DevTables::fx_*), where the variant has them
+    void (*fixed_tables)(int n1, const DevTables&, FxPair* hm, FxPair* gdb, FxLimb* lift,
+                         FxExp* exps, FxPair* normal, cudaStream_t);
+    bool has_fixed;
 };
 
 // kernels_fast.cu: FMA contraction, division-free Manning rate

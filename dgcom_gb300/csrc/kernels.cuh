@@ -58,6 +58,32 @@ __device__ __forceinline__ Q load_q(const DevBuf& in, const DevTables& T, const 
     return q;
 }
 
+__device__ __forceinline__ Sd load_side(const DevBuf& in, const DevTables& T, const Physics& P,
+                                        int64_t g) {
+    return {in.h[g], in.u[g], in.v[g], P.has_bed ? T.bed[g] : 0.0};
+}
+
+struct FacePair {
+    F3 a, b;
+};
+
+// hydro_hll of a face node along its geometry. With DGSWE_FAST, where the
+// interior faces mostly take fixed point, this is a call: the rest (sides not
+// both wet, super-critical flow, walls) then runs the same instructions in
+// every face kernel, the multiply-adds contracted alike, and its registers
+// are not the kernels'.
+#if DGSWE_FAST
+__device__ __noinline__
+#else
+__device__ __forceinline__
+#endif
+    FacePair face_hll(Sd qa, Sd qb, const double* geo, double g, double sqrt_g, double half_g,
+                      double h_min) {
+    FacePair f;
+    hydro_hll(qa, qb, geo[0], geo[1], geo[2], geo[3], geo[4], g, sqrt_g, half_g, h_min, f.a, f.b);
+    return f;
+}
+
 // An element's stage in a multirate pass (element_stage,
 // src/time/multirate.rs:169-200), every operation rounded on its own as the
 // reference's are (no contraction): its substep's start time and step, the
@@ -257,15 +283,29 @@ __global__ void __launch_bounds__(256) face_kernel(DevTables T, Physics P, DevBu
         const int fl = (int)(L & 3), fr = (int)(R & 3);
         const int rfi = N1 - 1 - fi;
         const int nl = P.face_node[fl][fi], nr = P.face_node[fr][rfi];
-        const Q ql = load_q(in, T, P, kl * NN + nl), qr = load_q(in, T, P, kr * NN + nr);
-        const double* geo = &T.edge_geo[e * 5];
+        const int64_t gl = kl * NN + nl, gr = kr * NN + nr;
         F3 fa, fbb;
         if (P.formulation == kWetDry) {
-            hydro_hll(side(ql), side(qr), geo[0], geo[1], geo[2], geo[3], geo[4], g, sqrt_g, half_g,
-                      h_min, fa, fbb);
-            fbb = {-fbb.h, -fbb.hu, -fbb.hv};
+            const Sd ql = load_side(in, T, P, gl), qr = load_side(in, T, P, gr);
+            bool done = false;
+#if DGSWE_FAST
+            fx::FaceFlux f;
+            if (T.fx_normal) done = fx::face_flux(ql, qr, T.fx_normal[e], T.fx_face, f);
+            if (done) {
+                fa = {f.h, f.hu_a, f.hv_a};
+                fbb = {-f.h, -f.hu_b, -f.hv_b};
+            }
+#endif
+            if (!done) {
+                const FacePair f =
+                    face_hll(ql, qr, &T.edge_geo[e * 5], g, sqrt_g, half_g, h_min);
+                fa = f.a;
+                fbb = {-f.b.h, -f.b.hu, -f.b.hv};
+            }
         } else {
-            entropy_surface(ql, qr, geo[0], geo[1], P, fa, fbb);
+            const double* geo = &T.edge_geo[e * 5];
+            entropy_surface(load_q(in, T, P, gl), load_q(in, T, P, gr), geo[0], geo[1], P, fa,
+                            fbb);
         }
         const int64_t sl = (L * N1) + fi, sr = (R * N1) + rfi;
         fb_h[sl] = fa.h;
@@ -294,8 +334,7 @@ __global__ void __launch_bounds__(256) face_kernel(DevTables T, Physics P, DevBu
         const Q qe = wall_ghost(qi, u, v, nx, ny, c.wall_h_min, h_min);
         F3 fdummy;
         if (P.formulation == kWetDry)
-            hydro_hll(side(qi), side(qe), nx, ny, geo[2], geo[3], geo[4], g, sqrt_g, half_g, h_min,
-                      fs, fdummy);
+            fs = face_hll(side(qi), side(qe), geo, g, sqrt_g, half_g, h_min).a;
         else
             entropy_surface(qi, qe, nx, ny, P, fs, fdummy);
     } else {
@@ -422,6 +461,94 @@ __device__ __forceinline__ void line_metric(const DevTables& T, int64_t k, int d
     }
 }
 
+#if DGSWE_FAST
+// A node's exponent fields (a negative depth's sign with it, which no scale
+// takes), two a word: depth and 4095 − depth, momentum and velocity, the mass
+// and momentum fluxes of its face slots. Their maxima over an element give
+// the element's fx::Exps.
+struct ExpWords {
+    unsigned w[3];
+};
+
+__device__ __forceinline__ int max_expo(double x, double y) {
+    return max(fx::expo(x), fx::expo(y));
+}
+
+__device__ __forceinline__ ExpWords node_exponents(double h, double hu, double hv, double u,
+                                                   double v, int64_t s_a, int64_t s_b,
+                                                   const double* fb_h, const double* fb_hu,
+                                                   const double* fb_hv) {
+    int fh = 0, fm = 0;
+    if (s_a >= 0) {
+        fh = fx::expo(fb_h[s_a]);
+        fm = max_expo(fb_hu[s_a], fb_hv[s_a]);
+    }
+    if (s_b >= 0) {
+        fh = max(fh, fx::expo(fb_h[s_b]));
+        fm = max(fm, max_expo(fb_hu[s_b], fb_hv[s_b]));
+    }
+    const unsigned hb = (unsigned)((uint64_t)fp::bits(h) >> 52);
+    return {{hb | (4095u - hb) << 16, (unsigned)(max_expo(hu, hv) | max_expo(u, v) << 16),
+             (unsigned)(fh | fm << 16)}};
+}
+
+// The maxima over each NN lanes of a warp
+template <int NN>
+__device__ __forceinline__ void warp_max(ExpWords& e) {
+#pragma unroll
+    for (int off = NN / 2; off > 0; off >>= 1)
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            e.w[q] = __vmaxu2(e.w[q], __shfl_xor_sync(0xffffffffu, e.w[q], off));
+}
+
+__device__ __forceinline__ fx::Exps exponents(const ExpWords& e) {
+    return {(int)(e.w[0] & 0xFFFFu), 4095 - (int)(e.w[0] >> 16), (int)(e.w[1] & 0xFFFFu),
+            (int)(e.w[1] >> 16),     (int)(e.w[2] & 0xFFFFu),    (int)(e.w[2] >> 16)};
+}
+
+// The edges' unit normals in fixed point
+__global__ void fixed_normals_kernel(DevTables T, FxPair* normal) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= T.n_edges) return;
+    const double* geo = &T.edge_geo[e * 5];
+    normal[e] = {fx::split(fx::to_fixed(geo[0], 1024)), fx::split(fx::to_fixed(geo[1], 1024))};
+}
+
+// The fixed-point tables of each element from its FP64 ones: a warp per
+// element takes the largest exponents, then cuts the entries to them
+template <int N1>
+__global__ void __launch_bounds__(256) fixed_tables_kernel(DevTables T, FxPair* hm, FxPair* gdb,
+                                                           FxLimb* lift, FxExp* exps) {
+    constexpr int NN = N1 * N1, NH = NN * (N1 - 1), NL = 4 * N1;
+    const int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31;
+    if (k >= T.K) return;
+    const double* m = &T.pair_hm[k * NH * 2];
+    const double* b = T.gdb ? &T.gdb[k * NN * 2] : nullptr;
+    const double* l = &T.lift_scale[k * NL];
+    int et = 0, eg = 0, el = 0;
+    for (int q = lane; q < NH * 2; q += 32) et = max(et, fx::expo(m[q]));
+    for (int q = lane; b && q < NN * 2; q += 32) eg = max(eg, fx::expo(b[q]));
+    for (int q = lane; q < NL; q += 32) el = max(el, fx::expo(l[q]));
+    et = __reduce_max_sync(0xffffffffu, et);
+    eg = __reduce_max_sync(0xffffffffu, eg);
+    el = __reduce_max_sync(0xffffffffu, el);
+    const bool ok = et >= fx::kExpLo && et <= fx::kExpHi && el >= fx::kExpLo && el <= fx::kExpHi &&
+                    eg <= fx::kExpHi;
+    eg = max(eg, fx::kExpLo - 400);  // a flat bed: no slope to scale by
+    auto pair = [](double x, double y, int K) {
+        return FxPair{fx::split(fx::to_fixed(x, K)), fx::split(fx::to_fixed(y, K))};
+    };
+    for (int q = lane; q < NH; q += 32)
+        hm[k * NH + q] = pair(m[2 * q], m[2 * q + 1], et + 1);
+    for (int q = lane; q < NN; q += 32)
+        gdb[k * NN + q] = b ? pair(b[2 * q], b[2 * q + 1], eg + 1) : FxPair{};
+    for (int q = lane; q < NL; q += 32) lift[k * NL + q] = fx::split(fx::to_fixed(l[q], el + 2));
+    if (lane == 0) exps[k] = {et - 1022, eg - 1022, el - 1022, ok ? 1 : 0};
+}
+#endif
+
 // LISTED: a multirate pass over lp's elements, each with its own stage
 template <int N1, bool LISTED, int SHAPE = 0>
 __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_BLOCKS)
@@ -431,10 +558,16 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
                  int check_finite, const int* active, DevBuf keep, LtsPass lp) {
     using C = Cfg<N1, SHAPE>;
     constexpr int NN = C::NN, NP = C::NP, NA = C::NA, EPB = C::EPB;
-    __shared__ double s_q[EPB][7][NN];  // h, hu, hv, u, v, b, 2g·h
+    __shared__ double s_q[EPB][6][NN];  // h, hu, hv, u, v, b
     __shared__ double s_x[EPB][C::X];
     __shared__ int s_flag[EPB][3];
     __shared__ double s_red[EPB][5];
+    // an element whose lanes share a warp finds its flags and largest
+    // exponents by votes and shuffles, else in shared memory
+    constexpr bool kInWarp = (NN & (NN - 1)) == 0;
+#if DGSWE_FAST
+    __shared__ unsigned s_exp[kInWarp ? 1 : EPB][6];
+#endif
 
     if (!*active) return;
     const int tid = threadIdx.x;
@@ -451,11 +584,6 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
     const int a = i % N1, j = i / N1;
     const double g = P.g, h_min = P.h_min, sqrt_g = P.sqrt_g, half_g = P.half_g;
 
-    if (i == 0) {
-        s_flag[e][0] = 0;
-        s_flag[e][1] = 0;
-        s_flag[e][2] = 0;
-    }
     double h = 0, hu = 0, hv = 0, u = 0, v = 0, b = 0;
     if (valid) {
         h = in.h[gi];
@@ -465,25 +593,109 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
         v = in.v[gi];
         b = P.has_bed ? T.bed[gi] : 0.0;
     }
-    s_q[e][0][i] = h;
-    s_q[e][1][i] = hu;
-    s_q[e][2][i] = hv;
-    s_q[e][3][i] = u;
-    s_q[e][4][i] = v;
-    s_q[e][5][i] = b;
-    s_q[e][6][i] = P.two_g * h;  // the pairs' pressure 2g·h_a·h_c takes one multiply
-    __syncthreads();
-    if (valid && P.formulation == kWetDry && fp::lt(h, P.subcell_depth)) {
-        atomicOr(&s_flag[e][0], 1);
-        if (!fp::nz(h)) atomicAdd(&s_flag[e][2], 1);
+    // A node lies on at most one s-face (0 or 2) and one r-face (1 or 3):
+    // its slots of the face fluxes in the reference's face order, −1: none
+    int64_t s_a = -1, s_b = -1;
+    if (valid) {
+        int f_a = j == 0 ? 0 : (j == N1 - 1 ? 2 : -1);
+        int f_b = a == N1 - 1 ? 1 : (a == 0 ? 3 : -1);
+        if (f_a == 2 && f_b == 1) {
+            f_a = 1;
+            f_b = 2;
+        }
+        const int64_t fbase = k * 4 * N1;
+        auto slot = [&](int f) -> int64_t {
+            const int fi = f == 0 ? a : (f == 1 ? j : (f == 2 ? N1 - 1 - a : N1 - 1 - j));
+            return fbase + f * N1 + fi;
+        };
+        if (f_a >= 0) s_a = slot(f_a);
+        if (f_b >= 0) s_b = slot(f_b);
+    }
+    // sub: an element with a node below the subcell depth.
+    // dry: a subcell element without water at any node (every h = ±0, so
+    // every u = v = 0): its reconstructed subcell faces are dry, so the
+    // interface fluxes, pressure and bed terms are all ±0, and it skips the
+    // subcell phases (they read only h, u, v and the bed)
+    const bool shallow = valid && P.formulation == kWetDry && fp::lt(h, P.subcell_depth);
+    bool sub, dry;
+#if DGSWE_FAST
+    ExpWords ew = node_exponents(h, hu, hv, u, v, s_a, s_b, fb_h, fb_hu, fb_hv);
+#endif
+    if (kInWarp) {
+        const unsigned lanes = ((1ull << NN) - 1) << ((tid & 31) / NN * NN);
+        sub = (__ballot_sync(0xffffffffu, shallow) & lanes) != 0;
+        dry = (__ballot_sync(0xffffffffu, shallow && !fp::nz(h)) & lanes) == lanes;
+        if (i == 0) s_flag[e][1] = 0;
+#if DGSWE_FAST
+        warp_max<NN>(ew);
+#endif
+    } else {
+        if (i == 0) {
+            s_flag[e][0] = 0;
+            s_flag[e][1] = 0;
+            s_flag[e][2] = 0;
+        }
+#if DGSWE_FAST
+        if (i < 6) s_exp[e][i] = 0;
+#endif
+        __syncthreads();
+        if (shallow) {
+            atomicOr(&s_flag[e][0], 1);
+            if (!fp::nz(h)) atomicAdd(&s_flag[e][2], 1);
+        }
+#if DGSWE_FAST
+        for (int q = 0; q < 3; ++q) {
+            atomicMax(&s_exp[e][2 * q], ew.w[q] & 0xFFFFu);
+            atomicMax(&s_exp[e][2 * q + 1], ew.w[q] >> 16);
+        }
+#endif
+        __syncthreads();
+        sub = s_flag[e][0] != 0;
+        dry = s_flag[e][2] == NN;
+#if DGSWE_FAST
+        for (int q = 0; q < 3; ++q) ew.w[q] = s_exp[e][2 * q] | s_exp[e][2 * q + 1] << 16;
+#endif
+    }
+    // fixed: the wet element's sums in fixed point (fixed64.hpp); an element
+    // whose depths or exponents spread too far for it, and every element of
+    // the exact numerics, takes the FP64 phases
+    bool fixed = false;
+#if DGSWE_FAST
+    fx::Scale sc;
+    FxLimb G{};                                   // 2g·h
+    FxLimb H{};                                   // h
+    int64_t m0 = 0, m1 = 0, u0 = 0, u1 = 0;       // hu, hv, u, v
+    FxLimb* const nd_h = (FxLimb*)&s_x[e][C::PAIR_DOUBLES];
+    int64_t* const nd = (int64_t*)&s_x[e][C::PAIR_DOUBLES + NN];
+    FxLimb* const pairs = (FxLimb*)&s_x[e][0];
+    static_assert(C::PAIR_DOUBLES + 5 * NN <= C::X, "the nodes' numbers fit behind the pairs'");
+    if (valid && !sub) {
+        sc = fx::scales(exponents(ew), T.fx_exp[k], T.fx_ec, T.fx_e2g);
+        fixed = sc.ok;
+    }
+    if (fixed) {
+        H = fx::split(fx::to_fixed(h, sc.kh));
+        G = fx::two_g_h(H, T.fx_two_g, sc);
+        m0 = fx::to_fixed(hu, sc.km);
+        m1 = fx::to_fixed(hv, sc.km);
+        u0 = fx::to_fixed(u, sc.ku);
+        u1 = fx::to_fixed(v, sc.ku);
+        nd_h[i] = H;
+        nd[i] = m0;
+        nd[NN + i] = m1;
+        nd[2 * NN + i] = u0;
+        nd[3 * NN + i] = u1;
+    }
+#endif
+    if (!fixed) {
+        s_q[e][0][i] = h;
+        s_q[e][1][i] = hu;
+        s_q[e][2][i] = hv;
+        s_q[e][3][i] = u;
+        s_q[e][4][i] = v;
+        s_q[e][5][i] = b;
     }
     __syncthreads();
-    const bool sub = s_flag[e][0] != 0;
-    // A subcell element without water at any node (every h = ±0, so every
-    // u = v = 0): its reconstructed subcell faces are dry, so the interface
-    // fluxes, pressure and bed terms are all ±0, and it skips the subcell
-    // phases (they read only h, u, v and the bed)
-    const bool dry = s_flag[e][2] == NN;
     double rh = 0.0, rhu = 0.0, rhv = 0.0;
     const bool affine = valid ? T.affine[k] != 0 : true;
 
@@ -494,7 +706,22 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
     double* ifl = &s_x[e][C::FACE_DOUBLES];          // [dir][line][pos][6]
 
     // ---- phase A: pair fluxes, or the subcells' reconstructed faces ----
-    if (valid && !sub) {
+    if (fixed) {
+#if DGSWE_FAST
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const int8_t* own = &T.sched_owned[(i * NP + q) * 5];
+            const int o = own[0] + own[1] - i;  // the pair's other node
+            const FxPair hm = T.fx_hm[gi * NP + q];
+            const fx::Flux f = fx::pair_flux(G, nd_h[o], m0 + nd[o], m1 + nd[NN + o],
+                                             u0 + nd[2 * NN + o], u1 + nd[3 * NN + o], hm.x, hm.y);
+            FxLimb* slot_f = &pairs[(i * NP + q) * 3];
+            slot_f[0] = f.h;
+            slot_f[1] = f.hu;
+            slot_f[2] = f.hv;
+        }
+#endif
+    } else if (valid && !sub) {
 #pragma unroll
         for (int q = 0; q < NP; ++q) {
             const int8_t* own = &T.sched_owned[(i * NP + q) * 5];
@@ -505,7 +732,7 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
             // ½·F#(q_a, q_c)·{{Ja}} scaled: mass, 2·F_hu, 2·F_hv
             const double mass = (s_q[e][1][na] + s_q[e][1][nc]) * hm0 +
                                 (s_q[e][2][na] + s_q[e][2][nc]) * hm1;
-            const double gp2 = s_q[e][6][na] * hc;
+            const double gp2 = P.two_g * s_q[e][0][na] * hc;
             const double g_hu = mass * (s_q[e][3][na] + s_q[e][3][nc]) + gp2 * hm0;
             const double g_hv = mass * (s_q[e][4][na] + s_q[e][4][nc]) + gp2 * hm1;
             double* slot_f = &s_x[e][(i * NP + q) * 3];
@@ -570,7 +797,30 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
     __syncthreads();
 
     // ---- phase B: sum the pairs; or the subcell interface fluxes ----
-    if (valid && !sub) {
+#if DGSWE_FAST
+    int64_t fh = 0, fhu = 0, fhv = 0;  // the sums in fixed point
+#endif
+    if (fixed) {
+#if DGSWE_FAST
+        fx::PairSum ah = fx::pair_sum(), au = ah, av = ah;
+#pragma unroll
+        for (int q = 0; q < NA; ++q) {
+            const FxLimb* f = &pairs[T.sched_slot[i * NA + q] * 3];
+            const FxLimb coef = T.fx_coef[i * NA + q];
+            fx::mac(ah, coef, f[0]);
+            fx::mac(au, coef, f[1]);
+            fx::mac(av, coef, f[2]);
+        }
+        fh = -fx::fold(ah);
+        fhu = -fx::fold(au);
+        fhv = -fx::fold(av);
+        if (P.has_bed) {
+            const FxPair slope = T.fx_gdb[gi];
+            fhu -= fx::bed_term(H, slope.x, sc);
+            fhv -= fx::bed_term(H, slope.y, sc);
+        }
+#endif
+    } else if (valid && !sub) {
 #pragma unroll
         for (int q = 0; q < NA; ++q) {
             const int slot_id = T.sched_slot[i * NA + q];
@@ -585,10 +835,12 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
             rhu -= h * T.gdb[gi * 2];
             rhv -= h * T.gdb[gi * 2 + 1];
         }
+    }
+    if (valid && !sub) {
         if (X.subcell_mass)  // no subcells: NaN (compute_rhs_swe_2d_mass_fluxes_into)
             for (int q = i; q < C::NSUB; q += NN)
                 X.subcell_mass[k * C::NSUB + q] = fp::from_bits(0x7FF8000000000000ll);
-    } else if (valid && sub && dry) {
+    } else if (valid && dry) {
         if (X.subcell_mass)  // the dry element's interface fluxes are ±0
             for (int q = i; q < C::NSUB; q += NN) X.subcell_mass[k * C::NSUB + q] = 0.0;
     } else if (valid && sub && !dry) {
@@ -673,54 +925,55 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
         }
     }
 
-    // ---- surface: −LIFT·sJ·F* of the node's faces ----
-    // A node lies on at most one s-face (0 or 2) and one r-face (1 or 3).
-    // Every lane takes two slots in face order, a missing one as zero, so
-    // the warp's FP64 instructions run on all lanes instead of once per
-    // face with only that face's nodes active. Subtracting +0 is exact.
+    // ---- surface: −LIFT·sJ·F* of the node's faces, and 1/J ----
+    // Every lane takes two slots, a missing one as zero, so the warp's
+    // instructions run on all lanes instead of once per face with only that
+    // face's nodes active. Subtracting +0 is exact.
+    double Fh = 0.0, Fhu = 0.0, Fhv = 0.0;
     if (valid) {
-        int f_a = j == 0 ? 0 : (j == N1 - 1 ? 2 : -1);
-        int f_b = a == N1 - 1 ? 1 : (a == 0 ? 3 : -1);
-        if (f_a == 2 && f_b == 1) {  // the reference's face order
-            f_a = 1;
-            f_b = 2;
-        }
-        const int64_t fbase = k * 4 * N1;
-        auto slot = [&](int f) -> int64_t {
-            const int fi = f == 0 ? a : (f == 1 ? j : (f == 2 ? N1 - 1 - a : N1 - 1 - j));
-            return fbase + f * N1 + fi;
-        };
-        double c_a = 0.0, h_a = 0.0, hu_a = 0.0, hv_a = 0.0;
-        double c_b = 0.0, h_b = 0.0, hu_b = 0.0, hv_b = 0.0;
-        if (f_a >= 0) {
-            const int64_t s_a = slot(f_a);
-            c_a = T.lift_scale[s_a];
+        double h_a = 0.0, hu_a = 0.0, hv_a = 0.0, h_b = 0.0, hu_b = 0.0, hv_b = 0.0;
+        if (s_a >= 0) {
             h_a = fb_h[s_a];
             hu_a = fb_hu[s_a];
             hv_a = fb_hv[s_a];
         }
-        if (f_b >= 0) {
-            const int64_t s_b = slot(f_b);
-            c_b = T.lift_scale[s_b];
+        if (s_b >= 0) {
             h_b = fb_h[s_b];
             hu_b = fb_hu[s_b];
             hv_b = fb_hv[s_b];
         }
-        rh -= c_a * h_a;
-        rhu -= c_a * hu_a;
-        rhv -= c_a * hv_a;
-        rh -= c_b * h_b;
-        rhu -= c_b * hu_b;
-        rhv -= c_b * hv_b;
+        const double jinv = T.jinv[gi];
+        if (fixed) {
+#if DGSWE_FAST
+            const FxLimb c_a = s_a >= 0 ? T.fx_lift[s_a] : FxLimb{0, 0};
+            const FxLimb c_b = s_b >= 0 ? T.fx_lift[s_b] : FxLimb{0, 0};
+            auto lift = [&](double x, double y, int K) {
+                fx::Acc s{fx::half<0>(), 0};
+                fx::mac(s, c_a, fx::split(fx::to_fixed(x, K)));
+                fx::mac(s, c_b, fx::split(fx::to_fixed(y, K)));
+                return fx::fold<0>(s);
+            };
+            Fh = fx::over_jacobian(fh - lift(h_a, h_b, sc.kfh), sc.sh, jinv);
+            Fhu = fx::over_jacobian(fhu - lift(hu_a, hu_b, sc.kfm), sc.sm, jinv);
+            Fhv = fx::over_jacobian(fhv - lift(hv_a, hv_b, sc.kfm), sc.sm, jinv);
+#endif
+        } else {
+            const double c_a = s_a >= 0 ? T.lift_scale[s_a] : 0.0;
+            const double c_b = s_b >= 0 ? T.lift_scale[s_b] : 0.0;
+            rh -= c_a * h_a;
+            rhu -= c_a * hu_a;
+            rhv -= c_a * hv_a;
+            rh -= c_b * h_b;
+            rhu -= c_b * hu_b;
+            rhv -= c_b * hv_b;
+            Fh = jinv * rh;
+            Fhu = jinv * rhu;
+            Fhv = jinv * rhv;
+        }
     }
 
-    // ---- 1/J and the sources ----
-    double Fh = 0.0, Fhu = 0.0, Fhv = 0.0;
+    // ---- the sources ----
     if (valid) {
-        const double jinv = T.jinv[gi];
-        Fh = jinv * rh;
-        Fhu = jinv * rhu;
-        Fhv = jinv * rhv;
         if (P.has_coriolis) {
             const double f = P.coriolis_field ? T.fcor[gi] : P.f0;
             Fhu += f * hv;

@@ -149,6 +149,15 @@ static void face_ready_n(const DevTables& T, const Physics& P, const DevBuf& in,
                                                      lp);
 }
 
+#if DGSWE_FAST
+template <int N1>
+static void fixed_tables_n(const DevTables& T, FxPair* hm, FxPair* gdb, FxLimb* lift, FxExp* exps,
+                           cudaStream_t s) {
+    if (T.K > 0)
+        fixed_tables_kernel<N1><<<(unsigned)((T.K + 7) / 8), 256, 0, s>>>(T, hm, gdb, lift, exps);
+}
+#endif
+
 #define DGSWE_BY_ORDER(fn, ...)            \
     switch (n1) {                          \
         case 2: fn<2>(__VA_ARGS__); break; \
@@ -262,6 +271,15 @@ static void face_adjoint(int n1, const DevTables& T, const Physics& P, const Dev
     DGSWE_BY_ORDER(face_adjoint_n, T, P, in, A, ctl, slot, s);
 }
 
+static void fixed_tables(int n1, const DevTables& T, FxPair* hm, FxPair* gdb, FxLimb* lift,
+                         FxExp* exps, FxPair* normal, cudaStream_t s) {
+#if DGSWE_FAST
+    if (T.n_edges > 0)
+        fixed_normals_kernel<<<(unsigned)((T.n_edges + 255) / 256), 256, 0, s>>>(T, normal);
+    DGSWE_BY_ORDER(fixed_tables_n, T, hm, gdb, lift, exps, s);
+#endif
+}
+
 #undef DGSWE_BY_ORDER
 
 static void adjoint_combine(const DevBuf& in, const AdjStage& A, double* out_h, double* out_hu,
@@ -330,7 +348,7 @@ static const KernelSet kSet = {face,          stage,         finish,          dt
                                 dt_fit,        end,           face_listed,     stage_listed,
                                 finish_listed, depth_flags,    subcell_list,
                                 implicit_damping, face_ready,  node_sources,
-                                dt_listed};
+                                dt_listed,     fixed_tables,  DGSWE_FAST};
 
 }  // namespace DGSWE_NS
 }  // namespace dgswe
