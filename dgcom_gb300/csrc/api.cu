@@ -599,10 +599,20 @@ int create_impl(dgswe_handle* h, const dgswe_form* f, int device) {
     UP(pair_coef, pair_coef_table(sched));
 
     fill_physics(*f, ops, !t.fcor.empty(), h->P, h->X);
+    {
+        // tables made on the device, on the uploads' own stream and done
+        // before any other stream reads them
+        double* metric = nullptr;
+        if ((s = device_array(h, (size_t)h->K * 4 * ops.n1 * (ops.n1 - 1), &metric))) return bail(s);
+        h->ks->sub_metrics(h->n1, T, h->P, metric, nullptr);
+        CK(cudaGetLastError());
+        T.sub_metric = metric;
+    }
     if (h->ks->has_fixed) {
         std::vector<FxLimb> coef;
         const bool usable = fixed_constants(sched, h->P, T, coef);
         UP(fx_coef, coef);
+        UP(fx_node, fixed_schedule(sched));
         const size_t nh = (size_t)h->n_values * (ops.n1 - 1), nl = (size_t)h->K * 4 * ops.n1;
         FxPair *hm = nullptr, *gdb = nullptr;
         FxLimb* lift = nullptr;
@@ -610,19 +620,21 @@ int create_impl(dgswe_handle* h, const dgswe_form* f, int device) {
         FxPair* normal = nullptr;
         if ((s = device_array(h, nh, &hm)) || (s = device_array(h, (size_t)h->n_values, &gdb)) ||
             (s = device_array(h, nl, &lift)) || (s = device_array(h, (size_t)h->K, &exps)) ||
+            (s = device_array(h, (size_t)h->K, &T.gen_list)) ||
+            (s = device_array(h, 2, &T.gen_count)) ||
             (s = device_array(h, (size_t)T.n_edges, &normal)))
             return bail(s);
-        // on the uploads' own stream, and done before any other stream reads them
         h->ks->fixed_tables(h->n1, T, hm, gdb, lift, exps, normal, nullptr);
         CK(cudaGetLastError());
         if (!usable) CK(cudaMemsetAsync(exps, 0, (size_t)h->K * sizeof(FxExp), nullptr));
-        CK(cudaStreamSynchronize(nullptr));
+        CK(cudaMemsetAsync(T.gen_count, 0, 2 * sizeof(unsigned), nullptr));
         T.fx_hm = hm;
         T.fx_gdb = gdb;
         T.fx_lift = lift;
         T.fx_exp = exps;
         if (usable) T.fx_normal = normal;  // null: every face in FP64
     }
+    CK(cudaStreamSynchronize(nullptr));
 #undef UP
     h->P.n_conditions = f->n_boundaries;
     for (int b = 0; b < f->n_boundaries; ++b) h->P.cond[b] = make_condition(f->boundaries[b]);

@@ -31,11 +31,16 @@ struct alignas(16) FxPair {
 struct alignas(16) FxExp {
     int32_t et, eg, el, ok;
 };
-// √g and g/2 at 2^(62 − e), their exponents and g's and h_min's (the least e
-// with x < 2^e)
+// A node's pairs, a byte each: the other nodes of the ones it owns, the slots
+// of all it is in
+struct alignas(16) FxNode {
+    uint64_t slots;
+    uint32_t others, unused;
+};
+// √g and g/2 at 2^(62 − e), their exponents and g's (the least e with x < 2^e)
 struct FxFaceConstants {
     FxLimb sqrt_g, half_g;
-    int e_sqrt_g, e_half_g, e_g, e_h_min;
+    int e_sqrt_g, e_half_g, e_g;
 };
 
 struct DevTables {
@@ -55,6 +60,7 @@ struct DevTables {
     const double* sched_coef;   // [nn][2(n1-1)]
     const double* sched_hcoef;  // [nn][2(n1-1)] sched_coef / 2
     const double* pair_coef;    // [nn·(n1-1)][4] per owned slot: both nodes' coefficients, halves
+    const double* sub_metric = nullptr;  // [K][2·n1·(n1−1)][2] the subcell interfaces' metrics
     // the wet stage's tables in fixed point (fixed64.hpp), made on the device
     // from the ones above: pair_hm, gdb and lift_scale as limbs with their
     // element's exponents {et, eg, el, usable}, sched_coef as limbs at
@@ -64,7 +70,12 @@ struct DevTables {
     const FxLimb* fx_lift = nullptr;  // [K·4·n1]
     const FxExp* fx_exp = nullptr;    // [K]
     const FxLimb* fx_coef = nullptr;  // [nn][2(n1−1)]
+    const FxNode* fx_node = nullptr;  // [nn]
     const FxPair* fx_normal = nullptr;  // [E] the edges' unit normals at 2^61
+    // the elements a stage leaves to general_kernel, and {their number, the
+    // blocks that have ended}; empty between stages
+    int32_t* gen_list = nullptr;     // [K]
+    unsigned* gen_count = nullptr;   // [2]
     FxLimb fx_two_g{};
     FxFaceConstants fx_face{};
     int fx_ec = 0, fx_e2g = 0;

@@ -205,10 +205,20 @@ int build_group(dgswe_ensemble* h, Group& G, std::vector<Tables>& tabs,
     UP(sched_hcoef, hcoef);
     UP(pair_coef, pair_coef_table(sched));
     fill_physics(h->form0, ops, fcor, G.P, G.X);
+    {
+        // tables made on the device, on the uploads' own stream and done
+        // before any other stream reads them
+        double* metric = nullptr;
+        if ((s = device_array(h, (size_t)G.K * 4 * ops.n1 * (ops.n1 - 1), &metric))) return s;
+        h->ks->sub_metrics(n1, T, G.P, metric, nullptr);
+        CK(cudaGetLastError());
+        T.sub_metric = metric;
+    }
     if (h->ks->has_fixed) {
         std::vector<FxLimb> coef;
         const bool usable = fixed_constants(sched, G.P, T, coef);
         UP(fx_coef, coef);
+        UP(fx_node, fixed_schedule(sched));
         FxPair *hm = nullptr, *gdb = nullptr;
         FxLimb* lift = nullptr;
         FxExp* exps = nullptr;
@@ -217,19 +227,21 @@ int build_group(dgswe_ensemble* h, Group& G, std::vector<Tables>& tabs,
             (s = device_array(h, (size_t)G.n_values, &gdb)) ||
             (s = device_array(h, (size_t)G.K * 4 * n1, &lift)) ||
             (s = device_array(h, (size_t)G.K, &exps)) ||
+            (s = device_array(h, (size_t)G.K, &T.gen_list)) ||
+            (s = device_array(h, 2, &T.gen_count)) ||
             (s = device_array(h, (size_t)T.n_edges, &normal)))
             return s;
-        // on the uploads' own stream, and done before any other stream reads them
         h->ks->fixed_tables(n1, T, hm, gdb, lift, exps, normal, nullptr);
         CK(cudaGetLastError());
         if (!usable) CK(cudaMemsetAsync(exps, 0, (size_t)G.K * sizeof(FxExp), nullptr));
-        CK(cudaStreamSynchronize(nullptr));
+        CK(cudaMemsetAsync(T.gen_count, 0, 2 * sizeof(unsigned), nullptr));
         T.fx_hm = hm;
         T.fx_gdb = gdb;
         T.fx_lift = lift;
         T.fx_exp = exps;
         if (usable) T.fx_normal = normal;  // null: every face in FP64
     }
+    CK(cudaStreamSynchronize(nullptr));
 #undef UP
     G.P.has_bed = h->form0.bathymetry ? 1 : 0;
     G.P.friction = friction ? DGSWE_FRICTION_MANNING_NODES : DGSWE_FRICTION_NONE;

@@ -282,6 +282,23 @@ DG_HD double from_fixed(int64_t v, int s) {
     return fp::from_bits((int64_t)(bits | ((uint64_t)sign & 0x8000000000000000ull)));
 }
 
+// Products of two numbers
+template <int K>
+DG_HD int64_t mul(const Lim& a, const Lim& b) {
+    Acc s{half<K>(), 0};
+    mac(s, a, b);
+    return fold<K>(s);
+}
+
+// x/y for normal x and y > 0 whose exponents lie within 2^±400 (the caller's
+// guard): x's mantissa times 1/y to 2^-59, rounded once
+DG_HD double div_pos(double x, double y) {
+    const uint64_t r = reciprocal61(mant(y) << 11);
+    const int64_t q = mul<3>(split((int64_t)(mant(x) << 9)), split((int64_t)r));  // 2^61·
+    const double v = from_fixed(q, 61 - expo(x) + expo(y));
+    return fp::bits(x) < 0 ? fp::neg(v) : v;
+}
+
 // ---- the wet element's right-hand side --------------------------------------
 //
 // Volume pairs, bed slope, surface lift and 1/J of a wet element, the FP64
@@ -387,16 +404,20 @@ DG_HD double over_jacobian(int64_t V, int s, double jinv) {
     return from_fixed(fold<1>(a), s + 1021 - expo(jinv));
 }
 
-// ---- the interior face's flux ------------------------------------------------
+// ---- the flux between two sides ----------------------------------------------
 //
-// hydro_hll (point.cuh) between two wet sides in sub-critical flow, each
+// hydro_hll (point.cuh) with at least one reconstructed side wet, each
 // quantity at a scale of the face node's own exponents (E: |x| < 2^E):
-//   depths 2^(61 − eh), velocities 2^(60 − ev), speeds of waves 2^(60 − eS),
-//   mass flux 2^(60 − eM), momentum flux 2^(59 − eQ), weights 2^61.
-// With α = S_R/(S_R − S_L), β = 1 − α and w = −α·S_L the star flux is
+//   surface sums 2^(60 − eL) (eL: depths and beds), reconstructed depths
+//   2^(61 − es), own depths 2^(61 − eh), velocities 2^(60 − ev), speeds of
+//   waves 2^(60 − eS), mass flux 2^(60 − eM), momentum flux 2^(59 − eQ),
+//   weights 2^61.
+// With S_L and S_R the wave speeds held to S_L ≤ 0 ≤ S_R, α = S_R/(S_R − S_L),
+// β = 1 − α and w = −α·S_L, the flux is
 //   α·F_l + β·F_r − w·(q_r − q_l),
-// whose differences of depths are exact, so that a face at rest has no mass
-// flux; eM follows the depths' difference, not their size.
+// the star flux in sub-critical flow and one side's (α or β = 1, w = 0)
+// otherwise. The differences of depths in it are exact, so that a face at
+// rest has no mass flux; eM follows the depths' difference, not their size.
 
 using FaceConstants = FxFaceConstants;
 
@@ -410,21 +431,14 @@ DG_HD int imax(int a, int b) { return a > b ? a : b; }
 DG_HD int64_t shr(int64_t v, int n) { return v >> (n > 63 ? 63 : n); }
 DG_HD int64_t abs64(int64_t v) { return v < 0 ? -v : v; }
 
-template <int K>
-DG_HD int64_t mul(const Lim& a, const Lim& b) {
-    Acc s{half<K>(), 0};
-    mac(s, a, b);
-    return fold<K>(s);
-}
-
-// √(g·x) at 2^(60 − eC) for x > 0 at 2^s (below 2^62), √(g·x) < 2^eC
+// √(g·x) at 2^(60 − eC) for 0 ≤ x at 2^s (below 2^62), √(g·x) < 2^eC
 DG_HD int64_t celerity(int64_t x, int s, const FaceConstants& c, int eC) {
     int up = clz64((uint64_t)x) - 2;     // x·2^up in [2^61, 2^62)
     up -= (60 - up - s) & 1;             // one less where that makes the exponent even
     const uint64_t X = up >= 0 ? (uint64_t)x << up : (uint64_t)x >> 1;
     const int p = 60 - up - s;           // x's value is X·2^(p − 60)
-    const int64_t v = mul<2>(split((int64_t)(root62(X) >> 1)), c.sqrt_g);
-    return shr(v, 1 - c.e_sqrt_g - p / 2 + eC);
+    const int64_t v = mul<2>(split((int64_t)(root62(x ? X : 1ull << 60) >> 1)), c.sqrt_g);
+    return x ? shr(v, 1 - c.e_sqrt_g - p / 2 + eC) : 0;
 }
 
 // a/(a + b) at 2^61 for 0 ≤ a, b < 2^61, not both 0
@@ -435,109 +449,130 @@ DG_HD int64_t share(int64_t a, int64_t b) {
     return mul<3>(split((int64_t)((uint64_t)a << up)), split((int64_t)q));
 }
 
-// False where the sides are not both wet, or the exponents spread too far:
-// nothing is written then
+// The flux along the unit normal n, times the vector m = |m|·n (each number
+// of m at 2^(61 − em); the mass flux times the length |m| by the caller), as
+// seen from both sides. Nothing is written where both reconstructed sides
+// are dry (kBothDry, but for two sides without any water) or the exponents
+// are out of range (kNoScale).
+enum FaceCase { kNoScale = 0, kDone = 1, kBothDry = 2 };
+
 template <class Side>
-DG_HD bool face_flux(const Side& qa, const Side& qb, const FxPair& n, const FaceConstants& c,
-                     FaceFlux& out) {
+DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const FxPair& n, const FxPair& m, int em,
+                     const FaceConstants& c, double h_min, FaceFlux& out) {
     const int xa = (int)((uint64_t)fp::bits(qa.h) >> 52), xb = (int)((uint64_t)fp::bits(qb.h) >> 52);
     const int xh = imax(xa, xb);
+    if (xh == 0) {  // depths of +0 or subnormal
+        out = {0.0, 0.0, 0.0, 0.0, 0.0};
+        return fp::bits(qa.h) == 0 && fp::bits(qb.h) == 0 ? kDone : kNoScale;
+    }
     const int xl = imax(xh, imax(expo(qa.b), expo(qb.b)));
     const int xv = imax(imax(expo(qa.u), expo(qa.v)), imax(expo(qb.u), expo(qb.v)));
-    // depths within 2^±120 (a negative one's sign field is above) and within
-    // 2^7 of the bed's elevation, so that the surface's sums hold them whole
-    if (xl > kExpHi || imax(xv, xh) > kExpHi || (xa < xb ? xa : xb) < imax(kExpLo, xl - 7))
-        return false;
-    const int eh = xh - 1022, up = xl - xh + 1;
-    // hydrostatic reconstruction: the surfaces over the higher bed, exact
-    const int64_t la = to_fixed(qa.h, xl + 3), lb = to_fixed(qb.h, xl + 3);  // 2^(60 − eL)
+    // within 2^±120 (a negative depth's sign field is above), h_min not above
+    // everything
+    if (imax(xv, xl) > kExpHi || xh < kExpLo || expo(h_min) > xl + 2) return kNoScale;
+    const int eL = xl - 1022, eh = xh - 1022;
+    // hydrostatic reconstruction: the surfaces over the higher bed
+    const int64_t la = to_fixed(qa.h, xl + 3), lb = to_fixed(qb.h, xl + 3);
     const int64_t ba = to_fixed(qa.b, xl + 3), bb = to_fixed(qb.b, xl + 3);
     const int64_t top = max64(ba, bb);
-    const int64_t ha = (int64_t)((uint64_t)la << up), hb = (int64_t)((uint64_t)lb << up);
-    const int64_t sa = (int64_t)((uint64_t)(la + ba - top) << up);
-    const int64_t sb = (int64_t)((uint64_t)(lb + bb - top) << up);
-    // every depth above twice h_min (its side wet beyond rounding)
-    const int64_t least = min64(sa, sb);
-    if (least <= 0 || 63 - clz64((uint64_t)least) + eh - 61 <= c.e_h_min) return false;
-    const int eC = (eh + c.e_g + 1) >> 1;
+    const int64_t ra = max64(la + ba - top, 0), rb = max64(lb + bb - top, 0);
+    const int64_t dry = to_fixed(h_min, xl + 3);
+    const bool wet_a = ra > dry, wet_b = rb > dry;
+    if (!wet_a && !wet_b) return kBothDry;
+    const int es = 64 - clz64((uint64_t)max64(ra, rb)) + eL - 60;
+    if (es < -60) return kNoScale;
+    const int64_t sa = (int64_t)((uint64_t)ra << (eL - es + 1));
+    const int64_t sb = (int64_t)((uint64_t)rb << (eL - es + 1));
+    const int eC = (es + c.e_g + 1) >> 1;
     const int ev = imax(xv - 1022, eC - 30);
     const int kv = 1024 + ev;
-    auto rotate = [&](const Lim& u, const Lim& v, int64_t& normal, int64_t& along) {
-        Acc a{half<2>(), 0}, t{half<2>(), 0};
+    auto rotate = [&](const Side& q, int64_t& normal, int64_t& along) {
+        const bool moves = fp::gt(q.h, h_min);
+        const Lim u = split(moves ? to_fixed(q.u, kv) : 0), v = split(moves ? to_fixed(q.v, kv) : 0);
+        Acc a{half<2>(), 0}, t{half<2>(), 0}, o{0, 0};
         mac(a, u, n.x);
         mac(a, v, n.y);
         normal = fold<2>(a);
         mac(t, v, n.x);
-        Acc o{0, 0};
         mac(o, u, n.y);
         t.t -= o.t;
         t.r -= o.r;
         along = fold<2>(t);
     };
     int64_t un_a, ut_a, un_b, ut_b;  // 2^(60 − ev)
-    rotate(split(to_fixed(qa.u, kv)), split(to_fixed(qa.v, kv)), un_a, ut_a);
-    rotate(split(to_fixed(qb.u, kv)), split(to_fixed(qb.v, kv)), un_b, ut_b);
-    // wave speeds (Einfeldt)
-    const int64_t c_a = celerity(sa, 61 - eh, c, eC), c_b = celerity(sb, 61 - eh, c, eC);
-    const int64_t c_m = celerity(sa + sb, 62 - eh, c, eC);
-    const Lim ul = split(un_a), ur = split(un_b);
-    const int64_t u_m = un_b + mul<3>(split(share(c_a, c_b)), split(un_a - un_b));
-    const int eS = imax(ev + 1, eC) + 1;
+    rotate(qa, un_a, ut_a);
+    rotate(qb, un_b, ut_b);
+    // wave speeds (Einfeldt; beside a dry side, the front's)
+    const int64_t c_a = celerity(sa, 61 - es, c, eC), c_b = celerity(sb, 61 - es, c, eC);
+    const int64_t c_m = celerity(sa + sb, 62 - es, c, eC);
+    const int64_t va = wet_a ? un_a : 0, vb = wet_b ? un_b : 0;
+    const int64_t u_m = vb + mul<3>(split(share(c_a, c_b)), split(va - vb));
+    const int eS = imax(ev, eC) + 2;
     const int dv = eS - ev, dc = eS - eC;
-    const int64_t s_l = min64(shr(un_a, dv) - shr(c_a, dc), shr(u_m, dv) - shr(c_m, dc));
-    const int64_t s_r = max64(shr(un_b, dv) + shr(c_b, dc), shr(u_m, dv) + shr(c_m, dc));
-    if (s_l >= 0 || s_r <= 0) return false;
+    const int64_t wa = shr(c_a, dc), wb = shr(c_b, dc), wm = shr(c_m, dc);
+    const int64_t xl_ = shr(va, dv), xr_ = shr(vb, dv), xm = shr(u_m, dv);
+    const int64_t s_l = min64(wet_a ? min64(xl_ - wa, xm - wm) : xr_ - 2 * wb, 0);
+    const int64_t s_r = max64(wet_b ? max64(xr_ + wb, xm + wm) : xl_ + 2 * wa, 0);
+    if (s_l == s_r) return kNoScale;
     const int64_t alpha = share(s_r, -s_l);
     const Lim al = split(alpha), be = split((1ll << 61) - alpha);
     const Lim w = split(mul<3>(al, split(-s_l)));  // 2^(60 − eS)
-    // momenta hs·un, hs·ut at 2^(60 − eh − ev)
+    // momenta hs·un, hs·ut at 2^(60 − es − ev); a dry side carries none in its
+    // own flux
     const Lim da = split(sa), db = split(sb);
+    const Lim ul = split(un_a), ur = split(un_b);
     const int64_t m_a = mul<3>(da, ul), m_b = mul<3>(db, ur);
     const Lim tl = split(ut_a), tr = split(ut_b);
     const int64_t t_a = mul<3>(da, tl), t_b = mul<3>(db, tr);
-    const Lim ml = split(m_a), mr = split(m_b);
+    const Lim ml = split(wet_a ? m_a : 0), mr = split(wet_b ? m_b : 0);
     // mass
     const int64_t dh = sb - sa;
     const int grow = clz64((uint64_t)abs64(dh)) - 3;  // dh·2^grow below 2^61
-    const int eD = eh - grow;
-    const int eM = imax(eh + ev + 1, eS + eD);
+    const int eD = es - grow;
+    const int eM = imax(es + ev + 1, eS + eD);
     Acc f{half<3>(), 0};
     mac(f, al, ml);
     mac(f, be, mr);
-    const int64_t f_h = shr(fold<3>(f), eM - eh - ev) -
+    const int64_t f_h = shr(fold<3>(f), eM - es - ev) -
                         shr(mul<3>(w, split((int64_t)((uint64_t)dh << grow))), eM - eS - eD);
     out.h = from_fixed(f_h, 60 - eM);
     // momentum
-    const int eP = 2 * eh + c.e_half_g;
-    const int eQ = imax(imax(eP, eh + 2 * ev + 1), eS + eh + ev - 1);
-    const int dp = 1 + eQ - eP, dm = 1 + eQ - eh - 2 * ev, dw = 1 + eQ - eS - eh - ev;
-    auto pressure = [&](int64_t x, int64_t y) {  // ½g·x·y of depths' scale, at 2^(59 − eQ)
-        return shr(mul<1>(split(mul<3>(split(x), split(y))), c.half_g), dp);
+    const int eQ = imax(imax(2 * eh + c.e_half_g, es + 2 * ev + 1), eS + es + ev - 1);
+    const int dm = 1 + eQ - es - 2 * ev, dw = 1 + eQ - eS - es - ev;
+    auto pressure = [&](int64_t x, int64_t y, int e) {  // ½g·x·y of depths at 2^(61 − e)
+        return shr(mul<1>(split(mul<3>(split(x), split(y))), c.half_g), 1 + eQ - 2 * e - c.e_half_g);
     };
     Acc g{half<3>(), 0};
-    mac(g, al, split(pressure(sa, sa) + shr(mul<4>(ml, ul), dm)));
-    mac(g, be, split(pressure(sb, sb) + shr(mul<4>(mr, ur), dm)));
+    mac(g, al, split(pressure(sa, sa, es) + shr(mul<4>(ml, ul), dm)));
+    mac(g, be, split(pressure(sb, sb, es) + shr(mul<4>(mr, ur), dm)));
     const int64_t f_n = fold<3>(g) - shr(mul<4>(w, split(m_b - m_a)), dw);
     Acc t{half<3>(), 0};
     mac(t, al, split(shr(mul<4>(ml, tl), dm)));
     mac(t, be, split(shr(mul<4>(mr, tr), dm)));
     const Lim f_t = split(fold<3>(t) - shr(mul<4>(w, split(t_b - t_a)), dw));
-    // each side's own pressure over the reconstructed one, and back
+    // each side's own pressure over the reconstructed one. Where a depth has
+    // bits below the surface sums' last place, the own one is taken whole
+    // and the pressure of its rounding cancels against the flux's.
+    const int down = eL - eh + 1;
+    const bool whole = (xa < xb ? xa : xb) >= xl - 7;
+    const int64_t ha = whole ? (int64_t)((uint64_t)la << down) : to_fixed(qa.h, xh + 2);
+    const int64_t hb = whole ? (int64_t)((uint64_t)lb << down) : to_fixed(qb.h, xh + 2);
+    const int64_t ga = (int64_t)((uint64_t)ra << down), gb = (int64_t)((uint64_t)rb << down);
     auto back = [&](int64_t normal, double& x, double& y) {
         const Lim fn = split(normal);
         Acc a{half<2>(), 0}, o{0, 0}, b{half<2>(), 0};
-        mac(a, fn, n.x);
-        mac(o, f_t, n.y);
+        mac(a, fn, m.x);
+        mac(o, f_t, m.y);
         a.t -= o.t;
         a.r -= o.r;
-        mac(b, fn, n.y);
-        mac(b, f_t, n.x);
-        x = from_fixed(fold<2>(a), 58 - eQ);
-        y = from_fixed(fold<2>(b), 58 - eQ);
+        mac(b, fn, m.y);
+        mac(b, f_t, m.x);
+        x = from_fixed(fold<2>(a), 58 - eQ - em);
+        y = from_fixed(fold<2>(b), 58 - eQ - em);
     };
-    back(f_n + pressure(ha - sa, ha + sa), out.hu_a, out.hv_a);
-    back(f_n + pressure(hb - sb, hb + sb), out.hu_b, out.hv_b);
-    return true;
+    back(f_n + pressure(ha - ga, ha + ga, eh), out.hu_a, out.hv_a);
+    back(f_n + pressure(hb - gb, hb + gb, eh), out.hu_b, out.hv_b);
+    return kDone;
 }
 
 }  // namespace fx

@@ -73,6 +73,8 @@ DG_HD bool le(double a, double b) { return key(a) <= key(b); }  // a <= b
 // a > b ? a : b and a < b ? a : b
 DG_HD double lmax(double a, double b) { return gt(a, b) ? a : b; }
 DG_HD double lmin(double a, double b) { return lt(a, b) ? a : b; }
+// -x
+DG_HD double neg(double x) { return from_bits((int64_t)((uint64_t)bits(x) ^ kNegZero)); }
 // x > 0 ? x : +0 (the depth floor max(x, 0) of the reference's selects)
 DG_HD double max0(double x) { return gt0(x) ? x : 0.0; }
 

@@ -265,10 +265,26 @@ inline std::vector<double> pair_coef_table(const PairSchedule& sched) {
     return pc;
 }
 
+// The schedule of the wet stage in fixed point, a word for each list
+inline std::vector<FxNode> fixed_schedule(const PairSchedule& sched) {
+    const int np = sched.n1 - 1;
+    std::vector<FxNode> nodes((size_t)sched.nn);
+    for (int i = 0; i < sched.nn; ++i) {
+        nodes[i] = {0, 0, 0};
+        for (int q = 0; q < np; ++q) {
+            const PairSlot& p = sched.owned[(size_t)i * np + q];
+            nodes[i].others |= (uint32_t)(p.a + p.c - i) << (8 * q);
+        }
+        for (int q = 0; q < 2 * np; ++q)
+            nodes[i].slots |= (uint64_t)sched.accum_slot[(size_t)i * 2 * np + q] << (8 * q);
+    }
+    return nodes;
+}
+
 // The fixed-point constants of the wet stage and of the interior faces
 // (fixed64.hpp): the accumulation coefficients as limbs at 2^(62 − fx_ec),
-// each node's adding up to at most 2^fx_ec in size, 2g, √g, g/2 and the
-// exponents of g and h_min; false where g is outside their range
+// each node's adding up to at most 2^fx_ec in size, 2g, √g, g/2 and g's
+// exponent; false where g is outside their range
 inline bool fixed_constants(const PairSchedule& sched, const Physics& P, DevTables& T,
                             std::vector<FxLimb>& coef) {
     const size_t na = 2 * ((size_t)sched.n1 - 1);
@@ -290,8 +306,6 @@ inline bool fixed_constants(const PairSchedule& sched, const Physics& P, DevTabl
     c.sqrt_g = constant(P.sqrt_g, c.e_sqrt_g);
     c.half_g = constant(P.half_g, c.e_half_g);
     std::frexp(P.g, &c.e_g);
-    std::frexp(P.h_min, &c.e_h_min);
-    if (P.h_min == 0.0) c.e_h_min = -1100;
     return T.fx_e2g >= -60 && T.fx_e2g <= 60;
 }
 

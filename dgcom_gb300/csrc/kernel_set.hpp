@@ -88,6 +88,8 @@ struct KernelSet {
     void (*fixed_tables)(int n1, const DevTables&, FxPair* hm, FxPair* gdb, FxLimb* lift,
                          FxExp* exps, FxPair* normal, cudaStream_t);
     bool has_fixed;
+    // the subcell interfaces' metrics (DevTables::sub_metric)
+    void (*sub_metrics)(int n1, const DevTables&, const Physics&, double* out, cudaStream_t);
 };
 
 // kernels_fast.cu: FMA contraction, division-free Manning rate

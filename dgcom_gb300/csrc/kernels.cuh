@@ -84,6 +84,34 @@ __device__ __forceinline__
     return f;
 }
 
+#if DGSWE_FAST
+__device__ __noinline__ FacePair face_dry(Sd qa, Sd qb, const double* geo, double g, double half_g,
+                                          double h_min) {
+    FacePair f;
+    hydro_dry(qa, qb, geo[0], geo[1], geo[3], geo[4], g, half_g, h_min, f.a, f.b);
+    return f;
+}
+
+// The flux of two sides along m = norm·(nx, ny): in fixed point, or the rest
+// (nf, mf: the two vectors as limbs, mf at 2^(61 − em); UNIT: both the unit
+// normal)
+template <bool UNIT>
+__device__ __forceinline__ FacePair face_pair(const DevTables& T, const Sd& qa, const Sd& qb,
+                                              const FxPair& nf, const FxPair& mf, int em,
+                                              const double* geo, double g, double sqrt_g,
+                                              double half_g, double h_min) {
+    fx::FaceFlux f;
+    const fx::FaceCase got = T.fx_normal ? fx::face_flux(qa, qb, nf, mf, em, T.fx_face, h_min, f)
+                                         : fx::kNoScale;
+    if (got == fx::kDone) {
+        const double h = UNIT ? f.h : geo[2] * f.h;
+        return {{h, f.hu_a, f.hv_a}, {h, f.hu_b, f.hv_b}};
+    }
+    if (got == fx::kBothDry) return face_dry(qa, qb, geo, g, half_g, h_min);
+    return face_hll(qa, qb, geo, g, sqrt_g, half_g, h_min);
+}
+#endif
+
 // An element's stage in a multirate pass (element_stage,
 // src/time/multirate.rs:169-200), every operation rounded on its own as the
 // reference's are (no contraction): its substep's start time and step, the
@@ -265,7 +293,7 @@ __device__ __forceinline__ double weather_level(const DevTables& T, const Physic
 // LISTED: a multirate pass's faces (lp's edge and boundary-face lists),
 // each boundary face at its element's stage time
 template <int N1, bool LISTED>
-__global__ void __launch_bounds__(256) face_kernel(DevTables T, Physics P, DevBuf in, double* fb_h,
+__global__ void __launch_bounds__(256, DGSWE_FAST ? 3 : 2) face_kernel(DevTables T, Physics P, DevBuf in, double* fb_h,
                                                    double* fb_hu, double* fb_hv,
                                                    const StepCtl* ctl, int slot,
                                                    const int* active, LtsPass lp) {
@@ -287,21 +315,16 @@ __global__ void __launch_bounds__(256) face_kernel(DevTables T, Physics P, DevBu
         F3 fa, fbb;
         if (P.formulation == kWetDry) {
             const Sd ql = load_side(in, T, P, gl), qr = load_side(in, T, P, gr);
-            bool done = false;
+            const double* geo = &T.edge_geo[e * 5];
 #if DGSWE_FAST
-            fx::FaceFlux f;
-            if (T.fx_normal) done = fx::face_flux(ql, qr, T.fx_normal[e], T.fx_face, f);
-            if (done) {
-                fa = {f.h, f.hu_a, f.hv_a};
-                fbb = {-f.h, -f.hu_b, -f.hv_b};
-            }
+            const FxPair n = T.fx_normal ? T.fx_normal[e] : FxPair{};
+            const FacePair f =
+                face_pair<true>(T, ql, qr, n, n, 0, geo, g, sqrt_g, half_g, h_min);
+#else
+            const FacePair f = face_hll(ql, qr, geo, g, sqrt_g, half_g, h_min);
 #endif
-            if (!done) {
-                const FacePair f =
-                    face_hll(ql, qr, &T.edge_geo[e * 5], g, sqrt_g, half_g, h_min);
-                fa = f.a;
-                fbb = {-f.b.h, -f.b.hu, -f.b.hv};
-            }
+            fa = f.a;
+            fbb = {fp::neg(f.b.h), fp::neg(f.b.hu), fp::neg(f.b.hv)};
         } else {
             const double* geo = &T.edge_geo[e * 5];
             entropy_surface(load_q(in, T, P, gl), load_q(in, T, P, gr), geo[0], geo[1], P, fa,
@@ -369,7 +392,7 @@ __global__ void __launch_bounds__(256) face_kernel(DevTables T, Physics P, DevBu
                 ut_e = -ue * ny + ve * nx;
             } else {
                 if (c.elevation_only == kIncomingWave)
-                    un_e = 2.0 * (sqrt(g * fmax(-qi.b, 0.0)) - sqrt(g * h_e));
+                    un_e = 2.0 * (vsqrt(g * fmax(-qi.b, 0.0)) - vsqrt(g * h_e));
                 ut_e = -u * ny + v * nx;
             }
             qb = characteristic_state_ext(qi, h_e, un_e, ut_e, nx, ny, g, h_min);
@@ -391,8 +414,8 @@ __global__ void __launch_bounds__(256) face_kernel(DevTables T, Physics P, DevBu
 
 // SHAPE 0: ⌊128/NN⌋ elements a block; SHAPE 1: ⌊64/NN⌋ elements a block
 // at twice the blocks per SM (the same registers and warps per SM); SHAPE 2:
-// ⌊128/NN⌋ elements a block at 6 blocks per SM (80 registers at N1 = 4,
-// with a few spilled). The launch shapes dgswe_autotune chooses between.
+// ⌊128/NN⌋ elements a block at 6 blocks per SM. The launch shapes
+// dgswe_autotune chooses between.
 template <int N1, int SHAPE = 0>
 struct Cfg {
     static constexpr int NN = N1 * N1;
@@ -401,17 +424,50 @@ struct Cfg {
     static constexpr int PER = SHAPE == 1 ? 64 : 128;
     static constexpr int EPB = (PER / NN) > 0 ? (PER / NN) : 1;
     static constexpr int THREADS = EPB * NN;
-    // stage_kernel blocks per SM: 5 caps it at ≤ 102 registers (96 at
-    // N1 = 4, no spills) for 20 warps per SM; it is bound by the FP64 pipe
-    // and waits on it, so more warps keep it busier (measured 5 % faster
-    // on the 1 M-quad N = 3 case than 4 blocks)
-    static constexpr int MIN_BLOCKS = SHAPE == 0 ? 5 : (SHAPE == 1 ? 10 : 6);
+    // stage_kernel blocks per SM. In fixed point the integer and FP64 pipes
+    // are each under half busy and the rest is latency: 28 warps an SM (72
+    // registers) against 20 (96) take the 200,000-quad N = 3 right-hand side
+    // from 0.226 to 0.210 ms, N = 4 at 100,000 from 0.354 to 0.310. The exact
+    // numerics wait on the FP64 pipe: 20 warps (≤ 102 registers, no spills)
+    // were 5 % faster than 16.
+    static constexpr int MIN_BLOCKS =
+        SHAPE == 2 ? 6 : (DGSWE_FAST ? 7 : 5) * (SHAPE == 1 ? 2 : 1);
     static constexpr int PAIR_DOUBLES = NN * NP * 3;
     static constexpr int FACE_DOUBLES = 2 * NN * 8;           // reconstructed faces
     static constexpr int NSUB = 2 * N1 * (N1 - 1);            // subcell interfaces
     static constexpr int IFL_DOUBLES = NSUB * 6;               // their fluxes
-    static constexpr int X = PAIR_DOUBLES > FACE_DOUBLES + IFL_DOUBLES ? PAIR_DOUBLES
-                                                                       : FACE_DOUBLES + IFL_DOUBLES;
+    // An element's scratch in FP64: its nodes' six values, and behind them the
+    // pair fluxes or the subcells' reconstructed faces. The interface fluxes
+    // come when the nodes' values are done with and lie over them.
+    static constexpr int NODES = 6 * NN;
+    static constexpr int AFTER = NODES > IFL_DOUBLES ? NODES : IFL_DOUBLES;
+    static constexpr int X =
+        AFTER + (PAIR_DOUBLES > FACE_DOUBLES ? PAIR_DOUBLES : FACE_DOUBLES);
+    // In fixed point: the pair fluxes, the nodes' numbers, the lifted fluxes
+    static constexpr int XF = PAIR_DOUBLES + 5 * NN + 12 * N1;
+};
+
+// LANES lanes work on an element; where that is a power of two they share a
+// warp, and the element's exchanges through shared memory order that warp alone
+template <int LANES>
+constexpr bool kElementInWarp = LANES <= 32 && (LANES & (LANES - 1)) == 0;
+
+template <int LANES>
+__device__ __forceinline__ void element_sync() {
+    if (kElementInWarp<LANES>) __syncwarp();
+    else __syncthreads();
+}
+
+// Asks for the line at p to be in the L2 cache by the time it is read
+__device__ __forceinline__ void prefetch(const void* p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+// general_kernel: two lanes a node
+template <int N1>
+struct GenCfg {
+    static constexpr int EPB = 128 / (2 * N1 * N1) > 0 ? 128 / (2 * N1 * N1) : 1;
+    static constexpr int THREADS = EPB * 2 * N1 * N1;
 };
 
 __device__ __forceinline__ int line_node(int n1, int dir, int line, int pos) {
@@ -461,35 +517,340 @@ __device__ __forceinline__ void line_metric(const DevTables& T, int64_t k, int d
     }
 }
 
-#if DGSWE_FAST
-// A node's exponent fields (a negative depth's sign with it, which no scale
-// takes), two a word: depth and 4095 − depth, momentum and velocity, the mass
-// and momentum fluxes of its face slots. Their maxima over an element give
-// the element's fx::Exps.
-struct ExpWords {
-    unsigned w[3];
-};
-
 __device__ __forceinline__ int max_expo(double x, double y) {
     return max(fx::expo(x), fx::expo(y));
 }
 
-__device__ __forceinline__ ExpWords node_exponents(double h, double hu, double hv, double u,
-                                                   double v, int64_t s_a, int64_t s_b,
-                                                   const double* fb_h, const double* fb_hu,
-                                                   const double* fb_hv) {
-    int fh = 0, fm = 0;
+// The subcell interfaces' metrics of every element, [K][2·N1·(N1−1)][2] in
+// the order of the subcell mass fluxes: what `telescoped` sums (72 FP64
+// operations a direction at N = 3, twice per node of a subcell element)
+template <int N1>
+__global__ void __launch_bounds__(256) sub_metric_kernel(DevTables T, Physics P, double* out) {
+    constexpr int NSUB = 2 * N1 * (N1 - 1);
+    const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (item >= T.K * 2 * N1) return;
+    const int64_t k = item / (2 * N1);
+    const int dir = (int)(item % (2 * N1)) / N1, line = (int)(item % N1);
+    double m0[N1], m1[N1], i0[N1 + 1], i1[N1 + 1];
+    line_metric<N1>(T, k, dir, line, m0, m1);
+    telescoped<N1>(P, m0, m1, T.affine[k] != 0, i0, i1);
+    double* o = &out[(k * NSUB + (dir * N1 + line) * (N1 - 1)) * 2];
+#pragma unroll
+    for (int pos = 0; pos + 1 < N1; ++pos) {
+        o[2 * pos] = i0[pos + 1];
+        o[2 * pos + 1] = i1[pos + 1];
+    }
+}
+
+// The two slots of an element's face fluxes that a node takes, in the
+// reference's face order, −1: none. A node lies on at most one s-face (0 or
+// 2) and one r-face (1 or 3).
+template <int N1>
+__device__ __forceinline__ void node_slots(int a, int j, int& s_a, int& s_b) {
+    int f_a = j == 0 ? 0 : (j == N1 - 1 ? 2 : -1);
+    int f_b = a == N1 - 1 ? 1 : (a == 0 ? 3 : -1);
+    if (f_a == 2 && f_b == 1) {
+        f_a = 1;
+        f_b = 2;
+    }
+    auto slot = [&](int f) {
+        return f * N1 + (f == 0 ? a : (f == 1 ? j : (f == 2 ? N1 - 1 - a : N1 - 1 - j)));
+    };
+    s_a = f_a >= 0 ? slot(f_a) : -1;
+    s_b = f_b >= 0 ? slot(f_b) : -1;
+}
+
+// −LIFT·sJ·F* of the node's faces added to its volume term r, over J. Every
+// lane takes two slots, a missing one as zero, so the warp's instructions run
+// on all lanes instead of once per face with only that face's nodes active.
+// Subtracting +0 is exact.
+template <int N1>
+__device__ __forceinline__ F3 lift_only(const DevTables& T, const double* fb_h,
+                                        const double* fb_hu, const double* fb_hv, int64_t k, int i,
+                                        F3 r) {
+    double c_a = 0.0, h_a = 0.0, hu_a = 0.0, hv_a = 0.0;
+    double c_b = 0.0, h_b = 0.0, hu_b = 0.0, hv_b = 0.0;
+    const int64_t fbase = k * 4 * N1;
+    int s_a, s_b;
+    node_slots<N1>(i % N1, i / N1, s_a, s_b);
     if (s_a >= 0) {
-        fh = fx::expo(fb_h[s_a]);
-        fm = max_expo(fb_hu[s_a], fb_hv[s_a]);
+        c_a = T.lift_scale[fbase + s_a];
+        h_a = fb_h[fbase + s_a];
+        hu_a = fb_hu[fbase + s_a];
+        hv_a = fb_hv[fbase + s_a];
     }
     if (s_b >= 0) {
-        fh = max(fh, fx::expo(fb_h[s_b]));
-        fm = max(fm, max_expo(fb_hu[s_b], fb_hv[s_b]));
+        c_b = T.lift_scale[fbase + s_b];
+        h_b = fb_h[fbase + s_b];
+        hu_b = fb_hu[fbase + s_b];
+        hv_b = fb_hv[fbase + s_b];
     }
+    r.h -= c_a * h_a;
+    r.hu -= c_a * hu_a;
+    r.hv -= c_a * hv_a;
+    r.h -= c_b * h_b;
+    r.hu -= c_b * hu_b;
+    r.hv -= c_b * hv_b;
+    const double jinv = T.jinv[k * N1 * N1 + i];
+    return {jinv * r.h, jinv * r.hu, jinv * r.hv};
+}
+
+// A node's right-hand side by the FP64 formulas, before the sources: an
+// element with subcells (sub; dry: without water at any node), or a wet one.
+// s_x is the element's scratch and holds its nodes' h, hu, hv, u, v and bed.
+// SPLIT 2: two lanes a node (`half` 0 and 1), a direction of the subcells
+// each; the result is the first's. Every lane of the element, or of the block
+// where elements cross warps, calls it (take: the element takes part).
+template <int N1, int SPLIT>
+__device__ __forceinline__ F3 general_rhs(const DevTables& T, const Physics& P,
+                                          const StageExtra& X, const DevBuf& in,
+                                          const double* fb_h, const double* fb_hu,
+                                          const double* fb_hv, int64_t k, int i, int half,
+                                          bool take, bool sub, bool dry, double* s_x) {
+    using C = Cfg<N1>;
+    constexpr int NN = C::NN, NP = C::NP, NA = C::NA, LANES = SPLIT * NN;
+    double(*const s_q)[NN] = (double(*)[NN])s_x;
+    double* const pairs = s_x + C::AFTER;
+    const bool wet = take && !sub && half == 0;
+    const int a = i % N1, j = i / N1;
+    const int64_t gi = k * NN + i;
+    const double g = P.g, h_min = P.h_min, sqrt_g = P.sqrt_g, half_g = P.half_g;
+    double h = 0.0, b = 0.0;
+    if (take) {
+        h = s_q[0][i];
+        b = s_q[5][i];
+    }
+    double rh = 0.0, rhu = 0.0, rhv = 0.0;
+    const bool affine = take ? T.affine[k] != 0 : true;
+
+    auto node_side = [&](int n) { return Sd{s_q[0][n], s_q[3][n], s_q[4][n], s_q[5][n]}; };
+    double* const faces = s_x + C::AFTER;  // [dir][line][pos][8]
+    double* const ifl = s_x;               // [dir][line][pos][6]
+
+    // ---- phase A: pair fluxes, or the subcells' reconstructed faces ----
+    if (wet) {
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const int8_t* own = &T.sched_owned[(i * NP + q) * 5];
+            const int na = own[0], nc = own[1];
+            const double hm0 = T.pair_hm[(gi * NP + q) * 2];
+            const double hm1 = T.pair_hm[(gi * NP + q) * 2 + 1];
+            const double hc = s_q[0][nc];
+            // ½·F#(q_a, q_c)·{{Ja}} scaled: mass, 2·F_hu, 2·F_hv
+            const double mass = (s_q[1][na] + s_q[1][nc]) * hm0 +
+                                (s_q[2][na] + s_q[2][nc]) * hm1;
+            const double gp2 = P.two_g * s_q[0][na] * hc;
+            const double g_hu = mass * (s_q[3][na] + s_q[3][nc]) + gp2 * hm0;
+            const double g_hv = mass * (s_q[4][na] + s_q[4][nc]) + gp2 * hm1;
+            double* slot_f = &pairs[(i * NP + q) * 3];
+            slot_f[0] = mass;
+            slot_f[1] = g_hu;
+            slot_f[2] = g_hv;
+        }
+    } else if (take && sub && !dry) {
+        // subcell faces of this node's subcell on its r-line and s-line
+#pragma unroll 1
+        for (int dir = half; dir < 2; dir += SPLIT) {
+            const int line = dir == 0 ? j : a;
+            const int pos = dir == 0 ? a : j;
+            const Sd q = node_side(i);
+            Sd l{}, r{};
+            double x_l = 0.0, x_r = 0.0;
+            bool have_l = true, have_r = true;
+            if (pos > 0) {
+                l = node_side(line_node(N1, dir, line, pos - 1));
+                x_l = P.x[pos - 1];
+            } else {
+                // r-lines end on faces 3 (reversed) and 1; s-lines on 0 and 2 (reversed)
+                const int face = dir == 0 ? 3 : 0;
+                const int fi = dir == 0 ? N1 - 1 - line : line;
+                const int64_t o = (k * 4 + face) * N1 + fi;
+                const int64_t og = T.outer_idx[o];
+                have_l = og >= 0;
+                if (have_l) {
+                    l = Sd{in.h[og], in.u[og], in.v[og], P.has_bed ? T.bed[og] : 0.0};
+                    x_l = -1.0 - T.outer_dist[o];
+                }
+            }
+            if (pos + 1 < N1) {
+                r = node_side(line_node(N1, dir, line, pos + 1));
+                x_r = P.x[pos + 1];
+            } else {
+                const int face = dir == 0 ? 1 : 2;
+                const int fi = dir == 0 ? line : N1 - 1 - line;
+                const int64_t o = (k * 4 + face) * N1 + fi;
+                const int64_t og = T.outer_idx[o];
+                have_r = og >= 0;
+                if (have_r) {
+                    r = Sd{in.h[og], in.u[og], in.v[og], P.has_bed ? T.bed[og] : 0.0};
+                    x_r = 1.0 + T.outer_dist[o];
+                }
+            }
+            Sd fl = q, fr = q;
+            if (have_l && have_r)
+                reconstruct(l, q, r, x_l, P.x[pos], x_r, X.xl[pos], X.xr[pos], P.subcell_h_dry,
+                            fl, fr);
+            double* f = &faces[((dir * N1 + line) * N1 + pos) * 8];
+            f[0] = fl.h;
+            f[1] = fl.u;
+            f[2] = fl.v;
+            f[3] = fl.b;
+            f[4] = fr.h;
+            f[5] = fr.u;
+            f[6] = fr.v;
+            f[7] = fr.b;
+        }
+    }
+    element_sync<LANES>();
+
+    // ---- phase B: sum the pairs; or the subcell interface fluxes ----
+    if (wet) {
+#pragma unroll
+        for (int q = 0; q < NA; ++q) {
+            const int slot_id = T.sched_slot[i * NA + q];
+            const double coef = T.sched_coef[i * NA + q];
+            const double hcoef = T.sched_hcoef[i * NA + q];  // coef / 2
+            const double* f = &pairs[slot_id * 3];
+            rh -= coef * f[0];
+            rhu -= hcoef * f[1];
+            rhv -= hcoef * f[2];
+        }
+        if (P.has_bed) {
+            rhu -= h * T.gdb[gi * 2];
+            rhv -= h * T.gdb[gi * 2 + 1];
+        }
+    } else if (take && dry) {
+        if (X.subcell_mass)  // the dry element's interface fluxes are ±0
+            for (int q = i + half * NN; q < C::NSUB; q += LANES)
+                X.subcell_mass[k * C::NSUB + q] = 0.0;
+    } else if (take && sub && !dry) {
+#pragma unroll 1
+        for (int dir = half; dir < 2; dir += SPLIT) {
+            const int line = dir == 0 ? j : a;
+            const int pos = dir == 0 ? a : j;
+            if (pos + 1 >= N1) continue;
+            const int64_t at = k * C::NSUB + (dir * N1 + line) * (N1 - 1) + pos;
+            const double mx = T.sub_metric[2 * at], my = T.sub_metric[2 * at + 1];
+            const double norm = vsqrt(mx * mx + my * my);
+            const double inv = vrcp(norm);
+            const double geo[5] = {mx, my, norm, mx * inv, my * inv};
+            const double* fa_ = &faces[((dir * N1 + line) * N1 + pos) * 8 + 4];   // right face of pos
+            const double* fb_ = &faces[((dir * N1 + line) * N1 + pos + 1) * 8];   // left face of pos+1
+            const Sd qa{fa_[0], fa_[1], fa_[2], fa_[3]}, qb{fb_[0], fb_[1], fb_[2], fb_[3]};
+#if DGSWE_FAST
+            auto pair = [](double x, double y, int K) {
+                return FxPair{fx::split(fx::to_fixed(x, K)), fx::split(fx::to_fixed(y, K))};
+            };
+            const int em = max_expo(mx, my);
+            const FacePair f =
+                face_pair<false>(T, qa, qb, pair(geo[3], geo[4], 1024), pair(mx, my, em + 2),
+                                 em - 1022, geo, g, sqrt_g, half_g, h_min);
+#else
+            const FacePair f = face_hll(qa, qb, geo, g, sqrt_g, half_g, h_min);
+#endif
+            const F3 fa = f.a, fb = f.b;
+            double* o = &ifl[((dir * N1 + line) * (N1 - 1) + pos) * 6];
+            if (X.subcell_mass)  // subcell_slot (src/solver/rhs/subcells.rs:37-42)
+                X.subcell_mass[at] = fa.h;
+            o[0] = fa.h;
+            o[1] = fa.hu;
+            o[2] = fa.hv;
+            o[3] = fb.h;
+            o[4] = fb.hu;
+            o[5] = fb.hv;
+        }
+    }
+    element_sync<LANES>();
+
+    // ---- phase C: the subcells' fluxes and bed terms at this node ----
+    if (take && sub && !dry) {
+#pragma unroll 1
+        for (int dir = half; dir < 2; dir += SPLIT) {
+            const int line = dir == 0 ? j : a;
+            const int pos = dir == 0 ? a : j;
+            const double iw = X.inv_w[pos];
+            if (pos + 1 < N1) {
+                const double* o = &ifl[((dir * N1 + line) * (N1 - 1) + pos) * 6];
+                rh -= iw * o[0];
+                rhu -= iw * o[1];
+                rhv -= iw * o[2];
+            }
+            if (pos > 0) {
+                const double* o = &ifl[((dir * N1 + line) * (N1 - 1) + pos - 1) * 6];
+                rh += iw * o[3];
+                rhu += iw * o[4];
+                rhv += iw * o[5];
+            }
+            const double* f = &faces[((dir * N1 + line) * N1 + pos) * 8];
+            const double lh = f[0], lb = f[3], rhh = f[4], rb = f[7];
+            const double w_a = P.w[pos];
+#if DGSWE_FAST
+            (void)w_a;
+            const double bed = -0.5 * g * (lh + rhh) * (rb - lb) * iw;  // iw = 1/w_a
+#else
+            const double bed = -0.5 * g * (lh + rhh) * (rb - lb) / w_a;
+#endif
+            double fx, fy;
+            // the metric at the subcell's two ends: of the interfaces, and of
+            // the line's end nodes
+            auto metric_at = [&](int at, int c) {
+                if (at > 0 && at < N1)
+                    return T.sub_metric[2 * (k * C::NSUB + (dir * N1 + line) * (N1 - 1) + at - 1) + c];
+                const int n = line_node(N1, dir, line, at == 0 ? 0 : N1 - 1);
+                return T.contra[(k * NN + n) * 4 + 2 * dir + c];
+            };
+            if (affine) {
+                fx = bed * metric_at(0, 0);
+                fy = bed * metric_at(0, 1);
+            } else {
+                const double ml0 = metric_at(pos, 0), ml1 = metric_at(pos, 1);
+                const double mr0 = metric_at(pos + 1, 0), mr1 = metric_at(pos + 1, 1);
+                const double metric =
+#if DGSWE_FAST
+                    0.25 * g * ((rhh + h) * (b - rb) + (lh + h) * (b - lb)) * iw;
+#else
+                    0.25 * g * ((rhh + h) * (b - rb) + (lh + h) * (b - lb)) / w_a;
+#endif
+                fx = bed * 0.5 * (ml0 + mr0) + metric * (mr0 - ml0);
+                fy = bed * 0.5 * (ml1 + mr1) + metric * (mr1 - ml1);
+            }
+            rhu += fx;
+            rhv += fy;
+        }
+    }
+
+    if (SPLIT == 2) {  // the second direction's sums to the node's first lane
+        element_sync<LANES>();  // the faces are done with
+        if (half == 1) {
+            faces[3 * i] = rh;
+            faces[3 * i + 1] = rhu;
+            faces[3 * i + 2] = rhv;
+        }
+        element_sync<LANES>();
+        if (half == 0 && !wet) {
+            rh += faces[3 * i];
+            rhu += faces[3 * i + 1];
+            rhv += faces[3 * i + 2];
+        }
+    }
+
+    if (!take || half != 0) return {0.0, 0.0, 0.0};
+    return lift_only<N1>(T, fb_h, fb_hu, fb_hv, k, i, F3{rh, rhu, rhv});
+}
+
+#if DGSWE_FAST
+// Exponent fields (a negative depth's sign with it, which no scale takes),
+// two a word: depth and 4095 − depth, momentum and velocity, the mass and
+// momentum of face fluxes. Their maxima over an element's nodes and face
+// slots give the element's fx::Exps.
+struct ExpWords {
+    unsigned w[3];
+};
+
+__device__ __forceinline__ ExpWords node_exponents(double h, double hu, double hv, double u,
+                                                   double v) {
     const unsigned hb = (unsigned)((uint64_t)fp::bits(h) >> 52);
-    return {{hb | (4095u - hb) << 16, (unsigned)(max_expo(hu, hv) | max_expo(u, v) << 16),
-             (unsigned)(fh | fm << 16)}};
+    return {{hb | (4095u - hb) << 16, (unsigned)(max_expo(hu, hv) | max_expo(u, v) << 16), 0u}};
 }
 
 // The maxima over each NN lanes of a warp
@@ -549,430 +910,33 @@ __global__ void __launch_bounds__(256) fixed_tables_kernel(DevTables T, FxPair* 
 }
 #endif
 
-// LISTED: a multirate pass over lp's elements, each with its own stage
-template <int N1, bool LISTED, int SHAPE = 0>
-__global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_BLOCKS)
-    stage_kernel(DevTables T, Physics P, StageExtra X, DevBuf in, DevBuf base, DevBuf out,
-                 DevBuf acc, const double* __restrict__ fb_h, const double* __restrict__ fb_hu,
-                 const double* __restrict__ fb_hv, StepCtl* ctl, int slot, int mode,
-                 int check_finite, const int* active, DevBuf keep, LtsPass lp) {
-    using C = Cfg<N1, SHAPE>;
-    constexpr int NN = C::NN, NP = C::NP, NA = C::NA, EPB = C::EPB;
-    __shared__ double s_q[EPB][6][NN];  // h, hu, hv, u, v, b
-    __shared__ double s_x[EPB][C::X];
-    __shared__ int s_flag[EPB][3];
-    __shared__ double s_red[EPB][5];
-    // an element whose lanes share a warp finds its flags and largest
-    // exponents by votes and shuffles, else in shared memory
-    constexpr bool kInWarp = (NN & (NN - 1)) == 0;
-#if DGSWE_FAST
-    __shared__ unsigned s_exp[kInWarp ? 1 : EPB][6];
-#endif
-
-    if (!*active) return;
+// A node's stage from its right-hand side F: the sources, the combination,
+// the damping, then the accumulation or the wet/dry correction and the
+// output. LANES lanes an element, of which the first NN hold its nodes
+// (valid); s_q is scratch of the element's, s_flag and s_red its own.
+template <int N1, bool LISTED, int LANES>
+__device__ __forceinline__ void finish_node(const DevTables& T, const Physics& P,
+                                            const DevBuf& in, const DevBuf& base,
+                                            const DevBuf& out, const DevBuf& acc,
+                                            const DevBuf& keep, StepCtl* cm, const LtsPass& lp,
+                                            int slot, int mode, int check_finite, int64_t k, int i,
+                                            bool valid, const F3& F, double (*s_q)[N1 * N1],
+                                            int* s_flag, double* s_red) {
+    constexpr int NN = N1 * N1;
     const int tid = threadIdx.x;
-    const int e = tid / NN, i = tid % NN;
-    int64_t k = (int64_t)blockIdx.x * EPB + e;
-    if (LISTED) k = k < lp.n ? (int64_t)lp.list[k] : T.K;
-    else k += X.k_first;
-    const int64_t k_end = (LISTED || X.k_last > T.K) ? T.K : X.k_last;
-    // the element's member (its StepCtl); an ensemble member that has
-    // stopped keeps its state: its elements take no part
-    StepCtl* const cm = ctl + ((T.elem_member && k < k_end) ? T.elem_member[k] : 0);
-    const bool valid = k < k_end && (!T.elem_member || cm->active);
     const int64_t gi = k * NN + i;
-    const int a = i % N1, j = i / N1;
-    const double g = P.g, h_min = P.h_min, sqrt_g = P.sqrt_g, half_g = P.half_g;
-
-    double h = 0, hu = 0, hv = 0, u = 0, v = 0, b = 0;
+    const double h_min = P.h_min;
+    // read (again, from the cache: ten registers fewer until here)
+    double h = 0.0, hu = 0.0, hv = 0.0, u = 0.0, v = 0.0;
     if (valid) {
         h = in.h[gi];
         hu = in.hu[gi];
         hv = in.hv[gi];
         u = in.u[gi];
         v = in.v[gi];
-        b = P.has_bed ? T.bed[gi] : 0.0;
     }
-    // A node lies on at most one s-face (0 or 2) and one r-face (1 or 3):
-    // its slots of the face fluxes in the reference's face order, −1: none
-    int64_t s_a = -1, s_b = -1;
-    if (valid) {
-        int f_a = j == 0 ? 0 : (j == N1 - 1 ? 2 : -1);
-        int f_b = a == N1 - 1 ? 1 : (a == 0 ? 3 : -1);
-        if (f_a == 2 && f_b == 1) {
-            f_a = 1;
-            f_b = 2;
-        }
-        const int64_t fbase = k * 4 * N1;
-        auto slot = [&](int f) -> int64_t {
-            const int fi = f == 0 ? a : (f == 1 ? j : (f == 2 ? N1 - 1 - a : N1 - 1 - j));
-            return fbase + f * N1 + fi;
-        };
-        if (f_a >= 0) s_a = slot(f_a);
-        if (f_b >= 0) s_b = slot(f_b);
-    }
-    // sub: an element with a node below the subcell depth.
-    // dry: a subcell element without water at any node (every h = ±0, so
-    // every u = v = 0): its reconstructed subcell faces are dry, so the
-    // interface fluxes, pressure and bed terms are all ±0, and it skips the
-    // subcell phases (they read only h, u, v and the bed)
-    const bool shallow = valid && P.formulation == kWetDry && fp::lt(h, P.subcell_depth);
-    bool sub, dry;
-#if DGSWE_FAST
-    ExpWords ew = node_exponents(h, hu, hv, u, v, s_a, s_b, fb_h, fb_hu, fb_hv);
-#endif
-    if (kInWarp) {
-        const unsigned lanes = ((1ull << NN) - 1) << ((tid & 31) / NN * NN);
-        sub = (__ballot_sync(0xffffffffu, shallow) & lanes) != 0;
-        dry = (__ballot_sync(0xffffffffu, shallow && !fp::nz(h)) & lanes) == lanes;
-        if (i == 0) s_flag[e][1] = 0;
-#if DGSWE_FAST
-        warp_max<NN>(ew);
-#endif
-    } else {
-        if (i == 0) {
-            s_flag[e][0] = 0;
-            s_flag[e][1] = 0;
-            s_flag[e][2] = 0;
-        }
-#if DGSWE_FAST
-        if (i < 6) s_exp[e][i] = 0;
-#endif
-        __syncthreads();
-        if (shallow) {
-            atomicOr(&s_flag[e][0], 1);
-            if (!fp::nz(h)) atomicAdd(&s_flag[e][2], 1);
-        }
-#if DGSWE_FAST
-        for (int q = 0; q < 3; ++q) {
-            atomicMax(&s_exp[e][2 * q], ew.w[q] & 0xFFFFu);
-            atomicMax(&s_exp[e][2 * q + 1], ew.w[q] >> 16);
-        }
-#endif
-        __syncthreads();
-        sub = s_flag[e][0] != 0;
-        dry = s_flag[e][2] == NN;
-#if DGSWE_FAST
-        for (int q = 0; q < 3; ++q) ew.w[q] = s_exp[e][2 * q] | s_exp[e][2 * q + 1] << 16;
-#endif
-    }
-    // fixed: the wet element's sums in fixed point (fixed64.hpp); an element
-    // whose depths or exponents spread too far for it, and every element of
-    // the exact numerics, takes the FP64 phases
-    bool fixed = false;
-#if DGSWE_FAST
-    fx::Scale sc;
-    FxLimb G{};                                   // 2g·h
-    FxLimb H{};                                   // h
-    int64_t m0 = 0, m1 = 0, u0 = 0, u1 = 0;       // hu, hv, u, v
-    FxLimb* const nd_h = (FxLimb*)&s_x[e][C::PAIR_DOUBLES];
-    int64_t* const nd = (int64_t*)&s_x[e][C::PAIR_DOUBLES + NN];
-    FxLimb* const pairs = (FxLimb*)&s_x[e][0];
-    static_assert(C::PAIR_DOUBLES + 5 * NN <= C::X, "the nodes' numbers fit behind the pairs'");
-    if (valid && !sub) {
-        sc = fx::scales(exponents(ew), T.fx_exp[k], T.fx_ec, T.fx_e2g);
-        fixed = sc.ok;
-    }
-    if (fixed) {
-        H = fx::split(fx::to_fixed(h, sc.kh));
-        G = fx::two_g_h(H, T.fx_two_g, sc);
-        m0 = fx::to_fixed(hu, sc.km);
-        m1 = fx::to_fixed(hv, sc.km);
-        u0 = fx::to_fixed(u, sc.ku);
-        u1 = fx::to_fixed(v, sc.ku);
-        nd_h[i] = H;
-        nd[i] = m0;
-        nd[NN + i] = m1;
-        nd[2 * NN + i] = u0;
-        nd[3 * NN + i] = u1;
-    }
-#endif
-    if (!fixed) {
-        s_q[e][0][i] = h;
-        s_q[e][1][i] = hu;
-        s_q[e][2][i] = hv;
-        s_q[e][3][i] = u;
-        s_q[e][4][i] = v;
-        s_q[e][5][i] = b;
-    }
-    __syncthreads();
-    double rh = 0.0, rhu = 0.0, rhv = 0.0;
-    const bool affine = valid ? T.affine[k] != 0 : true;
-
-    auto node_side = [&](int n) {
-        return Sd{s_q[e][0][n], s_q[e][3][n], s_q[e][4][n], s_q[e][5][n]};
-    };
-    double* faces = &s_x[e][0];                      // [dir][line][pos][8]
-    double* ifl = &s_x[e][C::FACE_DOUBLES];          // [dir][line][pos][6]
-
-    // ---- phase A: pair fluxes, or the subcells' reconstructed faces ----
-    if (fixed) {
-#if DGSWE_FAST
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-            const int8_t* own = &T.sched_owned[(i * NP + q) * 5];
-            const int o = own[0] + own[1] - i;  // the pair's other node
-            const FxPair hm = T.fx_hm[gi * NP + q];
-            const fx::Flux f = fx::pair_flux(G, nd_h[o], m0 + nd[o], m1 + nd[NN + o],
-                                             u0 + nd[2 * NN + o], u1 + nd[3 * NN + o], hm.x, hm.y);
-            FxLimb* slot_f = &pairs[(i * NP + q) * 3];
-            slot_f[0] = f.h;
-            slot_f[1] = f.hu;
-            slot_f[2] = f.hv;
-        }
-#endif
-    } else if (valid && !sub) {
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-            const int8_t* own = &T.sched_owned[(i * NP + q) * 5];
-            const int na = own[0], nc = own[1];
-            const double hm0 = T.pair_hm[(gi * NP + q) * 2];
-            const double hm1 = T.pair_hm[(gi * NP + q) * 2 + 1];
-            const double hc = s_q[e][0][nc];
-            // ½·F#(q_a, q_c)·{{Ja}} scaled: mass, 2·F_hu, 2·F_hv
-            const double mass = (s_q[e][1][na] + s_q[e][1][nc]) * hm0 +
-                                (s_q[e][2][na] + s_q[e][2][nc]) * hm1;
-            const double gp2 = P.two_g * s_q[e][0][na] * hc;
-            const double g_hu = mass * (s_q[e][3][na] + s_q[e][3][nc]) + gp2 * hm0;
-            const double g_hv = mass * (s_q[e][4][na] + s_q[e][4][nc]) + gp2 * hm1;
-            double* slot_f = &s_x[e][(i * NP + q) * 3];
-            slot_f[0] = mass;
-            slot_f[1] = g_hu;
-            slot_f[2] = g_hv;
-        }
-    } else if (valid && sub && !dry) {
-        // subcell faces of this node's subcell on its r-line and s-line
-#pragma unroll
-        for (int dir = 0; dir < 2; ++dir) {
-            const int line = dir == 0 ? j : a;
-            const int pos = dir == 0 ? a : j;
-            const Sd q = node_side(i);
-            Sd l{}, r{};
-            double x_l = 0.0, x_r = 0.0;
-            bool have_l = true, have_r = true;
-            if (pos > 0) {
-                l = node_side(line_node(N1, dir, line, pos - 1));
-                x_l = P.x[pos - 1];
-            } else {
-                // r-lines end on faces 3 (reversed) and 1; s-lines on 0 and 2 (reversed)
-                const int face = dir == 0 ? 3 : 0;
-                const int fi = dir == 0 ? N1 - 1 - line : line;
-                const int64_t o = (k * 4 + face) * N1 + fi;
-                const int64_t og = T.outer_idx[o];
-                have_l = og >= 0;
-                if (have_l) {
-                    l = Sd{in.h[og], in.u[og], in.v[og], P.has_bed ? T.bed[og] : 0.0};
-                    x_l = -1.0 - T.outer_dist[o];
-                }
-            }
-            if (pos + 1 < N1) {
-                r = node_side(line_node(N1, dir, line, pos + 1));
-                x_r = P.x[pos + 1];
-            } else {
-                const int face = dir == 0 ? 1 : 2;
-                const int fi = dir == 0 ? line : N1 - 1 - line;
-                const int64_t o = (k * 4 + face) * N1 + fi;
-                const int64_t og = T.outer_idx[o];
-                have_r = og >= 0;
-                if (have_r) {
-                    r = Sd{in.h[og], in.u[og], in.v[og], P.has_bed ? T.bed[og] : 0.0};
-                    x_r = 1.0 + T.outer_dist[o];
-                }
-            }
-            Sd fl = q, fr = q;
-            if (have_l && have_r)
-                reconstruct(l, q, r, x_l, P.x[pos], x_r, X.xl[pos], X.xr[pos], P.subcell_h_dry,
-                            fl, fr);
-            double* f = &faces[((dir * N1 + line) * N1 + pos) * 8];
-            f[0] = fl.h;
-            f[1] = fl.u;
-            f[2] = fl.v;
-            f[3] = fl.b;
-            f[4] = fr.h;
-            f[5] = fr.u;
-            f[6] = fr.v;
-            f[7] = fr.b;
-        }
-    }
-    __syncthreads();
-
-    // ---- phase B: sum the pairs; or the subcell interface fluxes ----
-#if DGSWE_FAST
-    int64_t fh = 0, fhu = 0, fhv = 0;  // the sums in fixed point
-#endif
-    if (fixed) {
-#if DGSWE_FAST
-        fx::PairSum ah = fx::pair_sum(), au = ah, av = ah;
-#pragma unroll
-        for (int q = 0; q < NA; ++q) {
-            const FxLimb* f = &pairs[T.sched_slot[i * NA + q] * 3];
-            const FxLimb coef = T.fx_coef[i * NA + q];
-            fx::mac(ah, coef, f[0]);
-            fx::mac(au, coef, f[1]);
-            fx::mac(av, coef, f[2]);
-        }
-        fh = -fx::fold(ah);
-        fhu = -fx::fold(au);
-        fhv = -fx::fold(av);
-        if (P.has_bed) {
-            const FxPair slope = T.fx_gdb[gi];
-            fhu -= fx::bed_term(H, slope.x, sc);
-            fhv -= fx::bed_term(H, slope.y, sc);
-        }
-#endif
-    } else if (valid && !sub) {
-#pragma unroll
-        for (int q = 0; q < NA; ++q) {
-            const int slot_id = T.sched_slot[i * NA + q];
-            const double coef = T.sched_coef[i * NA + q];
-            const double hcoef = T.sched_hcoef[i * NA + q];  // coef / 2
-            const double* f = &s_x[e][slot_id * 3];
-            rh -= coef * f[0];
-            rhu -= hcoef * f[1];
-            rhv -= hcoef * f[2];
-        }
-        if (P.has_bed) {
-            rhu -= h * T.gdb[gi * 2];
-            rhv -= h * T.gdb[gi * 2 + 1];
-        }
-    }
-    if (valid && !sub) {
-        if (X.subcell_mass)  // no subcells: NaN (compute_rhs_swe_2d_mass_fluxes_into)
-            for (int q = i; q < C::NSUB; q += NN)
-                X.subcell_mass[k * C::NSUB + q] = fp::from_bits(0x7FF8000000000000ll);
-    } else if (valid && dry) {
-        if (X.subcell_mass)  // the dry element's interface fluxes are ±0
-            for (int q = i; q < C::NSUB; q += NN) X.subcell_mass[k * C::NSUB + q] = 0.0;
-    } else if (valid && sub && !dry) {
-#pragma unroll
-        for (int dir = 0; dir < 2; ++dir) {
-            const int line = dir == 0 ? j : a;
-            const int pos = dir == 0 ? a : j;
-            if (pos + 1 >= N1) continue;
-            double m0[N1], m1[N1], i0[N1 + 1], i1[N1 + 1];
-            line_metric<N1>(T, k, dir, line, m0, m1);
-            telescoped<N1>(P, m0, m1, affine, i0, i1);
-            const double mx = i0[pos + 1], my = i1[pos + 1];
-            const double norm = vsqrt(mx * mx + my * my);
-            const double inv = vrcp(norm);
-            const double* fa_ = &faces[((dir * N1 + line) * N1 + pos) * 8 + 4];   // right face of pos
-            const double* fb_ = &faces[((dir * N1 + line) * N1 + pos + 1) * 8];   // left face of pos+1
-            F3 fa, fb;
-            hydro_hll(Sd{fa_[0], fa_[1], fa_[2], fa_[3]}, Sd{fb_[0], fb_[1], fb_[2], fb_[3]}, mx, my,
-                      norm, mx * inv, my * inv, g, sqrt_g, half_g, h_min, fa, fb);
-            double* o = &ifl[((dir * N1 + line) * (N1 - 1) + pos) * 6];
-            if (X.subcell_mass)  // subcell_slot (src/solver/rhs/subcells.rs:37-42)
-                X.subcell_mass[k * C::NSUB + (dir * N1 + line) * (N1 - 1) + pos] = fa.h;
-            o[0] = fa.h;
-            o[1] = fa.hu;
-            o[2] = fa.hv;
-            o[3] = fb.h;
-            o[4] = fb.hu;
-            o[5] = fb.hv;
-        }
-    }
-    __syncthreads();
-
-    // ---- phase C: the subcells' fluxes and bed terms at this node ----
-    if (valid && sub && !dry) {
-#pragma unroll
-        for (int dir = 0; dir < 2; ++dir) {
-            const int line = dir == 0 ? j : a;
-            const int pos = dir == 0 ? a : j;
-            const double iw = X.inv_w[pos];
-            if (pos + 1 < N1) {
-                const double* o = &ifl[((dir * N1 + line) * (N1 - 1) + pos) * 6];
-                rh -= iw * o[0];
-                rhu -= iw * o[1];
-                rhv -= iw * o[2];
-            }
-            if (pos > 0) {
-                const double* o = &ifl[((dir * N1 + line) * (N1 - 1) + pos - 1) * 6];
-                rh += iw * o[3];
-                rhu += iw * o[4];
-                rhv += iw * o[5];
-            }
-            const double* f = &faces[((dir * N1 + line) * N1 + pos) * 8];
-            const double lh = f[0], lb = f[3], rhh = f[4], rb = f[7];
-            const double w_a = P.w[pos];
-#if DGSWE_FAST
-            (void)w_a;
-            const double bed = -0.5 * g * (lh + rhh) * (rb - lb) * iw;  // iw = 1/w_a
-#else
-            const double bed = -0.5 * g * (lh + rhh) * (rb - lb) / w_a;
-#endif
-            double m0[N1], m1[N1];
-            line_metric<N1>(T, k, dir, line, m0, m1);
-            double fx, fy;
-            if (affine) {
-                fx = bed * m0[0];
-                fy = bed * m1[0];
-            } else {
-                double i0[N1 + 1], i1[N1 + 1];
-                telescoped<N1>(P, m0, m1, false, i0, i1);
-                const double ml0 = i0[pos], ml1 = i1[pos], mr0 = i0[pos + 1], mr1 = i1[pos + 1];
-                const double metric =
-#if DGSWE_FAST
-                    0.25 * g * ((rhh + h) * (b - rb) + (lh + h) * (b - lb)) * iw;
-#else
-                    0.25 * g * ((rhh + h) * (b - rb) + (lh + h) * (b - lb)) / w_a;
-#endif
-                fx = bed * 0.5 * (ml0 + mr0) + metric * (mr0 - ml0);
-                fy = bed * 0.5 * (ml1 + mr1) + metric * (mr1 - ml1);
-            }
-            rhu += fx;
-            rhv += fy;
-        }
-    }
-
-    // ---- surface: −LIFT·sJ·F* of the node's faces, and 1/J ----
-    // Every lane takes two slots, a missing one as zero, so the warp's
-    // instructions run on all lanes instead of once per face with only that
-    // face's nodes active. Subtracting +0 is exact.
-    double Fh = 0.0, Fhu = 0.0, Fhv = 0.0;
-    if (valid) {
-        double h_a = 0.0, hu_a = 0.0, hv_a = 0.0, h_b = 0.0, hu_b = 0.0, hv_b = 0.0;
-        if (s_a >= 0) {
-            h_a = fb_h[s_a];
-            hu_a = fb_hu[s_a];
-            hv_a = fb_hv[s_a];
-        }
-        if (s_b >= 0) {
-            h_b = fb_h[s_b];
-            hu_b = fb_hu[s_b];
-            hv_b = fb_hv[s_b];
-        }
-        const double jinv = T.jinv[gi];
-        if (fixed) {
-#if DGSWE_FAST
-            const FxLimb c_a = s_a >= 0 ? T.fx_lift[s_a] : FxLimb{0, 0};
-            const FxLimb c_b = s_b >= 0 ? T.fx_lift[s_b] : FxLimb{0, 0};
-            auto lift = [&](double x, double y, int K) {
-                fx::Acc s{fx::half<0>(), 0};
-                fx::mac(s, c_a, fx::split(fx::to_fixed(x, K)));
-                fx::mac(s, c_b, fx::split(fx::to_fixed(y, K)));
-                return fx::fold<0>(s);
-            };
-            Fh = fx::over_jacobian(fh - lift(h_a, h_b, sc.kfh), sc.sh, jinv);
-            Fhu = fx::over_jacobian(fhu - lift(hu_a, hu_b, sc.kfm), sc.sm, jinv);
-            Fhv = fx::over_jacobian(fhv - lift(hv_a, hv_b, sc.kfm), sc.sm, jinv);
-#endif
-        } else {
-            const double c_a = s_a >= 0 ? T.lift_scale[s_a] : 0.0;
-            const double c_b = s_b >= 0 ? T.lift_scale[s_b] : 0.0;
-            rh -= c_a * h_a;
-            rhu -= c_a * hu_a;
-            rhv -= c_a * hv_a;
-            rh -= c_b * h_b;
-            rhu -= c_b * hu_b;
-            rhv -= c_b * hv_b;
-            Fh = jinv * rh;
-            Fhu = jinv * rhu;
-            Fhv = jinv * rhv;
-        }
-    }
-
     // ---- the sources ----
+    double Fh = F.h, Fhu = F.hu, Fhv = F.hv;
     if (valid) {
         if (P.has_coriolis) {
             const double f = P.coriolis_field ? T.fcor[gi] : P.f0;
@@ -997,7 +961,11 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
     const StageArgs sa = LISTED ? (valid ? lts_stage(lp, k) : StageArgs{}) : cm->stage[slot];
     double vh = 0.0, vhu = 0.0, vhv = 0.0;
     if (valid) {
-        if (fp::nz(sa.a)) {
+        if (fp::bits(sa.a) == 0x3FF0000000000000ll) {  // 1: no multiply
+            vh = base.h[gi];
+            vhu = base.hu[gi];
+            vhv = base.hv[gi];
+        } else if (fp::nz(sa.a)) {
             vh = sa.a * base.h[gi];
             vhu = sa.a * base.hu[gi];
             vhv = sa.a * base.hv[gi];
@@ -1049,49 +1017,60 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
 
     // ---- wet/dry correction (wetting_drying.rs:194-215) ----
     if (P.has_wet_dry) {
-        __syncthreads();  // s_q is free again
-        if (valid && fp::lt(vh, P.h_dry)) atomicOr(&s_flag[e][1], 1);
-        s_q[e][0][i] = vh;
-        s_q[e][1][i] = vhu;
-        s_q[e][2][i] = vhv;
-        __syncthreads();
-        const bool needs = s_flag[e][1] != 0;
-        if (valid && needs && i == 0) {
-            // element_mean and positivity_limit_element
-            // (src/solver/limiters/swe_2d.rs:135-203), in node order
-            const double* mass = &T.mass[k * NN];
-            double sh = 0.0, shu = 0.0, shv = 0.0, hmin = INFINITY;
-            for (int p = 0; p < NN; ++p) {
-                sh += mass[p] * s_q[e][0][p];
-                shu += mass[p] * s_q[e][1][p];
-                shv += mass[p] * s_q[e][2][p];
-                hmin = lmin(s_q[e][0][p], hmin);
-            }
-            const double inv_area = T.inv_area[k];
-            const double h_avg = sh * inv_area;
-            s_red[e][0] = h_avg;
-            s_red[e][1] = shu * inv_area;
-            s_red[e][2] = shv * inv_area;
-            double theta = 1.0;
-            if (fp::gt0(h_avg) && fp::lt0(hmin)) {
-                theta = h_avg / (h_avg - hmin);
-                theta = fp::lt0(theta) ? 0.0 : (fp::gt(theta, 1.0) ? 1.0 : theta);
-            }
-            s_red[e][3] = theta;
-            s_red[e][4] = hmin;
-            if (fp::lt0(h_avg)) atomicAdd((unsigned long long*)&cm->clips, 1ull);
+        const bool thin = valid && fp::lt(vh, P.h_dry);
+        bool needs, some;  // the element's, and some element's of the group
+        if (kElementInWarp<LANES>) {
+            const unsigned lanes = (unsigned)(((1ull << LANES) - 1) << ((tid & 31) / LANES * LANES));
+            const unsigned votes = __ballot_sync(0xffffffffu, thin);
+            needs = (votes & lanes) != 0;
+            some = votes != 0;
+            __syncwarp();  // the element's scratch is free again
+        } else {
+            if (i == 0 && valid) *s_flag = 0;
+            __syncthreads();
+            if (thin) atomicOr(&*s_flag, 1);
+            some = __syncthreads_or(thin) != 0;
+            needs = *s_flag != 0;
         }
-        __syncthreads();
+        if (some) {
+            if (valid) {
+                s_q[0][i] = vh;
+                s_q[1][i] = vhu;
+                s_q[2][i] = vhv;
+            }
+            element_sync<LANES>();
+        }
+        if (valid && needs && i < 4) {
+            // element_mean and positivity_limit_element
+            // (src/solver/limiters/swe_2d.rs:135-203), in node order: a lane
+            // for each mean, one for the smallest depth
+            if (i < 3) {
+                const double* mass = &T.mass[k * NN];
+                double sum = 0.0;
+#pragma unroll
+                for (int p = 0; p < NN; ++p) sum += mass[p] * s_q[i][p];
+                s_red[i] = sum * T.inv_area[k];
+                if (i == 0 && fp::lt0(s_red[0]))
+                    atomicAdd((unsigned long long*)&cm->clips, 1ull);
+            } else {
+                double hmin = INFINITY;
+                for (int p = 0; p < NN; ++p) hmin = lmin(s_q[0][p], hmin);
+                s_red[3] = hmin;
+            }
+        }
+        if (some) element_sync<LANES>();
         if (valid && needs) {
-            const double h_avg = s_red[e][0];
+            const double h_avg = s_red[0];
             if (fp::le0(h_avg)) {
                 vh = vhu = vhv = 0.0;
             } else {
-                if (fp::lt0(s_red[e][4])) {
-                    const double th = s_red[e][3];
+                const double hmin = s_red[3];
+                if (fp::lt0(hmin)) {
+                    double th = vdiv(h_avg, h_avg - hmin);
+                    th = fp::lt0(th) ? 0.0 : (fp::gt(th, 1.0) ? 1.0 : th);
                     vh = th * (vh - h_avg) + h_avg;
-                    vhu = th * (vhu - s_red[e][1]) + s_red[e][1];
-                    vhv = th * (vhv - s_red[e][2]) + s_red[e][2];
+                    vhu = th * (vhu - s_red[1]) + s_red[1];
+                    vhv = th * (vhv - s_red[2]) + s_red[2];
                     vh = fp::max0(vh);
                 }
                 if (fp::lt(h_avg, P.h_dry)) vhu = vhv = 0.0;
@@ -1112,6 +1091,326 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
     }
 }
 
+#if DGSWE_FAST
+// The wet elements of a stage in fixed point, and those without water at any
+// node, which only their faces' fluxes reach (their reconstructed subcell
+// faces are dry, so the interface fluxes, pressure and bed terms are all ±0).
+// Any other with subcells, and one whose depths or exponents spread too far,
+// goes into T.gen_list for general_kernel, launched behind: inside this kernel its few hundred FP64
+// operations in a row (a call, so spills on the wet path; one busy warp to a
+// block's end) cost 17 % of a 50,000-quad coastal box's stage.
+// LISTED: a multirate pass over lp's elements, each with its own stage
+template <int N1, bool LISTED, int SHAPE = 0>
+__global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_BLOCKS)
+    stage_kernel(DevTables T, Physics P, StageExtra X, DevBuf in, DevBuf base, DevBuf out,
+                 DevBuf acc, const double* __restrict__ fb_h, const double* __restrict__ fb_hu,
+                 const double* __restrict__ fb_hv, StepCtl* ctl, int slot, int mode,
+                 int check_finite, const int* active, DevBuf keep, LtsPass lp) {
+    using C = Cfg<N1, SHAPE>;
+    constexpr int NN = C::NN, NP = C::NP, NA = C::NA, EPB = C::EPB;
+    // an element whose lanes share a warp finds its flags and largest
+    // exponents by votes and shuffles, else in shared memory
+    constexpr bool kInWarp = kElementInWarp<NN>;
+    __shared__ double s_x[EPB][C::XF];
+    __shared__ int s_flag[EPB][3];
+    __shared__ double s_red[EPB][4];
+    __shared__ unsigned s_exp[kInWarp ? 1 : EPB][6];
+
+    const int run = *active;
+    const int tid = threadIdx.x;
+    const int e = tid / NN, i = tid % NN;
+    int64_t k = (int64_t)blockIdx.x * EPB + e;
+    if (LISTED) k = k < lp.n ? (int64_t)lp.list[k] : T.K;
+    else k += X.k_first;
+    const int64_t k_end = (LISTED || X.k_last > T.K) ? T.K : X.k_last;
+    // the element's member (its StepCtl); an ensemble member that has
+    // stopped keeps its state: its elements take no part
+    StepCtl* const cm = ctl + ((T.elem_member && k < k_end) ? T.elem_member[k] : 0);
+    const bool valid = k < k_end && (!T.elem_member || cm->active);
+    const int64_t gi = k * NN + i;
+    const int64_t fbase = k * 4 * N1;  // the element's face slots
+    double(*const s_q)[NN] = (double(*)[NN])s_x[e];
+
+    // the node, and the element's 4·N1 face slots dealt out to its nodes
+    constexpr int NS = (4 * N1 + NN - 1) / NN;
+    double h = 0, hu = 0, hv = 0, u = 0, v = 0, flux[NS][3];
+    if (valid) {
+        h = in.h[gi];
+        hu = in.hu[gi];
+        hv = in.hv[gi];
+        u = in.u[gi];
+        v = in.v[gi];
+    }
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+        const int sl = i + q * NN;
+        const bool has = valid && sl < 4 * N1;
+        flux[q][0] = has ? fb_h[fbase + sl] : 0.0;
+        flux[q][1] = has ? fb_hu[fbase + sl] : 0.0;
+        flux[q][2] = has ? fb_hv[fbase + sl] : 0.0;
+    }
+    if (valid) {
+        // what the later phases read, on its way from DRAM meanwhile
+        prefetch(&T.fx_hm[gi * NP]);
+        prefetch(&T.fx_gdb[gi]);
+        prefetch(&T.jinv[gi]);
+        prefetch(&T.fx_lift[fbase + i % (4 * N1)]);
+        prefetch(&T.fx_exp[k]);
+        if (mode != kRhsOnly && base.h) {
+            prefetch(&base.h[gi]);
+            prefetch(&base.hu[gi]);
+            prefetch(&base.hv[gi]);
+        }
+        if (P.friction == 2) prefetch(&T.g_n2[gi]);
+    }
+    if (!run) return;
+    ExpWords ew = node_exponents(h, hu, hv, u, v);
+#pragma unroll
+    for (int q = 0; q < NS; ++q)
+        ew.w[2] = __vmaxu2(ew.w[2], (unsigned)(fx::expo(flux[q][0]) |
+                                               max_expo(flux[q][1], flux[q][2]) << 16));
+    const bool shallow = valid && P.formulation == kWetDry && fp::lt(h, P.subcell_depth);
+    // sub: the element has a node below the subcell depth; dry: no water at any
+    bool sub, dry;
+    if (kInWarp) {
+        const unsigned lanes = (unsigned)(((1ull << NN) - 1) << ((tid & 31) / NN * NN));
+        sub = (__ballot_sync(0xffffffffu, shallow) & lanes) != 0;
+        dry = (__ballot_sync(0xffffffffu, shallow && !fp::nz(h)) & lanes) == lanes;
+        warp_max<NN>(ew);
+    } else {
+        if (i < 2) s_flag[e][i] = 0;
+        if (i < 6) s_exp[e][i] = 0;
+        __syncthreads();
+        if (shallow) {
+            atomicOr(&s_flag[e][0], 1);
+            if (!fp::nz(h)) atomicAdd(&s_flag[e][1], 1);
+        }
+        for (int q = 0; q < 3; ++q) {
+            atomicMax(&s_exp[e][2 * q], ew.w[q] & 0xFFFFu);
+            atomicMax(&s_exp[e][2 * q + 1], ew.w[q] >> 16);
+        }
+        __syncthreads();
+        sub = s_flag[e][0] != 0;
+        dry = s_flag[e][1] == NN;
+        for (int q = 0; q < 3; ++q) ew.w[q] = s_exp[e][2 * q] | s_exp[e][2 * q + 1] << 16;
+    }
+    bool fixed = false;
+    fx::Scale sc;
+    if (valid && !sub) {
+        sc = fx::scales(exponents(ew), T.fx_exp[k], T.fx_ec, T.fx_e2g);
+        fixed = sc.ok;
+    }
+    if (valid && !fixed && !dry && i == 0) T.gen_list[atomicAdd(&T.gen_count[0], 1u)] = (int32_t)k;
+
+    FxLimb G{}, H{};                         // 2g·h, h
+    int64_t m0 = 0, m1 = 0, u0 = 0, u1 = 0;  // hu, hv, u, v
+    FxLimb* const pairs = (FxLimb*)&s_x[e][0];
+    FxLimb* const nd_h = (FxLimb*)&s_x[e][C::PAIR_DOUBLES];
+    int64_t* const nd = (int64_t*)&s_x[e][C::PAIR_DOUBLES + NN];
+    int64_t* const lifted = (int64_t*)&s_x[e][C::PAIR_DOUBLES + 5 * NN];
+    if (fixed) {
+        H = fx::split(fx::to_fixed(h, sc.kh));
+        G = fx::two_g_h(H, T.fx_two_g, sc);
+        m0 = fx::to_fixed(hu, sc.km);
+        m1 = fx::to_fixed(hv, sc.km);
+        u0 = fx::to_fixed(u, sc.ku);
+        u1 = fx::to_fixed(v, sc.ku);
+        nd_h[i] = H;
+        nd[i] = m0;
+        nd[NN + i] = m1;
+        nd[2 * NN + i] = u0;
+        nd[3 * NN + i] = u1;
+#pragma unroll
+        for (int q = 0; q < NS; ++q) {
+            const int sl = i + q * NN;
+            if (sl >= 4 * N1) continue;
+            const FxLimb c = T.fx_lift[fbase + sl];
+            lifted[sl] = fx::mul<0>(c, fx::split(fx::to_fixed(flux[q][0], sc.kfh)));
+            lifted[4 * N1 + sl] = fx::mul<0>(c, fx::split(fx::to_fixed(flux[q][1], sc.kfm)));
+            lifted[8 * N1 + sl] = fx::mul<0>(c, fx::split(fx::to_fixed(flux[q][2], sc.kfm)));
+        }
+    }
+    const FxNode node = T.fx_node[i];
+    element_sync<NN>();
+
+    // ---- the pair fluxes ----
+    if (fixed) {
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const int o = (node.others >> (8 * q)) & 0xFF;  // the pair's other node
+            const FxPair hm = T.fx_hm[gi * NP + q];
+            const fx::Flux f = fx::pair_flux(G, nd_h[o], m0 + nd[o], m1 + nd[NN + o],
+                                             u0 + nd[2 * NN + o], u1 + nd[3 * NN + o], hm.x, hm.y);
+            FxLimb* slot_f = &pairs[(i * NP + q) * 3];
+            slot_f[0] = f.h;
+            slot_f[1] = f.hu;
+            slot_f[2] = f.hv;
+        }
+    }
+    element_sync<NN>();
+
+    // ---- their sums, the bed slope, the lift and 1/J ----
+    F3 F{0.0, 0.0, 0.0};
+    if (fixed) {
+        fx::PairSum ah = fx::pair_sum(), au = ah, av = ah;
+#pragma unroll
+        for (int q = 0; q < NA; ++q) {
+            const FxLimb* f = &pairs[(int)((node.slots >> (8 * q)) & 0xFF) * 3];
+            const FxLimb coef = T.fx_coef[i * NA + q];
+            fx::mac(ah, coef, f[0]);
+            fx::mac(au, coef, f[1]);
+            fx::mac(av, coef, f[2]);
+        }
+        int64_t fh = -fx::fold(ah), fhu = -fx::fold(au), fhv = -fx::fold(av);
+        if (P.has_bed) {
+            const FxPair slope = T.fx_gdb[gi];
+            fhu -= fx::bed_term(H, slope.x, sc);
+            fhv -= fx::bed_term(H, slope.y, sc);
+        }
+        int s_a, s_b;
+        node_slots<N1>(i % N1, i / N1, s_a, s_b);
+        for (const int sl : {s_a, s_b})
+            if (sl >= 0) {
+                fh -= lifted[sl];
+                fhu -= lifted[4 * N1 + sl];
+                fhv -= lifted[8 * N1 + sl];
+            }
+        const double jinv = T.jinv[gi];
+        F.h = fx::over_jacobian(fh, sc.sh, jinv);
+        F.hu = fx::over_jacobian(fhu, sc.sm, jinv);
+        F.hv = fx::over_jacobian(fhv, sc.sm, jinv);
+        if (X.subcell_mass)  // no subcells: NaN (compute_rhs_swe_2d_mass_fluxes_into)
+            for (int q = i; q < C::NSUB; q += NN)
+                X.subcell_mass[k * C::NSUB + q] = fp::from_bits(0x7FF8000000000000ll);
+    }
+    if (dry) {
+        F = lift_only<N1>(T, fb_h, fb_hu, fb_hv, k, i, F3{0.0, 0.0, 0.0});
+        if (X.subcell_mass)  // its interface fluxes are ±0
+            for (int q = i; q < C::NSUB; q += NN) X.subcell_mass[k * C::NSUB + q] = 0.0;
+    }
+    finish_node<N1, LISTED, NN>(T, P, in, base, out, acc, keep, cm, lp, slot, mode, check_finite, k,
+                                i, fixed || dry, F, s_q, &s_flag[e][2], s_red[e]);
+}
+
+// The elements of a stage that stage_kernel left (T.gen_list): those with
+// subcells, and wet ones whose scales spread too far. Few and long (some 200
+// FP64 operations in a row), so two lanes a node, a subcell direction each.
+// The last block to end empties the list for the next stage.
+template <int N1, bool LISTED>
+__global__ void __launch_bounds__(GenCfg<N1>::THREADS, 4)
+    general_kernel(const __grid_constant__ DevTables T, const __grid_constant__ Physics P,
+                   const __grid_constant__ StageExtra X, const __grid_constant__ DevBuf in,
+                   DevBuf base, DevBuf out, DevBuf acc, const double* __restrict__ fb_h,
+                   const double* __restrict__ fb_hu, const double* __restrict__ fb_hv, StepCtl* ctl,
+                   int slot, int mode, int check_finite, DevBuf keep, LtsPass lp) {
+    constexpr int NN = N1 * N1, LANES = 2 * NN, EPB = GenCfg<N1>::EPB;
+    using C = Cfg<N1>;
+    __shared__ double s_x[EPB][C::X];
+    __shared__ int s_flag[EPB][2];
+    __shared__ double s_red[EPB][4];
+    const int tid = threadIdx.x;
+    const int e = tid / LANES, lane = tid % LANES, half = lane / NN, i = lane % NN;
+    double(*const s_q)[NN] = (double(*)[NN])s_x[e];
+    const unsigned n = *(volatile unsigned*)&T.gen_count[0];
+    for (unsigned first = blockIdx.x * EPB; first < n; first += gridDim.x * EPB) {
+        const bool take = first + e < n;
+        const int64_t k = take ? (int64_t)T.gen_list[first + e] : 0;
+        StepCtl* const cm = ctl + ((T.elem_member && take) ? T.elem_member[k] : 0);
+        const int64_t gi = k * NN + i;
+        double h = 0.0;
+        if (take && half == 0) {
+            h = in.h[gi];
+            s_q[0][i] = h;
+            s_q[1][i] = in.hu[gi];
+            s_q[2][i] = in.hv[gi];
+            s_q[3][i] = in.u[gi];
+            s_q[4][i] = in.v[gi];
+            s_q[5][i] = P.has_bed ? T.bed[gi] : 0.0;
+        }
+        // sub: an element with a node below the subcell depth
+        const bool shallow =
+            take && half == 0 && P.formulation == kWetDry && fp::lt(h, P.subcell_depth);
+        if (lane == 0) s_flag[e][0] = 0;
+        element_sync<LANES>();
+        if (shallow) atomicOr(&s_flag[e][0], 1);
+        element_sync<LANES>();
+        const bool sub = s_flag[e][0] != 0;
+        const F3 F = general_rhs<N1, 2>(T, P, X, in, fb_h, fb_hu, fb_hv, k, i, half, take, sub,
+                                        false, s_x[e]);
+        if (X.subcell_mass && take && !sub)  // no subcells: NaN
+            for (int q = lane; q < C::NSUB; q += LANES)
+                X.subcell_mass[k * C::NSUB + q] = fp::from_bits(0x7FF8000000000000ll);
+        finish_node<N1, LISTED, LANES>(T, P, in, base, out, acc, keep, cm, lp, slot, mode,
+                                       check_finite, k, i, take && half == 0, F, s_q,
+                                       &s_flag[e][1], s_red[e]);
+        element_sync<LANES>();
+    }
+    __syncthreads();
+    if (tid == 0 && atomicAdd(&T.gen_count[1], 1u) == gridDim.x - 1) {
+        T.gen_count[0] = 0;
+        T.gen_count[1] = 0;
+    }
+}
+#else
+// LISTED: a multirate pass over lp's elements, each with its own stage
+template <int N1, bool LISTED, int SHAPE = 0>
+__global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_BLOCKS)
+    stage_kernel(DevTables T, Physics P, StageExtra X, DevBuf in, DevBuf base, DevBuf out,
+                 DevBuf acc, const double* __restrict__ fb_h, const double* __restrict__ fb_hu,
+                 const double* __restrict__ fb_hv, StepCtl* ctl, int slot, int mode,
+                 int check_finite, const int* active, DevBuf keep, LtsPass lp) {
+    using C = Cfg<N1, SHAPE>;
+    constexpr int NN = C::NN, EPB = C::EPB;
+    __shared__ double s_x[EPB][C::X];
+    __shared__ int s_flag[EPB][3];
+    __shared__ double s_red[EPB][4];
+
+    if (!*active) return;
+    const int tid = threadIdx.x;
+    const int e = tid / NN, i = tid % NN;
+    int64_t k = (int64_t)blockIdx.x * EPB + e;
+    if (LISTED) k = k < lp.n ? (int64_t)lp.list[k] : T.K;
+    else k += X.k_first;
+    const int64_t k_end = (LISTED || X.k_last > T.K) ? T.K : X.k_last;
+    // the element's member (its StepCtl); an ensemble member that has
+    // stopped keeps its state: its elements take no part
+    StepCtl* const cm = ctl + ((T.elem_member && k < k_end) ? T.elem_member[k] : 0);
+    const bool valid = k < k_end && (!T.elem_member || cm->active);
+    const int64_t gi = k * NN + i;
+    double(*const s_q)[NN] = (double(*)[NN])s_x[e];
+    double h = 0.0;
+    if (valid) {
+        h = in.h[gi];
+        s_q[0][i] = h;
+        s_q[1][i] = in.hu[gi];
+        s_q[2][i] = in.hv[gi];
+        s_q[3][i] = in.u[gi];
+        s_q[4][i] = in.v[gi];
+        s_q[5][i] = P.has_bed ? T.bed[gi] : 0.0;
+    }
+    if (i < 2) s_flag[e][i] = 0;
+    // sub: an element with a node below the subcell depth; dry: without water
+    // at any node (every h = ±0, so every u = v = 0): its reconstructed subcell
+    // faces are dry, so the interface fluxes, pressure and bed terms are all
+    // ±0, and it skips the subcell phases
+    const bool shallow = valid && P.formulation == kWetDry && fp::lt(h, P.subcell_depth);
+    element_sync<NN>();
+    if (shallow) {
+        atomicOr(&s_flag[e][0], 1);
+        if (!fp::nz(h)) atomicAdd(&s_flag[e][1], 1);
+    }
+    element_sync<NN>();
+    const bool sub = s_flag[e][0] != 0, dry = s_flag[e][1] == NN;
+    const F3 F =
+        general_rhs<N1, 1>(T, P, X, in, fb_h, fb_hu, fb_hv, k, i, 0, valid, sub, dry, s_x[e]);
+    if (X.subcell_mass && valid && !sub)  // no subcells: NaN (compute_rhs_swe_2d_mass_fluxes_into)
+        for (int q = i; q < C::NSUB; q += NN)
+            X.subcell_mass[k * C::NSUB + q] = fp::from_bits(0x7FF8000000000000ll);
+    finish_node<N1, LISTED, NN>(T, P, in, base, out, acc, keep, cm, lp, slot, mode, check_finite, k,
+                                i, valid, F, s_q, &s_flag[e][2], s_red[e]);
+}
+#endif
+
 // finish_where over every element: state ← acc, then the wet/dry correction
 // LISTED: the end of the substeps of lp's elements, and a non-finite
 // result flagged in ctl
@@ -1122,7 +1421,7 @@ __global__ void __launch_bounds__(Cfg<N1>::THREADS)
     constexpr int NN = C::NN, EPB = C::EPB;
     __shared__ double s_v[EPB][3][NN];
     __shared__ int s_flag[EPB];
-    __shared__ double s_red[EPB][5];
+    __shared__ double s_red[EPB][4];
     const int tid = threadIdx.x;
     const int e = tid / NN, i = tid % NN;
     int64_t k = (int64_t)blockIdx.x * EPB + e;
@@ -1145,28 +1444,23 @@ __global__ void __launch_bounds__(Cfg<N1>::THREADS)
         if (valid && fp::lt(vh, P.h_dry)) atomicOr(&s_flag[e], 1);
         __syncthreads();
         const bool needs = s_flag[e] != 0;
-        if (valid && needs && i == 0) {
-            const double* mass = &T.mass[k * NN];
-            double sh = 0.0, shu = 0.0, shv = 0.0, hmin = INFINITY;
-            for (int p = 0; p < NN; ++p) {
-                sh += mass[p] * s_v[e][0][p];
-                shu += mass[p] * s_v[e][1][p];
-                shv += mass[p] * s_v[e][2][p];
-                hmin = lmin(s_v[e][0][p], hmin);
+        if (valid && needs && i < 4) {
+            // element_mean and positivity_limit_element
+            // (src/solver/limiters/swe_2d.rs:135-203), in node order: a lane
+            // for each mean, one for the smallest depth
+            if (i < 3) {
+                const double* mass = &T.mass[k * NN];
+                double sum = 0.0;
+#pragma unroll
+                for (int p = 0; p < NN; ++p) sum += mass[p] * s_v[e][i][p];
+                s_red[e][i] = sum * T.inv_area[k];
+                if (i == 0 && fp::lt0(s_red[e][0]))
+                    atomicAdd((unsigned long long*)&cm->clips, 1ull);
+            } else {
+                double hmin = INFINITY;
+                for (int p = 0; p < NN; ++p) hmin = lmin(s_v[e][0][p], hmin);
+                s_red[e][3] = hmin;
             }
-            const double inv_area = T.inv_area[k];
-            const double h_avg = sh * inv_area;
-            s_red[e][0] = h_avg;
-            s_red[e][1] = shu * inv_area;
-            s_red[e][2] = shv * inv_area;
-            double theta = 1.0;
-            if (fp::gt0(h_avg) && fp::lt0(hmin)) {
-                theta = h_avg / (h_avg - hmin);
-                theta = fp::lt0(theta) ? 0.0 : (fp::gt(theta, 1.0) ? 1.0 : theta);
-            }
-            s_red[e][3] = theta;
-            s_red[e][4] = hmin;
-            if (fp::lt0(h_avg)) atomicAdd((unsigned long long*)&cm->clips, 1ull);
         }
         __syncthreads();
         if (valid && needs) {
@@ -1174,8 +1468,10 @@ __global__ void __launch_bounds__(Cfg<N1>::THREADS)
             if (fp::le0(h_avg)) {
                 vh = vhu = vhv = 0.0;
             } else {
-                if (fp::lt0(s_red[e][4])) {
-                    const double th = s_red[e][3];
+                const double hmin = s_red[e][3];
+                if (fp::lt0(hmin)) {
+                    double th = vdiv(h_avg, h_avg - hmin);
+                    th = fp::lt0(th) ? 0.0 : (fp::gt(th, 1.0) ? 1.0 : th);
                     vh = th * (vh - h_avg) + h_avg;
                     vhu = th * (vhu - s_red[e][1]) + s_red[e][1];
                     vhv = th * (vhv - s_red[e][2]) + s_red[e][2];

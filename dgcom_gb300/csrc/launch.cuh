@@ -48,6 +48,16 @@ static void face_listed_n(const DevTables& T, const Physics& P, const DevBuf& in
                                                      lp);
 }
 
+#if DGSWE_FAST
+// general_kernel's blocks for a pass of `count` elements, of which it takes
+// those listed: enough for all, four a multiprocessor at most
+template <int N1>
+static unsigned general_blocks(int64_t count) {
+    const int64_t all = (count + GenCfg<N1>::EPB - 1) / GenCfg<N1>::EPB;
+    return (unsigned)(all < 608 ? all : 608);
+}
+#endif
+
 template <int N1>
 static void stage_n(const DevTables& T, const Physics& P, const StageExtra& X, const DevBuf& in,
                     const DevBuf& base, const DevBuf& out, const DevBuf& acc, const double* fh,
@@ -57,27 +67,27 @@ static void stage_n(const DevTables& T, const Physics& P, const StageExtra& X, c
     const int64_t k1 = X.k_last < T.K ? X.k_last : T.K;
     const int64_t count = k1 - X.k_first;
     if (count <= 0) return;
+    auto blocks = [&](int epb) { return (unsigned)((count + epb - 1) / epb); };
     if (P.stage_shape == 1) {
         using C1 = Cfg<N1, 1>;
-        const unsigned blocks = (unsigned)((count + C1::EPB - 1) / C1::EPB);
-        stage_kernel<N1, false, 1><<<blocks, C1::THREADS, 0, s>>>(
+        stage_kernel<N1, false, 1><<<blocks(C1::EPB), C1::THREADS, 0, s>>>(
             T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, slot, mode, check_finite, active, keep,
             LtsPass{});
-        return;
-    }
-    if (P.stage_shape == 2) {
+    } else if (P.stage_shape == 2) {
         using C2 = Cfg<N1, 2>;
-        const unsigned blocks = (unsigned)((count + C2::EPB - 1) / C2::EPB);
-        stage_kernel<N1, false, 2><<<blocks, C2::THREADS, 0, s>>>(
+        stage_kernel<N1, false, 2><<<blocks(C2::EPB), C2::THREADS, 0, s>>>(
             T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, slot, mode, check_finite, active, keep,
             LtsPass{});
-        return;
+    } else {
+        using C = Cfg<N1>;
+        stage_kernel<N1, false><<<blocks(C::EPB), C::THREADS, 0, s>>>(
+            T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, slot, mode, check_finite, active, keep,
+            LtsPass{});
     }
-    using C = Cfg<N1>;
-    const unsigned blocks = (unsigned)((count + C::EPB - 1) / C::EPB);
-    stage_kernel<N1, false><<<blocks, C::THREADS, 0, s>>>(T, P, X, in, base, out, acc, fh, fhu, fhv,
-                                                          ctl, slot, mode, check_finite, active,
-                                                          keep, LtsPass{});
+#if DGSWE_FAST
+    general_kernel<N1, false><<<general_blocks<N1>(count), GenCfg<N1>::THREADS, 0, s>>>(
+        T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, slot, mode, check_finite, keep, LtsPass{});
+#endif
 }
 
 template <int N1>
@@ -92,6 +102,10 @@ static void stage_listed_n(const DevTables& T, const Physics& P, const StageExtr
     stage_kernel<N1, true><<<blocks, C::THREADS, 0, s>>>(T, P, X, in, base, out, acc, fh, fhu, fhv,
                                                          ctl, 0, mode, 0, &ctl->always, DevBuf{},
                                                          lp);
+#if DGSWE_FAST
+    general_kernel<N1, true><<<general_blocks<N1>(lp.n), GenCfg<N1>::THREADS, 0, s>>>(
+        T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, 0, mode, 0, DevBuf{}, lp);
+#endif
 }
 
 template <int N1>
@@ -147,6 +161,13 @@ static void face_ready_n(const DevTables& T, const Physics& P, const DevBuf& in,
     const unsigned blocks = (unsigned)((items + threads - 1) / threads);
     face_kernel<N1, true><<<blocks, threads, 0, s>>>(T, P, in, fh, fhu, fhv, ctl, slot, active,
                                                      lp);
+}
+
+template <int N1>
+static void sub_metrics_n(const DevTables& T, const Physics& P, double* out, cudaStream_t s) {
+    const int64_t items = T.K * 2 * N1;
+    if (items > 0)
+        sub_metric_kernel<N1><<<(unsigned)((items + 255) / 256), 256, 0, s>>>(T, P, out);
 }
 
 #if DGSWE_FAST
@@ -271,6 +292,11 @@ static void face_adjoint(int n1, const DevTables& T, const Physics& P, const Dev
     DGSWE_BY_ORDER(face_adjoint_n, T, P, in, A, ctl, slot, s);
 }
 
+static void sub_metrics(int n1, const DevTables& T, const Physics& P, double* out,
+                        cudaStream_t s) {
+    DGSWE_BY_ORDER(sub_metrics_n, T, P, out, s);
+}
+
 static void fixed_tables(int n1, const DevTables& T, FxPair* hm, FxPair* gdb, FxLimb* lift,
                          FxExp* exps, FxPair* normal, cudaStream_t s) {
 #if DGSWE_FAST
@@ -348,7 +374,8 @@ static const KernelSet kSet = {face,          stage,         finish,          dt
                                 dt_fit,        end,           face_listed,     stage_listed,
                                 finish_listed, depth_flags,    subcell_list,
                                 implicit_damping, face_ready,  node_sources,
-                                dt_listed,     fixed_tables,  DGSWE_FAST};
+                                dt_listed,     fixed_tables,  DGSWE_FAST,
+                                sub_metrics};
 
 }  // namespace DGSWE_NS
 }  // namespace dgswe

@@ -51,10 +51,17 @@ using fp::lmin;
 // Arguments outside the range where the seed is a normal float (zero,
 // subnormal, negative, huge, non-finite) take the IEEE operation. Otherwise,
 // and always without DGSWE_FAST, the IEEE operation.
+#if defined(__CUDACC__) && DGSWE_FAST
+// the IEEE operations as calls, out of the kernels' code
+static __device__ __noinline__ double ieee_sqrt(double x) { return sqrt(x); }
+static __device__ __noinline__ double ieee_div(double x, double y) { return x / y; }
+static __device__ __noinline__ double ieee_cbrt(double x) { return cbrt(x); }
+#endif
+
 DG_PT double vsqrt(double x) {
 #if DGSWE_FAST_PATH
     const int64_t b = fp::bits(x);
-    if (b < 0x3810000000000000ll || b >= 0x47E0000000000000ll) return sqrt(x);  // 2^-126, 2^127
+    if (b < 0x3810000000000000ll || b >= 0x47E0000000000000ll) return ieee_sqrt(x);  // 2^-126, 2^127
     return fx::sqrt_pos(x);
 #else
     return sqrt(x);
@@ -64,7 +71,7 @@ DG_PT double vsqrt(double x) {
 DG_PT double vrcp(double y) {
 #if DGSWE_FAST_PATH
     const int64_t b = fp::bits(y);
-    if (b < 0x3820000000000000ll || b >= 0x47C0000000000000ll) return 1.0 / y;  // 2^-125, 2^125
+    if (b < 0x3820000000000000ll || b >= 0x47C0000000000000ll) return ieee_div(1.0, y);  // 2^±125
     return fx::rcp_pos(y);
 #else
     return 1.0 / y;
@@ -73,7 +80,9 @@ DG_PT double vrcp(double y) {
 
 DG_PT double vdiv(double x, double y) {
 #if DGSWE_FAST_PATH
-    return x * vrcp(y);
+    const unsigned ex = (unsigned)fx::expo(x) - 623u, ey = (unsigned)((uint64_t)fp::bits(y) >> 52) - 623u;
+    if (ex > 800u || ey > 800u) return ieee_div(x, y);  // 2^±400, y > 0
+    return fx::div_pos(x, y);
 #else
     return x / y;
 #endif
@@ -146,7 +155,7 @@ DG_PT F3 hll_aligned(double h_l, double hun_l, double hut_l, double un_l,
 DG_PT double wall_ram(double h, double un, double sill, double g) {
     un = fp::max0(un);
     const double head = un * un * (0.5 / g);
-    const double ram = (1.0 - head / sill) * h * un * (2.0 * un + sqrt(g * h));
+    const double ram = (1.0 - vdiv(head, sill)) * h * un * (2.0 * un + vsqrt(g * h));
     return fp::gt(sill, head) ? ram : 0.0;
 }
 
@@ -184,6 +193,26 @@ DG_PT void hydro_hll(const Sd& qa, const Sd& qb, double m0, double m1,
     const double dp_b = half_g * (qb.h * qb.h - hsb * hsb) + wall_b;
     fa = {f_h, f_hu + dp_a * m0, f_hv + dp_a * m1};
     fb = {f_h, f_hu + dp_b * m0, f_hv + dp_b * m1};
+}
+
+// hydro_hll where both reconstructed sides are dry: no flux, and each side's
+// own pressure with the momentum of water that runs against the sill
+DG_PT void hydro_dry(const Sd& qa, const Sd& qb, double m0, double m1, double nx, double ny,
+                     double g, double half_g, double h_min, F3& fa, F3& fb) {
+    const double b_face = lmax(qa.b, qb.b);
+    double wall_a = 0.0, wall_b = 0.0;
+    if (fp::gt(qa.h, h_min)) {
+        const double un = qa.u * nx + qa.v * ny;
+        if (fp::gt0(un)) wall_a = wall_ram(qa.h, un, b_face - (qa.h + qa.b), g);
+    }
+    if (fp::gt(qb.h, h_min)) {
+        const double un = qb.u * nx + qb.v * ny;
+        if (fp::lt0(un)) wall_b = wall_ram(qb.h, -un, b_face - (qb.h + qb.b), g);
+    }
+    const double dp_a = half_g * (qa.h * qa.h) + wall_a;
+    const double dp_b = half_g * (qb.h * qb.h) + wall_b;
+    fa = {0.0, dp_a * m0, dp_a * m1};
+    fb = {0.0, dp_b * m0, dp_b * m1};
 }
 
 // HarmonicTide::elevation (src/boundary/harmonic_tide.rs:124-136)
@@ -228,7 +257,11 @@ DG_PT double vpow_m43(double h) {
     const int64_t b = fp::bits(h);
     if (b >= 0x3820000000000000ll && b < 0x47C0000000000000ll) return fx::pow_m43(h);  // 2^±125
 #endif
+#if DGSWE_FAST_PATH
+    const double z = ieee_div(1.0, ieee_cbrt(h));
+#else
     const double z = 1.0 / cbrt(h);
+#endif
     return (z * z) * (z * z);
 }
 
@@ -266,21 +299,21 @@ DG_PT void damp(const Physics& P, double g_n2, double h, double& hu,
                     u = from.u;
                     v = from.v;
                 } else {
-                    const double inv = 1.0 / from.h;
+                    const double inv = vrcp(from.h);
                     u = from.hu * inv;
                     v = from.hv * inv;
                 }
             } else {
-                const double r = from.h / P.h_dry;
+                const double r = vdiv(from.h, P.h_dry);
                 const double factor =
-                    1.4142135623730951 * r / (P.h_dry * sqrt(1.0 + r * r * r * r));
+                    vdiv(1.4142135623730951 * r, P.h_dry * vsqrt(1.0 + r * r * r * r));
                 u = factor * from.hu;
                 v = factor * from.hv;
             }
         } else {
             // SWEState2D::velocity (src/solver/state/swe_2d.rs:54-61)
             const double h_reg = lmax(from.h, P.h_min);
-            const double inv_d = 1.0 / (from.h * from.h + h_reg * h_reg);
+            const double inv_d = vrcp(from.h * from.h + h_reg * h_reg);
             const double factor = 2.0 * from.h * inv_d;
             u = from.hu * factor;
             v = from.hv * factor;
@@ -290,8 +323,8 @@ DG_PT void damp(const Physics& P, double g_n2, double h, double& hu,
     }
     if (P.has_wet_dry && fp::lt(h, P.h_dry)) {
         // thin_layer_rate (wetting_drying.rs:135-146); h > 0 here
-        const double excess = P.h_dry / h - 1.0;
-        rate += excess * excess / P.relaxation_time;
+        const double excess = vdiv(P.h_dry, h) - 1.0;
+        rate += vdiv(excess * excess, P.relaxation_time);
     }
     const double factor = vrcp(1.0 + dt * rate);
     hu *= factor;
@@ -306,8 +339,9 @@ DG_PT void correct_node(const Physics& P, double h, double& hu, double& hv) {
         return;
     }
     if (fp::lt(h, P.h_dry)) {
-        const double r = h / P.h_dry;
-        const double factor = 1.4142135623730951 * r / (P.h_dry * sqrt(1.0 + r * r * r * r));
+        const double r = vdiv(h, P.h_dry);
+        const double factor =
+            vdiv(1.4142135623730951 * r, P.h_dry * vsqrt(1.0 + r * r * r * r));
         hu = h * (factor * hu);
         hv = h * (factor * hv);
     }
@@ -323,9 +357,9 @@ DG_PT void correct_node(const Physics& P, double h, double& hu, double& hv) {
     const double m2 = hu * hu + hv * hv;
     const double cap = P.max_velocity * h;
     if (fp::gt(m2, 0.99 * (cap * cap))) {
-        const double momentum = sqrt(m2);
+        const double momentum = vsqrt(m2);
         if (fp::gt(momentum, cap)) {
-            const double scale = cap / momentum;
+            const double scale = vdiv(cap, momentum);
             hu *= scale;
             hv *= scale;
         }
@@ -337,7 +371,11 @@ DG_PT void correct_node(const Physics& P, double h, double& hu, double& hv) {
 DG_PT double limited_slope(double q0, double q1, double q2, double ic,
                                                 double im, double ip) {
     const double dm = q1 - q0, dp = q2 - q1;
+#if DGSWE_FAST_PATH
+    const bool extremum = !fp::nz(dm) || !fp::nz(dp) || (fp::bits(dm) ^ fp::bits(dp)) < 0;
+#else
     const bool extremum = fp::le0(dm * dp);
+#endif
     const double central = (q2 - q0) * ic;
     const double bound = fp::min_nn(fabs(dm * im), fabs(dp * ip));
     const double sign = fp::lt0(central) ? -1.0 : 1.0;
@@ -408,7 +446,7 @@ DG_PT void interior_velocity(const Q& qi, double h_min, double& u, double& v) {
     u = 0.0;
     v = 0.0;
     if (fp::gt(qi.h, h_min)) {
-        const double inv = 1.0 / qi.h;
+        const double inv = vrcp(qi.h);
         u = qi.hu * inv;
         v = qi.hv * inv;
     }
@@ -441,11 +479,11 @@ DG_PT Q characteristic_state_ext(const Q& qi, double h_e, double un_e, double ut
     const double h_i = fmax(qi.h, 0.0);
     double un_i = 0.0, ut_i = 0.0;
     if (h_i > h_min) {
-        const double ui = qi.hu / h_i, vi = qi.hv / h_i;
+        const double ui = vdiv(qi.hu, h_i), vi = vdiv(qi.hv, h_i);
         un_i = ui * nx + vi * ny;
         ut_i = -ui * ny + vi * nx;
     }
-    const double c_i = sqrt(g * h_i), c_e = sqrt(g * h_e);
+    const double c_i = vsqrt(g * h_i), c_e = vsqrt(g * h_e);
     const double w_out = un_i + 2.0 * c_i, w_in = un_e - 2.0 * c_e;
     const bool wi = h_i > h_min, we = h_e > h_min;
     double h_b, un_b;
@@ -459,16 +497,16 @@ DG_PT Q characteristic_state_ext(const Q& qi, double h_e, double un_e, double ut
         h_b = h_e;
         un_b = un_e;
     } else if (wi && !we) {
-        const double cc = fmax(w_out / 3.0, 0.0);
-        h_b = cc * cc / g;
+        const double cc = fmax(vdiv(w_out, 3.0), 0.0);
+        h_b = vdiv(cc * cc, g);
         un_b = cc;
     } else if (!wi && we) {
-        const double cc = fmax(-w_in / 3.0, 0.0);
-        h_b = cc * cc / g;
+        const double cc = fmax(vdiv(-w_in, 3.0), 0.0);
+        h_b = vdiv(cc * cc, g);
         un_b = -cc;
     } else {
         const double cc = fmax(0.25 * (w_out - w_in), 0.0);
-        h_b = cc * cc / g;
+        h_b = vdiv(cc * cc, g);
         un_b = 0.5 * (w_out + w_in);
     }
     const double ut_b = un_b > 0.0 ? ut_i : ut_e;
@@ -490,7 +528,7 @@ DG_PT Q characteristic_state(const Q& qi, double u, double v, double eta, double
     const double bathy = qi.b;
     const double h_e = fmax(eta - bathy, 0.0);
     double un_e = 0.0;
-    if (elevation_only == kIncomingWave) un_e = 2.0 * (sqrt(g * fmax(-bathy, 0.0)) - sqrt(g * h_e));
+    if (elevation_only == kIncomingWave) un_e = 2.0 * (vsqrt(g * fmax(-bathy, 0.0)) - vsqrt(g * h_e));
     const double ut_e = -u * ny + v * nx;
     return characteristic_state_ext(qi, h_e, un_e, ut_e, nx, ny, g, h_min);
 }

@@ -1,4 +1,4 @@
-// Holds sqrt_pos, rcp_pos and pow_m43 of dgcom_gb300/csrc/fixed64.hpp to
+// Holds sqrt_pos, rcp_pos, div_pos and pow_m43 of dgcom_gb300/csrc/fixed64.hpp to
 // 0.75 ulp of the long double value, over their whole argument ranges:
 // random mantissas, mantissas at both ends, every exponent (parity and
 // remainder by three). Compiled with several DGSWE_SEED_ERROR, which stand
@@ -18,7 +18,7 @@ static double ulps(double got, long double want) {
 
 int main() {
     std::mt19937_64 rng(1);
-    double worst[3] = {0.0, 0.0, 0.0};
+    double worst[4] = {0.0, 0.0, 0.0, 0.0};
     long checks = 0;
     for (int e = 1023 - 124; e < 1023 + 124; ++e)
         for (int i = 0; i < 3000; ++i) {
@@ -27,10 +27,14 @@ int main() {
             if (i % 7 == 1) m = fx::kMantissa - rng() % 64;
             const double x = fp::from_bits((int64_t)(((uint64_t)e << 52) | m));
             const long double c = cbrtl((long double)x);
-            const double off[3] = {ulps(fx::sqrt_pos(x), sqrtl((long double)x)),
+            const double y = fp::from_bits((int64_t)(((uint64_t)(1023 - 200 + rng() % 400) << 52) |
+                                                     (i % 5 ? rng() & fx::kMantissa : m)));
+            const double n = i % 2 ? x : -x;
+            const double off[4] = {ulps(fx::sqrt_pos(x), sqrtl((long double)x)),
                                    ulps(fx::rcp_pos(x), 1.0L / (long double)x),
-                                   ulps(fx::pow_m43(x), 1.0L / (c * c * c * c))};
-            for (int k = 0; k < 3; ++k) {
+                                   ulps(fx::pow_m43(x), 1.0L / (c * c * c * c)),
+                                   ulps(fx::div_pos(n, y), (long double)n / (long double)y)};
+            for (int k = 0; k < 4; ++k) {
                 if (!(off[k] <= 0.75)) {
                     std::printf("function %d at %a: %g ulp\n", k, x, off[k]);
                     return 1;
@@ -39,5 +43,6 @@ int main() {
                 ++checks;
             }
         }
-    std::printf("ok %ld checks; worst %.4f %.4f %.4f ulp\n", checks, worst[0], worst[1], worst[2]);
+    std::printf("ok %ld checks; worst %.4f %.4f %.4f %.4f ulp\n", checks, worst[0],
+                worst[1], worst[2], worst[3]);
 }
