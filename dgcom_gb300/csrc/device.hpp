@@ -71,7 +71,7 @@ struct DevTables {
     const FxExp* fx_exp = nullptr;    // [K]
     const FxLimb* fx_coef = nullptr;  // [nn][2(n1−1)]
     const FxNode* fx_node = nullptr;  // [nn]
-    const FxPair* fx_normal = nullptr;  // [E] the edges' unit normals at 2^61
+    const FxPair* fx_normal = nullptr;  // [E] the edges' unit normals at 2^62
     // the elements a stage leaves to general_kernel, and {their number, the
     // blocks that have ended}; empty between stages
     int32_t* gen_list = nullptr;     // [K]

@@ -409,15 +409,18 @@ DG_HD double over_jacobian(int64_t V, int s, double jinv) {
 // hydro_hll (point.cuh) with at least one reconstructed side wet, each
 // quantity at a scale of the face node's own exponents (E: |x| < 2^E):
 //   surface sums 2^(60 − eL) (eL: depths and beds), reconstructed depths
-//   2^(61 − es), own depths 2^(61 − eh), velocities 2^(60 − ev), speeds of
-//   waves 2^(60 − eS), mass flux 2^(60 − eM), momentum flux 2^(59 − eQ),
-//   weights 2^61.
+//   2^(62 − es), own depths 2^(62 − eh), velocities 2^(60 − ev) and 2^(62 − ev),
+//   speeds of waves 2^(60 − eS), momenta 2^(60 − es − ev), mass flux
+//   2^(58 − eM), momentum flux 2^(58 − eQ), weights 2^62.
 // With S_L and S_R the wave speeds held to S_L ≤ 0 ≤ S_R, α = S_R/(S_R − S_L),
 // β = 1 − α and w = −α·S_L, the flux is
 //   α·F_l + β·F_r − w·(q_r − q_l),
 // the star flux in sub-critical flow and one side's (α or β = 1, w = 0)
 // otherwise. The differences of depths in it are exact, so that a face at
 // rest has no mass flux; eM follows the depths' difference, not their size.
+// The integer pipe that shifts and selects is the bound, so the scales are
+// such that most products end at theirs (fold<0>, one shift), and the results
+// become doubles on the idle FP64 pipe.
 
 using FaceConstants = FxFaceConstants;
 
@@ -429,36 +432,47 @@ DG_HD int64_t min64(int64_t a, int64_t b) { return a < b ? a : b; }
 DG_HD int64_t max64(int64_t a, int64_t b) { return a > b ? a : b; }
 DG_HD int imax(int a, int b) { return a > b ? a : b; }
 DG_HD int64_t shr(int64_t v, int n) { return v >> (n > 63 ? 63 : n); }
+DG_HD int64_t shl(int64_t v, int n) { return (int64_t)((uint64_t)v << n); }
 DG_HD int64_t abs64(int64_t v) { return v < 0 ? -v : v; }
 
-// √(g·x) at 2^(60 − eC) for 0 ≤ x at 2^s (below 2^62), √(g·x) < 2^eC
+// from_fixed by the conversion instruction, which runs on the FP64 pipe
+DG_HD double convert(int64_t v, int s) {
+#if defined(__CUDA_ARCH__)
+    const double x = __ll2double_rn(v);
+    return v ? fp::from_bits(fp::bits(x) - ((int64_t)s << 52)) : 0.0;
+#else
+    return from_fixed(v, s);
+#endif
+}
+
+// √(g·x) at 2^(58 − eC) for 0 ≤ x at 2^s (below 2^62), √(g·x) < 2^eC
 DG_HD int64_t celerity(int64_t x, int s, const FaceConstants& c, int eC) {
     int up = clz64((uint64_t)x) - 2;     // x·2^up in [2^61, 2^62)
     up -= (60 - up - s) & 1;             // one less where that makes the exponent even
     const uint64_t X = up >= 0 ? (uint64_t)x << up : (uint64_t)x >> 1;
     const int p = 60 - up - s;           // x's value is X·2^(p − 60)
-    const int64_t v = mul<2>(split((int64_t)(root62(x ? X : 1ull << 60) >> 1)), c.sqrt_g);
+    const int64_t v = mul<0>(split((int64_t)(root62(x ? X : 1ull << 60) >> 1)), c.sqrt_g);
     return x ? shr(v, 1 - c.e_sqrt_g - p / 2 + eC) : 0;
 }
 
-// a/(a + b) at 2^61 for 0 ≤ a, b < 2^61, not both 0
+// a/(a + b) at 2^62 for 0 ≤ a, b < 2^61, not both 0
 DG_HD int64_t share(int64_t a, int64_t b) {
     const uint64_t d = (uint64_t)(a + b);
     const int up = clz64(d) - 2;  // (a + b)·2^up in [2^61, 2^62)
     const uint64_t q = reciprocal61(d << (up + 2));
-    return mul<3>(split((int64_t)((uint64_t)a << up)), split((int64_t)q));
+    return mul<4>(split(shl(a, up)), split((int64_t)q));
 }
 
-// The flux along the unit normal n, times the vector m = |m|·n (each number
-// of m at 2^(61 − em); the mass flux times the length |m| by the caller), as
-// seen from both sides. Nothing is written where both reconstructed sides
-// are dry (kBothDry, but for two sides without any water) or the exponents
-// are out of range (kNoScale).
+// The flux along the unit normal n (at 2^62), times the vector m = |m|·n (at
+// 2^(62 − em), each number below 2^(em − 1), or n itself with em 0; the mass
+// flux times the length |m| by the caller), as seen from both sides. Nothing
+// is written where both reconstructed sides are dry (kBothDry, but for two
+// sides without any water) or the exponents are out of range (kNoScale).
 enum FaceCase { kNoScale = 0, kDone = 1, kBothDry = 2 };
 
 template <class Side>
 DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const FxPair& n, const FxPair& m, int em,
-                     const FaceConstants& c, double h_min, FaceFlux& out) {
+                         const FaceConstants& c, double h_min, FaceFlux& out) {
     const int xa = (int)((uint64_t)fp::bits(qa.h) >> 52), xb = (int)((uint64_t)fp::bits(qb.h) >> 52);
     const int xh = imax(xa, xb);
     if (xh == 0) {  // depths of +0 or subnormal
@@ -479,99 +493,99 @@ DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const FxPair& n, const 
     const int64_t dry = to_fixed(h_min, xl + 3);
     const bool wet_a = ra > dry, wet_b = rb > dry;
     if (!wet_a && !wet_b) return kBothDry;
-    const int es = 64 - clz64((uint64_t)max64(ra, rb)) + eL - 60;
-    if (es < -60) return kNoScale;
-    const int64_t sa = (int64_t)((uint64_t)ra << (eL - es + 1));
-    const int64_t sb = (int64_t)((uint64_t)rb << (eL - es + 1));
+    const int es = 4 + eL - clz64((uint64_t)(ra | rb));
     const int eC = (es + c.e_g + 1) >> 1;
     const int ev = imax(xv - 1022, eC - 30);
-    const int kv = 1024 + ev;
+    if (es < -60 || ev > eC + 30) return kNoScale;
+    const int64_t sa = shl(ra, eL - es + 2), sb = shl(rb, eL - es + 2);
+    const int kv = 1023 + ev;
     auto rotate = [&](const Side& q, int64_t& normal, int64_t& along) {
         const bool moves = fp::gt(q.h, h_min);
         const Lim u = split(moves ? to_fixed(q.u, kv) : 0), v = split(moves ? to_fixed(q.v, kv) : 0);
-        Acc a{half<2>(), 0}, t{half<2>(), 0}, o{0, 0};
+        Acc a{half<0>(), 0}, t{half<0>(), 0}, o{0, 0};
         mac(a, u, n.x);
         mac(a, v, n.y);
-        normal = fold<2>(a);
+        normal = fold<0>(a);
         mac(t, v, n.x);
         mac(o, u, n.y);
         t.t -= o.t;
         t.r -= o.r;
-        along = fold<2>(t);
+        along = fold<0>(t);
     };
     int64_t un_a, ut_a, un_b, ut_b;  // 2^(60 − ev)
     rotate(qa, un_a, ut_a);
     rotate(qb, un_b, ut_b);
     // wave speeds (Einfeldt; beside a dry side, the front's)
-    const int64_t c_a = celerity(sa, 61 - es, c, eC), c_b = celerity(sb, 61 - es, c, eC);
-    const int64_t c_m = celerity(sa + sb, 62 - es, c, eC);
+    const int64_t c_a = celerity(sa, 62 - es, c, eC), c_b = celerity(sb, 62 - es, c, eC);
+    const int64_t c_m = celerity((sa >> 1) + (sb >> 1), 62 - es, c, eC);
     const int64_t va = wet_a ? un_a : 0, vb = wet_b ? un_b : 0;
-    const int64_t u_m = vb + mul<3>(split(share(c_a, c_b)), split(va - vb));
+    const int64_t u_m = vb + mul<2>(split(share(c_a, c_b)), split(va - vb));
     const int eS = imax(ev, eC) + 2;
-    const int dv = eS - ev, dc = eS - eC;
-    const int64_t wa = shr(c_a, dc), wb = shr(c_b, dc), wm = shr(c_m, dc);
-    const int64_t xl_ = shr(va, dv), xr_ = shr(vb, dv), xm = shr(u_m, dv);
+    const int dv = eS - ev, dc = eS - eC - 2;  // at most 32
+    const int64_t wa = c_a >> dc, wb = c_b >> dc, wm = c_m >> dc;
+    const int64_t xl_ = va >> dv, xr_ = vb >> dv, xm = u_m >> dv;
     const int64_t s_l = min64(wet_a ? min64(xl_ - wa, xm - wm) : xr_ - 2 * wb, 0);
     const int64_t s_r = max64(wet_b ? max64(xr_ + wb, xm + wm) : xl_ + 2 * wa, 0);
     if (s_l == s_r) return kNoScale;
     const int64_t alpha = share(s_r, -s_l);
-    const Lim al = split(alpha), be = split((1ll << 61) - alpha);
-    const Lim w = split(mul<3>(al, split(-s_l)));  // 2^(60 − eS)
-    // momenta hs·un, hs·ut at 2^(60 − es − ev); a dry side carries none in its
-    // own flux
+    const Lim al = split(alpha), be = split((1ll << 62) - alpha);
+    const Lim w = split(mul<4>(al, split(-s_l)));  // 2^(62 − eS), below 2^61
+    // momenta hs·un, hs·ut; a dry side carries none in its own flux
     const Lim da = split(sa), db = split(sb);
-    const Lim ul = split(un_a), ur = split(un_b);
-    const int64_t m_a = mul<3>(da, ul), m_b = mul<3>(db, ur);
-    const Lim tl = split(ut_a), tr = split(ut_b);
-    const int64_t t_a = mul<3>(da, tl), t_b = mul<3>(db, tr);
+    const Lim ul = split(shl(un_a, 2)), ur = split(shl(un_b, 2));  // 2^(62 − ev)
+    const int64_t m_a = mul<0>(da, ul), m_b = mul<0>(db, ur);
+    const Lim tl = split(shl(ut_a, 2)), tr = split(shl(ut_b, 2));
+    const int64_t t_a = mul<0>(da, tl), t_b = mul<0>(db, tr);
     const Lim ml = split(wet_a ? m_a : 0), mr = split(wet_b ? m_b : 0);
     // mass
     const int64_t dh = sb - sa;
-    const int grow = clz64((uint64_t)abs64(dh)) - 3;  // dh·2^grow below 2^61
+    const int grow = clz64((uint64_t)abs64(dh)) - 2;  // dh·2^grow below 2^62
     const int eD = es - grow;
     const int eM = imax(es + ev + 1, eS + eD);
-    Acc f{half<3>(), 0};
+    Acc f{half<0>(), 0};
     mac(f, al, ml);
     mac(f, be, mr);
-    const int64_t f_h = shr(fold<3>(f), eM - es - ev) -
-                        shr(mul<3>(w, split((int64_t)((uint64_t)dh << grow))), eM - eS - eD);
-    out.h = from_fixed(f_h, 60 - eM);
+    const int64_t f_h = shr(fold<0>(f), eM - es - ev) -
+                        shr(mul<0>(w, split(shl(dh, grow))), 2 + eM - eS - eD);
+    out.h = convert(f_h, 58 - eM);
     // momentum
-    const int eQ = imax(imax(2 * eh + c.e_half_g, es + 2 * ev + 1), eS + es + ev - 1);
-    const int dm = 1 + eQ - es - 2 * ev, dw = 1 + eQ - eS - es - ev;
-    auto pressure = [&](int64_t x, int64_t y, int e) {  // ½g·x·y of depths at 2^(61 − e)
-        return shr(mul<1>(split(mul<3>(split(x), split(y))), c.half_g), 1 + eQ - 2 * e - c.e_half_g);
+    const int eQ = imax(imax(2 * eh + c.e_half_g + 1, es + 2 * ev + 1), eS + es + ev);
+    const int dm = eQ - es - 2 * ev, dw = eQ - eS - es - ev;
+    auto pressure = [&](int64_t x, int64_t y, int e) {  // ½g·x·y of depths at 2^(62 − e)
+        return shr(mul<0>(split(mul<0>(split(x), split(y))), c.half_g), eQ - 2 * e - c.e_half_g);
     };
-    Acc g{half<3>(), 0};
-    mac(g, al, split(pressure(sa, sa, es) + shr(mul<4>(ml, ul), dm)));
-    mac(g, be, split(pressure(sb, sb, es) + shr(mul<4>(mr, ur), dm)));
-    const int64_t f_n = fold<3>(g) - shr(mul<4>(w, split(m_b - m_a)), dw);
-    Acc t{half<3>(), 0};
-    mac(t, al, split(shr(mul<4>(ml, tl), dm)));
-    mac(t, be, split(shr(mul<4>(mr, tr), dm)));
-    const Lim f_t = split(fold<3>(t) - shr(mul<4>(w, split(t_b - t_a)), dw));
-    // each side's own pressure over the reconstructed one. Where a depth has
-    // bits below the surface sums' last place, the own one is taken whole
-    // and the pressure of its rounding cancels against the flux's.
-    const int down = eL - eh + 1;
+    Acc g{half<2>(), 0};
+    mac(g, al, split(pressure(sa, sa, es) + shr(mul<0>(ml, ul), dm)));
+    mac(g, be, split(pressure(sb, sb, es) + shr(mul<0>(mr, ur), dm)));
+    const int64_t f_n = fold<2>(g) - shr(mul<0>(w, split(m_b - m_a)), dw);
+    Acc t{half<2>(), 0};
+    mac(t, al, split(shr(mul<0>(ml, tl), dm)));
+    mac(t, be, split(shr(mul<0>(mr, tr), dm)));
+    const Lim f_t = split(shl(fold<2>(t) - shr(mul<0>(w, split(t_b - t_a)), dw), 2));
+    // each side's own pressure over the reconstructed one: ½g(h − hs)(h + hs).
+    // Where a depth has bits below the surface sums' last place, the own one is
+    // taken whole and the pressure of its rounding cancels against the flux's.
+    const int down = eL - eh + 2;
     const bool whole = (xa < xb ? xa : xb) >= xl - 7;
-    const int64_t ha = whole ? (int64_t)((uint64_t)la << down) : to_fixed(qa.h, xh + 2);
-    const int64_t hb = whole ? (int64_t)((uint64_t)lb << down) : to_fixed(qb.h, xh + 2);
-    const int64_t ga = (int64_t)((uint64_t)ra << down), gb = (int64_t)((uint64_t)rb << down);
-    auto back = [&](int64_t normal, double& x, double& y) {
-        const Lim fn = split(normal);
-        Acc a{half<2>(), 0}, o{0, 0}, b{half<2>(), 0};
+    auto back = [&](const Side& q, int64_t own, int64_t surface, double& x, double& y) {
+        const int64_t hq = whole ? shl(own, down) : to_fixed(q.h, xh + 1);
+        const int64_t gq = shl(surface, down);
+        const int64_t p = shr(mul<0>(split(mul<0>(split(hq - gq), split((hq >> 1) + (gq >> 1)))),
+                                     c.half_g),
+                              eQ - 2 * eh - c.e_half_g - 1);
+        const Lim fn = split(shl(f_n + p, 2));
+        Acc a{half<0>(), 0}, o{0, 0}, b{half<0>(), 0};
         mac(a, fn, m.x);
         mac(o, f_t, m.y);
         a.t -= o.t;
         a.r -= o.r;
         mac(b, fn, m.y);
         mac(b, f_t, m.x);
-        x = from_fixed(fold<2>(a), 58 - eQ - em);
-        y = from_fixed(fold<2>(b), 58 - eQ - em);
+        x = convert(fold<0>(a), 58 - eQ - em);
+        y = convert(fold<0>(b), 58 - eQ - em);
     };
-    back(f_n + pressure(ha - ga, ha + ga, eh), out.hu_a, out.hv_a);
-    back(f_n + pressure(hb - gb, hb + gb, eh), out.hu_b, out.hv_b);
+    back(qa, la, ra, out.hu_a, out.hv_a);
+    back(qb, lb, rb, out.hu_b, out.hv_b);
     return kDone;
 }
 

@@ -93,8 +93,8 @@ __device__ __noinline__ FacePair face_dry(Sd qa, Sd qb, const double* geo, doubl
 }
 
 // The flux of two sides along m = norm·(nx, ny): in fixed point, or the rest
-// (nf, mf: the two vectors as limbs, mf at 2^(61 − em); UNIT: both the unit
-// normal)
+// (nf, mf: the two vectors as limbs at 2^62 and 2^(62 − em); UNIT: both the
+// unit normal)
 template <bool UNIT>
 __device__ __forceinline__ FacePair face_pair(const DevTables& T, const Sd& qa, const Sd& qb,
                                               const FxPair& nf, const FxPair& mf, int em,
@@ -293,7 +293,8 @@ __device__ __forceinline__ double weather_level(const DevTables& T, const Physic
 // LISTED: a multirate pass's faces (lp's edge and boundary-face lists),
 // each boundary face at its element's stage time
 template <int N1, bool LISTED>
-__global__ void __launch_bounds__(256, DGSWE_FAST ? 3 : 2) face_kernel(DevTables T, Physics P, DevBuf in, double* fb_h,
+__global__ void __launch_bounds__(256, DGSWE_FAST ? 4 : 2)
+    face_kernel(DevTables T, Physics P, DevBuf in, double* fb_h,
                                                    double* fb_hu, double* fb_hv,
                                                    const StepCtl* ctl, int slot,
                                                    const int* active, LtsPass lp) {
@@ -743,8 +744,8 @@ __device__ __forceinline__ F3 general_rhs(const DevTables& T, const Physics& P,
             };
             const int em = max_expo(mx, my);
             const FacePair f =
-                face_pair<false>(T, qa, qb, pair(geo[3], geo[4], 1024), pair(mx, my, em + 2),
-                                 em - 1022, geo, g, sqrt_g, half_g, h_min);
+                face_pair<false>(T, qa, qb, pair(geo[3], geo[4], 1023), pair(mx, my, em + 2),
+                                 em - 1021, geo, g, sqrt_g, half_g, h_min);
 #else
             const FacePair f = face_hll(qa, qb, geo, g, sqrt_g, half_g, h_min);
 #endif
@@ -873,7 +874,7 @@ __global__ void fixed_normals_kernel(DevTables T, FxPair* normal) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= T.n_edges) return;
     const double* geo = &T.edge_geo[e * 5];
-    normal[e] = {fx::split(fx::to_fixed(geo[0], 1024)), fx::split(fx::to_fixed(geo[1], 1024))};
+    normal[e] = {fx::split(fx::to_fixed(geo[0], 1023)), fx::split(fx::to_fixed(geo[1], 1023))};
 }
 
 // The fixed-point tables of each element from its FP64 ones: a warp per

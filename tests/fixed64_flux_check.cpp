@@ -108,7 +108,7 @@ static long faces(std::mt19937_64& rng, Score& mass, Score& momentum) {
             if (i % 3 == 0) std::swap(a, b);
         }
         for (double* x : {&a.u, &a.v, &b.u, &b.v}) *x = speed * (U(rng) - 0.5);
-        const FxPair n{fx::split(fx::to_fixed(nx, 1024)), fx::split(fx::to_fixed(ny, 1024))};
+        const FxPair n{fx::split(fx::to_fixed(nx, 1023)), fx::split(fx::to_fixed(ny, 1023))};
         fx::FaceFlux f;
         if (fx::face_flux(a, b, n, n, 0, T.fx_face, kHMin, f) != fx::kDone) continue;
         ++done;
