@@ -119,6 +119,7 @@ struct dgswe_adjoint {
     // wet pass, forked from and joined to the target's stream
     cudaStream_t sub_stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
+    StageSide side;  // beside the forward's face and stage passes
 
     ~dgswe_adjoint() {
         if (h || ens) {
@@ -129,6 +130,7 @@ struct dgswe_adjoint {
             if (fork) cudaEventDestroy(fork);
             if (join) cudaEventDestroy(join);
             if (sub_stream) cudaStreamDestroy(sub_stream);
+            free_side(side);
         }
         if (h) dgswe_destroy(h);
         if (ens) dgswe_ensemble_destroy(ens);
@@ -265,10 +267,22 @@ void forward_step(dgswe_adjoint* a, const DevBuf& q) {
     const DevBuf* ins[3] = {&q, &a->S[1], &a->S[2]};
     const DevBuf* outs[3] = {&a->S[1], &a->S[2], &q};
     for (int s = 0; s < 3; ++s) {
-        t.ks->face(t.n1, *t.T, *t.P, *ins[s], t.fb_h, t.fb_hu, t.fb_hv, t.ctl, s, on, t.stream);
-        t.ks->stage(t.n1, *t.T, *t.P, *t.X, *ins[s], q, *outs[s], q, t.fb_h, t.fb_hu, t.fb_hv,
-                    t.ctl, s, kModePost, s == 2, on, t.stream);
+        t.ks->face_beside(t.n1, *t.T, *t.P, *ins[s], t.fb_h, t.fb_hu, t.fb_hv, t.ctl, s, on,
+                          t.stream, a->side);
+        t.ks->stage_beside(t.n1, *t.T, *t.P, *t.X, *ins[s], q, *outs[s], q, t.fb_h, t.fb_hu,
+                           t.fb_hv, t.ctl, s, kModePost, s == 2, on, DevBuf{}, t.stream, a->side);
     }
+}
+
+// One stage of a step with what its reverse needs kept
+void keep_stage(dgswe_adjoint* a, const DevBuf& in, const DevBuf& base, const DevBuf& out, int s,
+                const DevBuf& keep) {
+    const Target& t = a->tg;
+    const int* on = &t.ctl[0].always;
+    t.ks->face_beside(t.n1, *t.T, *t.P, in, t.fb_h, t.fb_hu, t.fb_hv, t.ctl, s, on, t.stream,
+                      a->side);
+    t.ks->stage_beside(t.n1, *t.T, *t.P, *t.X, in, base, out, base, t.fb_h, t.fb_hu, t.fb_hv,
+                       t.ctl, s, kModePost, 0, on, keep, t.stream, a->side);
 }
 
 // The three stages of a step reversed, the stage inputs in[0..2] and what
@@ -344,6 +358,7 @@ int setup(dgswe_adjoint* a, const dgswe_form* forms, const dgswe_adjoint_config*
     int least = 0, greatest = 0;
     ACK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     ACK(cudaStreamCreateWithPriority(&a->sub_stream, cudaStreamNonBlocking, greatest));
+    ACK(make_side(a->side));
     const int64_t nf = t.K * 4 * n1;
     // the bed slope's transpose: for node c, each line partner i's
     // ∂(g∇B)_i/∂B_c = g·D[pos_i][pos_c]·w(i, c), with w the forward's metric
@@ -803,10 +818,7 @@ int dgswe_adjoint_reverse(dgswe_adjoint* a, double* grad_h0, double* grad_hu0, d
                 // output's node velocities beside it
                 const DevBuf out[3] = {in[1], in[2], n + 1 < c1 ? view(n + 1, c0, 0) : a->S[3]};
                 for (int s = 0; s < 3; ++s) {
-                    t.ks->face(t.n1, *t.T, *t.P, in[s], t.fb_h, t.fb_hu, t.fb_hv, t.ctl, s, on,
-                               st);
-                    t.ks->stage_keep(t.n1, *t.T, *t.P, *t.X, in[s], in[0], out[s], t.fb_h, t.fb_hu,
-                                     t.fb_hv, t.ctl, s, 0, keep_view(n, c0, s), st);
+                    keep_stage(a, in[s], in[0], out[s], s, keep_view(n, c0, s));
                 }
                 recomputed += 1;
             }
@@ -845,9 +857,7 @@ int dgswe_adjoint_reverse(dgswe_adjoint* a, double* grad_h0, double* grad_hu0, d
             t.ks->velocity(q, nv, t.P->h_min, st);
             if (int s = args_to_ctl(a, n)) return s;
             for (int s = 0; s < 3; ++s) {
-                t.ks->face(t.n1, *t.T, *t.P, a->S[s], t.fb_h, t.fb_hu, t.fb_hv, t.ctl, s, on, st);
-                t.ks->stage_keep(t.n1, *t.T, *t.P, *t.X, a->S[s], q, a->S[s + 1], t.fb_h, t.fb_hu,
-                                 t.fb_hv, t.ctl, s, 0, a->Kp[s], st);
+                keep_stage(a, a->S[s], q, a->S[s + 1], s, a->Kp[s]);
             }
             if (int s = reverse_stages(a, a->S, a->Kp)) return s;
             recomputed += 1;

@@ -159,8 +159,8 @@ int dt_beside_first_face(dgswe_handle* h, const DtParams& D, const int* active) 
               h->dt_stream);
     h->ks->step_dt(h->ctl, 1, h->dt_stream);
     CK(cudaEventRecord(h->dt_join, h->dt_stream));
-    h->ks->face(h->n1, h->T, h->P, h->buf[DGSWE_STATE].view, h->fb_h, h->fb_hu, h->fb_hv, h->ctl,
-                0, active, h->stream);
+    h->ks->face_beside(h->n1, h->T, h->P, h->buf[DGSWE_STATE].view, h->fb_h, h->fb_hu, h->fb_hv,
+                       h->ctl, 0, active, h->stream, h->side);
     CK(cudaStreamWaitEvent(h->stream, h->dt_join, 0));
     return DGSWE_OK;
 }
@@ -177,6 +177,7 @@ int run_device_step_graph(dgswe_handle* h, int scheme, double cfl) {
         if (int s = ensure_buffer(h, b)) return s;
     const DtParams D = dt_params(h->form, cfl, scheme);
     if (int s = ensure_dt_stream(h)) return s;
+    CK(make_side(h->side));
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     const int* active = &h->ctl->active;
@@ -189,12 +190,13 @@ int run_device_step_graph(dgswe_handle* h, int scheme, double cfl) {
     for (int s = 0; s < n; ++s) {
         const int in = s == 0 ? DGSWE_STATE : s;
         const int out = s + 1 < n ? s + 1 : DGSWE_STATE;
-        if (s == 0)  // its face pass ran beside the dt pass
-            h->ks->stage(h->n1, h->T, h->P, h->X, h->buf[in].view, h->buf[DGSWE_STATE].view,
-                         h->buf[out].view, h->buf[DGSWE_STATE].view, h->fb_h, h->fb_hu, h->fb_hv,
-                         h->ctl, s, kModePost, s + 1 == n, active, h->stream);
-        else
-            launch_stage(h, in, DGSWE_STATE, out, DGSWE_STATE, s, kModePost, s + 1 == n, active);
+        const DevBuf& q = h->buf[DGSWE_STATE].view;
+        if (s > 0)  // the first face pass ran beside the dt pass
+            h->ks->face_beside(h->n1, h->T, h->P, h->buf[in].view, h->fb_h, h->fb_hu, h->fb_hv,
+                               h->ctl, s, active, h->stream, h->side);
+        h->ks->stage_beside(h->n1, h->T, h->P, h->X, h->buf[in].view, q, h->buf[out].view, q,
+                            h->fb_h, h->fb_hu, h->fb_hv, h->ctl, s, kModePost, s + 1 == n, active,
+                            DevBuf{}, h->stream, h->side);
     }
     h->ks->step_end(h->ctl, 1, h->stream);
     cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
@@ -620,14 +622,14 @@ int create_impl(dgswe_handle* h, const dgswe_form* f, int device) {
         FxPair* normal = nullptr;
         if ((s = device_array(h, nh, &hm)) || (s = device_array(h, (size_t)h->n_values, &gdb)) ||
             (s = device_array(h, nl, &lift)) || (s = device_array(h, (size_t)h->K, &exps)) ||
-            (s = device_array(h, (size_t)h->K, &T.gen_list)) ||
-            (s = device_array(h, 2, &T.gen_count)) ||
+            (s = device_array(h, 2 * (size_t)h->K, &T.gen_list)) ||
+            (s = device_array(h, 4, &T.gen_count)) ||
             (s = device_array(h, (size_t)T.n_edges, &normal)))
             return bail(s);
         h->ks->fixed_tables(h->n1, T, hm, gdb, lift, exps, normal, nullptr);
         CK(cudaGetLastError());
         if (!usable) CK(cudaMemsetAsync(exps, 0, (size_t)h->K * sizeof(FxExp), nullptr));
-        CK(cudaMemsetAsync(T.gen_count, 0, 2 * sizeof(unsigned), nullptr));
+        CK(cudaMemsetAsync(T.gen_count, 0, 4 * sizeof(unsigned), nullptr));
         T.fx_hm = hm;
         T.fx_gdb = gdb;
         T.fx_lift = lift;

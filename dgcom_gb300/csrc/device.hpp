@@ -72,10 +72,11 @@ struct DevTables {
     const FxLimb* fx_coef = nullptr;  // [nn][2(n1−1)]
     const FxNode* fx_node = nullptr;  // [nn]
     const FxPair* fx_normal = nullptr;  // [E] the edges' unit normals at 2^62
-    // the elements a stage leaves to general_kernel, and {their number, the
-    // blocks that have ended}; empty between stages
-    int32_t* gen_list = nullptr;     // [K]
-    unsigned* gen_count = nullptr;   // [2]
+    // the elements a stage leaves to general_kernel, in two lists (those with
+    // subcells, listed beforehand; what the stage kernel finds), and of each
+    // {its length, the blocks that have ended}: empty between stages
+    int32_t* gen_list = nullptr;     // [2][K]
+    unsigned* gen_count = nullptr;   // [2][2]
     FxLimb fx_two_g{};
     FxFaceConstants fx_face{};
     int fx_ec = 0, fx_e2g = 0;

@@ -227,14 +227,14 @@ int build_group(dgswe_ensemble* h, Group& G, std::vector<Tables>& tabs,
             (s = device_array(h, (size_t)G.n_values, &gdb)) ||
             (s = device_array(h, (size_t)G.K * 4 * n1, &lift)) ||
             (s = device_array(h, (size_t)G.K, &exps)) ||
-            (s = device_array(h, (size_t)G.K, &T.gen_list)) ||
-            (s = device_array(h, 2, &T.gen_count)) ||
+            (s = device_array(h, 2 * (size_t)G.K, &T.gen_list)) ||
+            (s = device_array(h, 4, &T.gen_count)) ||
             (s = device_array(h, (size_t)T.n_edges, &normal)))
             return s;
         h->ks->fixed_tables(n1, T, hm, gdb, lift, exps, normal, nullptr);
         CK(cudaGetLastError());
         if (!usable) CK(cudaMemsetAsync(exps, 0, (size_t)G.K * sizeof(FxExp), nullptr));
-        CK(cudaMemsetAsync(T.gen_count, 0, 2 * sizeof(unsigned), nullptr));
+        CK(cudaMemsetAsync(T.gen_count, 0, 4 * sizeof(unsigned), nullptr));
         T.fx_hm = hm;
         T.fx_gdb = gdb;
         T.fx_lift = lift;
@@ -413,6 +413,7 @@ int step_graph(dgswe_ensemble* h, int scheme, double cfl) {
     const int n = scheme_table(scheme, st);
     const int* on = h->always;
     cudaStream_t main = h->stream;
+    for (Group& G : h->groups) CK(make_side(G.beside));
     auto stream_of = [&](size_t g) { return g % 2 == 0 ? main : h->side; };
     auto fork = [&]() -> cudaError_t {
         cudaError_t e = cudaEventRecord(h->fork, main);
@@ -443,10 +444,11 @@ int step_graph(dgswe_ensemble* h, int scheme, double cfl) {
         for (size_t g = 0; g < h->groups.size(); ++g) {
             Group& G = h->groups[g];
             cudaStream_t sg = stream_of(g);
-            h->ks->face(G.n1, G.T, G.P, G.buf[in], G.fb_h, G.fb_hu, G.fb_hv, h->ctl, s, on, sg);
-            h->ks->stage(G.n1, G.T, G.P, G.X, G.buf[in], G.buf[DGSWE_STATE], G.buf[out],
-                         G.buf[DGSWE_STATE], G.fb_h, G.fb_hu, G.fb_hv, h->ctl, s, kModePost,
-                         s + 1 == n, on, sg);
+            h->ks->face_beside(G.n1, G.T, G.P, G.buf[in], G.fb_h, G.fb_hu, G.fb_hv, h->ctl, s, on,
+                               sg, G.beside);
+            h->ks->stage_beside(G.n1, G.T, G.P, G.X, G.buf[in], G.buf[DGSWE_STATE], G.buf[out],
+                                G.buf[DGSWE_STATE], G.fb_h, G.fb_hu, G.fb_hv, h->ctl, s, kModePost,
+                                s + 1 == n, on, DevBuf{}, sg, G.beside);
         }
         if (e == cudaSuccess) e = join();
     }
@@ -457,7 +459,8 @@ int step_graph(dgswe_ensemble* h, int scheme, double cfl) {
         return fail(h, DGSWE_ERR_CUDA, "stream capture: %s",
                     cudaGetErrorString(e != cudaSuccess ? e : e2));
     }
-    e = cudaGraphInstantiate(&h->graph, graph, 0);
+    // the kernel nodes keep the priority of the stream they were captured on
+    e = cudaGraphInstantiate(&h->graph, graph, cudaGraphInstantiateFlagUseNodePriority);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return fail(h, DGSWE_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
     h->graph_scheme = scheme;

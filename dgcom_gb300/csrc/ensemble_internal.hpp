@@ -28,6 +28,7 @@ struct Group {
     DevBuf buf[kEnsBuffers]{};
     double *fb_h = nullptr, *fb_hu = nullptr, *fb_hv = nullptr;
     std::vector<int> members;
+    StageSide beside;  // its stages' side stream (created on first use)
 };
 
 struct Member {
@@ -69,7 +70,10 @@ struct dgswe_ensemble {
             if (e) cudaEventDestroy(e);
         if (side) cudaStreamDestroy(side);
         if (stream) cudaStreamDestroy(stream);
-        for (Group& g : groups) delete g.ops;
+        for (Group& g : groups) {
+            dgswe::free_side(g.beside);
+            delete g.ops;
+        }
     }
 };
 

@@ -115,6 +115,7 @@ struct dgswe_handle {
     // fork and join between them (created on first use)
     cudaStream_t dt_stream = nullptr;
     cudaEvent_t dt_fork = nullptr, dt_join = nullptr;
+    dgswe::StageSide side;  // beside a step's face and stage passes (created on first use)
 
     ~dgswe_handle() {
         for (cudaEvent_t e : chunk_done)
@@ -123,6 +124,7 @@ struct dgswe_handle {
         for (cudaEvent_t e : {dt_fork, dt_join})
             if (e) cudaEventDestroy(e);
         if (dt_stream) cudaStreamDestroy(dt_stream);
+        dgswe::free_side(side);
         delete planner;
         if (dplan.host) cudaFreeHost(dplan.host);
         for (cudaEvent_t e : ev_lts)

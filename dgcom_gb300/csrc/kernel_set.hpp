@@ -8,6 +8,32 @@
 
 namespace dgswe {
 
+// A stream beside a pass's own, of a higher priority, and the events that
+// order the two
+struct StageSide {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, sources = nullptr, ready = nullptr, done = nullptr;
+};
+
+// A side stream with the highest priority, so that its few long blocks start
+// before the pass beside it fills the multiprocessors, and its events
+inline cudaError_t make_side(StageSide& side) {
+    if (side.stream) return cudaSuccess;
+    int least = 0, greatest = 0;
+    cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    for (cudaEvent_t* ev : {&side.fork, &side.sources, &side.ready, &side.done})
+        if (e == cudaSuccess && !*ev) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&side.stream, cudaStreamNonBlocking, greatest);
+    return e;
+}
+
+inline void free_side(StageSide& side) {
+    for (cudaEvent_t ev : {side.fork, side.sources, side.ready, side.done})
+        if (ev) cudaEventDestroy(ev);
+    if (side.stream) cudaStreamDestroy(side.stream);
+    side = StageSide{};
+}
+
 struct KernelSet {
     void (*face)(int n1, const DevTables&, const Physics&, const DevBuf& in, double* fh,
                  double* fhu, double* fhv, const StepCtl* ctl, int slot, const int* active,
@@ -21,12 +47,6 @@ struct KernelSet {
     void (*dt)(int n1, const DevTables&, const Physics&, const DevBuf& q, const DtParams&,
                double* dt_el, StepCtl* ctl, const int* active, cudaStream_t);
     void (*velocity)(const DevBuf&, int64_t n, double h_min, cudaStream_t);
-    // a kPost stage that also keeps the combination and the damped momentum
-    // (the adjoint's recomputation)
-    void (*stage_keep)(int n1, const DevTables&, const Physics&, const StageExtra&,
-                       const DevBuf& in, const DevBuf& base, const DevBuf& out, const double* fh,
-                       const double* fhu, const double* fhv, StepCtl* ctl, int slot,
-                       int check_finite, const DevBuf& keep, cudaStream_t);
     // the adjoint of one stage (adjoint_kernels.cuh): the wet elements'
     // pass (`subcells` 0) or the listed subcell elements' (1)
     void (*stage_adjoint)(int n1, const DevTables&, const Physics&, const StageExtra&,
@@ -88,6 +108,19 @@ struct KernelSet {
     void (*fixed_tables)(int n1, const DevTables&, FxPair* hm, FxPair* gdb, FxLimb* lift,
                          FxExp* exps, FxPair* normal, cudaStream_t);
     bool has_fixed;
+    // face and stage as above, for a pass over the whole mesh, one after the
+    // other: the node sources and the list of the elements with subcells run
+    // on the side stream beside the face pass, those elements' stage there
+    // beside the others'. `keep` (null: not) takes the combination and the
+    // damped momentum (the adjoint's recomputation)
+    void (*face_beside)(int n1, const DevTables&, const Physics&, const DevBuf& in, double* fh,
+                        double* fhu, double* fhv, const StepCtl* ctl, int slot, const int* active,
+                        cudaStream_t, const StageSide&);
+    void (*stage_beside)(int n1, const DevTables&, const Physics&, const StageExtra&,
+                         const DevBuf& in, const DevBuf& base, const DevBuf& out,
+                         const DevBuf& acc, const double* fh, const double* fhu,
+                         const double* fhv, StepCtl* ctl, int slot, int mode, int check_finite,
+                         const int* active, const DevBuf& keep, cudaStream_t, const StageSide&);
     // the subcell interfaces' metrics (DevTables::sub_metric)
     void (*sub_metrics)(int n1, const DevTables&, const Physics&, double* out, cudaStream_t);
 };

@@ -1097,7 +1097,9 @@ __device__ __forceinline__ void finish_node(const DevTables& T, const Physics& P
 // node, which only their faces' fluxes reach (their reconstructed subcell
 // faces are dry, so the interface fluxes, pressure and bed terms are all ±0).
 // Any other with subcells, and one whose depths or exponents spread too far,
-// goes into T.gen_list for general_kernel, launched behind: inside this kernel its few hundred FP64
+// goes into T.gen_list's second half for general_kernel, launched behind
+// (shallow_listed: those with subcells are in its first half already, and a
+// general_kernel takes them beside this kernel): inside this kernel its few hundred FP64
 // operations in a row (a call, so spills on the wet path; one busy warp to a
 // block's end) cost 17 % of a 50,000-quad coastal box's stage.
 // LISTED: a multirate pass over lp's elements, each with its own stage
@@ -1106,7 +1108,8 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
     stage_kernel(DevTables T, Physics P, StageExtra X, DevBuf in, DevBuf base, DevBuf out,
                  DevBuf acc, const double* __restrict__ fb_h, const double* __restrict__ fb_hu,
                  const double* __restrict__ fb_hv, StepCtl* ctl, int slot, int mode,
-                 int check_finite, const int* active, DevBuf keep, LtsPass lp) {
+                 int check_finite, const int* active, DevBuf keep, LtsPass lp,
+                 int shallow_listed) {
     using C = Cfg<N1, SHAPE>;
     constexpr int NN = C::NN, NP = C::NP, NA = C::NA, EPB = C::EPB;
     // an element whose lanes share a warp finds its flags and largest
@@ -1201,7 +1204,8 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
         sc = fx::scales(exponents(ew), T.fx_exp[k], T.fx_ec, T.fx_e2g);
         fixed = sc.ok;
     }
-    if (valid && !fixed && !dry && i == 0) T.gen_list[atomicAdd(&T.gen_count[0], 1u)] = (int32_t)k;
+    if (valid && !fixed && !dry && i == 0 && !(sub && shallow_listed))
+        T.gen_list[T.K + atomicAdd(&T.gen_count[2], 1u)] = (int32_t)k;
 
     FxLimb G{}, H{};                         // 2g·h, h
     int64_t m0 = 0, m1 = 0, u0 = 0, u1 = 0;  // hu, hv, u, v
@@ -1293,17 +1297,44 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
                                 i, fixed || dry, F, s_q, &s_flag[e][2], s_red[e]);
 }
 
-// The elements of a stage that stage_kernel left (T.gen_list): those with
-// subcells, and wet ones whose scales spread too far. Few and long (some 200
-// FP64 operations in a row), so two lanes a node, a subcell direction each.
-// The last block to end empties the list for the next stage.
+// A stage's elements with subcells and water, from its input, into T.gen_list's
+// first half: beside the face pass, so that general_kernel can take them
+// beside the stage pass
+template <int N1>
+__global__ void __launch_bounds__(256)
+    shallow_list_kernel(DevTables T, Physics P, DevBuf in, const StepCtl* ctl,
+                        const int* active) {
+    constexpr int NN = N1 * N1, EPB = 256 / NN;
+    __shared__ int s_flag[EPB][2];
+    if (!*active) return;
+    const int e = threadIdx.x / NN, i = threadIdx.x % NN;
+    const int64_t k = (int64_t)blockIdx.x * EPB + e;
+    const bool valid = e < EPB && k < T.K && (!T.elem_member || ctl[T.elem_member[k]].active);
+    const double h = valid ? in.h[k * NN + i] : 0.0;
+    if (e < EPB && i < 2) s_flag[e][i] = 0;
+    __syncthreads();
+    if (valid && fp::lt(h, P.subcell_depth)) {
+        atomicOr(&s_flag[e][0], 1);
+        if (!fp::nz(h)) atomicAdd(&s_flag[e][1], 1);
+    }
+    __syncthreads();
+    if (valid && i == 0 && s_flag[e][0] && s_flag[e][1] != NN)
+        T.gen_list[atomicAdd(&T.gen_count[0], 1u)] = (int32_t)k;
+}
+
+// The elements of a stage that stage_kernel leaves (a half of T.gen_list):
+// those with subcells, and wet ones whose scales spread too far. Few and long
+// (some 200 FP64 operations in a row, 20 µs for any number of them), so two
+// lanes a node, a subcell direction each. The last block to end empties the
+// list for the next stage.
 template <int N1, bool LISTED>
 __global__ void __launch_bounds__(GenCfg<N1>::THREADS, 4)
     general_kernel(const __grid_constant__ DevTables T, const __grid_constant__ Physics P,
                    const __grid_constant__ StageExtra X, const __grid_constant__ DevBuf in,
                    DevBuf base, DevBuf out, DevBuf acc, const double* __restrict__ fb_h,
                    const double* __restrict__ fb_hu, const double* __restrict__ fb_hv, StepCtl* ctl,
-                   int slot, int mode, int check_finite, DevBuf keep, LtsPass lp) {
+                   int slot, int mode, int check_finite, const int* active, DevBuf keep,
+                   LtsPass lp, int list) {
     constexpr int NN = N1 * N1, LANES = 2 * NN, EPB = GenCfg<N1>::EPB;
     using C = Cfg<N1>;
     __shared__ double s_x[EPB][C::X];
@@ -1312,11 +1343,14 @@ __global__ void __launch_bounds__(GenCfg<N1>::THREADS, 4)
     const int tid = threadIdx.x;
     const int e = tid / LANES, lane = tid % LANES, half = lane / NN, i = lane % NN;
     double(*const s_q)[NN] = (double(*)[NN])s_x[e];
-    const unsigned n = *(volatile unsigned*)&T.gen_count[0];
+    const int32_t* elements = T.gen_list + list * T.K;
+    unsigned* const count = T.gen_count + 2 * list;
+    const unsigned n = *active ? *(volatile unsigned*)count : 0u;
     for (unsigned first = blockIdx.x * EPB; first < n; first += gridDim.x * EPB) {
-        const bool take = first + e < n;
-        const int64_t k = take ? (int64_t)T.gen_list[first + e] : 0;
-        StepCtl* const cm = ctl + ((T.elem_member && take) ? T.elem_member[k] : 0);
+        const bool listed = first + e < n;
+        const int64_t k = listed ? (int64_t)elements[first + e] : 0;
+        StepCtl* const cm = ctl + ((T.elem_member && listed) ? T.elem_member[k] : 0);
+        const bool take = listed && (!T.elem_member || cm->active);
         const int64_t gi = k * NN + i;
         double h = 0.0;
         if (take && half == 0) {
@@ -1347,9 +1381,9 @@ __global__ void __launch_bounds__(GenCfg<N1>::THREADS, 4)
         element_sync<LANES>();
     }
     __syncthreads();
-    if (tid == 0 && atomicAdd(&T.gen_count[1], 1u) == gridDim.x - 1) {
-        T.gen_count[0] = 0;
-        T.gen_count[1] = 0;
+    if (tid == 0 && atomicAdd(&count[1], 1u) == gridDim.x - 1) {
+        count[0] = 0;
+        count[1] = 0;
     }
 }
 #else

@@ -25,8 +25,23 @@ static void relax(const DevTables& T, const Physics& P, const DevBuf& in, const 
 
 template <int N1>
 static void face_n(const DevTables& T, const Physics& P, const DevBuf& in, double* fh, double* fhu,
-                   double* fhv, const StepCtl* ctl, int slot, const int* active, cudaStream_t s) {
-    relax<false>(T, P, in, ctl, slot, LtsPass{}, s);
+                   double* fhv, const StepCtl* ctl, int slot, const int* active, cudaStream_t s,
+                   const StageSide* side = nullptr) {
+    if (!side) relax<false>(T, P, in, ctl, slot, LtsPass{}, s);
+#if DGSWE_FAST
+    if (side) {
+        cudaEventRecord(side->fork, s);
+        cudaStreamWaitEvent(side->stream, side->fork, 0);
+        if (T.rx_src) {
+            relax<false>(T, P, in, ctl, slot, LtsPass{}, side->stream);
+            cudaEventRecord(side->sources, side->stream);
+        }
+        constexpr int EPB = 256 / (N1 * N1);
+        if (P.formulation == kWetDry)
+            shallow_list_kernel<N1><<<(unsigned)((T.K + EPB - 1) / EPB), 256, 0, side->stream>>>(
+                T, P, in, ctl, active);
+    }
+#endif
     const int64_t items = (T.n_edges + T.n_bfaces) * N1;
     if (items == 0) return;
     const int threads = P.face_threads > 0 && P.face_threads <= 256 ? P.face_threads : 256;
@@ -62,31 +77,52 @@ template <int N1>
 static void stage_n(const DevTables& T, const Physics& P, const StageExtra& X, const DevBuf& in,
                     const DevBuf& base, const DevBuf& out, const DevBuf& acc, const double* fh,
                     const double* fhu, const double* fhv, StepCtl* ctl, int slot, int mode,
-                    int check_finite, const int* active, const DevBuf& keep, cudaStream_t s) {
+                    int check_finite, const int* active, const DevBuf& keep, cudaStream_t s,
+                    const StageSide* side = nullptr) {
     // the pass's elements: all, or the chunk [k_first, k_last) of X
     const int64_t k1 = X.k_last < T.K ? X.k_last : T.K;
     const int64_t count = k1 - X.k_first;
     if (count <= 0) return;
+#if DGSWE_FAST
+    auto general = [&](int list, cudaStream_t on) {
+        general_kernel<N1, false><<<general_blocks<N1>(count), GenCfg<N1>::THREADS, 0, on>>>(
+            T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, slot, mode, check_finite, active, keep,
+            LtsPass{}, list);
+    };
+    const int listed = side != nullptr;
+    if (side) {
+        cudaEventRecord(side->ready, s);
+        cudaStreamWaitEvent(side->stream, side->ready, 0);
+        if (T.rx_src) cudaStreamWaitEvent(s, side->sources, 0);
+        general(0, side->stream);
+        cudaEventRecord(side->done, side->stream);
+    }
+#define DGSWE_LISTED , listed
+#else
+    (void)side;
+#define DGSWE_LISTED
+#endif
     auto blocks = [&](int epb) { return (unsigned)((count + epb - 1) / epb); };
     if (P.stage_shape == 1) {
         using C1 = Cfg<N1, 1>;
         stage_kernel<N1, false, 1><<<blocks(C1::EPB), C1::THREADS, 0, s>>>(
             T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, slot, mode, check_finite, active, keep,
-            LtsPass{});
+            LtsPass{} DGSWE_LISTED);
     } else if (P.stage_shape == 2) {
         using C2 = Cfg<N1, 2>;
         stage_kernel<N1, false, 2><<<blocks(C2::EPB), C2::THREADS, 0, s>>>(
             T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, slot, mode, check_finite, active, keep,
-            LtsPass{});
+            LtsPass{} DGSWE_LISTED);
     } else {
         using C = Cfg<N1>;
         stage_kernel<N1, false><<<blocks(C::EPB), C::THREADS, 0, s>>>(
             T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, slot, mode, check_finite, active, keep,
-            LtsPass{});
+            LtsPass{} DGSWE_LISTED);
     }
+#undef DGSWE_LISTED
 #if DGSWE_FAST
-    general_kernel<N1, false><<<general_blocks<N1>(count), GenCfg<N1>::THREADS, 0, s>>>(
-        T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, slot, mode, check_finite, keep, LtsPass{});
+    if (side) cudaStreamWaitEvent(s, side->done, 0);
+    general(1, s);
 #endif
 }
 
@@ -101,10 +137,13 @@ static void stage_listed_n(const DevTables& T, const Physics& P, const StageExtr
     const unsigned blocks = (unsigned)((lp.n + C::EPB - 1) / C::EPB);
     stage_kernel<N1, true><<<blocks, C::THREADS, 0, s>>>(T, P, X, in, base, out, acc, fh, fhu, fhv,
                                                          ctl, 0, mode, 0, &ctl->always, DevBuf{},
-                                                         lp);
+                                                         lp
 #if DGSWE_FAST
+                                                         , 0);
     general_kernel<N1, true><<<general_blocks<N1>(lp.n), GenCfg<N1>::THREADS, 0, s>>>(
-        T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, 0, mode, 0, DevBuf{}, lp);
+        T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, 0, mode, 0, &ctl->always, DevBuf{}, lp, 1);
+#else
+    );
 #endif
 }
 
@@ -220,12 +259,21 @@ static void stage(int n1, const DevTables& T, const Physics& P, const StageExtra
                    check_finite, active, DevBuf{}, s);
 }
 
-static void stage_keep(int n1, const DevTables& T, const Physics& P, const StageExtra& X,
-                       const DevBuf& in, const DevBuf& base, const DevBuf& out, const double* fh,
-                       const double* fhu, const double* fhv, StepCtl* ctl, int slot,
-                       int check_finite, const DevBuf& keep, cudaStream_t s) {
-    DGSWE_BY_ORDER(stage_n, T, P, X, in, base, out, base, fh, fhu, fhv, ctl, slot, kPost,
-                   check_finite, &ctl->always, keep, s);
+static void face_beside(int n1, const DevTables& T, const Physics& P, const DevBuf& in, double* fh,
+                        double* fhu, double* fhv, const StepCtl* ctl, int slot, const int* active,
+                        cudaStream_t s, const StageSide& side) {
+    DGSWE_BY_ORDER(face_n, T, P, in, fh, fhu, fhv, ctl, slot, active, s,
+                   DGSWE_FAST ? &side : nullptr);
+}
+
+static void stage_beside(int n1, const DevTables& T, const Physics& P, const StageExtra& X,
+                         const DevBuf& in, const DevBuf& base, const DevBuf& out,
+                         const DevBuf& acc, const double* fh, const double* fhu,
+                         const double* fhv, StepCtl* ctl, int slot, int mode, int check_finite,
+                         const int* active, const DevBuf& keep, cudaStream_t s,
+                         const StageSide& side) {
+    DGSWE_BY_ORDER(stage_n, T, P, X, in, base, out, acc, fh, fhu, fhv, ctl, slot, mode,
+                   check_finite, active, keep, s, DGSWE_FAST ? &side : nullptr);
 }
 
 static void finish(int n1, const DevTables& T, const Physics& P, const DevBuf& acc,
@@ -369,12 +417,12 @@ static void end(StepCtl* c, int n, cudaStream_t s) {
 }
 
 static const KernelSet kSet = {face,          stage,         finish,          dt,
-                                velocity,      stage_keep,    stage_adjoint,   face_adjoint,
+                                velocity,      stage_adjoint,   face_adjoint,
                                 adjoint_combine, station_eval, station_seed,   begin,
                                 dt_fit,        end,           face_listed,     stage_listed,
                                 finish_listed, depth_flags,    subcell_list,
                                 implicit_damping, face_ready,  node_sources,
-                                dt_listed,     fixed_tables,  DGSWE_FAST,
+                                dt_listed,     fixed_tables,  DGSWE_FAST,     face_beside,   stage_beside,
                                 sub_metrics};
 
 }  // namespace DGSWE_NS
