@@ -1015,11 +1015,22 @@ int dgswe_step(dgswe_handle* h, int32_t scheme, double t, double dt) {
 
 namespace {
 
+// dgswe_step_host's element chunks: as many as keep each at 8 MiB of state or
+// more, up to kHostChunks. A chunk costs some 100 µs of calls (copies of
+// pageable memory come back when they are done), 8 MiB about 80 µs of copies:
+// a step of 60,000 quads at N = 3 in pageable memory takes 1.24 ms with chunks
+// of 2 MiB, 1.00 with 4, 0.85 with 8; one of 320 quads at N = 2 0.97 ms in
+// eight chunks, 0.26 in one.
+int host_chunks(const dgswe_handle* h) {
+    const int64_t fit = 3 * h->n_values * (int64_t)sizeof(double) / (8 << 20);
+    return (int)std::max<int64_t>(1, std::min<int64_t>(kHostChunks, fit));
+}
+
 // The ready lists of dgswe_step_host's upload chunks (ready_lists,
 // host_common.hpp), on the device
 int build_ready_lists(dgswe_handle* h) {
     if (h->ready_built) return DGSWE_OK;
-    const ReadyLists r = ready_lists(h->K, kHostChunks, h->nb, h->h_edge_left, h->h_edge_right,
+    const ReadyLists r = ready_lists(h->K, host_chunks(h), h->nb, h->h_edge_left, h->h_edge_right,
                                      h->h_bface);
     std::copy(r.elem_off.begin(), r.elem_off.end(), h->ready_elem_off);
     std::copy(r.edge_off.begin(), r.edge_off.end(), h->ready_edge_off);
@@ -1087,11 +1098,12 @@ int dgswe_step_host(dgswe_handle* h, int32_t scheme, double t, double cfl, doubl
     const DevBuf& q = h->buf[DGSWE_STATE].view;
     const int* active = &h->ctl->active;
     const DtParams D = dt_params(h->form, cfl, scheme);
-    const int64_t per = (h->K + kHostChunks - 1) / kHostChunks;
+    const int chunks = host_chunks(h);
+    const int64_t per = (h->K + chunks - 1) / chunks;
     h->ks->step_begin(h->ctl, 1, h->stream);  // the dt reset, the first stage's time
     CK(cudaEventRecord(h->chunk_done[0], h->stream));  // after the work queued before
     CK(cudaStreamWaitEvent(h->copy_stream, h->chunk_done[0], 0));
-    for (int c = 0; c < kHostChunks; ++c) {
+    for (int c = 0; c < chunks; ++c) {
         const int64_t k0 = std::min<int64_t>(h->K, c * per), k1 = std::min<int64_t>(h->K, k0 + per);
         if (k1 > k0) {
             const size_t off = (size_t)k0 * h->nn, cnt = (size_t)(k1 - k0) * h->nn;
@@ -1124,29 +1136,34 @@ int dgswe_step_host(dgswe_handle* h, int32_t scheme, double t, double cfl, doubl
         else
             launch_stage(h, in, DGSWE_STATE, s + 1, DGSWE_STATE, s, kModePost, 0, active);
     }
-    // the last stage in element chunks, each copied back while the next runs
+    // the last stage in element chunks, each copied back while the next runs;
+    // every launch comes before the first copy, since a copy into pageable
+    // memory holds the host until it is done
     const int last = n_st - 1;
     const DevBuf& in = h->buf[last].view;
     h->ks->face(h->n1, h->T, h->P, in, h->fb_h, h->fb_hu, h->fb_hv, h->ctl, last, active,
                 h->stream);
-    for (int c = 0; c < kHostChunks; ++c) {
-        const int64_t k0 = c * per, k1 = std::min<int64_t>(h->K, k0 + per);
-        if (k1 <= k0) break;
+    for (int c = 0; c < chunks; ++c) {
         StageExtra X = h->X;
-        X.k_first = k0;
-        X.k_last = k1;
+        X.k_first = std::min<int64_t>(h->K, c * per);
+        X.k_last = std::min<int64_t>(h->K, X.k_first + per);
+        if (X.k_last <= X.k_first) break;
         h->ks->stage(h->n1, h->T, h->P, X, in, q, q, q, h->fb_h, h->fb_hu, h->fb_hv, h->ctl, last,
                      kModePost, 1, active, h->stream);
         CK(cudaEventRecord(h->chunk_done[c], h->stream));
+    }
+    h->ks->step_end(h->ctl, 1, h->stream);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(h->h_ctl, h->ctl, sizeof(StepCtl), cudaMemcpyDeviceToHost, h->stream));
+    for (int c = 0; c < chunks; ++c) {
+        const int64_t k0 = c * per, k1 = std::min<int64_t>(h->K, k0 + per);
+        if (k1 <= k0) break;
         CK(cudaStreamWaitEvent(h->copy_stream, h->chunk_done[c], 0));
         const size_t off = (size_t)k0 * h->nn, len = (size_t)(k1 - k0) * h->nn * sizeof(double);
         CK(cudaMemcpyAsync(hh + off, q.h + off, len, cudaMemcpyDeviceToHost, h->copy_stream));
         CK(cudaMemcpyAsync(hu + off, q.hu + off, len, cudaMemcpyDeviceToHost, h->copy_stream));
         CK(cudaMemcpyAsync(hv + off, q.hv + off, len, cudaMemcpyDeviceToHost, h->copy_stream));
     }
-    h->ks->step_end(h->ctl, 1, h->stream);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(h->h_ctl, h->ctl, sizeof(StepCtl), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->copy_stream));
     if (int s = sync(h)) return s;
     const StepCtl& c = *h->h_ctl;
