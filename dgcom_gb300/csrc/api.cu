@@ -619,22 +619,20 @@ int create_impl(dgswe_handle* h, const dgswe_form* f, int device) {
         FxPair *hm = nullptr, *gdb = nullptr;
         FxLimb* lift = nullptr;
         FxExp* exps = nullptr;
-        FxPair* normal = nullptr;
         if ((s = device_array(h, nh, &hm)) || (s = device_array(h, (size_t)h->n_values, &gdb)) ||
             (s = device_array(h, nl, &lift)) || (s = device_array(h, (size_t)h->K, &exps)) ||
             (s = device_array(h, 2 * (size_t)h->K, &T.gen_list)) ||
-            (s = device_array(h, 4, &T.gen_count)) ||
-            (s = device_array(h, (size_t)T.n_edges, &normal)))
+            (s = device_array(h, 4, &T.gen_count)))
             return bail(s);
-        h->ks->fixed_tables(h->n1, T, hm, gdb, lift, exps, normal, nullptr);
+        h->ks->fixed_tables(h->n1, T, hm, gdb, lift, exps, nullptr);
         CK(cudaGetLastError());
-        if (!usable) CK(cudaMemsetAsync(exps, 0, (size_t)h->K * sizeof(FxExp), nullptr));
+        if (!usable)  // no element and no face takes them
+            CK(cudaMemsetAsync(exps, 0, (size_t)h->K * sizeof(FxExp), nullptr));
         CK(cudaMemsetAsync(T.gen_count, 0, 4 * sizeof(unsigned), nullptr));
         T.fx_hm = hm;
         T.fx_gdb = gdb;
         T.fx_lift = lift;
         T.fx_exp = exps;
-        if (usable) T.fx_normal = normal;  // null: every face in FP64
     }
     CK(cudaStreamSynchronize(nullptr));
 #undef UP

@@ -37,10 +37,11 @@ struct alignas(16) FxNode {
     uint64_t slots;
     uint32_t others, unused;
 };
-// √g and g/2 at 2^(62 − e), their exponents and g's (the least e with x < 2^e)
+// √g and g/2 at 2^(62 − e), their exponents and g's (the least e with x < 2^e);
+// whether g is within their range
 struct FxFaceConstants {
     FxLimb sqrt_g, half_g;
-    int e_sqrt_g, e_half_g, e_g;
+    int e_sqrt_g, e_half_g, e_g, usable;
 };
 
 struct DevTables {
@@ -71,7 +72,6 @@ struct DevTables {
     const FxExp* fx_exp = nullptr;    // [K]
     const FxLimb* fx_coef = nullptr;  // [nn][2(n1−1)]
     const FxNode* fx_node = nullptr;  // [nn]
-    const FxPair* fx_normal = nullptr;  // [E] the edges' unit normals at 2^62
     // the elements a stage leaves to general_kernel, in two lists (those with
     // subcells, listed beforehand; what the stage kernel finds), and of each
     // {its length, the blocks that have ended}: empty between stages

@@ -222,24 +222,22 @@ int build_group(dgswe_ensemble* h, Group& G, std::vector<Tables>& tabs,
         FxPair *hm = nullptr, *gdb = nullptr;
         FxLimb* lift = nullptr;
         FxExp* exps = nullptr;
-        FxPair* normal = nullptr;
         if ((s = device_array(h, (size_t)G.n_values * (n1 - 1), &hm)) ||
             (s = device_array(h, (size_t)G.n_values, &gdb)) ||
             (s = device_array(h, (size_t)G.K * 4 * n1, &lift)) ||
             (s = device_array(h, (size_t)G.K, &exps)) ||
             (s = device_array(h, 2 * (size_t)G.K, &T.gen_list)) ||
-            (s = device_array(h, 4, &T.gen_count)) ||
-            (s = device_array(h, (size_t)T.n_edges, &normal)))
+            (s = device_array(h, 4, &T.gen_count)))
             return s;
-        h->ks->fixed_tables(n1, T, hm, gdb, lift, exps, normal, nullptr);
+        h->ks->fixed_tables(n1, T, hm, gdb, lift, exps, nullptr);
         CK(cudaGetLastError());
-        if (!usable) CK(cudaMemsetAsync(exps, 0, (size_t)G.K * sizeof(FxExp), nullptr));
+        if (!usable)  // no element and no face takes them
+            CK(cudaMemsetAsync(exps, 0, (size_t)G.K * sizeof(FxExp), nullptr));
         CK(cudaMemsetAsync(T.gen_count, 0, 4 * sizeof(unsigned), nullptr));
         T.fx_hm = hm;
         T.fx_gdb = gdb;
         T.fx_lift = lift;
         T.fx_exp = exps;
-        if (usable) T.fx_normal = normal;  // null: every face in FP64
     }
     CK(cudaStreamSynchronize(nullptr));
 #undef UP

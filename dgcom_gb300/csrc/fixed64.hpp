@@ -206,6 +206,26 @@ DG_HD double pow_m43(double h) {
     return fp::from_bits((int64_t)(rounded + ((uint64_t)(field - 1) << 52)));
 }
 
+// Right shifts, everything out from 64 on (the instruction's own rule)
+DG_HD uint64_t shr_u(uint64_t v, int n) {
+#if defined(__CUDA_ARCH__)
+    uint64_t r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+    return r;
+#else
+    return n > 63 ? 0 : v >> n;
+#endif
+}
+DG_HD int64_t shr(int64_t v, int n) {
+#if defined(__CUDA_ARCH__)
+    int64_t r;
+    asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+    return r;
+#else
+    return v >> (n > 63 ? 63 : n);
+#endif
+}
+
 // ---- fixed-point numbers ----------------------------------------------------
 //
 // A number is an int64 whose scale (the power of two it is multiplied by) is
@@ -218,8 +238,8 @@ DG_HD double pow_m43(double h) {
 using Lim = FxLimb;  // hi·2^32 + lo
 
 DG_HD Lim split(int64_t v) {
-    const int32_t lo = (int32_t)v;
-    return {lo, (int32_t)(v >> 32) - (lo >> 31)};
+    const uint32_t lo = (uint32_t)v;
+    return {(int32_t)lo, (int32_t)((uint32_t)((uint64_t)v >> 32) + (lo >> 31))};
 }
 
 // A sum of products: r counts 2^64, t 2^32
@@ -261,12 +281,12 @@ DG_HD int64_t fold(const PairSum& p) {
 
 // x·2^(1085 − K), towards zero: |x| < 2^(K − 1023), so the result is below
 // 2^62. Subnormal x count as zero (K is far above their exponent).
+DG_HD int64_t to_fixed_nn(double x, int K) {  // x ≥ +0
+    return (int64_t)shr_u(mant(x) << 10, K - expo(x));
+}
 DG_HD int64_t to_fixed(double x, int K) {
-    const int64_t b = fp::bits(x);
-    const uint64_t m = mant(x) << 10;
-    const int r = K - expo(x);
-    const int64_t v = (int64_t)(m >> (r > 63 ? 63 : r));
-    const int64_t sign = b >> 63;
+    const int64_t v = to_fixed_nn(x, K);
+    const int64_t sign = fp::bits(x) >> 63;
     return (v ^ sign) - sign;
 }
 
@@ -297,6 +317,16 @@ DG_HD double div_pos(double x, double y) {
     const int64_t q = mul<3>(split((int64_t)(mant(x) << 9)), split((int64_t)r));  // 2^61·
     const double v = from_fixed(q, 61 - expo(x) + expo(y));
     return fp::bits(x) < 0 ? fp::neg(v) : v;
+}
+
+// from_fixed by the conversion instruction, which runs on the FP64 pipe
+DG_HD double convert(int64_t v, int s) {
+#if defined(__CUDA_ARCH__)
+    const double x = __ll2double_rn(v);
+    return v ? fp::from_bits(fp::bits(x) - ((int64_t)s << 52)) : 0.0;
+#else
+    return from_fixed(v, s);
+#endif
 }
 
 // ---- the wet element's right-hand side --------------------------------------
@@ -359,7 +389,7 @@ DG_HD Lim two_g_h(const Lim& H, const Lim& two_g, const Scale& s) {
     Acc a{half<2>(), 0};
     mac(a, H, two_g);
     const int64_t v = fold<2>(a);
-    return split(v >> (s.g_shift > 63 ? 63 : s.g_shift));
+    return split(shr(v, s.g_shift));
 }
 
 struct Flux {
@@ -394,14 +424,14 @@ DG_HD Flux pair_flux(const Lim& G, const Lim& H, int64_t M0, int64_t M1, int64_t
 DG_HD int64_t bed_term(const Lim& H, const Lim& slope, const Scale& s) {
     Acc a{half<0>(), 0};
     mac(a, H, slope);
-    return fold<0>(a) >> (s.b_shift > 63 ? 63 : s.b_shift);
+    return shr(fold<0>(a), s.b_shift);
 }
 
 // V·2^-s/J as a double
 DG_HD double over_jacobian(int64_t V, int s, double jinv) {
     Acc a{half<1>(), 0};
     mac(a, split(V), split((int64_t)(mant(jinv) << 9)));
-    return from_fixed(fold<1>(a), s + 1021 - expo(jinv));
+    return convert(fold<1>(a), s + 1021 - expo(jinv));
 }
 
 // ---- the flux between two sides ----------------------------------------------
@@ -431,19 +461,8 @@ struct FaceFlux {
 DG_HD int64_t min64(int64_t a, int64_t b) { return a < b ? a : b; }
 DG_HD int64_t max64(int64_t a, int64_t b) { return a > b ? a : b; }
 DG_HD int imax(int a, int b) { return a > b ? a : b; }
-DG_HD int64_t shr(int64_t v, int n) { return v >> (n > 63 ? 63 : n); }
 DG_HD int64_t shl(int64_t v, int n) { return (int64_t)((uint64_t)v << n); }
 DG_HD int64_t abs64(int64_t v) { return v < 0 ? -v : v; }
-
-// from_fixed by the conversion instruction, which runs on the FP64 pipe
-DG_HD double convert(int64_t v, int s) {
-#if defined(__CUDA_ARCH__)
-    const double x = __ll2double_rn(v);
-    return v ? fp::from_bits(fp::bits(x) - ((int64_t)s << 52)) : 0.0;
-#else
-    return from_fixed(v, s);
-#endif
-}
 
 // √(g·x) at 2^(58 − eC) for 0 ≤ x at 2^s (below 2^62), √(g·x) < 2^eC
 DG_HD int64_t celerity(int64_t x, int s, const FaceConstants& c, int eC) {
@@ -463,15 +482,16 @@ DG_HD int64_t share(int64_t a, int64_t b) {
     return mul<4>(split(shl(a, up)), split((int64_t)q));
 }
 
-// The flux along the unit normal n (at 2^62), times the vector m = |m|·n (at
-// 2^(62 − em), each number below 2^(em − 1), or n itself with em 0; the mass
-// flux times the length |m| by the caller), as seen from both sides. Nothing
-// is written where both reconstructed sides are dry (kBothDry, but for two
-// sides without any water) or the exponents are out of range (kNoScale).
+// The flux along the vector m = |m|·n (geo: m, |m|, n) as seen from both
+// sides. The rotations into the normal and back, 17 operations, and the
+// conversions of the results run on the FP64 pipe, which is idle here.
+// Nothing is written where both reconstructed sides are dry (kBothDry, but
+// for two sides without any water) or the exponents are out of range
+// (kNoScale).
 enum FaceCase { kNoScale = 0, kDone = 1, kBothDry = 2 };
 
 template <class Side>
-DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const FxPair& n, const FxPair& m, int em,
+DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const double* geo,
                          const FaceConstants& c, double h_min, FaceFlux& out) {
     const int xa = (int)((uint64_t)fp::bits(qa.h) >> 52), xb = (int)((uint64_t)fp::bits(qb.h) >> 52);
     const int xh = imax(xa, xb);
@@ -480,17 +500,26 @@ DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const FxPair& n, const 
         return fp::bits(qa.h) == 0 && fp::bits(qb.h) == 0 ? kDone : kNoScale;
     }
     const int xl = imax(xh, imax(expo(qa.b), expo(qb.b)));
-    const int xv = imax(imax(expo(qa.u), expo(qa.v)), imax(expo(qb.u), expo(qb.v)));
+    auto rotate = [&](const Side& q, double& normal, double& along) {
+        const bool moves = fp::gt(q.h, h_min);
+        const double u = moves ? q.u : 0.0, v = moves ? q.v : 0.0;
+        normal = fma(u, geo[3], v * geo[4]);
+        along = fma(v, geo[3], fp::neg(u) * geo[4]);
+    };
+    double na, ta, nb, tb;
+    rotate(qa, na, ta);
+    rotate(qb, nb, tb);
+    const int xv = imax(imax(expo(na), expo(ta)), imax(expo(nb), expo(tb)));
     // within 2^±120 (a negative depth's sign field is above), h_min not above
     // everything
     if (imax(xv, xl) > kExpHi || xh < kExpLo || expo(h_min) > xl + 2) return kNoScale;
     const int eL = xl - 1022, eh = xh - 1022;
     // hydrostatic reconstruction: the surfaces over the higher bed
-    const int64_t la = to_fixed(qa.h, xl + 3), lb = to_fixed(qb.h, xl + 3);
+    const int64_t la = to_fixed_nn(qa.h, xl + 3), lb = to_fixed_nn(qb.h, xl + 3);
     const int64_t ba = to_fixed(qa.b, xl + 3), bb = to_fixed(qb.b, xl + 3);
     const int64_t top = max64(ba, bb);
     const int64_t ra = max64(la + ba - top, 0), rb = max64(lb + bb - top, 0);
-    const int64_t dry = to_fixed(h_min, xl + 3);
+    const int64_t dry = to_fixed_nn(h_min, xl + 3);
     const bool wet_a = ra > dry, wet_b = rb > dry;
     if (!wet_a && !wet_b) return kBothDry;
     const int es = 4 + eL - clz64((uint64_t)(ra | rb));
@@ -498,23 +527,9 @@ DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const FxPair& n, const 
     const int ev = imax(xv - 1022, eC - 30);
     if (es < -60 || ev > eC + 30) return kNoScale;
     const int64_t sa = shl(ra, eL - es + 2), sb = shl(rb, eL - es + 2);
-    const int kv = 1023 + ev;
-    auto rotate = [&](const Side& q, int64_t& normal, int64_t& along) {
-        const bool moves = fp::gt(q.h, h_min);
-        const Lim u = split(moves ? to_fixed(q.u, kv) : 0), v = split(moves ? to_fixed(q.v, kv) : 0);
-        Acc a{half<0>(), 0}, t{half<0>(), 0}, o{0, 0};
-        mac(a, u, n.x);
-        mac(a, v, n.y);
-        normal = fold<0>(a);
-        mac(t, v, n.x);
-        mac(o, u, n.y);
-        t.t -= o.t;
-        t.r -= o.r;
-        along = fold<0>(t);
-    };
-    int64_t un_a, ut_a, un_b, ut_b;  // 2^(60 − ev)
-    rotate(qa, un_a, ut_a);
-    rotate(qb, un_b, ut_b);
+    const int kv = 1025 + ev;
+    const int64_t un_a = to_fixed(na, kv), ut_a = to_fixed(ta, kv);  // 2^(60 − ev)
+    const int64_t un_b = to_fixed(nb, kv), ut_b = to_fixed(tb, kv);
     // wave speeds (Einfeldt; beside a dry side, the front's)
     const int64_t c_a = celerity(sa, 62 - es, c, eC), c_b = celerity(sb, 62 - es, c, eC);
     const int64_t c_m = celerity((sa >> 1) + (sb >> 1), 62 - es, c, eC);
@@ -547,7 +562,7 @@ DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const FxPair& n, const 
     mac(f, be, mr);
     const int64_t f_h = shr(fold<0>(f), eM - es - ev) -
                         shr(mul<0>(w, split(shl(dh, grow))), 2 + eM - eS - eD);
-    out.h = convert(f_h, 58 - eM);
+    out.h = geo[2] * convert(f_h, 58 - eM);
     // momentum
     const int eQ = imax(imax(2 * eh + c.e_half_g + 1, es + 2 * ev + 1), eS + es + ev);
     const int dm = eQ - es - 2 * ev, dw = eQ - eS - es - ev;
@@ -561,28 +576,21 @@ DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const FxPair& n, const 
     Acc t{half<2>(), 0};
     mac(t, al, split(shr(mul<0>(ml, tl), dm)));
     mac(t, be, split(shr(mul<0>(mr, tr), dm)));
-    const Lim f_t = split(shl(fold<2>(t) - shr(mul<0>(w, split(t_b - t_a)), dw), 2));
+    const double f_t = convert(fold<2>(t) - shr(mul<0>(w, split(t_b - t_a)), dw), 58 - eQ);
     // each side's own pressure over the reconstructed one: ½g(h − hs)(h + hs).
     // Where a depth has bits below the surface sums' last place, the own one is
     // taken whole and the pressure of its rounding cancels against the flux's.
     const int down = eL - eh + 2;
     const bool whole = (xa < xb ? xa : xb) >= xl - 7;
     auto back = [&](const Side& q, int64_t own, int64_t surface, double& x, double& y) {
-        const int64_t hq = whole ? shl(own, down) : to_fixed(q.h, xh + 1);
+        const int64_t hq = whole ? shl(own, down) : to_fixed_nn(q.h, xh + 1);
         const int64_t gq = shl(surface, down);
         const int64_t p = shr(mul<0>(split(mul<0>(split(hq - gq), split((hq >> 1) + (gq >> 1)))),
                                      c.half_g),
                               eQ - 2 * eh - c.e_half_g - 1);
-        const Lim fn = split(shl(f_n + p, 2));
-        Acc a{half<0>(), 0}, o{0, 0}, b{half<0>(), 0};
-        mac(a, fn, m.x);
-        mac(o, f_t, m.y);
-        a.t -= o.t;
-        a.r -= o.r;
-        mac(b, fn, m.y);
-        mac(b, f_t, m.x);
-        x = convert(fold<0>(a), 58 - eQ - em);
-        y = convert(fold<0>(b), 58 - eQ - em);
+        const double fn = convert(f_n + p, 58 - eQ);
+        x = fma(fn, geo[0], fp::neg(f_t) * geo[1]);
+        y = fma(fn, geo[1], f_t * geo[0]);
     };
     back(qa, la, ra, out.hu_a, out.hv_a);
     back(qb, lb, rb, out.hu_b, out.hv_b);

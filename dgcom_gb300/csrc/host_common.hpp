@@ -306,7 +306,8 @@ inline bool fixed_constants(const PairSchedule& sched, const Physics& P, DevTabl
     c.sqrt_g = constant(P.sqrt_g, c.e_sqrt_g);
     c.half_g = constant(P.half_g, c.e_half_g);
     std::frexp(P.g, &c.e_g);
-    return T.fx_e2g >= -60 && T.fx_e2g <= 60;
+    c.usable = T.fx_e2g >= -60 && T.fx_e2g <= 60;
+    return c.usable != 0;
 }
 
 // The ready lists of a state uploaded in `chunks` element chunks of

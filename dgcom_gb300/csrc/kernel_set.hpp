@@ -103,10 +103,10 @@ struct KernelSet {
     void (*dt_listed)(int n1, const DevTables&, const Physics&, const DevBuf& q, const DtParams&,
                       double* dt_el, StepCtl* ctl, const int* active, const int32_t* list,
                       int64_t n, cudaStream_t);
-    // the fixed-point tables from pair_hm, gdb, lift_scale and edge_geo
+    // the fixed-point tables from pair_hm, gdb and lift_scale
     // (DevTables::fx_*), where the variant has them
     void (*fixed_tables)(int n1, const DevTables&, FxPair* hm, FxPair* gdb, FxLimb* lift,
-                         FxExp* exps, FxPair* normal, cudaStream_t);
+                         FxExp* exps, cudaStream_t);
     bool has_fixed;
     // face and stage as above, for a pass over the whole mesh, one after the
     // other: the node sources and the list of the elements with subcells run

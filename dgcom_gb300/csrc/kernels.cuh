@@ -93,20 +93,13 @@ __device__ __noinline__ FacePair face_dry(Sd qa, Sd qb, const double* geo, doubl
 }
 
 // The flux of two sides along m = norm·(nx, ny): in fixed point, or the rest
-// (nf, mf: the two vectors as limbs at 2^62 and 2^(62 − em); UNIT: both the
-// unit normal)
-template <bool UNIT>
 __device__ __forceinline__ FacePair face_pair(const DevTables& T, const Sd& qa, const Sd& qb,
-                                              const FxPair& nf, const FxPair& mf, int em,
                                               const double* geo, double g, double sqrt_g,
                                               double half_g, double h_min) {
     fx::FaceFlux f;
-    const fx::FaceCase got = T.fx_normal ? fx::face_flux(qa, qb, nf, mf, em, T.fx_face, h_min, f)
-                                         : fx::kNoScale;
-    if (got == fx::kDone) {
-        const double h = UNIT ? f.h : geo[2] * f.h;
-        return {{h, f.hu_a, f.hv_a}, {h, f.hu_b, f.hv_b}};
-    }
+    const fx::FaceCase got =
+        T.fx_face.usable ? fx::face_flux(qa, qb, geo, T.fx_face, h_min, f) : fx::kNoScale;
+    if (got == fx::kDone) return {{f.h, f.hu_a, f.hv_a}, {f.h, f.hu_b, f.hv_b}};
     if (got == fx::kBothDry) return face_dry(qa, qb, geo, g, half_g, h_min);
     return face_hll(qa, qb, geo, g, sqrt_g, half_g, h_min);
 }
@@ -318,9 +311,7 @@ __global__ void __launch_bounds__(256, DGSWE_FAST ? 4 : 2)
             const Sd ql = load_side(in, T, P, gl), qr = load_side(in, T, P, gr);
             const double* geo = &T.edge_geo[e * 5];
 #if DGSWE_FAST
-            const FxPair n = T.fx_normal ? T.fx_normal[e] : FxPair{};
-            const FacePair f =
-                face_pair<true>(T, ql, qr, n, n, 0, geo, g, sqrt_g, half_g, h_min);
+            const FacePair f = face_pair(T, ql, qr, geo, g, sqrt_g, half_g, h_min);
 #else
             const FacePair f = face_hll(ql, qr, geo, g, sqrt_g, half_g, h_min);
 #endif
@@ -358,7 +349,11 @@ __global__ void __launch_bounds__(256, DGSWE_FAST ? 4 : 2)
         const Q qe = wall_ghost(qi, u, v, nx, ny, c.wall_h_min, h_min);
         F3 fdummy;
         if (P.formulation == kWetDry)
+#if DGSWE_FAST
+            fs = face_pair(T, side(qi), side(qe), geo, g, sqrt_g, half_g, h_min).a;
+#else
             fs = face_hll(side(qi), side(qe), geo, g, sqrt_g, half_g, h_min).a;
+#endif
         else
             entropy_surface(qi, qe, nx, ny, P, fs, fdummy);
     } else {
@@ -739,13 +734,7 @@ __device__ __forceinline__ F3 general_rhs(const DevTables& T, const Physics& P,
             const double* fb_ = &faces[((dir * N1 + line) * N1 + pos + 1) * 8];   // left face of pos+1
             const Sd qa{fa_[0], fa_[1], fa_[2], fa_[3]}, qb{fb_[0], fb_[1], fb_[2], fb_[3]};
 #if DGSWE_FAST
-            auto pair = [](double x, double y, int K) {
-                return FxPair{fx::split(fx::to_fixed(x, K)), fx::split(fx::to_fixed(y, K))};
-            };
-            const int em = max_expo(mx, my);
-            const FacePair f =
-                face_pair<false>(T, qa, qb, pair(geo[3], geo[4], 1023), pair(mx, my, em + 2),
-                                 em - 1021, geo, g, sqrt_g, half_g, h_min);
+            const FacePair f = face_pair(T, qa, qb, geo, g, sqrt_g, half_g, h_min);
 #else
             const FacePair f = face_hll(qa, qb, geo, g, sqrt_g, half_g, h_min);
 #endif
@@ -867,14 +856,6 @@ __device__ __forceinline__ void warp_max(ExpWords& e) {
 __device__ __forceinline__ fx::Exps exponents(const ExpWords& e) {
     return {(int)(e.w[0] & 0xFFFFu), 4095 - (int)(e.w[0] >> 16), (int)(e.w[1] & 0xFFFFu),
             (int)(e.w[1] >> 16),     (int)(e.w[2] & 0xFFFFu),    (int)(e.w[2] >> 16)};
-}
-
-// The edges' unit normals in fixed point
-__global__ void fixed_normals_kernel(DevTables T, FxPair* normal) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= T.n_edges) return;
-    const double* geo = &T.edge_geo[e * 5];
-    normal[e] = {fx::split(fx::to_fixed(geo[0], 1023)), fx::split(fx::to_fixed(geo[1], 1023))};
 }
 
 // The fixed-point tables of each element from its FP64 ones: a warp per
@@ -1160,12 +1141,6 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
         prefetch(&T.jinv[gi]);
         prefetch(&T.fx_lift[fbase + i % (4 * N1)]);
         prefetch(&T.fx_exp[k]);
-        if (mode != kRhsOnly && base.h) {
-            prefetch(&base.h[gi]);
-            prefetch(&base.hu[gi]);
-            prefetch(&base.hv[gi]);
-        }
-        if (P.friction == 2) prefetch(&T.g_n2[gi]);
     }
     if (!run) return;
     ExpWords ew = node_exponents(h, hu, hv, u, v);
@@ -1214,7 +1189,7 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
     int64_t* const nd = (int64_t*)&s_x[e][C::PAIR_DOUBLES + NN];
     int64_t* const lifted = (int64_t*)&s_x[e][C::PAIR_DOUBLES + 5 * NN];
     if (fixed) {
-        H = fx::split(fx::to_fixed(h, sc.kh));
+        H = fx::split(fx::to_fixed_nn(h, sc.kh));
         G = fx::two_g_h(H, T.fx_two_g, sc);
         m0 = fx::to_fixed(hu, sc.km);
         m1 = fx::to_fixed(hv, sc.km);

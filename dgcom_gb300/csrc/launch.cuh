@@ -346,10 +346,8 @@ static void sub_metrics(int n1, const DevTables& T, const Physics& P, double* ou
 }
 
 static void fixed_tables(int n1, const DevTables& T, FxPair* hm, FxPair* gdb, FxLimb* lift,
-                         FxExp* exps, FxPair* normal, cudaStream_t s) {
+                         FxExp* exps, cudaStream_t s) {
 #if DGSWE_FAST
-    if (T.n_edges > 0)
-        fixed_normals_kernel<<<(unsigned)((T.n_edges + 255) / 256), 256, 0, s>>>(T, normal);
     DGSWE_BY_ORDER(fixed_tables_n, T, hm, gdb, lift, exps, s);
 #endif
 }

@@ -108,9 +108,9 @@ static long faces(std::mt19937_64& rng, Score& mass, Score& momentum) {
             if (i % 3 == 0) std::swap(a, b);
         }
         for (double* x : {&a.u, &a.v, &b.u, &b.v}) *x = speed * (U(rng) - 0.5);
-        const FxPair n{fx::split(fx::to_fixed(nx, 1023)), fx::split(fx::to_fixed(ny, 1023))};
+        const double geo[5] = {nx, ny, 1.0, nx, ny};
         fx::FaceFlux f;
-        if (fx::face_flux(a, b, n, n, 0, T.fx_face, kHMin, f) != fx::kDone) continue;
+        if (fx::face_flux(a, b, geo, T.fx_face, kHMin, f) != fx::kDone) continue;
         ++done;
         const Five<Q> q = hll<Q>(a, b, nx, ny, P.g, P.sqrt_g, P.half_g);
         const Five<double> d = hll<double>(a, b, nx, ny, P.g, P.sqrt_g, P.half_g);
