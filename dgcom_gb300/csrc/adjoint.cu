@@ -73,9 +73,7 @@ struct Target {
     std::vector<int> cond0, ncond;    // per member: first condition, count
     int n_cond = 0;
     // the parameters a calibration changes between sweeps: the tide
-    // constituents (in Physics::cond of one mesh, or the ensemble's device
-    // table) and g·n² per node (null: a uniform coefficient)
-    Physics* cond_host = nullptr;
+    // constituents (in the device's table of conditions) and g·n² per node (null: a uniform coefficient)
     Condition* cond_dev = nullptr;
     double* g_n2 = nullptr;
 };
@@ -569,7 +567,7 @@ int dgswe_adjoint_create(const dgswe_form* f, int device, const dgswe_adjoint_co
     t.cond0 = {0};
     t.ncond = {f->n_boundaries};
     t.n_cond = f->n_boundaries;
-    t.cond_host = &h->P;
+    t.cond_dev = const_cast<Condition*>(h->T.cond);
     t.g_n2 = const_cast<double*>(h->T.g_n2);
     return setup(a, f, cfg);
 }
@@ -906,10 +904,7 @@ int dgswe_adjoint_set_parameters(dgswe_adjoint* a, const double* manning_n, cons
     }
     if (tide && t.n_cond > 0) {
         std::vector<Condition> c((size_t)t.n_cond);
-        if (t.cond_dev)
-            ACK(cudaMemcpy(c.data(), t.cond_dev, c.size() * sizeof(Condition), cudaMemcpyDeviceToHost));
-        else
-            std::copy(t.cond_host->cond, t.cond_host->cond + t.n_cond, c.begin());
+        ACK(cudaMemcpy(c.data(), t.cond_dev, c.size() * sizeof(Condition), cudaMemcpyDeviceToHost));
         for (int ci = 0; ci < t.n_cond; ++ci)
             for (int i = 0; i < c[ci].n_constituents; ++i) {
                 const double amp = tide[((size_t)ci * kMaxConstituents + i) * 2];
@@ -919,10 +914,7 @@ int dgswe_adjoint_set_parameters(dgswe_adjoint* a, const double* manning_n, cons
                 c[ci].c[i].amplitude = amp;
                 c[ci].c[i].phase = ph;
             }
-        if (t.cond_dev)
-            ACK(cudaMemcpy(t.cond_dev, c.data(), c.size() * sizeof(Condition), cudaMemcpyHostToDevice));
-        else
-            std::copy(c.begin(), c.end(), t.cond_host->cond);
+        ACK(cudaMemcpy(t.cond_dev, c.data(), c.size() * sizeof(Condition), cudaMemcpyHostToDevice));
     }
     a->forward_done = false;
     return DGSWE_OK;

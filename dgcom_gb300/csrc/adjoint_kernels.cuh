@@ -46,8 +46,12 @@ struct AdjCfg {
     static constexpr int NN = N1 * N1;
     static constexpr int NP = N1 - 1;
     static constexpr int NA = 2 * (N1 - 1);
-    static constexpr int EPB = (64 / NN) > 0 ? (64 / NN) : 1;
-    static constexpr int THREADS = EPB * NN;
+    // the subcell pass: two lanes a node, a subcell direction each (an
+    // element's reverse is one long chain of FP64 instructions)
+    static constexpr int SPLIT = PATH == kAdjSub ? 2 : 1;
+    static constexpr int LANES = NN * SPLIT;
+    static constexpr int EPB = (64 / LANES) > 0 ? (64 / LANES) : 1;
+    static constexpr int THREADS = EPB * LANES;
     // per pair slot a row of 7, the pair's factors for its two nodes; the
     // bed-slope weights (2 per node); each node's λ of the RHS (3 per node)
     static constexpr int ROW = 7;
@@ -87,9 +91,10 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
     stage_adjoint_kernel(DevTables T, Physics P, StageExtra X, DevBuf in, DevBuf keep, AdjStage A,
                          const StepCtl* ctl, int slot) {
     using C = AdjCfg<N1, PATH>;
-    constexpr int NN = C::NN, NP = C::NP, NA = C::NA, EPB = C::EPB;
+    constexpr int NN = C::NN, NP = C::NP, NA = C::NA, EPB = C::EPB, SPLIT = C::SPLIT;
     __shared__ double s_q[EPB][6][NN];        // stage input: h, hu, hv, u, v, b
     __shared__ double s_l[EPB][6][C::LAND];   // λ landing from the element's other nodes
+    __shared__ double s_r[EPB][3][C::LAND];   // λ of the RHS, for the second lanes
     __shared__ double s_x[EPB][C::X];         // limiter, then the pair or subcell scratch
     __shared__ int s_flag[EPB][2];
     __shared__ double s_red[EPB][12];
@@ -97,24 +102,23 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
     __shared__ int s_live[EPB];
 
     const int tid = threadIdx.x;
-    const int e = tid / NN, i = tid % NN;
-    // the subcell pass takes its elements from the stage's subcell list;
-    // its blocks past the list's end leave at once
-    int64_t k;
-    if (PATH == kAdjSub) {
-        const unsigned long long n_sub = A.sub_count[slot];
-        const unsigned long long at = (unsigned long long)blockIdx.x * EPB;
-        if (at >= n_sub) return;
-        k = at + e < n_sub ? A.sub_list[slot * T.K + (int64_t)(at + e)] : T.K;
-    } else {
-        k = (int64_t)blockIdx.x * EPB + e;
-    }
-    bool valid = k < T.K;
-    const int64_t gi = k * NN + i;
+    const int e = tid / C::LANES, half = tid % C::LANES / NN, i = tid % NN;
     const int a = i % N1, j = i / N1;
     const double g = P.g, h_min = P.h_min, sqrt_g = P.sqrt_g, half_g = P.half_g;
-
-    if (i == 0) {
+    // the wet pass: one element each; the subcell pass: the stage's list, in
+    // strides of the grid
+    const unsigned long long n_sub = PATH == kAdjSub ? A.sub_count[slot] : 1ull;
+    for (unsigned long long at = (PATH == kAdjSub ? blockIdx.x : 0) * (unsigned long long)EPB;
+         at < n_sub; at += (unsigned long long)gridDim.x * EPB) {
+    int64_t k;
+    if (PATH == kAdjSub)
+        k = at + e < n_sub ? A.sub_list[slot * T.K + (int64_t)(at + e)] : T.K;
+    else
+        k = (int64_t)blockIdx.x * EPB + e;
+    const bool mine = k < T.K;
+    bool valid = mine && half == 0;  // holds a node
+    const int64_t gi = k * NN + i;
+    if (i == 0 && half == 0) {
         s_flag[e][0] = 0;
         s_flag[e][1] = 0;
         s_live[e] = 0;
@@ -140,13 +144,15 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
         dhu = keep.u[gi];
         dhv = keep.v[gi];
     }
-    s_q[e][0][i] = h;
-    s_q[e][1][i] = hu;
-    s_q[e][2][i] = hv;
-    s_q[e][3][i] = u;
-    s_q[e][4][i] = v;
-    s_q[e][5][i] = b;
-    if (PATH == kAdjSub) {
+    if (half == 0) {
+        s_q[e][0][i] = h;
+        s_q[e][1][i] = hu;
+        s_q[e][2][i] = hv;
+        s_q[e][3][i] = u;
+        s_q[e][4][i] = v;
+        s_q[e][5][i] = b;
+    }
+    if (PATH == kAdjSub && half == 0) {
 #pragma unroll
         for (int c = 0; c < 6; ++c) s_l[e][c][i] = 0.0;
     }
@@ -174,9 +180,9 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
         if (s_b >= 0) A.lf_h[s_b] = A.lf_hu[s_b] = A.lf_hv[s_b] = 0.0;
         valid = false;
     }
-    if (!__syncthreads_or(valid ? 1 : 0)) return;
+    if (!__syncthreads_or(valid ? 1 : 0)) continue;
     constexpr bool sub = PATH == kAdjSub;
-    const bool affine = valid ? T.affine[k] != 0 : true;
+    const bool affine = mine ? T.affine[k] != 0 : true;
     // the element's member's stage weights (an ensemble: one StepCtl each)
     const StageArgs sa = ctl[(T.elem_member && valid) ? T.elem_member[k] : 0].stage[slot];
 
@@ -188,9 +194,11 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
     double ldh = lo_h, ldhu = lo_hu, ldhv = lo_hv;  // λ of (vh, dhu, dhv)
     if (P.has_wet_dry) {
         if (valid && fp::lt(vh, P.h_dry)) atomicOr(&s_flag[e][1], 1);
-        s_x[e][0 * NN + i] = vh;
-        s_x[e][1 * NN + i] = dhu;
-        s_x[e][2 * NN + i] = dhv;
+        if (half == 0) {
+            s_x[e][0 * NN + i] = vh;
+            s_x[e][1 * NN + i] = dhu;
+            s_x[e][2 * NN + i] = dhv;
+        }
         __syncthreads();
         const bool needs = s_flag[e][1] != 0;
         if (valid && needs && i == 0) {
@@ -211,7 +219,7 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
             const double h_avg = sh * inv_area;
             double theta = 1.0, theta_raw = 1.0;
             if (fp::gt0(h_avg) && fp::lt0(hmin)) {
-                theta_raw = h_avg / (h_avg - hmin);
+                theta_raw = vdiv(h_avg, h_avg - hmin);
                 theta = fp::lt0(theta_raw) ? 0.0 : (fp::gt(theta_raw, 1.0) ? 1.0 : theta_raw);
             }
             s_red[e][0] = h_avg;
@@ -260,9 +268,11 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
             ldhu = lwhu;
             ldhv = lwhv;
         }
-        s_x[e][3 * NN + i] = lpre;
-        s_x[e][4 * NN + i] = lwhu;
-        s_x[e][5 * NN + i] = lwhv;
+        if (half == 0) {
+            s_x[e][3 * NN + i] = lpre;
+            s_x[e][4 * NN + i] = lwhu;
+            s_x[e][5 * NN + i] = lwhv;
+        }
         __syncthreads();
         if (valid && scaled && i == 0) {
             double tb = 0.0, sp = 0.0, spu = 0.0, spv = 0.0;
@@ -370,8 +380,21 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
     auto node_side = [&](int n) {
         return Sd{s_q[e][0][n], s_q[e][3][n], s_q[e][4][n], s_q[e][5][n]};
     };
+    if (PATH == kAdjSub && half == 0) {
+        s_r[e][0][i] = lrh;
+        s_r[e][1][i] = lrhu;
+        s_r[e][2][i] = lrhv;
+    }
     __syncthreads();
-    const bool work = valid;  // live elements only (above)
+    // live elements only (above): both lanes of a node in the subcell pass
+    const bool work = PATH == kAdjSub ? mine && s_flag[e][0] && s_live[e] : valid;
+    if (PATH == kAdjSub) {
+        lrh = s_r[e][0][i];
+        lrhu = s_r[e][1][i];
+        lrhv = s_r[e][2][i];
+        h = s_q[e][0][i];
+        b = s_q[e][5][i];
+    }
     // step 1: pair slots' λ, or the subcell faces (forward)
     if (work && !sub) {
         if (P.has_bed) {
@@ -383,8 +406,8 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
         s_lr[NN + i] = lrhu;
         s_lr[2 * NN + i] = lrhv;
     } else if (work && sub) {
-#pragma unroll
-        for (int dir = 0; dir < 2; ++dir) {
+#pragma unroll 1
+        for (int dir = half; dir < 2; dir += SPLIT) {
             const int line = dir == 0 ? j : a;
             const int pos = dir == 0 ? a : j;
             const Sd q = node_side(i);
@@ -466,8 +489,8 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
             o[6] = mass;
         }
     } else if (work && sub) {
-#pragma unroll
-        for (int dir = 0; dir < 2; ++dir) {
+#pragma unroll 1
+        for (int dir = half; dir < 2; dir += SPLIT) {
             const int line = dir == 0 ? j : a;
             const int pos = dir == 0 ? a : j;
             const double iw = X.inv_w[pos];
@@ -495,16 +518,15 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
             const double kb = -0.5 * g / w_a;
             const double km = 0.25 * g / w_a;
 #endif
-            double m0[N1], m1[N1];
-            line_metric<N1>(T, k, dir, line, m0, m1);
             double lbed;
             double llh = 0.0, llb = 0.0, lrh_ = 0.0, lrb = 0.0;
+            const double ml0 = subcell_metric<N1>(T, k, dir, line, pos, 0);
+            const double ml1 = subcell_metric<N1>(T, k, dir, line, pos, 1);
             if (affine) {
-                lbed = lrhu * m0[0] + lrhv * m1[0];
+                lbed = lrhu * ml0 + lrhv * ml1;
             } else {
-                double i0[N1 + 1], i1[N1 + 1];
-                telescoped<N1>(P, m0, m1, false, i0, i1);
-                const double ml0 = i0[pos], ml1 = i1[pos], mr0 = i0[pos + 1], mr1 = i1[pos + 1];
+                const double mr0 = subcell_metric<N1>(T, k, dir, line, pos + 1, 0);
+                const double mr1 = subcell_metric<N1>(T, k, dir, line, pos + 1, 1);
                 lbed = lrhu * 0.5 * (ml0 + mr0) + lrhv * 0.5 * (ml1 + mr1);
                 const double lmet = lrhu * (mr0 - ml0) + lrhv * (mr1 - ml1);
                 // metric = km·((rhh + h)(b − rb) + (lh + h)(b − lb))
@@ -563,15 +585,13 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
             }
         }
     } else if (work && sub) {
-#pragma unroll
-        for (int dir = 0; dir < 2; ++dir) {
+#pragma unroll 1
+        for (int dir = half; dir < 2; dir += SPLIT) {
             const int line = dir == 0 ? j : a;
             const int pos = dir == 0 ? a : j;
             if (pos + 1 >= N1) continue;
-            double m0[N1], m1[N1], i0[N1 + 1], i1[N1 + 1];
-            line_metric<N1>(T, k, dir, line, m0, m1);
-            telescoped<N1>(P, m0, m1, affine, i0, i1);
-            const double mx = i0[pos + 1], my = i1[pos + 1];
+            const double mx = subcell_metric<N1>(T, k, dir, line, pos + 1, 0);
+            const double my = subcell_metric<N1>(T, k, dir, line, pos + 1, 1);
             const double norm = vsqrt(mx * mx + my * my);
             const double inv = vrcp(norm);
             const double* fa_ = &faces[((dir * N1 + line) * N1 + pos) * 8 + 4];
@@ -596,8 +616,8 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
     __syncthreads();
     // step 4: the subcell reconstructions, reversed
     if (work && sub) {
-#pragma unroll
-        for (int dir = 0; dir < 2; ++dir) {
+#pragma unroll 1
+        for (int dir = half; dir < 2; dir += SPLIT) {
             const int line = dir == 0 ? j : a;
             const int pos = dir == 0 ? a : j;
             const Sd q = node_side(i);
@@ -676,6 +696,12 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
             }
         }
     }
+    if (PATH == kAdjSub && work && half == 1) {  // the second direction's sums
+        atomicAdd(&s_l[e][0][i], Lh);
+        atomicAdd(&s_l[e][3][i], Lu);
+        atomicAdd(&s_l[e][4][i], Lv);
+        atomicAdd(&s_l[e][5][i], Lb);
+    }
     __syncthreads();
     if (valid) {
         // λ landed from the element's other nodes (the subcell pass only)
@@ -686,7 +712,9 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
         A.li_u[gi] = Lu + land(3);
         A.li_v[gi] = Lv + land(4);
         const double lb_all = Lb + land(5);
-        if (P.has_bed && A.lbed && lb_all != 0.0) atomicAdd(&A.lbed[gi], lb_all);
+        if (P.has_bed && A.lbed && fp::nz(lb_all)) atomicAdd(&A.lbed[gi], lb_all);
+    }
+    if (PATH == kAdjSub) __syncthreads();  // the scratch is free again
     }
 }
 
@@ -703,12 +731,12 @@ __global__ void __launch_bounds__(256)
     const double g = P.g, h_min = P.h_min, sqrt_g = P.sqrt_g, half_g = P.half_g;
     auto add = [&](int64_t gn, double lh, double lhu, double lhv, double lu, double lv,
                    double lb) {
-        if (lh != 0.0) atomicAdd(&A.lx_h[gn], lh);
-        if (lhu != 0.0) atomicAdd(&A.lx_hu[gn], lhu);
-        if (lhv != 0.0) atomicAdd(&A.lx_hv[gn], lhv);
-        if (lu != 0.0) atomicAdd(&A.lx_u[gn], lu);
-        if (lv != 0.0) atomicAdd(&A.lx_v[gn], lv);
-        if (P.has_bed && A.lbed && lb != 0.0) atomicAdd(&A.lbed[gn], lb);
+        if (fp::nz(lh)) atomicAdd(&A.lx_h[gn], lh);
+        if (fp::nz(lhu)) atomicAdd(&A.lx_hu[gn], lhu);
+        if (fp::nz(lhv)) atomicAdd(&A.lx_hv[gn], lhv);
+        if (fp::nz(lu)) atomicAdd(&A.lx_u[gn], lu);
+        if (fp::nz(lv)) atomicAdd(&A.lx_v[gn], lv);
+        if (P.has_bed && A.lbed && fp::nz(lb)) atomicAdd(&A.lbed[gn], lb);
     };
     if (item < n_int) {
         const int64_t e = item / N1;
@@ -720,7 +748,7 @@ __global__ void __launch_bounds__(256)
         const int64_t sl = (L * N1) + fi, sr = (R * N1) + rfi;
         // the right slot stored −fb
         const F3 la{A.lf_h[sl], A.lf_hu[sl], A.lf_hv[sl]};
-        const F3 lb{-A.lf_h[sr], -A.lf_hu[sr], -A.lf_hv[sr]};
+        const F3 lb{fp::neg(A.lf_h[sr]), fp::neg(A.lf_hu[sr]), fp::neg(A.lf_hv[sr])};
         // (the states are loaded before the test below, so that one memory
         // latency covers both)
         const int64_t gl = kl * NN + P.face_node[fl][fi], gr = kr * NN + P.face_node[fr][rfi];
@@ -750,7 +778,7 @@ __global__ void __launch_bounds__(256)
     const double* geo = &T.bface_geo[bfi * 5];
     const double nx = geo[0], ny = geo[1];
     const int ci = T.bface_cond[bfi];
-    const Condition& c = T.cond ? T.cond[ci] : P.cond[ci];
+    const Condition& c = T.cond[ci];
     double u, v;
     interior_velocity(qi, h_min, u, v);
     if (c.kind == kBcWall) {
@@ -774,7 +802,7 @@ __global__ void __launch_bounds__(256)
         characteristic_state_rev(qi, u, v, eta, nx, ny, c.elevation_only, g, h_min, qbb, qib, ub,
                                  vb, etab);
         add(gn, qib.h, qib.hu, qib.hv, ub, vb, qib.b);
-        if (A.ltide && etab != 0.0) {
+        if (A.ltide && fp::nz(etab)) {
             double gr[2 * kMaxConstituents] = {};
             tide_elevation_rev(c, t, etab, gr);
             for (int m = 0; m < 2 * c.n_constituents; ++m)

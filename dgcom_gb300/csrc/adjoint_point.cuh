@@ -155,13 +155,13 @@ DG_PT void wall_ram_rev(double h, double un, double sill, double g, double ramb,
     const double up = fp::max0(un);
     const double head = up * up * (0.5 / g);
     if (!fp::gt(sill, head)) return;
-    const double c = sqrt(g * h);
-    const double a = 1.0 - head / sill, p = h * up, q = 2.0 * up + c;
+    const double c = vsqrt(g * h);
+    const double a = 1.0 - vdiv(head, sill), p = h * up, q = 2.0 * up + c;
     const double ab = ramb * p * q, pb = ramb * a * q, qb = ramb * a * p;
-    const double headb = -ab / sill;
-    sillb += ab * head / (sill * sill);
+    const double headb = vdiv(-ab, sill);
+    sillb += vdiv(ab * head, sill * sill);
     hb += pb * up;
-    if (fp::gt0(c)) hb += qb * g * 0.5 / c;
+    if (fp::gt0(c)) hb += vdiv(qb * g * 0.5, c);
     const double upb = pb * h + 2.0 * qb + headb * 2.0 * up * (0.5 / g);
     if (fp::gt0(un)) unb += upb;
 }
@@ -305,18 +305,18 @@ DG_PT void characteristic_state_rev(const Q& qi, double u, double v, double eta,
     const double h_e = fmax(e_arg, 0.0);
     double un_e = 0.0;
     const double neg_b = fmax(-bathy, 0.0);
-    if (elevation_only == kIncomingWave) un_e = 2.0 * (sqrt(g * neg_b) - sqrt(g * h_e));
+    if (elevation_only == kIncomingWave) un_e = 2.0 * (vsqrt(g * neg_b) - vsqrt(g * h_e));
     const double ut_e = -u * ny + v * nx;
     const double h_i = fmax(qi.h, 0.0);
     double un_i = 0.0, ut_i = 0.0, ui = 0.0, vi = 0.0;
     const bool moving = h_i > h_min;
     if (moving) {
-        ui = qi.hu / h_i;
-        vi = qi.hv / h_i;
+        ui = vdiv(qi.hu, h_i);
+        vi = vdiv(qi.hv, h_i);
         un_i = ui * nx + vi * ny;
         ut_i = -ui * ny + vi * nx;
     }
-    const double c_i = sqrt(g * h_i), c_e = sqrt(g * h_e);
+    const double c_i = vsqrt(g * h_i), c_e = vsqrt(g * h_e);
     const double w_out = un_i + 2.0 * c_i, w_in = un_e - 2.0 * c_e;
     const bool wi = h_i > h_min, we = h_e > h_min;
     int branch;
@@ -335,18 +335,18 @@ DG_PT void characteristic_state_rev(const Q& qi, double u, double v, double eta,
         un_b = un_e;
     } else if (wi && !we) {
         branch = 3;
-        cc = fmax(w_out / 3.0, 0.0);
-        h_b = cc * cc / g;
+        cc = fmax(vdiv(w_out, 3.0), 0.0);
+        h_b = vdiv(cc * cc, g);
         un_b = cc;
     } else if (!wi && we) {
         branch = 4;
-        cc = fmax(-w_in / 3.0, 0.0);
-        h_b = cc * cc / g;
+        cc = fmax(vdiv(-w_in, 3.0), 0.0);
+        h_b = vdiv(cc * cc, g);
         un_b = -cc;
     } else {
         branch = 5;
         cc = fmax(0.25 * (w_out - w_in), 0.0);
-        h_b = cc * cc / g;
+        h_b = vdiv(cc * cc, g);
         un_b = 0.5 * (w_out + w_in);
     }
     const bool t_in = un_b > 0.0;
@@ -373,15 +373,15 @@ DG_PT void characteristic_state_rev(const Q& qi, double u, double v, double eta,
             un_eb += un_bb;
             break;
         case 3: {
-            const double ccb = h_bb * 2.0 * cc / g + un_bb;
+            const double ccb = vdiv(h_bb * 2.0 * cc, g) + un_bb;
             if (w_out / 3.0 > 0.0) w_outb += ccb / 3.0;
         } break;
         case 4: {
-            const double ccb = h_bb * 2.0 * cc / g - un_bb;
+            const double ccb = vdiv(h_bb * 2.0 * cc, g) - un_bb;
             if (-w_in / 3.0 > 0.0) w_inb -= ccb / 3.0;
         } break;
         case 5: {
-            const double ccb = h_bb * 2.0 * cc / g;
+            const double ccb = vdiv(h_bb * 2.0 * cc, g);
             if (0.25 * (w_out - w_in) > 0.0) {
                 w_outb += 0.25 * ccb;
                 w_inb -= 0.25 * ccb;
@@ -395,21 +395,21 @@ DG_PT void characteristic_state_rev(const Q& qi, double u, double v, double eta,
     const double c_ib = 2.0 * w_outb;
     un_eb += w_inb;
     const double c_eb = -2.0 * w_inb;
-    if (c_i > 0.0) h_ib += c_ib * g * 0.5 / c_i;
-    if (c_e > 0.0) h_eb += c_eb * g * 0.5 / c_e;
+    if (c_i > 0.0) h_ib += vdiv(c_ib * g * 0.5, c_i);
+    if (c_e > 0.0) h_eb += vdiv(c_eb * g * 0.5, c_e);
     if (moving) {
         const double uib = un_ib * nx - ut_ib * ny, vib = un_ib * ny + ut_ib * nx;
-        qib.hu += uib / h_i;
-        qib.hv += vib / h_i;
-        h_ib -= (uib * ui + vib * vi) / h_i;
+        qib.hu += vdiv(uib, h_i);
+        qib.hv += vdiv(vib, h_i);
+        h_ib -= vdiv(uib * ui + vib * vi, h_i);
     }
     if (qi.h > 0.0) qib.h += h_ib;
     ub_i -= ut_eb * ny;
     vb_i += ut_eb * nx;
     double bathyb = 0.0;
     if (elevation_only == kIncomingWave) {
-        if (neg_b > 0.0) bathyb -= un_eb * 2.0 * g * 0.5 / sqrt(g * neg_b);
-        if (h_e > 0.0) h_eb -= un_eb * 2.0 * g * 0.5 / sqrt(g * h_e);
+        if (neg_b > 0.0) bathyb -= vdiv(un_eb * 2.0 * g * 0.5, vsqrt(g * neg_b));
+        if (h_e > 0.0) h_eb -= vdiv(un_eb * 2.0 * g * 0.5, vsqrt(g * h_e));
     }
     if (e_arg > 0.0) {
         etab += h_eb;
@@ -459,19 +459,20 @@ DG_PT void damp_velocity(const Physics& P, const DampIn& from, double& u, double
                 u = from.u;
                 v = from.v;
             } else {
-                const double inv = 1.0 / from.h;
+                const double inv = vrcp(from.h);
                 u = from.hu * inv;
                 v = from.hv * inv;
             }
         } else {
-            const double r = from.h / P.h_dry;
-            const double factor = 1.4142135623730951 * r / (P.h_dry * sqrt(1.0 + r * r * r * r));
+            const double r = vdiv(from.h, P.h_dry);
+            const double factor =
+                vdiv(1.4142135623730951 * r, P.h_dry * vsqrt(1.0 + r * r * r * r));
             u = factor * from.hu;
             v = factor * from.hv;
         }
     } else {
         const double h_reg = lmax(from.h, P.h_min);
-        const double inv_d = 1.0 / (from.h * from.h + h_reg * h_reg);
+        const double inv_d = vrcp(from.h * from.h + h_reg * h_reg);
         const double factor = 2.0 * from.h * inv_d;
         u = from.hu * factor;
         v = from.hv * factor;
@@ -480,9 +481,9 @@ DG_PT void damp_velocity(const Physics& P, const DampIn& from, double& u, double
 
 // d/dh of the desingularising factor √2 r/(h_dry √(1 + r⁴)), r = h/h_dry
 DG_PT double desing_factor_dh(double h, double h_dry) {
-    const double r = h / h_dry, r4 = r * r * r * r;
-    const double s = sqrt(1.0 + r4);
-    return 1.4142135623730951 * (1.0 - r4) / (h_dry * h_dry * s * s * s);
+    const double r = vdiv(h, h_dry), r4 = r * r * r * r;
+    const double s = vsqrt(1.0 + r4);
+    return vdiv(1.4142135623730951 * (1.0 - r4), h_dry * h_dry * s * s * s);
 }
 
 DG_PT void damp_velocity_rev(const Physics& P, const DampIn& from, double ub, double vb,
@@ -494,15 +495,16 @@ DG_PT void damp_velocity_rev(const Physics& P, const DampIn& from, double ub, do
                 fromb.u += ub;
                 fromb.v += vb;
             } else {
-                const double inv = 1.0 / from.h;
+                const double inv = vrcp(from.h);
                 const double u = from.hu * inv, v = from.hv * inv;
                 fromb.hu += ub * inv;
                 fromb.hv += vb * inv;
                 fromb.h -= (ub * u + vb * v) * inv;
             }
         } else {
-            const double r = from.h / P.h_dry;
-            const double factor = 1.4142135623730951 * r / (P.h_dry * sqrt(1.0 + r * r * r * r));
+            const double r = vdiv(from.h, P.h_dry);
+            const double factor =
+                vdiv(1.4142135623730951 * r, P.h_dry * vsqrt(1.0 + r * r * r * r));
             fromb.hu += ub * factor;
             fromb.hv += vb * factor;
             fromb.h += (ub * from.hu + vb * from.hv) * desing_factor_dh(from.h, P.h_dry);
@@ -511,7 +513,7 @@ DG_PT void damp_velocity_rev(const Physics& P, const DampIn& from, double ub, do
         const bool reg = !fp::gt(from.h, P.h_min);  // lmax(h, h_min) took h_min
         const double h_reg = lmax(from.h, P.h_min);
         const double den = from.h * from.h + h_reg * h_reg;
-        const double factor = 2.0 * from.h / den;
+        const double factor = vdiv(2.0 * from.h, den);
         fromb.hu += ub * factor;
         fromb.hv += vb * factor;
         const double fb = ub * from.hu + vb * from.hv;
@@ -542,8 +544,8 @@ DG_PT void damp_rev(const Physics& P, double g_n2, double h, double hu, double h
         }
     }
     const bool thin = P.has_wet_dry && fp::lt(h, P.h_dry);
-    const double excess = thin ? P.h_dry / h - 1.0 : 0.0;
-    if (thin) rate += excess * excess / P.relaxation_time;
+    const double excess = thin ? vdiv(P.h_dry, h) - 1.0 : 0.0;
+    if (thin) rate += vdiv(excess * excess, P.relaxation_time);
     const double factor = vrcp(1.0 + dt * rate);
     hub += factor * hub_o;
     hvb += factor * hvb_o;

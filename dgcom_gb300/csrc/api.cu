@@ -319,7 +319,7 @@ int boundary_node_tables(dgswe_handle* h, const dgswe_form& f, const Operators& 
     for (int b = 0; b < f.n_boundaries; ++b) {
         if (f.boundaries[b].kind == DGSWE_BC_PARENT) {
             const dgswe_parent_series& ps = *f.boundaries[b].parent;
-            Condition& c = h->P.cond[b];
+            Condition& c = h->conditions[b];
             c.nt_slot0 = slot0[b] = (int64_t)depth.size();
             c.pt_time0 = (int64_t)ptimes.size();
             c.pt_val0 = (int64_t)pvalues.size();
@@ -333,7 +333,7 @@ int boundary_node_tables(dgswe_handle* h, const dgswe_form& f, const Operators& 
         }
         if (f.boundaries[b].kind != DGSWE_BC_NODE_TIDES) continue;
         const dgswe_node_tides& nt = *f.boundaries[b].node_tides;
-        Condition& c = h->P.cond[b];
+        Condition& c = h->conditions[b];
         c.nt_omega0 = (int)omega.size();
         c.nt_slot0 = slot0[b] = (int64_t)mean.size();
         c.nt_coef0 = (int64_t)coef.size();
@@ -636,9 +636,10 @@ int create_impl(dgswe_handle* h, const dgswe_form* f, int device) {
     }
     CK(cudaStreamSynchronize(nullptr));
 #undef UP
-    h->P.n_conditions = f->n_boundaries;
-    for (int b = 0; b < f->n_boundaries; ++b) h->P.cond[b] = make_condition(f->boundaries[b]);
+    for (int b = 0; b < f->n_boundaries; ++b)
+        h->conditions.push_back(make_condition(f->boundaries[b]));
     if ((s = boundary_node_tables(h, *f, ops, topo, t))) return bail(s);
+    if ((s = upload_vec(h, h->conditions, &T.cond))) return bail(s);
     if ((s = relaxation_tables(h, *f))) return bail(s);
     if ((s = atmosphere_tables(h, *f))) return bail(s);
 

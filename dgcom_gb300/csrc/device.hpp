@@ -81,9 +81,11 @@ struct DevTables {
     FxFaceConstants fx_face{};
     int fx_ec = 0, fx_e2g = 0;
     // An ensemble's concatenated members: each element's member (its
-    // StepCtl is ctl[member]) and the members' boundary conditions, which
-    // bface_cond indexes. Both null for one mesh (ctl[0], Physics::cond).
+    // StepCtl is ctl[member]); null for one mesh (ctl[0])
     const int32_t* elem_member = nullptr;
+    // the boundary conditions (an ensemble's: its members' back to back),
+    // which bface_cond indexes: in memory, since 5 KB of them among a
+    // kernel's arguments cost every launch of it
     const struct Condition* cond = nullptr;
     // The adjoint's transpose of the bed slope: per node c, for each
     // direction and line position p, g·D[p][pos_c]·w (x and y) of the node i
@@ -165,8 +167,6 @@ struct Physics {
     double g_n2, manning_h_min;
     int has_coriolis, coriolis_field;
     double f0;
-    int n_conditions;
-    Condition cond[kMaxConditions];
     double x[5], w[5], d[25];  // GLL nodes, weights, D
     int face_node[4][5];
     // launch shapes (dgswe_autotune): the face kernel's threads per block

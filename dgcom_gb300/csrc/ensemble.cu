@@ -243,7 +243,6 @@ int build_group(dgswe_ensemble* h, Group& G, std::vector<Tables>& tabs,
 #undef UP
     G.P.has_bed = h->form0.bathymetry ? 1 : 0;
     G.P.friction = friction ? DGSWE_FRICTION_MANNING_NODES : DGSWE_FRICTION_NONE;
-    G.P.n_conditions = 0;  // the conditions are in T.cond
     // state and stage buffers, face fluxes
     for (int b = 0; b < kEnsBuffers; ++b) {
         double* p = nullptr;

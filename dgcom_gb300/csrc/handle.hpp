@@ -54,6 +54,7 @@ struct dgswe_handle {
     const KernelSet* ks = nullptr;
     DevTables T{};
     Physics P{};
+    std::vector<dgswe::Condition> conditions;  // as uploaded to T.cond
     StageExtra X{};
     std::vector<void*> allocations;
     dgswe::host::DeviceBuffer buf[DGSWE_N_BUFFERS + 1];

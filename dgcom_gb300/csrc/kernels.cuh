@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(256, DGSWE_FAST ? 4 : 2)
     const Q qi = load_q(in, T, P, k * NN + node);
     const double* geo = &T.bface_geo[bfi * 5];
     const double nx = geo[0], ny = geo[1];
-    const Condition& c = T.cond ? T.cond[T.bface_cond[bfi]] : P.cond[T.bface_cond[bfi]];
+    const Condition& c = T.cond[T.bface_cond[bfi]];
     F3 fs;
     double u, v;
     interior_velocity(qi, h_min, u, v);
@@ -538,6 +538,17 @@ __global__ void __launch_bounds__(256) sub_metric_kernel(DevTables T, Physics P,
     }
 }
 
+// The metric at end `at` of a line's subcells: of the interfaces, and of the
+// line's end nodes (0, N1)
+template <int N1>
+__device__ __forceinline__ double subcell_metric(const DevTables& T, int64_t k, int dir, int line,
+                                                 int at, int c) {
+    if (at > 0 && at < N1)
+        return T.sub_metric[2 * ((k * 2 + dir) * N1 * (N1 - 1) + line * (N1 - 1) + at - 1) + c];
+    const int n = line_node(N1, dir, line, at == 0 ? 0 : N1 - 1);
+    return T.contra[(k * N1 * N1 + n) * 4 + 2 * dir + c];
+}
+
 // The two slots of an element's face fluxes that a node takes, in the
 // reference's face order, −1: none. A node lies on at most one s-face (0 or
 // 2) and one r-face (1 or 3).
@@ -726,7 +737,8 @@ __device__ __forceinline__ F3 general_rhs(const DevTables& T, const Physics& P,
             const int pos = dir == 0 ? a : j;
             if (pos + 1 >= N1) continue;
             const int64_t at = k * C::NSUB + (dir * N1 + line) * (N1 - 1) + pos;
-            const double mx = T.sub_metric[2 * at], my = T.sub_metric[2 * at + 1];
+            const double mx = subcell_metric<N1>(T, k, dir, line, pos + 1, 0);
+            const double my = subcell_metric<N1>(T, k, dir, line, pos + 1, 1);
             const double norm = vsqrt(mx * mx + my * my);
             const double inv = vrcp(norm);
             const double geo[5] = {mx, my, norm, mx * inv, my * inv};
@@ -781,20 +793,14 @@ __device__ __forceinline__ F3 general_rhs(const DevTables& T, const Physics& P,
             const double bed = -0.5 * g * (lh + rhh) * (rb - lb) / w_a;
 #endif
             double fx, fy;
-            // the metric at the subcell's two ends: of the interfaces, and of
-            // the line's end nodes
-            auto metric_at = [&](int at, int c) {
-                if (at > 0 && at < N1)
-                    return T.sub_metric[2 * (k * C::NSUB + (dir * N1 + line) * (N1 - 1) + at - 1) + c];
-                const int n = line_node(N1, dir, line, at == 0 ? 0 : N1 - 1);
-                return T.contra[(k * NN + n) * 4 + 2 * dir + c];
-            };
             if (affine) {
-                fx = bed * metric_at(0, 0);
-                fy = bed * metric_at(0, 1);
+                fx = bed * subcell_metric<N1>(T, k, dir, line, 0, 0);
+                fy = bed * subcell_metric<N1>(T, k, dir, line, 0, 1);
             } else {
-                const double ml0 = metric_at(pos, 0), ml1 = metric_at(pos, 1);
-                const double mr0 = metric_at(pos + 1, 0), mr1 = metric_at(pos + 1, 1);
+                const double ml0 = subcell_metric<N1>(T, k, dir, line, pos, 0);
+                const double ml1 = subcell_metric<N1>(T, k, dir, line, pos, 1);
+                const double mr0 = subcell_metric<N1>(T, k, dir, line, pos + 1, 0);
+                const double mr1 = subcell_metric<N1>(T, k, dir, line, pos + 1, 1);
                 const double metric =
 #if DGSWE_FAST
                     0.25 * g * ((rhh + h) * (b - rb) + (lh + h) * (b - lb)) * iw;

@@ -314,10 +314,11 @@ static void stage_adjoint_n(const DevTables& T, const Physics& P, const StageExt
         stage_adjoint_kernel<N1, kAdjWet><<<(unsigned)((T.K + CW::EPB - 1) / CW::EPB),
                                             CW::THREADS, 0, s>>>(T, P, X, in, keep, A, ctl, slot);
     } else {
-        // sized for every element; the blocks past the list's end leave at once
+        // enough for every element, eight blocks a multiprocessor at most
         using CS = AdjCfg<N1, kAdjSub>;
-        stage_adjoint_kernel<N1, kAdjSub><<<(unsigned)((T.K + CS::EPB - 1) / CS::EPB),
-                                            CS::THREADS, 0, s>>>(T, P, X, in, keep, A, ctl, slot);
+        const int64_t all = (T.K + CS::EPB - 1) / CS::EPB;
+        stage_adjoint_kernel<N1, kAdjSub><<<(unsigned)(all < 1216 ? all : 1216), CS::THREADS, 0,
+                                            s>>>(T, P, X, in, keep, A, ctl, slot);
     }
 }
 

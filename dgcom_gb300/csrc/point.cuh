@@ -61,7 +61,8 @@ static __device__ __noinline__ double ieee_cbrt(double x) { return cbrt(x); }
 DG_PT double vsqrt(double x) {
 #if DGSWE_FAST_PATH
     const int64_t b = fp::bits(x);
-    if (b < 0x3810000000000000ll || b >= 0x47E0000000000000ll) return ieee_sqrt(x);  // 2^-126, 2^127
+    if (b < 0x3810000000000000ll || b >= 0x47E0000000000000ll)  // 2^-126, 2^127
+        return b == 0 ? 0.0 : ieee_sqrt(x);
     return fx::sqrt_pos(x);
 #else
     return sqrt(x);
