@@ -193,6 +193,7 @@ struct StageExtra {
 struct DtParams {
     double cfl;
     double bound_cfl, max_cfl, max_cfl_subcells, shallow;
+    float cfl32, bound_cfl32, max_cfl32, max_cfl_subcells32;  // rounded
     int positivity;
 };
 
@@ -228,6 +229,7 @@ struct StepCtl {
     double dt_max, dt_min, cfl;
     double dt_min_used, dt_max_used;
     unsigned long long dt_bits;  // atomicMin of the element steps
+    unsigned dt_up;              // and of upper bounds of them (float bits; dt_min_kernel)
     long long steps, max_steps, clips;
     int active;     // the current step runs
     int landed;

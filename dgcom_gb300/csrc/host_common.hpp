@@ -51,6 +51,10 @@ inline DtParams dt_params(const dgswe_form& f, double cfl, int scheme) {
     d.max_cfl = std::fmax(bound, 0.9 * lin);
     d.max_cfl_subcells = std::fmax(bound, 0.9 * sub);
     d.shallow = 100.0 * f.positivity_h_dry;
+    d.cfl32 = (float)d.cfl;
+    d.bound_cfl32 = (float)d.bound_cfl;
+    d.max_cfl32 = (float)d.max_cfl;
+    d.max_cfl_subcells32 = (float)d.max_cfl_subcells;
     return d;
 }
 

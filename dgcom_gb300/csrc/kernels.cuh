@@ -1589,23 +1589,11 @@ struct DtCfg {
 // The element's dt from its largest rate and its nodes' depths and mass
 // weights (element_dt, swe_2d.rs:2072-2115, with PositivityBound::element_cfl
 // and positivity_relaxation, swe_2d.rs:2220-2258)
-template <int N1>
 __device__ __forceinline__ double element_dt(const DtParams& D, int order, double weight_ratio,
-                                             double rmax, const double* h, const double* mass) {
-    constexpr int NN = N1 * N1;
+                                             double rmax, double water, double water_b,
+                                             bool shallow) {
     double cfl = D.cfl;
     if (D.positivity) {
-        double water = 0.0, water_b = 0.0;
-        bool shallow = false;
-#pragma unroll
-        for (int p = 0; p < NN; ++p) {
-            const double hp = h[p];
-            shallow = shallow || fp::le(hp, D.shallow);
-            const double wi = mass[p] * fp::max0(hp);
-            water += wi;
-            constexpr int last = N1 - 1;
-            if (p % N1 == 0 || p % N1 == last || p / N1 == 0 || p / N1 == last) water_b += wi;
-        }
         // f64::min drops the NaN of 0/0
         const double ratio =
             fp::le0(water_b) ? weight_ratio : lmin(water / water_b, weight_ratio);
@@ -1614,6 +1602,21 @@ __device__ __forceinline__ double element_dt(const DtParams& D, int order, doubl
         cfl = lmin(cfl, lmin(D.bound_cfl * rho, cap));
     }
     return fp::lt(rmax, 1e-14) ? INFINITY : cfl / ((2.0 * (double)order + 1.0) * rmax);
+}
+
+// Whether node p lies on the element's boundary
+template <int N1>
+__device__ __forceinline__ constexpr bool boundary_node(int p) {
+    return p % N1 == 0 || p % N1 == N1 - 1 || p / N1 == 0 || p / N1 == N1 - 1;
+}
+
+// The water over the element's nodes and over its boundary nodes, in node
+// order, every product and sum rounded on its own (two kernels take it and
+// the step must have the same bits from both)
+__device__ __forceinline__ void add_water(double wi, bool boundary, double& water,
+                                          double& water_b) {
+    water = __dadd_rn(water, wi);
+    if (boundary) water_b = __dadd_rn(water_b, wi);
 }
 
 // LISTED: the elements list[0..n_list) (any order, any subset), else all
@@ -1721,8 +1724,17 @@ __global__ void __launch_bounds__(DtCfg<N1>::THREADS)
     int member = -1;
     if (kl < T.K) {
         const double rmax = fp::from_bits((int64_t)s_rmax[tid]);
-        const double dt = element_dt<N1>(D, P.order, T.weight_ratio[kl], rmax, &s_h[tid * PITCH],
-                                         &s_mass[tid * PITCH]);
+        double water = 0.0, water_b = 0.0;
+        bool shallow = false;
+        if (D.positivity)
+#pragma unroll
+            for (int p = 0; p < NN; ++p) {
+                const double hp = s_h[tid * PITCH + p];
+                shallow = shallow || fp::le(hp, D.shallow);
+                add_water(__dmul_rn(s_mass[tid * PITCH + p], fp::max0(hp)), boundary_node<N1>(p),
+                          water, water_b);
+            }
+        const double dt = element_dt(D, P.order, T.weight_ratio[kl], rmax, water, water_b, shallow);
         if (dt_el) dt_el[kl] = dt;
         dt_bits = (unsigned long long)fp::bits(dt);
         member = T.elem_member ? T.elem_member[kl] : 0;
@@ -1741,6 +1753,139 @@ __global__ void __launch_bounds__(DtCfg<N1>::THREADS)
     if (member >= 0 && (tid == 0 || below != member)) atomicMin(&ctl[member].dt_bits, dt_bits);
 }
 
+// The smallest step alone, where no element's own is asked for: the same
+// bits as dt_kernel's minimum. Every element's step is bracketed in single
+// precision (its largest rate between max(r₃₂ ∓ δ·B), its water ratio within
+// 2⁻¹⁶); the smallest upper end so far, of all blocks, is kept beside the
+// smallest step, and only an element whose lower end is not above it is
+// taken in FP64. A few hundred elements are, and what remains is memory: 112 B
+// a node. An element has LANES lanes of one warp, each with at most a node
+// and a face slot.
+template <int N1>
+struct DtLanes {
+    static constexpr int LANES = N1 == 2 ? 8 : (N1 == 5 ? 32 : 16);
+    static constexpr int EPB = 256 / LANES;
+};
+
+template <int N1, bool LISTED>
+__global__ void __launch_bounds__(256)
+    dt_min_kernel(DevTables T, Physics P, DevBuf q, DtParams D, StepCtl* ctl, const int* active,
+                  const int32_t* list, int64_t n_list) {
+    constexpr int NN = N1 * N1, LANES = DtLanes<N1>::LANES, EPB = DtLanes<N1>::EPB;
+    if (!*active) return;
+    const int lane = threadIdx.x % LANES;
+    const int64_t at = (int64_t)blockIdx.x * EPB + threadIdx.x / LANES;
+    const int64_t k = LISTED ? (at < n_list ? (int64_t)list[at] : T.K) : at;
+    const bool mine = k < T.K;
+    StepCtl* const cm = ctl + ((T.elem_member && mine) ? T.elem_member[k] : 0);
+    constexpr float kDelta = 1.0f / 65536.0f, kFloor = 1e-30f;  // δ = 2⁻¹⁶, as dt_kernel's
+    const float g32 = f32_trunc(P.g);
+    const int64_t gi = k * NN + lane, o = k * 4 * N1 + lane;
+    const bool node = mine && lane < NN, slot = mine && lane < 4 * N1;
+    double h = 0.0, mass = 0.0, u = 0.0, v = 0.0;
+    double hf = 0.0, uf = 0.0, vf = 0.0;
+    float m[6], mf[6];
+    const int64_t nb = slot ? T.nb_face_node[o] : -1;
+    if (node) {
+        h = q.h[gi];
+        u = q.u[gi];
+        v = q.v[gi];
+        mass = T.mass[gi];
+        const float2* t = (const float2*)&T.dtm32_own[gi * 6];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float2 x = t[c];
+            m[2 * c] = x.x;
+            m[2 * c + 1] = x.y;
+        }
+    }
+    if (nb >= 0) {
+        hf = q.h[nb];
+        uf = q.u[nb];
+        vf = q.v[nb];
+        const float2* t = (const float2*)&T.dtm32_face[o * 6];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float2 x = t[c];
+            mf[2 * c] = x.x;
+            mf[2 * c + 1] = x.y;
+        }
+    }
+    // the rates in single precision, −1 for a dry or missing node
+    float r = -1.0f, b = 0.0f, rf = -1.0f, bf = 0.0f;
+    if (node && fp::gt(h, P.h_min)) {
+        node_rate_f32(h, u, v, m, g32, r, b);
+        b = kDelta * b + kFloor;
+    }
+    if (nb >= 0 && fp::gt(hf, P.h_min)) {
+        node_rate_f32(hf, uf, vf, mf, g32, rf, bf);
+        bf = kDelta * bf + kFloor;
+    }
+    float lo = fmaxf(fmaxf(r - b, rf - bf), 0.0f), up = fmaxf(fmaxf(r + b, rf + bf), 0.0f);
+    const bool edge = boundary_node<N1>(lane);
+    const float w32 = node ? f32_trunc(mass) * f32_trunc(fp::max0(h)) : 0.0f;
+    float water32 = w32, water_b32 = edge ? w32 : 0.0f;
+    unsigned thin = node && fp::le(h, D.shallow) ? 1u : 0u;
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) {
+        lo = fmaxf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+        up = fmaxf(up, __shfl_xor_sync(0xffffffffu, up, off));
+        water32 += __shfl_xor_sync(0xffffffffu, water32, off);
+        water_b32 += __shfl_xor_sync(0xffffffffu, water_b32, off);
+        thin |= __shfl_xor_sync(0xffffffffu, thin, off);
+    }
+    // the step between its bounds; each factor's rounding is within 2⁻²⁰
+    const double weight_ratio = mine ? T.weight_ratio[k] : 1.0;
+    float cfl_lo = D.cfl32, cfl_up = D.cfl32;
+    if (D.positivity) {
+        constexpr float kRatio = 1.0f / 65536.0f;
+        const float wr = f32_trunc(weight_ratio);
+        const float cap = thin ? D.max_cfl_subcells32 : D.max_cfl32;
+        // water that single precision flushes: any ratio from 0 to the weights'
+        const bool some = water_b32 > 1e-30f;
+        const float ratio = some ? fminf(water32 / water_b32, wr) : wr;
+        const float rho_lo = some ? fmaxf(0.9f * ratio * (1.0f - kRatio), 1.0f) : 1.0f;
+        const float rho_up = fmaxf(0.9f * ratio * (1.0f + kRatio), 1.0f);
+        cfl_lo = fminf(cfl_lo, fminf(D.bound_cfl32 * rho_lo, cap));
+        cfl_up = fminf(cfl_up, fminf(D.bound_cfl32 * rho_up, cap));
+    }
+    constexpr float kStep = 1.0f / 131072.0f;  // 2⁻¹⁷
+    const float n21 = 2.0f * (float)P.order + 1.0f;
+    const float dt_lo = up > 0.0f ? cfl_lo / (n21 * up) * (1.0f - kStep) : INFINITY;
+    const float dt_up = lo > 1e-13f ? cfl_up / (n21 * lo) * (1.0f + kStep) : INFINITY;
+    unsigned best = 0x7F800000u;  // +∞; the bits of floats ≥ 0 order as they do
+    if (mine) {
+        best = *(volatile unsigned*)&cm->dt_up;
+        if (lane == 0 && __float_as_uint(dt_up) < best) atomicMin(&cm->dt_up, __float_as_uint(dt_up));
+        best = min(best, __float_as_uint(dt_up));
+    }
+    const bool exact = mine && __float_as_uint(dt_lo) <= best;
+    if (!__any_sync(0xffffffffu, exact)) return;
+    unsigned long long rmax = 0ull;  // the bits of rates ≥ +0
+    if (exact && r >= 0.0f && r + b >= lo)
+        rmax = (unsigned long long)fp::bits(node_rate(h, u, v, &T.dtm_own[gi * 6], P.g));
+    if (exact && rf >= 0.0f && rf + bf >= lo) {
+        const unsigned long long x =
+            (unsigned long long)fp::bits(node_rate(hf, uf, vf, &T.dtm_face[o * 6], P.g));
+        rmax = x > rmax ? x : rmax;
+    }
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, rmax, off);
+        rmax = x > rmax ? x : rmax;
+    }
+    const double wi = __dmul_rn(mass, fp::max0(h));
+    double water = 0.0, water_b = 0.0;
+    if (D.positivity)
+        for (int p = 0; p < NN; ++p)
+            add_water(__shfl_sync(0xffffffffu, wi, p, LANES), boundary_node<N1>(p), water, water_b);
+    if (exact && lane == 0) {
+        const double dt = element_dt(D, P.order, weight_ratio, fp::from_bits((int64_t)rmax), water,
+                                     water_b, thin != 0u);
+        atomicMin(&cm->dt_bits, (unsigned long long)fp::bits(dt));
+    }
+}
+
 // ---------------------------------------------------------------------------
 // the run's clock on the device (Simulation::run_with_callback's loop body,
 // src/simulation/runner.rs:355-450)
@@ -1753,6 +1898,7 @@ __global__ void step_begin(StepCtl* ctl, int n) {
     if (m >= n) return;
     StepCtl* c = ctl + m;
     c->dt_bits = 0x7FF0000000000000ull;  // +∞
+    c->dt_up = 0x7F800000u;
     bool run = c->failure == 0 && c->t < c->target;
     if (run && c->max_steps > 0 && c->steps >= c->max_steps) {
         c->failure = kFailMaxSteps;

@@ -167,6 +167,12 @@ static void finish_listed_n(const DevTables& T, const Physics& P, const DevBuf& 
 template <int N1>
 static void dt_n(const DevTables& T, const Physics& P, const DevBuf& q, const DtParams& D,
                  double* dt_el, StepCtl* ctl, const int* active, cudaStream_t s) {
+    if (!dt_el) {
+        constexpr int EPB = DtLanes<N1>::EPB;
+        dt_min_kernel<N1, false><<<(unsigned)((T.K + EPB - 1) / EPB), 256, 0, s>>>(
+            T, P, q, D, ctl, active, nullptr, 0);
+        return;
+    }
     using C = DtCfg<N1>;
     const unsigned blocks = (unsigned)((T.K + C::EPB - 1) / C::EPB);
     dt_kernel<N1, false><<<blocks, C::THREADS, 0, s>>>(T, P, q, D, dt_el, ctl, active, nullptr, 0);
@@ -176,8 +182,14 @@ template <int N1>
 static void dt_listed_n(const DevTables& T, const Physics& P, const DevBuf& q, const DtParams& D,
                         double* dt_el, StepCtl* ctl, const int* active, const int32_t* list,
                         int64_t n, cudaStream_t s) {
-    using C = DtCfg<N1>;
     if (n <= 0) return;
+    if (!dt_el) {
+        constexpr int EPB = DtLanes<N1>::EPB;
+        dt_min_kernel<N1, true><<<(unsigned)((n + EPB - 1) / EPB), 256, 0, s>>>(T, P, q, D, ctl,
+                                                                               active, list, n);
+        return;
+    }
+    using C = DtCfg<N1>;
     const unsigned blocks = (unsigned)((n + C::EPB - 1) / C::EPB);
     dt_kernel<N1, true><<<blocks, C::THREADS, 0, s>>>(T, P, q, D, dt_el, ctl, active, list, n);
 }

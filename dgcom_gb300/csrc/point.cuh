@@ -418,8 +418,13 @@ DG_PT void reconstruct(const Sd& m, const Sd& c, const Sd& p, double x0,
 DG_PT double node_rate(double h, double u, double v, const double* m,
                                             double g) {
     const double c = vsqrt(g * fp::max0(h));
+#if DGSWE_FAST_PATH  // two kernels take it: the same contraction in both
+    const double lr = fma(c, m[4], fabs(fma(u, m[0], v * m[1])));
+    const double ls = fma(c, m[5], fabs(fma(u, m[2], v * m[3])));
+#else
     const double lr = fabs(u * m[0] + v * m[1]) + c * m[4];
     const double ls = fabs(u * m[2] + v * m[3]) + c * m[5];
+#endif
     return lr + ls;
 }
 
