@@ -46,12 +46,14 @@ UNIT = "DOF-updates/s"
 BYTES_PER_NODE_STAGE = {2: 81.8, 3: 77.5}  # algorithmic bytes (state, bed, mesh), N=2 / N=3
 # stage_kernel<4>'s DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per
 # node-stage in one ncu capture of the 200k-quad coastal box, for scaling by nodes
-STAGE_TRAFFIC_PER_NODE_STAGE = {3: 187.3}
+STAGE_TRAFFIC_PER_NODE_STAGE = {3: 179.3}
 # FP64 floating-point operations the step's kernels execute per node (an FMA
 # as 2): ncu's dadd + dmul + 2·dfma instruction counts of one capture of the
-# 200k-quad coastal box at N = 3 — the stage and face kernels per stage (three
-# a step) and the dt kernel once a step
-FP64_FLOPS_PER_NODE = {3: {"stage": 157.4, "face": 77.1, "dt": 11.4}}
+# 200k-quad coastal box at N = 3 — the stage (with the subcell elements'
+# kernel) and face kernels per stage (three a step) and the dt kernel once a
+# step. The rest of the stage's and the faces' arithmetic is fixed point on
+# the integer pipes (157.4 + 77.1 a node-stage with all of it in FP64).
+FP64_FLOPS_PER_NODE = {3: {"stage": 23.7, "face": 14.3, "dt": 4.1}}
 
 
 def fp64_gemm_tflops(device: int, n: int = 6144, reps: int = 5) -> float | None:
@@ -438,8 +440,9 @@ def run_ours(args, rank: int, world: int, local: int):
                          "traffic": (STAGE_TRAFFIC_PER_NODE_STAGE[args.order] * nodes
                                      if args.order in STAGE_TRAFFIC_PER_NODE_STAGE else None),
                          "peak_kind": peak_kind, "kernel": f"stage_kernel<{args.order + 1}>",
-                         "note": "bound by the FP64 pipe (86.9 % of it in ncu), not HBM; traffic "
-                                 "from an ncu capture at 200k quads scaled by nodes"},
+                         "note": "bound by the integer and FP64 pipes together (50 to 53 % of "
+                                 "each in ncu, 60 % of issue slots), not HBM; traffic from an "
+                                 "ncu capture at 200k quads scaled by nodes"},
             "fp64": fp64,
             "kernel_ms": {"stage": timed.stage_ms / args.steps, "face": timed.face_ms / args.steps,
                           "dt": timed.dt_ms / args.steps, "control": timed.control_ms / args.steps},

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(AdjCfg<N1, PATH>::THREADS, AdjCfg<N1, PATH>::M
     const int a = i % N1, j = i / N1;
     const double g = P.g, h_min = P.h_min, sqrt_g = P.sqrt_g, half_g = P.half_g;
     // the wet pass: one element each; the subcell pass: the stage's list, in
-    // strides of the grid
+    // strides of the grid (the loop is the whole kernel, not indented for it)
     const unsigned long long n_sub = PATH == kAdjSub ? A.sub_count[slot] : 1ull;
     for (unsigned long long at = (PATH == kAdjSub ? blockIdx.x : 0) * (unsigned long long)EPB;
          at < n_sub; at += (unsigned long long)gridDim.x * EPB) {

@@ -149,8 +149,8 @@ int ensure_dt_stream(dgswe_handle* h) {
 
 // A step's dt pass and fit on the dt stream beside its first stage's face
 // pass on the handle's stream: both read the step's start state; the face
-// pass is held by the FP64 pipe and the dt pass by memory, so the one hides
-// the other. The first stage's time comes from step_begin, so the face pass
+// pass is held by the arithmetic pipes and the dt pass by memory, so the one
+// hides the other. The first stage's time comes from step_begin, so the face pass
 // needs nothing from the fit. The stage pass that follows waits for both.
 int dt_beside_first_face(dgswe_handle* h, const DtParams& D, const int* active) {
     CK(cudaEventRecord(h->dt_fork, h->stream));
@@ -1118,7 +1118,7 @@ int dgswe_step_host(dgswe_handle* h, int32_t scheme, double t, double cfl, doubl
             h->ks->velocity(part, (int64_t)cnt, h->P.h_min, h->stream);
         }
         const int64_t e0 = h->ready_elem_off[c], e1 = h->ready_elem_off[c + 1];
-        h->ks->dt_listed(h->n1, h->T, h->P, q, D, nullptr, h->ctl, active, h->ready_elems + e0,
+        h->ks->dt_listed(h->n1, h->T, h->P, q, D, h->ctl, active, h->ready_elems + e0,
                          e1 - e0, h->stream);
         const int64_t f0 = h->ready_edge_off[c], f1 = h->ready_edge_off[c + 1];
         const int64_t b0 = h->ready_bface_off[c], b1 = h->ready_bface_off[c + 1];

@@ -170,8 +170,8 @@ struct Physics {
     double x[5], w[5], d[25];  // GLL nodes, weights, D
     int face_node[4][5];
     // launch shapes (dgswe_autotune): the face kernel's threads per block
-    // and the stage kernel's shape (0: ⌊128/nn⌋ elements a block, 5 blocks
-    // per SM; 1: ⌊64/nn⌋ elements a block, 10 blocks per SM)
+    // and the stage kernel's shape (0: ⌊128/nn⌋ elements a block; 1: ⌊64/nn⌋
+    // at twice the blocks per SM; 2: ⌊128/nn⌋ at 6 blocks per SM)
     int face_threads = 256;
     int stage_shape = 0;
 };

@@ -2,9 +2,13 @@
 //
 // This file is compiled twice (kernels_fast.cu, kernels_exact.cu) into two
 // namespaces: DGSWE_FAST = 1 lets the compiler contract multiply-adds into
-// FMA (-fmad=true) and evaluates the Manning rate without divisions; 0 keeps
-// every multiply and add separately rounded (-fmad=false) and follows the
-// reference's arithmetic, its cube root included. Both are FP64 throughout.
+// FMA (-fmad=true), evaluates the Manning rate without divisions, and does
+// the wet elements' volume term, the wet faces' fluxes and every square root
+// and quotient in 62-bit fixed point on the integer pipes (fixed64.hpp: an
+// FP64 warp instruction holds its pipe for 64 cycles here, the time of some
+// thirty integer multiply-adds); 0 keeps every multiply and add separately
+// rounded FP64 (-fmad=false) and follows the reference's arithmetic, its cube
+// root included. Neither holds or sums anything in less than FP64's 53 bits.
 //
 // Kernels of one stage (one RK stage of every element):
 //  - face_kernel: the numerical flux F* of every interior edge node once,
@@ -20,10 +24,15 @@
 //    Coriolis, the Shu–Osher combination, the point-implicit damping and the
 //    wet/dry correction or the accumulation (the reference's fused
 //    stage_where, src/physics/builder.rs:652-737), and the node velocities
-//    the next stage reads.
-// Per step: dt_kernel<N1> (element steps, atomic minimum) and three
-// one-thread kernels that run the step's clock on the device, so that a
-// whole step is one CUDA graph.
+//    the next stage reads;
+//  - with DGSWE_FAST, general_kernel<N1>: the same for the elements that fixed
+//    point leaves (subcells with water, depths spread too far), listed by
+//    stage_kernel or, beside the face pass, by shallow_list_kernel.
+// Per step: dt_min_kernel<N1> (the smallest element step; dt_kernel<N1> where
+// every element's is asked for) and three one-thread kernels that run the
+// step's clock on the device, so that a whole step is one CUDA graph. Once
+// per handle, fixed_tables_kernel (the mesh's fixed-point tables) and
+// sub_metric_kernel (the subcells' geometry).
 //
 // The volume and surface terms use the summation-by-parts identity of the
 // GLL operators: at a line end the volume term's 2·D₀₀·F(q)·Ja and the
@@ -283,14 +292,17 @@ __device__ __forceinline__ double weather_level(const DevTables& T, const Physic
     return inverse_barometer_level(p, tidal_ramp(t, T.at_ramp), T.at_rho_water);
 }
 
+// A thread a face node. In FP64 the pipe was full (86 % of it; 0.348 ms for
+// 200,000 quads at N = 3); in fixed point the integer pipes and the FP64
+// pipe (the rotations, the conversions, faces that fixed point leaves) share
+// the work at 62-65 % each and 0.111 ms. Four blocks an SM (64 registers)
+// against three or two: 10.48, 10.72, 11.16 ms over 60 passes.
 // LISTED: a multirate pass's faces (lp's edge and boundary-face lists),
 // each boundary face at its element's stage time
 template <int N1, bool LISTED>
 __global__ void __launch_bounds__(256, DGSWE_FAST ? 4 : 2)
-    face_kernel(DevTables T, Physics P, DevBuf in, double* fb_h,
-                                                   double* fb_hu, double* fb_hv,
-                                                   const StepCtl* ctl, int slot,
-                                                   const int* active, LtsPass lp) {
+    face_kernel(DevTables T, Physics P, DevBuf in, double* fb_h, double* fb_hu, double* fb_hv,
+                const StepCtl* ctl, int slot, const int* active, LtsPass lp) {
     if (!*active) return;
     const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t n_int = (LISTED ? lp.n_edges : T.n_edges) * N1;
@@ -1619,11 +1631,11 @@ __device__ __forceinline__ void add_water(double wi, bool boundary, double& wate
     if (boundary) water_b = __dadd_rn(water_b, wi);
 }
 
-// LISTED: the elements list[0..n_list) (any order, any subset), else all
-template <int N1, bool LISTED>
+// Every element's step into dt_el, and the smallest
+template <int N1>
 __global__ void __launch_bounds__(DtCfg<N1>::THREADS)
     dt_kernel(DevTables T, Physics P, DevBuf q, DtParams D, double* dt_el, StepCtl* ctl,
-              const int* active, const int32_t* list, int64_t n_list) {
+              const int* active) {
     using C = DtCfg<N1>;
     constexpr int NN = C::NN, EPB = C::EPB, PITCH = C::PITCH, SLOTS = C::SLOTS;
     __shared__ int64_t s_k[EPB];                      // the block's elements
@@ -1638,8 +1650,7 @@ __global__ void __launch_bounds__(DtCfg<N1>::THREADS)
     if (!*active) return;
     const int tid = threadIdx.x;
     const int e = tid / NN, i = tid % NN;
-    const int64_t at = (int64_t)blockIdx.x * EPB + e;
-    const int64_t k = LISTED ? (at < n_list ? (int64_t)list[at] : T.K) : at;
+    const int64_t k = (int64_t)blockIdx.x * EPB + e;
     if (i == 0) s_k[e] = k;
     const int64_t gi = k * NN + i;
     const double g = P.g, h_min = P.h_min;
@@ -1735,7 +1746,7 @@ __global__ void __launch_bounds__(DtCfg<N1>::THREADS)
                           water, water_b);
             }
         const double dt = element_dt(D, P.order, T.weight_ratio[kl], rmax, water, water_b, shallow);
-        if (dt_el) dt_el[kl] = dt;
+        dt_el[kl] = dt;
         dt_bits = (unsigned long long)fp::bits(dt);
         member = T.elem_member ? T.elem_member[kl] : 0;
     }
@@ -1759,8 +1770,10 @@ __global__ void __launch_bounds__(DtCfg<N1>::THREADS)
 // 2⁻¹⁶); the smallest upper end so far, of all blocks, is kept beside the
 // smallest step, and only an element whose lower end is not above it is
 // taken in FP64. A few hundred elements are, and what remains is memory: 112 B
-// a node. An element has LANES lanes of one warp, each with at most a node
-// and a face slot.
+// a node, read at 58 % of the DRAM's rate (0.062 ms for 200,000 quads at
+// N = 3, where dt_kernel takes 0.146). An element has LANES lanes of one warp,
+// each with at most a node and a face slot.
+// LISTED: the elements list[0..n_list) (any order, any subset), else all
 template <int N1>
 struct DtLanes {
     static constexpr int LANES = N1 == 2 ? 8 : (N1 == 5 ? 32 : 16);

@@ -65,7 +65,9 @@ static void face_listed_n(const DevTables& T, const Physics& P, const DevBuf& in
 
 #if DGSWE_FAST
 // general_kernel's blocks for a pass of `count` elements, of which it takes
-// those listed: enough for all, four a multiprocessor at most
+// those listed: enough for all, and at most the four on each of the 152
+// multiprocessors that run at once (the rest of a longer list comes in their
+// next rounds; an empty list then costs 608 blocks' start, 2.5 µs)
 template <int N1>
 static unsigned general_blocks(int64_t count) {
     const int64_t all = (count + GenCfg<N1>::EPB - 1) / GenCfg<N1>::EPB;
@@ -175,23 +177,17 @@ static void dt_n(const DevTables& T, const Physics& P, const DevBuf& q, const Dt
     }
     using C = DtCfg<N1>;
     const unsigned blocks = (unsigned)((T.K + C::EPB - 1) / C::EPB);
-    dt_kernel<N1, false><<<blocks, C::THREADS, 0, s>>>(T, P, q, D, dt_el, ctl, active, nullptr, 0);
+    dt_kernel<N1><<<blocks, C::THREADS, 0, s>>>(T, P, q, D, dt_el, ctl, active);
 }
 
 template <int N1>
 static void dt_listed_n(const DevTables& T, const Physics& P, const DevBuf& q, const DtParams& D,
-                        double* dt_el, StepCtl* ctl, const int* active, const int32_t* list,
-                        int64_t n, cudaStream_t s) {
+                        StepCtl* ctl, const int* active, const int32_t* list, int64_t n,
+                        cudaStream_t s) {
     if (n <= 0) return;
-    if (!dt_el) {
-        constexpr int EPB = DtLanes<N1>::EPB;
-        dt_min_kernel<N1, true><<<(unsigned)((n + EPB - 1) / EPB), 256, 0, s>>>(T, P, q, D, ctl,
-                                                                               active, list, n);
-        return;
-    }
-    using C = DtCfg<N1>;
-    const unsigned blocks = (unsigned)((n + C::EPB - 1) / C::EPB);
-    dt_kernel<N1, true><<<blocks, C::THREADS, 0, s>>>(T, P, q, D, dt_el, ctl, active, list, n);
+    constexpr int EPB = DtLanes<N1>::EPB;
+    dt_min_kernel<N1, true><<<(unsigned)((n + EPB - 1) / EPB), 256, 0, s>>>(T, P, q, D, ctl,
+                                                                           active, list, n);
 }
 
 // The face fluxes of the listed interior edges and boundary faces of a
@@ -258,9 +254,9 @@ static void node_sources(const DevTables& T, const Physics& P, const DevBuf& in,
 }
 
 static void dt_listed(int n1, const DevTables& T, const Physics& P, const DevBuf& q,
-                      const DtParams& D, double* dt_el, StepCtl* ctl, const int* active,
-                      const int32_t* list, int64_t n, cudaStream_t s) {
-    DGSWE_BY_ORDER(dt_listed_n, T, P, q, D, dt_el, ctl, active, list, n, s);
+                      const DtParams& D, StepCtl* ctl, const int* active, const int32_t* list,
+                      int64_t n, cudaStream_t s) {
+    DGSWE_BY_ORDER(dt_listed_n, T, P, q, D, ctl, active, list, n, s);
 }
 
 static void stage(int n1, const DevTables& T, const Physics& P, const StageExtra& X,

@@ -39,7 +39,7 @@ constexpr int kIncomingWave = 1;
 //
 // Every compare, minimum and maximum of doubles on the per-node paths goes
 // through fp:: (fp64_bits.hpp): the same result on the integer pipes, which
-// leaves the FP64 pipe, the stage's bound, to arithmetic.
+// leaves the FP64 pipe, the slowest by far, to arithmetic.
 
 using fp::lmax;
 using fp::lmin;

@@ -101,9 +101,11 @@ enum dgswe_scheme {
 };
 
 /* Device arithmetic, FP64 throughout. FAST contracts multiply-adds into FMA,
- * takes square roots and reciprocals within an ulp of the correctly rounded
- * value (a single-precision seed refined in FP64) and the Manning rate's
- * h^(-4/3) from one third-order FP64 step, with no division; EXACT keeps
+ * takes square roots, reciprocals and the Manning rate's h^(-4/3) within an
+ * ulp of the correctly rounded value in 64-bit fixed point, and the wet
+ * elements' volume terms and the wet faces' fluxes in 62-bit fixed point
+ * scaled per element and face node (their error against an extended-precision result is
+ * below FP64's); EXACT keeps
  * every multiply and add separately rounded, uses IEEE division and square
  * root and follows the reference's cube root
  * (src/source/swe_2d/friction.rs:39-70). */
@@ -617,8 +619,8 @@ int dgswe_planner_spread(dgswe_planner* planner, uint8_t* levels, int32_t limit,
 /* Launch shapes of a handle's kernels, chosen by timing them on its own
  * mesh and state (an autotuner): the face kernel's threads per
  * block (64, 128 or 256) and the stage kernel's elements per block
- * (shape 0: ⌊128/(N+1)²⌋ at 5 blocks per SM; 1: ⌊64/(N+1)²⌋ at 10; 2:
- * ⌊128/(N+1)²⌋ at 6). The shapes change no result (tests compare them bit
+ * (shape 0: ⌊128/(N+1)²⌋ at 7 blocks per SM, EXACT at 5; 1:
+ * ⌊64/(N+1)²⌋ at twice that; 2: ⌊128/(N+1)²⌋ at 6). The shapes change no result (tests compare them bit
  * for bit). No reference counterpart. */
 typedef struct dgswe_tuning {
     int32_t face_threads;      /* chosen */
