@@ -474,8 +474,17 @@ __device__ __forceinline__ void prefetch(const void* p) {
 // general_kernel: two lanes a node
 template <int N1>
 struct GenCfg {
-    static constexpr int EPB = 128 / (2 * N1 * N1) > 0 ? 128 / (2 * N1 * N1) : 1;
-    static constexpr int THREADS = EPB * 2 * N1 * N1;
+    static constexpr int LANES = 2 * N1 * N1;
+    static constexpr int EPB = 128 / LANES > 0 ? 128 / LANES : 1;
+    static constexpr int THREADS = EPB * LANES;
+    // Where an element's lanes straddle warps (N1 = 3), a warp waits for the
+    // branches of up to three; as few elements as two a sub-partition have a
+    // warp each instead (the block's last, two lanes short, holds one too): a
+    // 4,000-quad drying channel's run 89.0 → 82.7 ms, a 50,000-quad box's the
+    // same. At N1 = 2, where four fit a warp, that was 2 % slower (a
+    // 90,000-quad storm, 129.9 → 132.7 ms).
+    static constexpr bool SPREAD = LANES < 32 && 32 % LANES != 0;
+    static constexpr unsigned FEW = 2 * 4 * 152;
 };
 
 __device__ __forceinline__ int line_node(int n1, int dir, int line, int pos) {
@@ -1334,13 +1343,18 @@ __global__ void __launch_bounds__(GenCfg<N1>::THREADS, 4)
     __shared__ int s_flag[EPB][2];
     __shared__ double s_red[EPB][4];
     const int tid = threadIdx.x;
-    const int e = tid / LANES, lane = tid % LANES, half = lane / NN, i = lane % NN;
-    double(*const s_q)[NN] = (double(*)[NN])s_x[e];
     const int32_t* elements = T.gen_list + list * T.K;
     unsigned* const count = T.gen_count + 2 * list;
     const unsigned n = *active ? *(volatile unsigned*)count : 0u;
-    for (unsigned first = blockIdx.x * EPB; first < n; first += gridDim.x * EPB) {
-        const bool listed = first + e < n;
+    // where they are few, a warp each
+    constexpr int WARPS = (GenCfg<N1>::THREADS + 31) / 32;
+    const bool spread = GenCfg<N1>::SPREAD && n <= GenCfg<N1>::FEW && n <= gridDim.x * WARPS;
+    const int stride = spread ? 32 : LANES;
+    const unsigned per_block = spread ? WARPS : EPB;
+    const int e = tid / stride, lane = tid % stride, half = lane / NN, i = lane % NN;
+    double(*const s_q)[NN] = (double(*)[NN])s_x[e];
+    for (unsigned first = blockIdx.x * per_block; first < n; first += gridDim.x * per_block) {
+        const bool listed = first + e < n && lane < LANES;
         const int64_t k = listed ? (int64_t)elements[first + e] : 0;
         StepCtl* const cm = ctl + ((T.elem_member && listed) ? T.elem_member[k] : 0);
         const bool take = listed && (!T.elem_member || cm->active);

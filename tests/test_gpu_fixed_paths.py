@@ -101,6 +101,28 @@ def test_a_runs_step_is_the_smallest_element_step(numerics, order, kind):
         dev.close()
 
 
+@pytest.mark.parametrize("nx, ny, shallow", [(37, 5, 0), (37, 5, 1), (37, 5, 107), (37, 5, 108),
+                                             (37, 5, 109), (37, 5, 185), (400, 20, 1216),
+                                             (400, 20, 1217)])
+def test_subcell_lists_of_any_length(nx, ny, shallow):
+    """At order 2 a short list of subcell elements has a warp for each (up to
+    four a block of the launch, and 1216 in all), a longer one packs them."""
+    form = cases.tidal_channel(nx=nx, ny=ny, order=2).form
+    dev, ref = SWEPhysics2D(form, 0), oracle(form)
+    try:
+        rng = np.random.default_rng(11)
+        h = 0.5 + rng.random((nx * ny, 9))
+        h[rng.permutation(nx * ny)[:shallow], 4] = 1e-4
+        h = h.reshape(-1)
+        for s in (dev, ref):
+            s.upload(h, 0.4 * h, -0.2 * h)
+        err = rel_err(dev.compute_rhs_into(0.0), ref.compute_rhs_into(0.0))
+        assert err <= TOL_RHS, f"relative RHS difference {err:.3e}"
+    finally:
+        dev.close()
+        ref.close()
+
+
 @pytest.mark.parametrize("members", [1, 3])
 @pytest.mark.parametrize("order", [2, 3])
 def test_a_run_equals_its_calls(order, members):
