@@ -29,7 +29,8 @@ struct alignas(16) FxPair {
     FxLimb x, y;
 };
 struct alignas(16) FxExp {
-    int32_t et, eg, el, ok;
+    int32_t et, eg, el;
+    int32_t ok;  // 0: not usable; else fx::own_deficits
 };
 // A node's pairs, a byte each: the other nodes of the ones it owns, the slots
 // of all it is in

@@ -337,17 +337,23 @@ DG_HD double convert(int64_t v, int s) {
 //   h          2^(62 − eh)       exact: the element's depths lie within 2^9
 //   hu, hv     2^(60 − em)       (u, v at 2^(61 − ev)); exact down to 2^-8
 //   pair metric 2^(62 − et), bed slope 2^(62 − eg), lift 2^(61 − el)
-//   mass flux of a pair 2^(58 − em − et), its momentum flux 2^(58 − eP − et),
+//   mass flux of a pair 2^(58 − em − et), its momentum flux 2^(59 − eP − et),
 //   eP covering 2g·h² and the advected momentum, whichever is larger
-// Every sum stays below 2^63 with its last place below 2^-57 of the largest
-// term, where FP64 rounds each operation at 2^-53 of its result.
+// Every sum stays below 2^63. Its last place is one for all of an element's
+// nodes, where FP64 rounds each node's operations at 2^-53 of their own
+// results: where a node's own terms are so small beside the element's that FP64
+// would be closer (thin_depth, thin and own_mass_small below), it is FP64 that
+// takes them.
 
 struct Exps {  // biased exponent fields over an element; 0: all zero
     int h_max, h_min, m, v, fh, fm;  // depth, momentum, velocity, face fluxes
+    int h_top = 15;                  // the deepest node's four bits after the leading one
+    int h_key = 0, m_key = 0;        // the smallest node's depth and momentum as key() has them
 };
 
 struct Scale {
     bool ok;
+    int eP, em;
     int kh, km, ku;   // to_fixed's K of h, of hu and hv, of u and v
     int g_shift;      // of 2g·h, and of the bed slope's products
     int b_shift;
@@ -358,7 +364,21 @@ struct Scale {
 // exponent fields within 2^±120 (beyond it the element takes FP64)
 constexpr int kExpLo = 1023 - 120, kExpHi = 1023 + 120;
 
-DG_HD Scale scales(const Exps& x, const FxExp& t, int ec, int e2g) {
+// The sign, the exponent field and four bits of the mantissa: for x > 0 a
+// lower bound of 16·(log2 x + 1023), at most 2.4 below it
+DG_HD int key(double x) { return (int)((uint64_t)fp::bits(x) >> 48); }
+constexpr int kKeyOne = 16 * 1023;
+
+// The least e with 2g·h² < 2^e by the deepest node's leading bits (top of the
+// 64ths above 2g·2^-e2g): e2g + 2·eh, or up to two less
+DG_HD int pressure_exponent(int h_max, int h_top, int e2g, int two_g_64ths) {
+    const unsigned x = 17u + (unsigned)h_top;  // h < x·2^(eh − 5)
+    const unsigned p = x * x * (unsigned)two_g_64ths;  // 2g·h² < p·2^(e2g + 2·eh − 16)
+    return e2g + 2 * (h_max - 1022) + (int)(p > 16384u) + (int)(p > 32768u) +
+           (int)(p > 65536u) - 2;
+}
+
+DG_HD Scale scales(const Exps& x, const FxExp& t, int ec, int e2g, int two_g_64ths = 64) {
     Scale s;
     s.ok = t.ok && x.h_max <= kExpHi && x.h_max >= kExpLo && x.h_min >= x.h_max - 9 &&
            x.m <= kExpHi && (x.m == 0 || x.m >= kExpLo) && x.v <= kExpHi && x.fh <= kExpHi &&
@@ -367,29 +387,119 @@ DG_HD Scale scales(const Exps& x, const FxExp& t, int ec, int e2g) {
     const int lift = t.el - t.et - ec - 1022;
     int em = (x.m > kExpLo ? x.m : kExpLo) - 1022;
     if (x.fh && em < x.fh + lift + 1) em = x.fh + lift + 1;
-    int eP = e2g + 2 * eh;
+    int eP = pressure_exponent(x.h_max, x.h_top, e2g, two_g_64ths);
     if (x.v && eP < em + x.v - 1022 + 3) eP = em + x.v - 1022 + 3;
-    if (x.fm && eP < x.fm + lift + 2) eP = x.fm + lift + 2;
+    if (x.fm && eP < x.fm + lift + 3) eP = x.fm + lift + 3;
     const int steep = t.eg + eh + 1 - t.et - ec;
     if (eP < steep) eP = steep;
+    s.eP = eP;
+    s.em = em;
     s.kh = 1023 + eh;
     s.km = 1025 + em;
     s.ku = 1021 + eP - em;
     s.g_shift = eP - e2g - 2 * eh;
     s.b_shift = eP - steep;
     s.sh = 60 - em - t.et - ec;
-    s.sm = 61 - eP - t.et - ec;
+    s.sm = 62 - eP - t.et - ec;
     s.kfh = 1082 - s.sh - t.el;
     s.kfm = 1082 - s.sm - t.el;
     return s;
 }
 
-// 2g·h at 2^(62 − eP + eh) from h and 2g (two_g: at 2^(62 − e2g))
+// Whether FP64 is closer to an element's nodes than these sums. Fixed point
+// rounds a node's sum at its last place, FP64 at 2^-53 of the node's largest
+// term, so the line is drawn at how many of these places that term has: over
+// elements of orders 1 to 4 with depths in the ratio 1 to 512, sides in the
+// ratio 1 to 32, sheared and still currents (tests/fixed64_nodes_check.cpp) the
+// root mean square error against extended precision passes FP64's at 2^52 to
+// 2^52.3 places and halves with each further bit. A lower bound of the term
+// stands for it, in sixteenths of its log2, and metrics that are made with the
+// tables (FxExp::ok):
+//  - momentum: the pressure of the shallowest node with itself, 2g·h_min²·W, W
+//    the smallest over the nodes and both components of the largest
+//    ½|coefficient·metric|;
+//  - mass: twice the slowest node's momentum across its lines, 4·m_min·V, V the
+//    least over the nodes and the directions of a current. The bound is far
+//    below the term where a few nodes are at rest among moving ones, so where it
+//    fails each node looks at its fluxes themselves (own_mass_small).
+// An element whose momentum is too close takes FP64 whole, a node whose mass is
+// takes that alone.
+// Elements of even depth have 53.3 bits or more on the meshes here, so that
+// depths in the ratio 1.3 (order 4, the least favourable scale) to 2 still stay.
+constexpr int kMomentumBits = 16 * 52 + 4, kMassBits = 16 * 52 + 8;
+
+// How much smaller than 2^(et + ec) W and V are, a half word each: FxExp::ok of
+// a usable element (not 0)
+struct OwnMetric {
+    int w, v;  // the keys of a node's, then of an element's
+};
+DG_HD OwnMetric own_metric(const double* hm, const int32_t* slots, const double* coefs, int na) {
+    double w0 = 0.0, w1 = 0.0, v = 0.0;
+    for (int q = 0; q < na; ++q) {
+        const double c = 0.5 * fabs(coefs[q]);
+        const double a0 = c * hm[2 * slots[q]], a1 = c * hm[2 * slots[q] + 1];
+        w0 = fmax(w0, fabs(a0));
+        w1 = fmax(w1, fabs(a1));
+        for (int p = 0; p < q; ++p) {  // a current across at most one of two lines
+            const double d = 0.5 * fabs(coefs[p]);
+            const double b0 = d * hm[2 * slots[p]], b1 = d * hm[2 * slots[p] + 1];
+            const double size = fabs(a0) + fabs(a1) + fabs(b0) + fabs(b1);
+            if (size > 0.0) v = fmax(v, fabs(a0 * b1 - a1 * b0) / size);
+        }
+    }
+    return {key(fmin(w0, w1)), key(v)};
+}
+DG_HD int own_deficits(const OwnMetric& m, int et, int ec) {
+    int w = 16 * (et + ec) - (m.w - kKeyOne), v = 16 * (et + ec) - (m.v - kKeyOne);
+    w = w < 0 ? 0 : (w > 0x7FFE ? 0x7FFE : w);
+    v = v < 0 ? 0 : (v > 0x7FFF ? 0x7FFF : v);
+    return (v << 16) | (w + 1);
+}
+
+DG_HD bool thin_at(int eP, int h_key, const FxExp& t, int two_g_key) {
+    return 16 * (62 - eP) + (two_g_key - kKeyOne) + 2 * (h_key - kKeyOne) -
+               ((t.ok & 0x7FFF) - 1) < kMomentumBits;
+}
+
+// By the depths alone, which are known before the face fluxes
+DG_HD bool thin_depth(const Exps& x, const FxExp& t, int e2g, int two_g_64ths, int two_g_key) {
+    return thin_at(pressure_exponent(x.h_max, x.h_top, e2g, two_g_64ths), x.h_key, t, two_g_key);
+}
+
+// By all that goes into the scale
+DG_HD bool thin(const Exps& x, const Scale& s, const FxExp& t, int two_g_key) {
+    return thin_at(s.eP, x.h_key, t, two_g_key);
+}
+
+// Whether the mass fluxes have to be looked at
+DG_HD bool slow_node(const Exps& x, const Scale& s, const FxExp& t) {
+    return (x.m | x.fh) != 0 && 16 * (62 - s.em) + (x.m_key - kKeyOne) - (t.ok >> 16) < kMassBits;
+}
+
+// A node's largest mass term so far (in 2^4 places of its sum), from a pair's
+// coefficient and flux, and from a lifted face flux
+DG_HD void own_mass(int64_t& own, const Lim& coef, const Lim& f) {
+    const int64_t p = mads(coef.hi, f.hi, 0);
+    const int64_t a = (p < 0 ? -p : p) | ((f.lo | f.hi) != 0);
+    own = own > a ? own : a;
+}
+DG_HD void own_mass(int64_t& own, int64_t lifted) {
+    const int64_t v = lifted < 0 ? -lifted : lifted;
+    const int64_t a = (v >> 4) | (v != 0);
+    own = own > a ? own : a;
+}
+// too small, unless the node has no flux at all
+DG_HD bool own_mass_small(int64_t own) {
+    return own != 0 && own < 398000000000000ll;  // 2^48.5
+}
+
+// 2g·h at 2^(62 − eP + eh), below 2^63, from h and 2g (two_g: at 2^(62 − e2g))
 DG_HD Lim two_g_h(const Lim& H, const Lim& two_g, const Scale& s) {
     Acc a{half<2>(), 0};
     mac(a, H, two_g);
     const int64_t v = fold<2>(a);
-    return split(shr(v, s.g_shift));
+    const int up = s.g_shift < 0 ? -s.g_shift : 0;
+    return split(shr((int64_t)((uint64_t)v << up), s.g_shift + up));
 }
 
 struct Flux {
@@ -409,22 +519,22 @@ DG_HD Flux pair_flux(const Lim& G, const Lim& H, int64_t M0, int64_t M1, int64_t
     Acc p{half<0>(), 0};
     mac(p, G, H);
     const Lim gp = split(fold<0>(p));
-    Acc b{half<0>(), 0};
+    Acc b{half<1>(), 0};
     mac(b, f.h, split(U0));
     mac(b, gp, m0);
-    f.hu = split(fold<0>(b));
-    Acc c{half<0>(), 0};
+    f.hu = split(fold<1>(b));
+    Acc c{half<1>(), 0};
     mac(c, f.h, split(U1));
     mac(c, gp, m1);
-    f.hv = split(fold<0>(c));
+    f.hv = split(fold<1>(c));
     return f;
 }
 
 // h times the bed slope at the momentum sums' scale
 DG_HD int64_t bed_term(const Lim& H, const Lim& slope, const Scale& s) {
-    Acc a{half<0>(), 0};
+    Acc a{half<1>(), 0};
     mac(a, H, slope);
-    return shr(fold<0>(a), s.b_shift);
+    return shr(fold<1>(a), s.b_shift);
 }
 
 // V·2^-s/J as a double

@@ -8,7 +8,10 @@
 // FP64 warp instruction holds its pipe for 64 cycles here, the time of some
 // thirty integer multiply-adds); 0 keeps every multiply and add separately
 // rounded FP64 (-fmad=false) and follows the reference's arithmetic, its cube
-// root included. Neither holds or sums anything in less than FP64's 53 bits.
+// root included. A wet element's sums have one last place for all its nodes in
+// fixed point; where that is further from a node's result than FP64's rounding,
+// FP64 takes the element or the node (fixed64.hpp), so that no node's error is
+// above FP64's.
 //
 // Kernels of one stage (one RK stage of every element):
 //  - face_kernel: the numerical flux F* of every interior edge node once,
@@ -856,18 +859,44 @@ __device__ __forceinline__ F3 general_rhs(const DevTables& T, const Physics& P,
 }
 
 #if DGSWE_FAST
-// Exponent fields (a negative depth's sign with it, which no scale takes),
-// two a word: depth and 4095 − depth, momentum and velocity, the mass and
-// momentum of face fluxes. Their maxima over an element's nodes and face
-// slots give the element's fx::Exps.
+// A node's pair and lift terms of the mass by the FP64 formulas, for a slow node
+// of an element in fixed point (a few in a thousand; listing the element for
+// general_kernel instead made its launch behind every stage 6 µs longer)
+template <int N1>
+__device__ __forceinline__ double mass_sum(const DevTables& T, const DevBuf& in,
+                                           const double* fb_h, uint64_t slots, int64_t k, int i,
+                                           int s_a, int s_b) {
+    constexpr int NN = N1 * N1, NP = N1 - 1, NA = 2 * NP;
+    const double hu = in.hu[k * NN + i], hv = in.hv[k * NN + i];
+    double r = 0.0;
+#pragma unroll 2
+    for (int q = 0; q < NA; ++q) {
+        const int slot = (int)((slots >> (8 * q)) & 0xFF), owner = slot / NP;
+        const int other = (T.fx_node[owner].others >> (8 * (slot - owner * NP))) & 0xFF;
+        const int64_t o = k * NN + (owner == i ? other : owner);
+        const double* hm = &T.pair_hm[(k * NN * NP + slot) * 2];
+        r -= T.sched_coef[i * NA + q] * ((hu + in.hu[o]) * hm[0] + (hv + in.hv[o]) * hm[1]);
+    }
+    const int64_t fbase = k * 4 * N1;
+    if (s_a >= 0) r -= T.lift_scale[fbase + s_a] * fb_h[fbase + s_a];
+    if (s_b >= 0) r -= T.lift_scale[fbase + s_b] * fb_h[fbase + s_b];
+    return r;
+}
+
+// Two a word: the depth's key (a negative depth's sign with it, which no scale
+// takes) and 65535 less it, the same of the momentum, the exponent fields of the
+// velocity and of the face fluxes' mass and momentum. Their maxima over an
+// element's nodes and face slots give the element's fx::Exps.
 struct ExpWords {
-    unsigned w[3];
+    unsigned w[4];
 };
+
+__device__ __forceinline__ unsigned both_ends(unsigned key) { return key | (65535u - key) << 16; }
 
 __device__ __forceinline__ ExpWords node_exponents(double h, double hu, double hv, double u,
                                                    double v) {
-    const unsigned hb = (unsigned)((uint64_t)fp::bits(h) >> 52);
-    return {{hb | (4095u - hb) << 16, (unsigned)(max_expo(hu, hv) | max_expo(u, v) << 16), 0u}};
+    const unsigned m = max(fx::key(hu) & 0x7FFF, fx::key(hv) & 0x7FFF);
+    return {{both_ends((unsigned)fx::key(h)), both_ends(m), (unsigned)max_expo(u, v), 0u}};
 }
 
 // The maxima over each NN lanes of a warp
@@ -876,13 +905,38 @@ __device__ __forceinline__ void warp_max(ExpWords& e) {
 #pragma unroll
     for (int off = NN / 2; off > 0; off >>= 1)
 #pragma unroll
-        for (int q = 0; q < 3; ++q)
+        for (int q = 0; q < 4; ++q)
             e.w[q] = __vmaxu2(e.w[q], __shfl_xor_sync(0xffffffffu, e.w[q], off));
 }
 
+// The depths' part of an element's exponents from their keys' maxima
+__device__ __forceinline__ fx::Exps depth_exponents(unsigned w) {
+    fx::Exps x{};
+    const int deepest = (int)(w & 0xFFFFu);
+    x.h_key = 65535 - (int)(w >> 16);
+    x.h_max = deepest >> 4;
+    x.h_min = x.h_key >> 4;
+    x.h_top = deepest & 15;
+    return x;
+}
+
 __device__ __forceinline__ fx::Exps exponents(const ExpWords& e) {
-    return {(int)(e.w[0] & 0xFFFFu), 4095 - (int)(e.w[0] >> 16), (int)(e.w[1] & 0xFFFFu),
-            (int)(e.w[1] >> 16),     (int)(e.w[2] & 0xFFFFu),    (int)(e.w[2] >> 16)};
+    fx::Exps x = depth_exponents(e.w[0]);
+    x.m = (int)(e.w[1] & 0xFFFFu) >> 4;
+    x.m_key = 65535 - (int)(e.w[1] >> 16);
+    x.v = (int)e.w[2];
+    x.fh = (int)(e.w[3] & 0xFFFFu);
+    x.fm = (int)(e.w[3] >> 16);
+    return x;
+}
+
+// Of 2g, the 64ths above it and its key (fx::scales)
+__device__ __forceinline__ int two_g_64ths(const DevTables& T) { return (T.fx_two_g.hi >> 24) + 1; }
+
+// Whether an element's depths alone take it to FP64 (fx::thin_depth)
+__device__ __forceinline__ bool thin_depth(const DevTables& T, const Physics& P, const FxExp& t,
+                                           const fx::Exps& x) {
+    return t.ok != 0 && fx::thin_depth(x, t, T.fx_e2g, two_g_64ths(T), fx::key(P.two_g));
 }
 
 // The fixed-point tables of each element from its FP64 ones: a warp per
@@ -890,7 +944,7 @@ __device__ __forceinline__ fx::Exps exponents(const ExpWords& e) {
 template <int N1>
 __global__ void __launch_bounds__(256) fixed_tables_kernel(DevTables T, FxPair* hm, FxPair* gdb,
                                                            FxLimb* lift, FxExp* exps) {
-    constexpr int NN = N1 * N1, NH = NN * (N1 - 1), NL = 4 * N1;
+    constexpr int NN = N1 * N1, NH = NN * (N1 - 1), NL = 4 * N1, NA = 2 * (N1 - 1);
     const int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (k >= T.K) return;
@@ -904,6 +958,12 @@ __global__ void __launch_bounds__(256) fixed_tables_kernel(DevTables T, FxPair* 
     et = __reduce_max_sync(0xffffffffu, et);
     eg = __reduce_max_sync(0xffffffffu, eg);
     el = __reduce_max_sync(0xffffffffu, el);
+    fx::OwnMetric own{0x7FFF, 0x7FFF};
+    for (int n = lane; n < NN; n += 32) {
+        const fx::OwnMetric o = fx::own_metric(m, &T.sched_slot[n * NA], &T.sched_coef[n * NA], NA);
+        own = {min(own.w, o.w), min(own.v, o.v)};
+    }
+    own = {__reduce_min_sync(0xffffffffu, own.w), __reduce_min_sync(0xffffffffu, own.v)};
     const bool ok = et >= fx::kExpLo && et <= fx::kExpHi && el >= fx::kExpLo && el <= fx::kExpHi &&
                     eg <= fx::kExpHi;
     eg = max(eg, fx::kExpLo - 400);  // a flat bed: no slope to scale by
@@ -915,7 +975,9 @@ __global__ void __launch_bounds__(256) fixed_tables_kernel(DevTables T, FxPair* 
     for (int q = lane; q < NN; q += 32)
         gdb[k * NN + q] = b ? pair(b[2 * q], b[2 * q + 1], eg + 1) : FxPair{};
     for (int q = lane; q < NL; q += 32) lift[k * NL + q] = fx::split(fx::to_fixed(l[q], el + 2));
-    if (lane == 0) exps[k] = {et - 1022, eg - 1022, el - 1022, ok ? 1 : 0};
+    if (lane == 0)
+        exps[k] = {et - 1022, eg - 1022, el - 1022,
+                   ok ? fx::own_deficits(own, et - 1022, T.fx_ec) : 0};
 }
 #endif
 
@@ -1104,9 +1166,10 @@ __device__ __forceinline__ void finish_node(const DevTables& T, const Physics& P
 // The wet elements of a stage in fixed point, and those without water at any
 // node, which only their faces' fluxes reach (their reconstructed subcell
 // faces are dry, so the interface fluxes, pressure and bed terms are all ±0).
-// Any other with subcells, and one whose depths or exponents spread too far,
+// Any other with subcells, and one that fixed point leaves to FP64 (fixed64.hpp),
 // goes into T.gen_list's second half for general_kernel, launched behind
-// (shallow_listed: those with subcells are in its first half already, and a
+// (shallow_listed: those with subcells, and those left by their depths, are in its
+// first half already, and a
 // general_kernel takes them beside this kernel): inside this kernel its few hundred FP64
 // operations in a row (a call, so spills on the wet path; one busy warp to a
 // block's end) cost 17 % of a 50,000-quad coastal box's stage.
@@ -1126,7 +1189,7 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
     __shared__ double s_x[EPB][C::XF];
     __shared__ int s_flag[EPB][3];
     __shared__ double s_red[EPB][4];
-    __shared__ unsigned s_exp[kInWarp ? 1 : EPB][6];
+    __shared__ unsigned s_exp[kInWarp ? 1 : EPB][8];
 
     const int run = *active;
     const int tid = threadIdx.x;
@@ -1173,7 +1236,7 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
     ExpWords ew = node_exponents(h, hu, hv, u, v);
 #pragma unroll
     for (int q = 0; q < NS; ++q)
-        ew.w[2] = __vmaxu2(ew.w[2], (unsigned)(fx::expo(flux[q][0]) |
+        ew.w[3] = __vmaxu2(ew.w[3], (unsigned)(fx::expo(flux[q][0]) |
                                                max_expo(flux[q][1], flux[q][2]) << 16));
     const bool shallow = valid && P.formulation == kWetDry && fp::lt(h, P.subcell_depth);
     // sub: the element has a node below the subcell depth; dry: no water at any
@@ -1185,28 +1248,35 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
         warp_max<NN>(ew);
     } else {
         if (i < 2) s_flag[e][i] = 0;
-        if (i < 6) s_exp[e][i] = 0;
+        for (int q = i; q < 8; q += NN) s_exp[e][q] = 0;
         __syncthreads();
         if (shallow) {
             atomicOr(&s_flag[e][0], 1);
             if (!fp::nz(h)) atomicAdd(&s_flag[e][1], 1);
         }
-        for (int q = 0; q < 3; ++q) {
+        for (int q = 0; q < 4; ++q) {
             atomicMax(&s_exp[e][2 * q], ew.w[q] & 0xFFFFu);
-            atomicMax(&s_exp[e][2 * q + 1], ew.w[q] >> 16);
+            if (q != 2) atomicMax(&s_exp[e][2 * q + 1], ew.w[q] >> 16);
         }
         __syncthreads();
         sub = s_flag[e][0] != 0;
         dry = s_flag[e][1] == NN;
-        for (int q = 0; q < 3; ++q) ew.w[q] = s_exp[e][2 * q] | s_exp[e][2 * q + 1] << 16;
+        for (int q = 0; q < 4; ++q) ew.w[q] = s_exp[e][2 * q] | s_exp[e][2 * q + 1] << 16;
     }
-    bool fixed = false;
+    // fixed: the element's right-hand side comes from here; slow: the mass of a
+    // node may not; by_depth: its depths alone leave it
+    bool fixed = false, slow = false, by_depth = false;
     fx::Scale sc;
     if (valid && !sub) {
-        sc = fx::scales(exponents(ew), T.fx_exp[k], T.fx_ec, T.fx_e2g);
-        fixed = sc.ok;
+        const FxExp t = T.fx_exp[k];
+        const fx::Exps x = exponents(ew);
+        sc = fx::scales(x, t, T.fx_ec, T.fx_e2g, two_g_64ths(T));
+        fixed = sc.ok && !fx::thin(x, sc, t, fx::key(P.two_g));
+        slow = fixed && fx::slow_node(x, sc, t);
+        if (slow) prefetch(&T.pair_hm[gi * NP * 2]);
+        by_depth = P.formulation == kWetDry && thin_depth(T, P, t, x);
     }
-    if (valid && !fixed && !dry && i == 0 && !(sub && shallow_listed))
+    if (valid && !fixed && !dry && i == 0 && !((sub || by_depth) && shallow_listed))
         T.gen_list[T.K + atomicAdd(&T.gen_count[2], 1u)] = (int32_t)k;
 
     FxLimb G{}, H{};                         // 2g·h, h
@@ -1284,6 +1354,17 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
             }
         const double jinv = T.jinv[gi];
         F.h = fx::over_jacobian(fh, sc.sh, jinv);
+        if (slow) {  // a node whose own mass terms are too small takes them in FP64
+            int64_t own = 0;
+#pragma unroll 1
+            for (int q = 0; q < NA; ++q)
+                fx::own_mass(own, T.fx_coef[i * NA + q],
+                             pairs[(int)((node.slots >> (8 * q)) & 0xFF) * 3]);
+            if (s_a >= 0) fx::own_mass(own, lifted[s_a]);
+            if (s_b >= 0) fx::own_mass(own, lifted[s_b]);
+            if (fx::own_mass_small(own))
+                F.h = jinv * mass_sum<N1>(T, in, fb_h, node.slots, k, i, s_a, s_b);
+        }
         F.hu = fx::over_jacobian(fhu, sc.sm, jinv);
         F.hv = fx::over_jacobian(fhv, sc.sm, jinv);
         if (X.subcell_mass)  // no subcells: NaN (compute_rhs_swe_2d_mass_fluxes_into)
@@ -1299,28 +1380,49 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
                                 i, fixed || dry, F, s_q, &s_flag[e][2], s_red[e]);
 }
 
-// A stage's elements with subcells and water, from its input, into T.gen_list's
-// first half: beside the face pass, so that general_kernel can take them
-// beside the stage pass
+// A stage's elements with subcells and water and those whose depths leave them
+// to FP64, from its input, into T.gen_list's first half: beside the face pass, so
+// that general_kernel can take them beside the stage pass
 template <int N1>
 __global__ void __launch_bounds__(256)
     shallow_list_kernel(DevTables T, Physics P, DevBuf in, const StepCtl* ctl,
                         const int* active) {
     constexpr int NN = N1 * N1, EPB = 256 / NN;
     __shared__ int s_flag[EPB][2];
+    __shared__ unsigned s_key[EPB][2];
     if (!*active) return;
     const int e = threadIdx.x / NN, i = threadIdx.x % NN;
     const int64_t k = (int64_t)blockIdx.x * EPB + e;
     const bool valid = e < EPB && k < T.K && (!T.elem_member || ctl[T.elem_member[k]].active);
     const double h = valid ? in.h[k * NN + i] : 0.0;
-    if (e < EPB && i < 2) s_flag[e][i] = 0;
-    __syncthreads();
-    if (valid && fp::lt(h, P.subcell_depth)) {
-        atomicOr(&s_flag[e][0], 1);
-        if (!fp::nz(h)) atomicAdd(&s_flag[e][1], 1);
+    const bool shallow = valid && fp::lt(h, P.subcell_depth);
+    unsigned ends = both_ends((unsigned)fx::key(h));
+    bool sub, dry;
+    if (kElementInWarp<NN>) {
+        const unsigned lanes = (unsigned)(((1ull << NN) - 1) << ((threadIdx.x & 31) / NN * NN));
+        sub = (__ballot_sync(0xffffffffu, shallow) & lanes) != 0;
+        dry = (__ballot_sync(0xffffffffu, shallow && !fp::nz(h)) & lanes) == lanes;
+#pragma unroll
+        for (int off = NN / 2; off > 0; off >>= 1)
+            ends = __vmaxu2(ends, __shfl_xor_sync(0xffffffffu, ends, off));
+    } else {
+        if (e < EPB && i < 2) s_flag[e][i] = 0, s_key[e][i] = 0;
+        __syncthreads();
+        if (e < EPB) {
+            atomicMax(&s_key[e][0], ends & 0xFFFFu);
+            atomicMax(&s_key[e][1], ends >> 16);
+        }
+        if (shallow) {
+            atomicOr(&s_flag[e][0], 1);
+            if (!fp::nz(h)) atomicAdd(&s_flag[e][1], 1);
+        }
+        __syncthreads();
+        if (e >= EPB) return;
+        sub = s_flag[e][0] != 0;
+        dry = s_flag[e][1] == NN;
+        ends = s_key[e][0] | s_key[e][1] << 16;
     }
-    __syncthreads();
-    if (valid && i == 0 && s_flag[e][0] && s_flag[e][1] != NN)
+    if (valid && i == 0 && (sub ? !dry : thin_depth(T, P, T.fx_exp[k], depth_exponents(ends))))
         T.gen_list[atomicAdd(&T.gen_count[0], 1u)] = (int32_t)k;
 }
 

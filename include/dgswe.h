@@ -104,8 +104,10 @@ enum dgswe_scheme {
  * takes square roots, reciprocals and the Manning rate's h^(-4/3) within an
  * ulp of the correctly rounded value in 64-bit fixed point, and the wet
  * elements' volume terms and the wet faces' fluxes in 62-bit fixed point
- * scaled per element and face node (their error against an extended-precision result is
- * below FP64's); EXACT keeps
+ * scaled per element and face node, or in FP64 where that is closer to a node's
+ * result (shallow or slow nodes of elements whose depths or currents vary
+ * strongly): against an extended-precision result no node's error is above
+ * FP64's; EXACT keeps
  * every multiply and add separately rounded, uses IEEE division and square
  * root and follows the reference's cube root
  * (src/source/swe_2d/friction.rs:39-70). */
