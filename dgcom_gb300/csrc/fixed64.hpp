@@ -548,10 +548,10 @@ DG_HD double over_jacobian(int64_t V, int s, double jinv) {
 //
 // hydro_hll (point.cuh) with at least one reconstructed side wet, each
 // quantity at a scale of the face node's own exponents (E: |x| < 2^E):
-//   surface sums 2^(60 − eL) (eL: depths and beds), reconstructed depths
-//   2^(62 − es), own depths 2^(62 − eh), velocities 2^(60 − ev) and 2^(62 − ev),
-//   speeds of waves 2^(60 − eS), momenta 2^(60 − es − ev), mass flux
-//   2^(58 − eM), momentum flux 2^(58 − eQ), weights 2^62.
+//   surface sums 2^(62 − eL) (eL: depths and beds), reconstructed depths
+//   2^(62 − es), velocities 2^(60 − ev) and 2^(62 − ev), speeds of waves
+//   2^(60 − eS), momenta 2^(60 − es − ev), mass flux 2^(58 − eM), momentum flux
+//   2^(59 − eQ), weights 2^62.
 // With S_L and S_R the wave speeds held to S_L ≤ 0 ≤ S_R, α = S_R/(S_R − S_L),
 // β = 1 − α and w = −α·S_L, the flux is
 //   α·F_l + β·F_r − w·(q_r − q_l),
@@ -571,6 +571,7 @@ struct FaceFlux {
 DG_HD int64_t min64(int64_t a, int64_t b) { return a < b ? a : b; }
 DG_HD int64_t max64(int64_t a, int64_t b) { return a > b ? a : b; }
 DG_HD int imax(int a, int b) { return a > b ? a : b; }
+DG_HD int imin(int a, int b) { return a < b ? a : b; }
 DG_HD int64_t shl(int64_t v, int n) { return (int64_t)((uint64_t)v << n); }
 DG_HD int64_t abs64(int64_t v) { return v < 0 ? -v : v; }
 
@@ -622,21 +623,25 @@ DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const double* geo,
     const int xv = imax(imax(expo(na), expo(ta)), imax(expo(nb), expo(tb)));
     // within 2^±120 (a negative depth's sign field is above), h_min not above
     // everything
-    if (imax(xv, xl) > kExpHi || xh < kExpLo || expo(h_min) > xl + 2) return kNoScale;
-    const int eL = xl - 1022, eh = xh - 1022;
-    // hydrostatic reconstruction: the surfaces over the higher bed
-    const int64_t la = to_fixed_nn(qa.h, xl + 3), lb = to_fixed_nn(qb.h, xl + 3);
-    const int64_t ba = to_fixed(qa.b, xl + 3), bb = to_fixed(qb.b, xl + 3);
+    if (imax(xv, xl) > kExpHi || xh < kExpLo || expo(h_min) > xl) return kNoScale;
+    const int eL = xl - 1022;
+    // hydrostatic reconstruction: the depths less the step up to the higher bed
+    const int64_t la = to_fixed_nn(qa.h, xl + 1), lb = to_fixed_nn(qb.h, xl + 1);
+    const int64_t ba = to_fixed(qa.b, xl + 1), bb = to_fixed(qb.b, xl + 1);
     const int64_t top = max64(ba, bb);
-    const int64_t ra = max64(la + ba - top, 0), rb = max64(lb + bb - top, 0);
-    const int64_t dry = to_fixed_nn(h_min, xl + 3);
+    const int64_t ra = max64(la + (ba - top), 0), rb = max64(lb + (bb - top), 0);
+    const int64_t dry = to_fixed_nn(h_min, xl + 1);
     const bool wet_a = ra > dry, wet_b = rb > dry;
     if (!wet_a && !wet_b) return kBothDry;
-    const int es = 4 + eL - clz64((uint64_t)(ra | rb));
+    const int es = 2 + eL - clz64((uint64_t)(ra | rb));
     const int eC = (es + c.e_g + 1) >> 1;
-    const int ev = imax(xv - 1022, eC - 30);
+    const int ev = imax(xv - 1022, -120);
     if (es < -60 || ev > eC + 30) return kNoScale;
-    const int64_t sa = shl(ra, eL - es + 2), sb = shl(rb, eL - es + 2);
+    // films left of much deeper water by a step, their surface at the datum: the
+    // FP64 sums h + B are exact there, these only to 2^-62 of the deep side
+    if (ba != bb && es < eL - 6 && (max64(abs64(la + ba), abs64(lb + bb)) >> 56) == 0)
+        return kNoScale;
+    const int64_t sa = shl(ra, eL - es), sb = shl(rb, eL - es);
     const int kv = 1025 + ev;
     const int64_t un_a = to_fixed(na, kv), ut_a = to_fixed(ta, kv);  // 2^(60 − ev)
     const int64_t un_b = to_fixed(nb, kv), ut_b = to_fixed(tb, kv);
@@ -646,9 +651,9 @@ DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const double* geo,
     const int64_t va = wet_a ? un_a : 0, vb = wet_b ? un_b : 0;
     const int64_t u_m = vb + mul<2>(split(share(c_a, c_b)), split(va - vb));
     const int eS = imax(ev, eC) + 2;
-    const int dv = eS - ev, dc = eS - eC - 2;  // at most 32
+    const int dv = eS - ev, dc = eS - eC - 2;  // dc at most 30
     const int64_t wa = c_a >> dc, wb = c_b >> dc, wm = c_m >> dc;
-    const int64_t xl_ = va >> dv, xr_ = vb >> dv, xm = u_m >> dv;
+    const int64_t xl_ = shr(va, dv), xr_ = shr(vb, dv), xm = shr(u_m, dv);
     const int64_t s_l = min64(wet_a ? min64(xl_ - wa, xm - wm) : xr_ - 2 * wb, 0);
     const int64_t s_r = max64(wet_b ? max64(xr_ + wb, xm + wm) : xl_ + 2 * wa, 0);
     if (s_l == s_r) return kNoScale;
@@ -665,7 +670,7 @@ DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const double* geo,
     // mass
     const int64_t dh = sb - sa;
     const int grow = clz64((uint64_t)abs64(dh)) - 2;  // dh·2^grow below 2^62
-    const int eD = es - grow;
+    const int eD = dh ? es - grow : es - 300;
     const int eM = imax(es + ev + 1, eS + eD);
     Acc f{half<0>(), 0};
     mac(f, al, ml);
@@ -674,36 +679,42 @@ DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const double* geo,
                         shr(mul<0>(w, split(shl(dh, grow))), 2 + eM - eS - eD);
     out.h = geo[2] * convert(f_h, 58 - eM);
     // momentum
-    const int eQ = imax(imax(2 * eh + c.e_half_g + 1, es + 2 * ev + 1), eS + es + ev);
-    const int dm = eQ - es - 2 * ev, dw = eQ - eS - es - ev;
-    auto pressure = [&](int64_t x, int64_t y, int e) {  // ½g·x·y of depths at 2^(62 − e)
-        return shr(mul<0>(split(mul<0>(split(x), split(y))), c.half_g), eQ - 2 * e - c.e_half_g);
+    const int eQ = imax(imax(2 * es + c.e_half_g + 1, es + 2 * ev + 1), eS + es + ev);
+    const int dp = eQ - 2 * es - c.e_half_g, dm = eQ - es - 2 * ev, dw = eQ - eS - es - ev;
+    auto pressure = [&](int64_t x) {  // ½g·x² of a depth at 2^(62 − es)
+        const Lim l = split(x);
+        return shr(mul<1>(split(mul<0>(l, l)), c.half_g), dp);
     };
     Acc g{half<2>(), 0};
-    mac(g, al, split(pressure(sa, sa, es) + shr(mul<0>(ml, ul), dm)));
-    mac(g, be, split(pressure(sb, sb, es) + shr(mul<0>(mr, ur), dm)));
-    const int64_t f_n = fold<2>(g) - shr(mul<0>(w, split(m_b - m_a)), dw);
+    mac(g, al, split(pressure(sa) + shr(mul<1>(ml, ul), dm)));
+    mac(g, be, split(pressure(sb) + shr(mul<1>(mr, ur), dm)));
+    const double f_n = convert(fold<2>(g) - shr(mul<1>(w, split(m_b - m_a)), dw), 59 - eQ);
     Acc t{half<2>(), 0};
-    mac(t, al, split(shr(mul<0>(ml, tl), dm)));
-    mac(t, be, split(shr(mul<0>(mr, tr), dm)));
-    const double f_t = convert(fold<2>(t) - shr(mul<0>(w, split(t_b - t_a)), dw), 58 - eQ);
-    // each side's own pressure over the reconstructed one: ½g(h − hs)(h + hs).
-    // Where a depth has bits below the surface sums' last place, the own one is
-    // taken whole and the pressure of its rounding cancels against the flux's.
-    const int down = eL - eh + 2;
-    const bool whole = (xa < xb ? xa : xb) >= xl - 7;
-    auto back = [&](const Side& q, int64_t own, int64_t surface, double& x, double& y) {
-        const int64_t hq = whole ? shl(own, down) : to_fixed_nn(q.h, xh + 1);
-        const int64_t gq = shl(surface, down);
-        const int64_t p = shr(mul<0>(split(mul<0>(split(hq - gq), split((hq >> 1) + (gq >> 1)))),
-                                     c.half_g),
-                              eQ - 2 * eh - c.e_half_g - 1);
-        const double fn = convert(f_n + p, 58 - eQ);
-        x = fma(fn, geo[0], fp::neg(f_t) * geo[1]);
-        y = fma(fn, geo[1], f_t * geo[0]);
+    mac(t, al, split(shr(mul<1>(ml, tl), dm)));
+    mac(t, be, split(shr(mul<1>(mr, tr), dm)));
+    const double f_t = convert(fold<2>(t) - shr(mul<1>(w, split(t_b - t_a)), dw), 59 - eQ);
+    const double along_x = f_t * geo[1], along_y = f_t * geo[0];
+    out.hu_a = out.hu_b = fma(f_n, geo[0], fp::neg(along_x));
+    out.hv_a = out.hv_b = fma(f_n, geo[1], along_y);
+    // Each side's own pressure over the reconstructed one, ½g(h − hs)(h + hs):
+    // none over one bed, where the depth reaches its last place in the surface
+    // sums; else at the side's own scale, which a step of the bed sets far from
+    // the other's, and added in FP64.
+    if (ba == bb && imin(xa, xb) >= xl - 9) return kDone;
+    auto own = [&](const Side& q, int x, int64_t s) {
+        const int e = x - 1022;
+        const int64_t hq = x ? (int64_t)(mant(q.h) << 9) : 0;  // at 2^(62 − e)
+        const int64_t gq = shl(s, imin(eL - e, 63)), d = hq - gq;
+        const int up = clz64((uint64_t)d) - 2;
+        const int64_t p = mul<2>(split(mul<2>(split(shl(d, up)), split((hq >> 1) + (gq >> 1)))),
+                                 c.half_g);
+        return convert(p, 61 - 2 * e + up - c.e_half_g);
     };
-    back(qa, la, ra, out.hu_a, out.hv_a);
-    back(qb, lb, rb, out.hu_b, out.hv_b);
+    const double f_a = f_n + own(qa, xa, ra), f_b = f_n + own(qb, xb, rb);
+    out.hu_a = fma(f_a, geo[0], fp::neg(along_x));
+    out.hv_a = fma(f_a, geo[1], along_y);
+    out.hu_b = fma(f_b, geo[0], fp::neg(along_x));
+    out.hv_b = fma(f_b, geo[1], along_y);
     return kDone;
 }
 

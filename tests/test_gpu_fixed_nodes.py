@@ -67,20 +67,13 @@ def own_terms(form, q, dy):
     return [m.reshape(-1) for m in (mass, 9.81 * along_x(times(h)), 9.81 * along_y(times(t(h))))]
 
 
-@pytest.mark.parametrize("order", [1, 2, 3, 4])
-@pytest.mark.parametrize("ratio, shear, aspect", [
-    (1.05, 1.0, 1.0), (1.5, 1.0, 1.0), (2.0, 1.0, 1.0), (2.5, 1.0, 1.0), (4.0, 1.0, 1.0),
-    (30.0, 1.0, 1.0), (1.05, 8.0, 1.0), (1.05, 64.0, 1.0), (1.05, 1.0, 30.0),
-    (8.0, 100.0, 4.0)])
-def test_every_node_to_its_own_terms(order, ratio, shear, aspect):
+def check_nodes(form, q, own):
     """Device and oracle both round a node's some thirty operations at 2^-53 of
     terms of this size: together 64 of these."""
-    form, q = rectangle(order, ratio, shear, aspect=aspect)
     dev, ref = SWEPhysics2D(form, 0), oracle(form)
     try:
         for s in (dev, ref):
             s.upload(*q)
-        own = own_terms(form, q, SIDE / aspect)
         for name, g, w, o in zip(("h", "hu", "hv"), dev.compute_rhs_into(0.0),
                                  ref.compute_rhs_into(0.0), own):
             err = (np.abs(g - w) / o).max()
@@ -88,6 +81,38 @@ def test_every_node_to_its_own_terms(order, ratio, shear, aspect):
     finally:
         dev.close()
         ref.close()
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("ratio, shear, aspect", [
+    (1.05, 1.0, 1.0), (1.5, 1.0, 1.0), (2.0, 1.0, 1.0), (2.5, 1.0, 1.0), (4.0, 1.0, 1.0),
+    (30.0, 1.0, 1.0), (1.05, 8.0, 1.0), (1.05, 64.0, 1.0), (1.05, 1.0, 30.0),
+    (8.0, 100.0, 4.0)])
+def test_every_node_to_its_own_terms(order, ratio, shear, aspect):
+    form, q = rectangle(order, ratio, shear, aspect=aspect)
+    check_nodes(form, q, own_terms(form, q, SIDE / aspect))
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("shear", [1e4, 1e6])
+def test_currents_far_below_the_waves(order, shear):
+    """Faces whose currents are 1e-13 to 1e-19 of the wave's speed."""
+    form, q = rectangle(order, 1.05, shear)
+    check_nodes(form, q, own_terms(form, q, SIDE))
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("shelf", [5.0, 0.1])
+def test_a_shelf_beside_deep_water(order, shelf):
+    """A step of the bed along an element edge, one surface over it: the shelf's
+    nodes to their own depth's terms."""
+    form, _ = rectangle(order, 1.0, 1.0)
+    x, _ = form.positions()
+    column = (x.mean(axis=1) > SIDE)[:, None] & np.ones_like(x, dtype=bool)
+    form.bathymetry = np.where(column, 0.137 - shelf, 0.137 - 20.0)
+    h = 0.137 - form.bathymetry
+    q = (h.reshape(-1), 0.01 * h.reshape(-1), 0.02 * h.reshape(-1))
+    check_nodes(form, q, own_terms(form, q, SIDE))
 
 
 @pytest.mark.parametrize("order", [1, 2, 3, 4])
