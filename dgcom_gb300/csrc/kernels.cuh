@@ -1982,12 +1982,16 @@ __global__ void __launch_bounds__(256)
     const float n21 = 2.0f * (float)P.order + 1.0f;
     const float dt_lo = up > 0.0f ? cfl_lo / (n21 * up) * (1.0f - kStep) : INFINITY;
     const float dt_up = lo > 1e-13f ? cfl_up / (n21 * lo) * (1.0f + kStep) : INFINITY;
-    unsigned best = 0x7F800000u;  // +∞; the bits of floats ≥ 0 order as they do
-    if (mine) {
+    // the smallest upper end so far (the bits of floats ≥ 0 order as they do),
+    // read once for the element: other blocks lower it meanwhile, and its lanes
+    // have to agree on whether it is taken
+    unsigned best = 0x7F800000u;  // +∞
+    if (mine && lane == 0) {
         best = *(volatile unsigned*)&cm->dt_up;
-        if (lane == 0 && __float_as_uint(dt_up) < best) atomicMin(&cm->dt_up, __float_as_uint(dt_up));
+        if (__float_as_uint(dt_up) < best) atomicMin(&cm->dt_up, __float_as_uint(dt_up));
         best = min(best, __float_as_uint(dt_up));
     }
+    best = __shfl_sync(0xffffffffu, best, 0, LANES);
     const bool exact = mine && __float_as_uint(dt_lo) <= best;
     if (!__any_sync(0xffffffffu, exact)) return;
     unsigned long long rmax = 0ull;  // the bits of rates ≥ +0
