@@ -661,13 +661,12 @@ int dgswe_adjoint_forward(dgswe_adjoint* a, const double* h0, const double* hu0,
     std::vector<StepCtl> c0((size_t)M);
     for (int m = 0; m < M; ++m) {
         StepCtl& c = c0[m];
-        std::memset(&c, 0, sizeof c);
+        c = StepCtl{};
         c.t = a->cfg.t_start;
         c.t_end = INFINITY;
         c.target = INFINITY;
         c.cfl = cfl;
         c.dt_min_used = INFINITY;
-        c.dt_bits = 0x7FF0000000000000ull;
         c.always = 1;
         c.active = 1;
         c.scheme_stages = n_stages;

@@ -109,7 +109,7 @@ int begin_run(dgswe_handle* h, const dgswe_run_config* run, double target) {
     StepCtl& c = *h->h_ctl;
     long long clips0 = 0;
     CK(cudaMemcpy(&clips0, &h->ctl->clips, sizeof clips0, cudaMemcpyDeviceToHost));
-    std::memset(&c, 0, sizeof c);
+    c = StepCtl{};
     c.t = run->t_start;
     c.t_end = run->t_end;
     c.target = target;
@@ -118,7 +118,6 @@ int begin_run(dgswe_handle* h, const dgswe_run_config* run, double target) {
     c.cfl = run->cfl;
     c.dt_min_used = INFINITY;
     c.dt_max_used = 0.0;
-    c.dt_bits = 0x7FF0000000000000ull;
     c.max_steps = run->max_steps > 0 ? run->max_steps : 0;
     c.clips = clips0;
     c.always = 1;
@@ -661,7 +660,7 @@ int create_impl(dgswe_handle* h, const dgswe_form* f, int device) {
     h->ctl = (StepCtl*)p;
     CK(cudaMallocHost(&p, sizeof(StepCtl)));
     h->h_ctl = (StepCtl*)p;
-    std::memset(h->h_ctl, 0, sizeof(StepCtl));
+    *h->h_ctl = StepCtl{};
     h->h_ctl->always = 1;
     h->h_ctl->active = 1;
     CK(cudaMemcpy(h->ctl, h->h_ctl, sizeof(StepCtl), cudaMemcpyHostToDevice));
@@ -970,9 +969,10 @@ int dgswe_element_dt(dgswe_handle* h, double cfl, int32_t scheme, double* dt_ele
     if (!(cfl > 0.0) || (scheme != DGSWE_SSP_RK3 && scheme != DGSWE_SSP_RK43))
         return fail(h, DGSWE_ERR_INVALID, "element_dt: cfl %g, scheme %d", cfl, scheme);
     CK(cudaSetDevice(h->device));
-    const unsigned long long inf_bits = 0x7FF0000000000000ull;
-    CK(cudaMemcpyAsync(&h->ctl->dt_bits, &inf_bits, sizeof inf_bits, cudaMemcpyHostToDevice,
-                       h->stream));
+    const StepCtl fresh{};
+    CK(cudaMemcpyAsync(&h->ctl->dt_bits, &fresh.dt_bits,
+                       offsetof(StepCtl, dt_up) + sizeof fresh.dt_up - offsetof(StepCtl, dt_bits),
+                       cudaMemcpyHostToDevice, h->stream));
     const DtParams D = dt_params(h->form, cfl, scheme);
     h->ks->dt(h->n1, h->T, h->P, h->buf[DGSWE_STATE].view, D, h->dt_el, h->ctl, always(h),
               h->stream);
@@ -1069,14 +1069,13 @@ int dgswe_step_host(dgswe_handle* h, int32_t scheme, double t, double cfl, doubl
     // count stays on the device: the record is written around it
     {
         StepCtl& c = *h->h_ctl;
-        std::memset(&c, 0, sizeof c);
+        c = StepCtl{};
         c.t = t;
         c.t_end = h->parent_range.second;
         c.target = h->parent_range.second;
         c.dt_max = dt_max;
         c.cfl = cfl;
         c.dt_min_used = INFINITY;
-        c.dt_bits = 0x7FF0000000000000ull;
         c.always = 1;
         c.scheme_stages = n_st;
         for (int s = 0; s < n_st; ++s) {

@@ -229,8 +229,10 @@ struct StepCtl {
     double t, dt, target, t_end;
     double dt_max, dt_min, cfl;
     double dt_min_used, dt_max_used;
-    unsigned long long dt_bits;  // atomicMin of the element steps
-    unsigned dt_up;              // and of upper bounds of them (float bits; dt_min_kernel)
+    // atomicMin of the element steps, and of upper bounds of them (float bits;
+    // dt_min_kernel): both +∞ where a dt pass starts, step_begin's work in a run
+    unsigned long long dt_bits = 0x7FF0000000000000ull;
+    unsigned dt_up = 0x7F800000u;
     long long steps, max_steps, clips;
     int active;     // the current step runs
     int landed;

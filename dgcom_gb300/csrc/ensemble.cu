@@ -342,7 +342,7 @@ int create_impl(dgswe_ensemble* h, const dgswe_form* forms, int n, int device) {
     void* p = nullptr;
     CK(cudaMallocHost(&p, (size_t)n * sizeof(StepCtl)));
     h->h_ctl = (StepCtl*)p;
-    std::memset(h->h_ctl, 0, (size_t)n * sizeof(StepCtl));
+    std::fill(h->h_ctl, h->h_ctl + n, StepCtl{});
     for (int m = 0; m < n; ++m) {
         h->h_ctl[m].always = 1;
         h->h_ctl[m].active = 1;
@@ -369,7 +369,7 @@ int begin_run(dgswe_ensemble* h, const dgswe_run_config* run, int64_t steps) {
         StepCtl& c = h->h_ctl[m];
         const double t_own = c.t;  // the mirror holds the device's state after each run
         const long long clips = c.clips;
-        std::memset(&c, 0, sizeof c);
+        c = StepCtl{};
         c.t = std::isnan(run->t_start) ? t_own : run->t_start;
         c.clips = clips;
         c.t_end = INFINITY;
@@ -379,7 +379,6 @@ int begin_run(dgswe_ensemble* h, const dgswe_run_config* run, int64_t steps) {
         c.cfl = run->cfl;
         c.dt_min_used = INFINITY;
         c.dt_max_used = 0.0;
-        c.dt_bits = 0x7FF0000000000000ull;
         c.max_steps = steps;
         c.always = 1;
         c.active = 1;

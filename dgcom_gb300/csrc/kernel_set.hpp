@@ -104,7 +104,8 @@ struct KernelSet {
                        int64_t n_bfaces, cudaStream_t);
     void (*node_sources)(const DevTables&, const Physics&, const DevBuf& in, const StepCtl* ctl,
                          int slot, cudaStream_t);
-    // the smallest step over the listed elements
+    // the smallest step over the listed elements; as `dt` without dt_el, it starts
+    // from the +∞ of StepCtl's dt_bits and dt_up
     void (*dt_listed)(int n1, const DevTables&, const Physics&, const DevBuf& q, const DtParams&,
                       StepCtl* ctl, const int* active, const int32_t* list, int64_t n,
                       cudaStream_t);

@@ -167,11 +167,10 @@ int run_multirate(dgswe_handle* h, const dgswe_run_config* run, dgswe_callback c
     StepCtl& c = *h->h_ctl;
     long long clips0 = 0;
     CK(cudaMemcpy(&clips0, &h->ctl->clips, sizeof clips0, cudaMemcpyDeviceToHost));
-    std::memset(&c, 0, sizeof c);
+    c = StepCtl{};
     c.clips = clips0;
     c.always = 1;
     c.active = 1;
-    c.dt_bits = 0x7FF0000000000000ull;
     CK(cudaMemcpyAsync(h->ctl, &c, sizeof c, cudaMemcpyHostToDevice, st));
     h->ks->velocity(h->buf[DGSWE_STATE].view, h->n_values, h->P.h_min, st);
     // the stage values, the last stage's and the sums start as the state
