@@ -78,6 +78,17 @@ DG_HD double neg(double x) { return from_bits((int64_t)((uint64_t)bits(x) ^ kNeg
 // x > 0 ? x : +0 (the depth floor max(x, 0) of the reference's selects)
 DG_HD double max0(double x) { return gt0(x) ? x : 0.0; }
 
+// a·b <= 0 of the rounded product, which is formed only where it may underflow
+// or where an operand is infinite or NaN
+DG_HD bool product_le0(double a, double b) {
+    const int ea = (int)((uint64_t)bits(a) >> 52) & 0x7FF;
+    const int eb = (int)((uint64_t)bits(b) >> 52) & 0x7FF;
+    const bool number = ea != 0x7FF && eb != 0x7FF;
+    if (number && (!nz(a) || !nz(b))) return true;
+    if (number && ea + eb >= 1025) return (bits(a) ^ bits(b)) < 0;  // 2^-1021 and above
+    return a * b <= 0.0;
+}
+
 // Both operands non-negative (sign bit clear, e.g. after max0, or depths
 // known to be ≥ +0): the raw patterns already order as the values
 DG_HD bool gt_nn(double a, double b) { return bits(a) > bits(b); }

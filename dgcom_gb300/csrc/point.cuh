@@ -373,7 +373,7 @@ DG_PT double limited_slope(double q0, double q1, double q2, double ic,
                                                 double im, double ip) {
     const double dm = q1 - q0, dp = q2 - q1;
 #if DGSWE_FAST_PATH
-    const bool extremum = !fp::nz(dm) || !fp::nz(dp) || (fp::bits(dm) ^ fp::bits(dp)) < 0;
+    const bool extremum = fp::product_le0(dm, dp);
 #else
     const bool extremum = fp::le0(dm * dp);
 #endif
