@@ -1264,8 +1264,8 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
         for (int q = 0; q < 4; ++q) ew.w[q] = s_exp[e][2 * q] | s_exp[e][2 * q + 1] << 16;
     }
     // fixed: the element's right-hand side comes from here; slow: the mass of a
-    // node may not; by_depth: its depths alone leave it
-    bool fixed = false, slow = false, by_depth = false;
+    // node may not
+    bool fixed = false, slow = false;
     fx::Scale sc;
     if (valid && !sub) {
         const FxExp t = T.fx_exp[k];
@@ -1274,10 +1274,13 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
         fixed = sc.ok && !fx::thin(x, sc, t, fx::key(P.two_g));
         slow = fixed && fx::slow_node(x, sc, t);
         if (slow) prefetch(&T.pair_hm[gi * NP * 2]);
-        by_depth = P.formulation == kWetDry && thin_depth(T, P, t, x);
     }
-    if (valid && !fixed && !dry && i == 0 && !((sub || by_depth) && shallow_listed))
-        T.gen_list[T.K + atomicAdd(&T.gen_count[2], 1u)] = (int32_t)k;
+    if (valid && !fixed && !dry && i == 0) {
+        const bool listed =
+            shallow_listed && (sub || (P.formulation == kWetDry &&
+                                       thin_depth(T, P, T.fx_exp[k], depth_exponents(ew.w[0]))));
+        if (!listed) T.gen_list[T.K + atomicAdd(&T.gen_count[2], 1u)] = (int32_t)k;
+    }
 
     FxLimb G{}, H{};                         // 2g·h, h
     int64_t m0 = 0, m1 = 0, u0 = 0, u1 = 0;  // hu, hv, u, v
@@ -1356,7 +1359,7 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
         F.h = fx::over_jacobian(fh, sc.sh, jinv);
         if (slow) {  // a node whose own mass terms are too small takes them in FP64
             int64_t own = 0;
-#pragma unroll 1
+#pragma unroll
             for (int q = 0; q < NA; ++q)
                 fx::own_mass(own, T.fx_coef[i * NA + q],
                              pairs[(int)((node.slots >> (8 * q)) & 0xFF) * 3]);
