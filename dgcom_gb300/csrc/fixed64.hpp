@@ -637,9 +637,11 @@ DG_HD FaceCase face_flux(const Side& qa, const Side& qb, const double* geo,
     const int eC = (es + c.e_g + 1) >> 1;
     const int ev = imax(xv - 1022, -120);
     if (es < -60 || ev > eC + 30) return kNoScale;
-    // films left of much deeper water by a step, their surface at the datum: the
-    // FP64 sums h + B are exact there, these only to 2^-62 of the deep side
-    if (ba != bb && es < eL - 6 && (max64(abs64(la + ba), abs64(lb + bb)) >> 56) == 0)
+    // films left of much deeper water by a step, their surface within 2^-9 of the
+    // datum: FP64's sums h + B round at the surface, these at 2^-62 of the deep
+    // side (at 2^-6 instead of 2^-8 and 2^-9, some lane of most shore elements
+    // took FP64: a 90,000-quad box's stage at N = 1 44 us, not 40)
+    if (ba != bb && es < eL - 8 && (max64(abs64(la + ba), abs64(lb + bb)) >> 53) == 0)
         return kNoScale;
     const int64_t sa = shl(ra, eL - es), sb = shl(rb, eL - es);
     const int kv = 1025 + ev;

@@ -93,24 +93,26 @@ int main() {
     DevTables T{};
     std::vector<FxLimb> coef;
     fixed_constants(PairSchedule(ops), P, T, coef);
-    const char* names[6] = {"one surface at the datum, a step", "one surface off it, a step",
+    const char* names[7] = {"one surface at the datum, a step", "one surface off it, a step",
                             "a jump, one bed",                  "films on a step",
-                            "steps and jumps",                  "slow currents, equal depths"};
+                            "steps and jumps",                  "slow currents, equal depths",
+                            "one surface near the datum, a step"};
     bool good = true;
-    for (int kind = 0; kind < 6; ++kind) {
+    for (int kind = 0; kind < 7; ++kind) {
         std::mt19937_64 rng(3 + kind);
         std::vector<Score> mass(24), momentum(24);
         long done = 0;
         for (int i = 0; i < 500000; ++i) {
             const double H = std::pow(10.0, -2.0 + 4.0 * U(rng)), turn = 6.283185307179586 * U(rng);
-            const double r = std::exp2(-20.0 * U(rng)), off = H * (U(rng) - 0.5);
+            const double r = std::exp2(-20.0 * U(rng));
+            const double off = H * (U(rng) - 0.5) * (kind == 6 ? std::exp2(-14.0 * U(rng)) : 1.0);
             double nx = std::cos(turn), ny = std::sin(turn);
             if (i % 2) nx = 1.0, ny = 0.0;
             Side a, b;
             a.h = H;
             b.h = H * r;
             a.b = kind == 0 ? -H : -H + off;
-            if (kind < 2) b.b = a.h + a.b + 1e-3 * b.h * (U(rng) - 0.5) - b.h;
+            if (kind < 2 || kind == 6) b.b = a.h + a.b + 1e-3 * b.h * (U(rng) - 0.5) - b.h;
             if (kind == 2) b.b = a.b;
             if (kind == 3) b.b = a.h + a.b + H * U(rng);
             if (kind == 4) b.b = a.b + H * (1.0 - r) * U(rng);
