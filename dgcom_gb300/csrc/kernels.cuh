@@ -1272,7 +1272,7 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
         const fx::Exps x = exponents(ew);
         sc = fx::scales(x, t, T.fx_ec, T.fx_e2g, two_g_64ths(T));
         fixed = sc.ok && !fx::thin(x, sc, t, fx::key(P.two_g));
-        slow = fixed && fx::slow_node(x, sc, t);
+        slow = fixed && fx::slow_node(x, sc, t, T.fx_e2g);
         if (slow) prefetch(&T.pair_hm[gi * NP * 2]);
     }
     if (valid && !fixed && !dry && i == 0) {

@@ -203,7 +203,7 @@ static void run(int order, int kind, int rounds, std::mt19937_64& rng, Group& g)
             lifted[i] = fx::mul<0>(fx::split(fx::to_fixed(x.lift[i / 3], el + 2)),
                                    fx::split(fx::to_fixed(x.flux[i], i % 3 ? sc.kfm : sc.kfh)));
         }
-        const bool slow = fx::slow_node(e, sc, t);
+        const bool slow = fx::slow_node(e, sc, t, T.fx_e2g);
         ++g.taken;
         std::vector<Q> want, own_q;
         std::vector<double> fp64, own_d;
