@@ -861,9 +861,11 @@ __device__ __forceinline__ F3 general_rhs(const DevTables& T, const Physics& P,
 #if DGSWE_FAST
 // A node's pair and lift terms of the mass by the FP64 formulas, for a slow node
 // of an element in fixed point (a few in a thousand; listing the element for
-// general_kernel instead made its launch behind every stage 6 µs longer)
+// general_kernel instead made its launch behind every stage 6 µs longer). A call,
+// out of the stage kernel's code and registers: 4.23 ms a step in it for a 1 M-quad
+// box, 4.38 inlined
 template <int N1>
-__device__ __forceinline__ double mass_sum(const DevTables& T, const DevBuf& in,
+__device__ __noinline__ double mass_sum(const DevTables& T, const DevBuf& in,
                                            const double* fb_h, uint64_t slots, int64_t k, int i,
                                            int s_a, int s_b) {
     constexpr int NN = N1 * N1, NP = N1 - 1, NA = 2 * NP;
@@ -1176,8 +1178,9 @@ __device__ __forceinline__ void finish_node(const DevTables& T, const Physics& P
 // LISTED: a multirate pass over lp's elements, each with its own stage
 template <int N1, bool LISTED, int SHAPE = 0>
 __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_BLOCKS)
-    stage_kernel(DevTables T, Physics P, StageExtra X, DevBuf in, DevBuf base, DevBuf out,
-                 DevBuf acc, const double* __restrict__ fb_h, const double* __restrict__ fb_hu,
+    stage_kernel(const __grid_constant__ DevTables T, Physics P, StageExtra X,
+                 const __grid_constant__ DevBuf in, DevBuf base, DevBuf out, DevBuf acc,
+                 const double* __restrict__ fb_h, const double* __restrict__ fb_hu,
                  const double* __restrict__ fb_hv, StepCtl* ctl, int slot, int mode,
                  int check_finite, const int* active, DevBuf keep, LtsPass lp,
                  int shallow_listed) {
