@@ -1290,9 +1290,10 @@ int dgswe_profile_steps(dgswe_handle* h, const dgswe_run_config* run, int64_t n_
     if (int s = ensure_dt_stream(h)) return s;
     const DtParams D = dt_params(h->form, run->cfl, run->scheme);
     const int* active = &h->ctl->active;
-    // per step, as the step graph runs it: begin; the dt pass and the fit on
-    // the dt stream beside the first face pass; then the first stage pass and
-    // n − 1 × (face, stage); end. Events: before begin, after begin (the
+    // per step, as the step graph runs it but for the elements that leave fixed
+    // point, which come behind the stage pass here and beside it there: begin; the
+    // dt pass and the fit on the dt stream beside the first face pass; then the
+    // first stage pass and n − 1 × (face, stage); end. Events: before begin, after begin (the
     // fork), after dt and after the fit (dt stream), after the first face
     // pass, after the join, after each later pass → 5 + 2n per step
     const int per_step = 5 + 2 * n;

@@ -434,20 +434,31 @@ struct OwnMetric {
     int w, v;  // the keys of a node's, then of an element's
 };
 DG_HD OwnMetric own_metric(const double* hm, const int32_t* slots, const double* coefs, int na) {
-    double w0 = 0.0, w1 = 0.0, v = 0.0;
+    double w0 = 0.0, w1 = 0.0, a0 = 0.0, a1 = 0.0, size = 0.0;  // a: the largest
     for (int q = 0; q < na; ++q) {
         const double c = 0.5 * fabs(coefs[q]);
-        const double a0 = c * hm[2 * slots[q]], a1 = c * hm[2 * slots[q] + 1];
-        w0 = fmax(w0, fabs(a0));
-        w1 = fmax(w1, fabs(a1));
-        for (int p = 0; p < q; ++p) {  // a current across at most one of two lines
-            const double d = 0.5 * fabs(coefs[p]);
-            const double b0 = d * hm[2 * slots[p]], b1 = d * hm[2 * slots[p] + 1];
-            const double size = fabs(a0) + fabs(a1) + fabs(b0) + fabs(b1);
-            if (size > 0.0) v = fmax(v, fabs(a0 * b1 - a1 * b0) / size);
+        const double x = c * hm[2 * slots[q]], y = c * hm[2 * slots[q] + 1];
+        w0 = fmax(w0, fabs(x));
+        w1 = fmax(w1, fabs(y));
+        if (fabs(x) + fabs(y) > size) {
+            size = fabs(x) + fabs(y);
+            a0 = x;
+            a1 = y;
         }
     }
-    return {key(fmin(w0, w1)), key(v)};
+    // a current lies along at most one of two lines: with the pair that is most
+    // across the largest, |a × b|/(|a| + |b|) of it is across one or the other
+    double across = 0.0, both = 1.0;
+    for (int q = 0; q < na; ++q) {
+        const double c = 0.5 * fabs(coefs[q]);
+        const double x = c * hm[2 * slots[q]], y = c * hm[2 * slots[q] + 1];
+        const double cross = fabs(a0 * y - a1 * x);
+        if (cross > across) {
+            across = cross;
+            both = size + fabs(x) + fabs(y);
+        }
+    }
+    return {key(fmin(w0, w1)), key(across / both)};
 }
 DG_HD int own_deficits(const OwnMetric& m, int et, int ec) {
     int w = 16 * (et + ec) - (m.w - kKeyOne), v = 16 * (et + ec) - (m.v - kKeyOne);

@@ -29,7 +29,7 @@
 //    stage_where, src/physics/builder.rs:652-737), and the node velocities
 //    the next stage reads;
 //  - with DGSWE_FAST, general_kernel<N1>: the same for the elements that fixed
-//    point leaves (subcells with water, depths spread too far), listed by
+//    point leaves (subcells with water, nodes that FP64 is closer to), listed by
 //    stage_kernel or, beside the face pass, by shallow_list_kernel.
 // Per step: dt_min_kernel<N1> (the smallest element step; dt_kernel<N1> where
 // every element's is asked for) and three one-thread kernels that run the
@@ -80,10 +80,10 @@ struct FacePair {
 };
 
 // hydro_hll of a face node along its geometry. With DGSWE_FAST, where the
-// interior faces mostly take fixed point, this is a call: the rest (sides not
-// both wet, super-critical flow, walls) then runs the same instructions in
-// every face kernel, the multiply-adds contracted alike, and its registers
-// are not the kernels'.
+// interior faces mostly take fixed point, this is a call: the rest (exponents
+// out of range, some films near the datum: fx::kNoScale) then runs the same
+// instructions in every face kernel, the multiply-adds contracted alike, and its
+// registers are not the kernels'.
 #if DGSWE_FAST
 __device__ __noinline__
 #else
@@ -1433,7 +1433,7 @@ __global__ void __launch_bounds__(256)
 }
 
 // The elements of a stage that stage_kernel leaves (a half of T.gen_list):
-// those with subcells, and wet ones whose scales spread too far. Few and long
+// those with subcells, and wet ones that FP64 is closer to. Few and long
 // (some 200 FP64 operations in a row, 20 µs for any number of them), so two
 // lanes a node, a subcell direction each. The last block to end empties the
 // list for the next stage.

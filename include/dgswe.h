@@ -101,15 +101,14 @@ enum dgswe_scheme {
 };
 
 /* Device arithmetic, FP64 throughout. FAST contracts multiply-adds into FMA,
- * takes square roots, reciprocals and the Manning rate's h^(-4/3) within an
- * ulp of the correctly rounded value in 64-bit fixed point, and the wet
- * elements' volume terms and the wet faces' fluxes in 62-bit fixed point
- * scaled per element and face node, or in FP64 where that is closer to a node's
- * result (shallow or slow nodes of elements whose depths or currents vary
- * strongly): against an extended-precision result no node's error is above
- * FP64's; EXACT keeps
- * every multiply and add separately rounded, uses IEEE division and square
- * root and follows the reference's cube root
+ * takes square roots, reciprocals, quotients and the Manning rate's h^(-4/3) in
+ * 64-bit fixed point (quotients within 0.52 ulp of the exact value, the others
+ * within 0.75), and the wet elements' volume terms and the faces' fluxes in
+ * 62-bit fixed point scaled per element and face node, or in FP64 where that is
+ * closer to a node's result (shallow or slow nodes of elements whose depths or
+ * currents vary strongly): against an extended-precision result no node's error
+ * is above FP64's. EXACT keeps every multiply and add separately rounded, uses
+ * IEEE division and square root and follows the reference's cube root
  * (src/source/swe_2d/friction.rs:39-70). */
 enum dgswe_numerics {
     DGSWE_NUMERICS_FAST = 0,
