@@ -53,7 +53,7 @@ STAGE_TRAFFIC_PER_NODE_STAGE = {3: 179.3}
 # kernel) and face kernels per stage (three a step) and the dt kernel once a
 # step. The rest of the stage's and the faces' arithmetic is fixed point on
 # the integer pipes (157.4 + 77.1 a node-stage with all of it in FP64).
-FP64_FLOPS_PER_NODE = {3: {"stage": 23.7, "face": 14.3, "dt": 4.1}}
+FP64_FLOPS_PER_NODE = {3: {"stage": 33.8, "face": 12.4, "dt": 4.0}}
 
 
 def fp64_gemm_tflops(device: int, n: int = 6144, reps: int = 5) -> float | None:
@@ -440,7 +440,7 @@ def run_ours(args, rank: int, world: int, local: int):
                          "traffic": (STAGE_TRAFFIC_PER_NODE_STAGE[args.order] * nodes
                                      if args.order in STAGE_TRAFFIC_PER_NODE_STAGE else None),
                          "peak_kind": peak_kind, "kernel": f"stage_kernel<{args.order + 1}>",
-                         "note": "bound by the integer and FP64 pipes together (50 to 53 % of "
+                         "note": "bound by the integer and FP64 pipes together (50 to 60 % of "
                                  "each in ncu, 60 % of issue slots), not HBM; traffic from an "
                                  "ncu capture at 200k quads scaled by nodes"},
             "fp64": fp64,

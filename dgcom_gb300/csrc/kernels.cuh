@@ -298,8 +298,9 @@ __device__ __forceinline__ double weather_level(const DevTables& T, const Physic
 // A thread a face node. In FP64 the pipe was full (86 % of it; 0.348 ms for
 // 200,000 quads at N = 3); in fixed point the integer pipes and the FP64
 // pipe (the rotations, the conversions, faces that fixed point leaves) share
-// the work at 62-65 % each and 0.111 ms. Four blocks an SM (64 registers)
-// against three or two: 10.48, 10.72, 11.16 ms over 60 passes.
+// the work at 59 to 64 % each and 0.106 ms. Four blocks an SM (64 registers, 112
+// to 148 bytes spilled) against three or two: 10.48, 10.72, 11.16 ms over 60
+// passes.
 // LISTED: a multirate pass's faces (lp's edge and boundary-face lists),
 // each boundary face at its element's stage time
 template <int N1, bool LISTED>
@@ -436,9 +437,12 @@ struct Cfg {
     static constexpr int EPB = (PER / NN) > 0 ? (PER / NN) : 1;
     static constexpr int THREADS = EPB * NN;
     // stage_kernel blocks per SM. In fixed point the integer and FP64 pipes
-    // are each under half busy and the rest is latency: 28 warps an SM (72
+    // are each about half busy and the rest is latency: 28 warps an SM (72
     // registers) against 20 (96) take the 200,000-quad N = 3 right-hand side
-    // from 0.226 to 0.210 ms, N = 4 at 100,000 from 0.354 to 0.310. The exact
+    // from 0.226 to 0.210 ms, N = 4 at 100,000 from 0.354 to 0.310. At 72
+    // registers orders 2 and 4 spill 24 and 16 bytes, 1 and 3 none; against 24
+    // warps (80 registers) N = 1 to 4 take 76, 164, 174, 244 µs and 80, 168, 183,
+    // 244 (400,000, 300,000, 200,000, 100,000 quads). The exact
     // numerics wait on the FP64 pipe: 20 warps (≤ 102 registers, no spills)
     // were 5 % faster than 16.
     static constexpr int MIN_BLOCKS =

@@ -67,7 +67,7 @@ static void face_listed_n(const DevTables& T, const Physics& P, const DevBuf& in
 // general_kernel's blocks for a pass of `count` elements, of which it takes
 // those listed: enough for all, and at most the four on each of the 152
 // multiprocessors that run at once (the rest of a longer list comes in their
-// next rounds; an empty list then costs 608 blocks' start, 2.5 µs)
+// next rounds; an empty list then costs 608 blocks' start, 3 to 4.5 µs)
 template <int N1>
 static unsigned general_blocks(int64_t count) {
     const int64_t all = (count + GenCfg<N1>::EPB - 1) / GenCfg<N1>::EPB;
