@@ -1386,6 +1386,9 @@ __global__ void __launch_bounds__(Cfg<N1, SHAPE>::THREADS, Cfg<N1, SHAPE>::MIN_B
         if (X.subcell_mass)  // its interface fluxes are ±0
             for (int q = i; q < C::NSUB; q += NN) X.subcell_mass[k * C::NSUB + q] = 0.0;
     }
+    // the buffer summed into may be the input, which a slow node's mass_sum reads
+    // at the element's other nodes
+    if (mode == kAccumulate) element_sync<NN>();
     finish_node<N1, LISTED, NN>(T, P, in, base, out, acc, keep, cm, lp, slot, mode, check_finite, k,
                                 i, fixed || dry, F, s_q, &s_flag[e][2], s_red[e]);
 }

@@ -117,6 +117,27 @@ def test_a_shelf_beside_deep_water(order, shelf):
 
 @pytest.mark.parametrize("order", [1, 2, 3, 4])
 @pytest.mark.parametrize("ratio, shear", [(2.5, 1.0), (1.05, 1e3)])
+def test_a_sum_into_the_stage_s_input(order, ratio, shear):
+    """The buffer that a stage is summed into may be its input: the same bits as
+    into a copy of it, though a slow node reads its element's other nodes."""
+    form, q = rectangle(order, ratio, shear, nx=40, ny=9)
+    dev = SWEPhysics2D(form, 0)
+    try:
+        got = []
+        for acc in (3, 1):
+            for buffer in (abi.STATE, 1, 3):
+                dev.upload(*q, buffer=buffer)
+            dev.stage_where(base=abi.STATE, input=1, out=2, time=0.0, a=1.0, b=0.0, c=0.01,
+                            acc=acc, w=0.5, keep=0.25)
+            got.append(dev.download(2) + dev.download(acc))
+        for g, w in zip(*got):
+            assert np.array_equal(g, w)
+    finally:
+        dev.close()
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("ratio, shear", [(2.5, 1.0), (1.05, 1e3)])
 def test_a_run_over_them_equals_its_calls(order, ratio, shear):
     """Listed before the stage (by their depths) or by it (by their fluxes), and
     taken beside it or behind it: the same bits."""
